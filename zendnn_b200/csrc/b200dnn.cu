@@ -16,6 +16,7 @@
 #include "decode_ring.cuh"
 #include "tc_gemm.cuh"
 #include "moe_kernels.cuh"
+#include "sdpa_flash_api.cuh"
 
 using namespace b200;
 
@@ -211,19 +212,6 @@ int32_t launch_quant_rows(const RowQuantArgs &a, int32_t src_dt, int64_t rows, c
 }
 
 // ------------------------------------------------------------------------------------ GEMM launchers
-// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per kernel and device: raises the limit to the largest size
-// the kernel is launched with and remembers that it did.
-int32_t ensure_max_smem(const void *fn, int bytes = 227 * 1024) {
-  DeviceShared &D = *rt().shared;
-  std::lock_guard<std::mutex> lk(D.attr_mu);
-  int &have = D.smem_limit[fn];
-  if (have < bytes) {
-    B2_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    have = bytes;
-  }
-  return B200DNN_SUCCESS;
-}
-
 int32_t launch_stream(const uint8_t *A, int64_t lda, bool a_unsigned, int M, int N, int K, const PackedWeight &pw,
                       const EpiParams &epi, cudaStream_t st) {
   Runtime &R = rt();

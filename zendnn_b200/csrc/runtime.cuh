@@ -264,6 +264,19 @@ inline Runtime *&current_rt() { static thread_local Runtime *r = nullptr; return
 // The context of the call in progress on this thread (set by CallGuard).
 inline Runtime &rt() { return *current_rt(); }
 
+// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per kernel and device: raises the limit to the largest size
+// the kernel is launched with and remembers that it did.
+inline int32_t ensure_max_smem(const void *fn, int bytes = 227 * 1024) {
+  DeviceShared &D = *rt().shared;
+  std::lock_guard<std::mutex> lk(D.attr_mu);
+  int &have = D.smem_limit[fn];
+  if (have < bytes) {
+    B2_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    have = bytes;
+  }
+  return B200DNN_SUCCESS;
+}
+
 // Entered at the top of every C-ABI entry point: finds (or creates) the context of (current device, stream), takes its
 // lock for the duration of the call and rewinds its workspace.
 struct CallGuard {

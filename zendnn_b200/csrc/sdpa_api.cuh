@@ -1,15 +1,16 @@
 // sdpa_direct: softmax(Q K^T * scale + mask) V per (batch, head), the attention operator beside the MoE block of a decoder
 // layer (reference: lowoha_operators/sdpa/lowoha_sdpa.hpp:48-55, sdpa_params lowoha_sdpa_common.hpp:57-103, checks
-// flash_sdpa/lowoha_flash_sdpa_utils.cpp:23-178).  Built here in the form of the reference's BMM backend
-// (bmm_sdpa/lowoha_sdpa_bmm.cpp: scores by matmul_direct, mask and causal mask on the f32 scores, softmax, matmul_direct
-// with V), every product on the tcgen05 kernel's bf16 form:
-//   S[seq, kv]  = Q_bh K_bh^T          bf16 x bf16 -> f32   (K_bh taken as a transposed weight, packed per head)
+// flash_sdpa/lowoha_flash_sdpa_utils.cpp:23-178).  The steps are those of the reference's BMM backend (bmm_sdpa/lowoha_sdpa_bmm.cpp):
+//   S[seq, kv]  = Q_bh K_bh^T          bf16 x bf16 -> f32
 //   P           = softmax(S * scale + mask) over kv, f32, rounded to bf16; causal: key j > query i is masked
 //   O_bh        = P V_bh               bf16 x bf16 -> out_dt
 // scale == 0 means 1 / sqrt(head_dim) (bmm_sdpa/lowoha_sdpa_utils.cpp:25-27).  A row whose keys are all masked gives zeros.
-// Not a flash kernel: the scores make a round trip through HBM (seq * kv * 6 bytes per head).  Tensors whose query rows
-// follow each other at one pitch over all heads ([batch, head, seq, dim] storage) take five launches for all heads (K and V
-// of every head into the tile layout, two grouped products, one softmax); other layouts go head by head.
+// One fused kernel (sdpa_flash.cuh) takes rows of 16-byte vectors with a head dimension of up to 128, in any storage order.  Measured
+// against the three-step form below: 32 heads x 2048 causal, head_dim 128: 62 us for 636; 256 heads x 1 query x 3000 keys: 64 us
+// for 569 (6.1 TB/s); [batch, seq, head, dim] storage, which went head by head: 61 us for 8.6 ms at 1280 heads x 4 queries.
+// Everything else runs the steps one after the other on the tcgen05 GEMM's bf16 form, the scores making a round trip through HBM
+// (seq * kv * 6 bytes per head): tensors whose query rows follow each other at one pitch over all heads in five launches for all
+// heads (K and V of every head into the tile layout, two grouped products, one softmax), other layouts head by head.
 // Included at the end of b200dnn.cu.
 #pragma once
 
@@ -111,6 +112,20 @@ extern "C" int32_t b200dnn_sdpa(const b200dnn_sdpa_t *d, void *stream) {
   const int64_t kvp = round_up(KV, 8);
   const float scale = d->scale == 0.0 ? 1.0f / std::sqrt((float)D) : (float)d->scale;
   const int64_t mb = msz[0] > 1 ? mst[0] : 0, mh = msz[1] > 1 ? mst[1] : 0, mi = msz[2] > 1 ? mst[2] : 0;
+
+  // ---- one fused kernel where it fits (B200DNN_SDPA_GROUPED=0 keeps the head-by-head form, B200DNN_SDPA_FUSED=0 the BMM forms)
+  if (env_int("B200DNN_SDPA_GROUPED", 1) != 0 && env_int("B200DNN_SDPA_FUSED", 1) != 0) {
+    SdpaCall c{};
+    c.B = B; c.H = H; c.S = S; c.KV = KV; c.D = D;
+    c.q = q; c.k = k; c.v = v; c.out = o_out.dev;
+    for (int i = 0; i < 3; ++i) { c.qs[i] = d->q_stride[i]; c.ks[i] = d->k_stride[i]; c.vs[i] = d->v_stride[i]; c.os[i] = d->o_stride[i]; }
+    c.scale = scale; c.causal = d->is_causal ? 1 : 0;
+    c.mask = mk; c.mask_dt = d->mask_dt; c.mb = mb; c.mh = mh; c.mi = mi;
+    c.test_no_loads = env_int("B200DNN_TEST_NO_LOADS", 0);
+    const int32_t rc = sdpa_fused(c, st);
+    if (rc == B200DNN_SUCCESS) return finish_out({&o_out}, st);
+    if (rc != B200DNN_UNIMPLEMENTED) return rc;
+  }
 
   // ---- all heads at once: when the query rows of all heads follow each other at one pitch, the two products are grouped
   // launches (one group per head, the head's K or V as its weight) and the softmax is one launch; several rounds when the

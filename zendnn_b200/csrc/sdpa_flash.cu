@@ -1,0 +1,146 @@
+// Launchers of the fused attention kernels (sdpa_flash.cuh): which form takes a call, tensor maps, grids.
+#include <cudaTypedefs.h>
+#include "runtime.cuh"
+#include "sdpa_flash.cuh"
+#include "sdpa_flash_api.cuh"
+
+namespace b200 {
+
+namespace {
+
+// [128 rows x 64 (128-byte swizzle) or 32 (no swizzle) elements] boxes of a bf16 tensor seen as (d, row, head, batch); an extent of
+// one takes any stride
+int32_t make_map_heads(CUtensorMap *m, const void *base, int64_t D, int64_t rows, int64_t H, int64_t B, int64_t st_row, int64_t st_h, int64_t st_b,
+                       uint32_t inner = 64) {
+  cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)rows, (cuuint64_t)H, (cuuint64_t)B};
+  auto bytes = [&](int64_t st, int64_t n) { return (cuuint64_t)((n > 1 ? st : st_row) * 2); };
+  cuuint64_t strides[3] = {(cuuint64_t)(st_row * 2), bytes(st_h, H), bytes(st_b, B)};
+  cuuint32_t box[4] = {inner, 128, 1, 1}, estr[4] = {1, 1, 1, 1};
+  CUresult r = rt().encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           inner == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  B2_CHECK(r == CUDA_SUCCESS, B200DNN_FAILURE, "cuTensorMapEncodeTiled (attention) failed with %d", (int)r);
+  return B200DNN_SUCCESS;
+}
+
+int walks(int64_t stride, int64_t n) { return n > 1 && stride != 0 ? 1 : 0; }     // 0: broadcast
+
+template <typename K, typename... Args>
+int32_t launch_pdl(K kern, unsigned grid, unsigned threads, size_t smem, unsigned cluster, cudaStream_t st, const Args &...args) {
+  B2_TRY(ensure_max_smem((const void *)kern, (int)smem));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 1;
+  if (cluster > 1) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
+  cfg.attrs = attr;
+  B2_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+  B2_LAUNCHED();
+  return B200DNN_SUCCESS;
+}
+
+// Few query rows: a cluster of CTAs per (batch, head), split over the keys.
+int32_t launch_sdpa_decode(const SdpaCall &c, cudaStream_t st) {
+  SdpaDecodeArgs a{};
+  a.q = (const uint16_t *)c.q; a.out = (uint16_t *)c.out;
+  a.qb = c.qs[0]; a.qh = c.qs[1]; a.qs = c.qs[2]; a.ob = c.os[0]; a.oh = c.os[1]; a.os = c.os[2];
+  a.kb = walks(c.ks[0], c.B); a.kh = walks(c.ks[1], c.H); a.vb = walks(c.vs[0], c.B); a.vh = walks(c.vs[1], c.H);
+  a.S = (int)c.S; a.KV = (int)c.KV; a.D = (int)c.D; a.H = (int)c.H;
+  a.scale_log2 = c.scale * 1.44269504088896340736f; a.causal = c.causal;
+  a.mask = SdpaMask{c.mask, c.mask_dt, c.mb, c.mh, c.mi};
+  a.status = rt().status;
+  const int64_t heads = c.B * c.H;
+  const int db = c.D <= 64 ? 1 : 2;
+  // CTAs per head: the busiest SM's keys, plus about 300 keys' worth of time (3 us) for the start and the exchange of each round of
+  // CTAs that it runs one after the other (two are resident where their shared memory allows)
+  auto chunk_of = [&](int s) { return (int)round_up((c.KV + s - 1) / s, 128); };
+  auto smem_of = [&](int s) {
+    const size_t scores = (size_t)c.S * (chunk_of(s) + 8) * 4, red = (size_t)kSdpaDecodeWarps * c.S * c.D * 4;
+    return sdpa_decode_ring_bytes(db) + (scores > red ? scores : red) + 1024;
+  };
+  int split = 0;
+  int64_t best = 0;
+  for (int s = 1; s <= 8; s *= 2) {
+    if (smem_of(s) > (size_t)220 * 1024) continue;
+    const int64_t resident = smem_of(s) <= (size_t)112 * 1024 ? 2 : 1, per_sm = (heads * s + rt().sm_count - 1) / rt().sm_count;
+    const int64_t cost = per_sm * chunk_of(s) + (per_sm + resident - 1) / resident * 300;
+    if (split == 0 || cost <= best) { split = s; best = cost; }
+  }
+  if (split == 0 || heads * split > (1ll << 30)) return B200DNN_UNIMPLEMENTED;
+  const size_t smem = smem_of(split);
+  a.chunk = chunk_of(split);
+  a.sc_stride = a.chunk + 8;             // rows start 8 banks apart: the fragments' eight-byte reads are free of conflicts
+  CUtensorMap mk, mv;
+  B2_TRY(make_map_heads(&mk, c.k, c.D, c.KV, a.kh ? c.H : 1, a.kb ? c.B : 1, c.ks[2], c.ks[1], c.ks[0], 32));
+  B2_TRY(make_map_heads(&mv, c.v, c.D, c.KV, a.vh ? c.H : 1, a.vb ? c.B : 1, c.vs[2], c.vs[1], c.vs[0], 64));
+  const unsigned grid = (unsigned)(heads * split);
+  if (db == 1) {
+    if (c.S <= 8) return launch_pdl(sdpa_decode_kernel<1, false>, grid, kSdpaDecodeThreads, smem, split, st, mk, mv, a);
+    return launch_pdl(sdpa_decode_kernel<1, true>, grid, kSdpaDecodeThreads, smem, split, st, mk, mv, a);
+  }
+  if (c.S <= 8) return launch_pdl(sdpa_decode_kernel<2, false>, grid, kSdpaDecodeThreads, smem, split, st, mk, mv, a);
+  return launch_pdl(sdpa_decode_kernel<2, true>, grid, kSdpaDecodeThreads, smem, split, st, mk, mv, a);
+}
+
+int32_t launch_sdpa_flash(const SdpaCall &c, cudaStream_t st) {
+  SdpaFlashArgs a{};
+  const int sms = rt().sm_count;
+  const int64_t heads = c.B * c.H;
+  a.S = (int)c.S; a.KV = (int)c.KV; a.D = (int)c.D; a.H = (int)c.H; a.n_bh = (int)heads;
+  // 256 query rows per CTA, or 128 where that would leave SMs without work
+  a.tiles = (c.S <= 128 || heads * ((c.S + 255) / 256) < sms) ? 1 : 2;
+  a.n_qt = (int)((c.S + a.tiles * 128 - 1) / (a.tiles * 128));
+  if (heads * a.n_qt >= (1ll << 31)) return B200DNN_UNIMPLEMENTED;
+  // Longest query tiles of all heads first (under a causal mask their lengths differ by the sequence length) while every head's K
+  // and V stay in the L2 together; head after head otherwise.
+  a.bh_major = !c.causal || 4 * heads * c.KV * c.D > (64ll << 20);
+  a.scale_log2 = c.scale * 1.44269504088896340736f; a.causal = c.causal;
+  a.mask = SdpaMask{c.mask, c.mask_dt, c.mb, c.mh, c.mi};
+  const int64_t mstep = c.mask_dt == B200DNN_F32 ? 4 : 8;
+  a.mask_vec = (reinterpret_cast<uintptr_t>(c.mask) & 15) == 0 && c.mb % mstep == 0 && c.mh % mstep == 0 && c.mi % mstep == 0;
+  a.kb = walks(c.ks[0], c.B); a.kh = walks(c.ks[1], c.H); a.vb = walks(c.vs[0], c.B); a.vh = walks(c.vs[1], c.H);
+  a.out = (uint16_t *)c.out; a.ob = c.os[0]; a.oh = c.os[1]; a.os = c.os[2];
+  const uintptr_t al = reinterpret_cast<uintptr_t>(c.out) | (uintptr_t)(c.os[2] * 2) | (c.H > 1 ? (uintptr_t)(c.os[1] * 2) : 0) | (c.B > 1 ? (uintptr_t)(c.os[0] * 2) : 0);
+  a.out_align = (al & 31) == 0 ? 32 : ((al & 15) == 0 ? 16 : 2);
+  a.status = rt().status; a.test_no_loads = c.test_no_loads;
+  CUtensorMap mq, mk, mv;
+  B2_TRY(make_map_heads(&mq, c.q, c.D, c.S, c.H, c.B, c.qs[2], c.qs[1], c.qs[0]));
+  B2_TRY(make_map_heads(&mk, c.k, c.D, c.KV, a.kh ? c.H : 1, a.kb ? c.B : 1, c.ks[2], c.ks[1], c.ks[0]));
+  B2_TRY(make_map_heads(&mv, c.v, c.D, c.KV, a.vh ? c.H : 1, a.vb ? c.B : 1, c.vs[2], c.vs[1], c.vs[0]));
+  const int db = c.D <= 64 ? 1 : 2;
+  const size_t smem = (size_t)(a.tiles + kFlashSlots) * db * 16384 + 1024;
+  const unsigned grid = (unsigned)(heads * a.n_qt);
+  if (db == 1) {
+    if (c.mask) return launch_pdl(sdpa_flash_kernel<1, true>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
+    return launch_pdl(sdpa_flash_kernel<1, false>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
+  }
+  if (c.mask) return launch_pdl(sdpa_flash_kernel<2, true>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
+  return launch_pdl(sdpa_flash_kernel<2, false>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
+}
+
+}  // namespace
+
+int32_t sdpa_fused(const SdpaCall &c, cudaStream_t st) {
+  // both kernels read rows as 16-byte vectors (the copy engine's rule as well) and hold a head dimension of up to 128; the
+  // row maximum is taken before the scale is applied
+  if (c.D % 8 != 0 || c.D > 128 || !(c.scale > 0.f)) return B200DNN_UNIMPLEMENTED;
+  auto ok = [](const void *p, const int64_t (&s)[3], int64_t B, int64_t H, bool broadcast) {
+    if ((reinterpret_cast<uintptr_t>(p) & 15) != 0 || s[2] <= 0 || s[2] % 8 != 0) return false;
+    if (H > 1 && (s[1] % 8 != 0 || s[1] < 0 || (s[1] == 0 && !broadcast))) return false;
+    return B <= 1 || (s[0] % 8 == 0 && s[0] >= 0 && (s[0] != 0 || broadcast));
+  };
+  if (!ok(c.q, c.qs, c.B, c.H, false) || !ok(c.k, c.ks, c.B, c.H, true) || !ok(c.v, c.vs, c.B, c.H, true)) return B200DNN_UNIMPLEMENTED;
+  if (c.B * c.H > (1ll << 28)) return B200DNN_UNIMPLEMENTED;
+  if (c.S <= 16 && !c.test_no_loads) {
+    const int32_t rc = launch_sdpa_decode(c, st);
+    if (rc != B200DNN_UNIMPLEMENTED) return rc;
+  }
+  return launch_sdpa_flash(c, st);
+}
+
+}  // namespace b200

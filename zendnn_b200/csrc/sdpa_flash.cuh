@@ -1,0 +1,773 @@
+// Fused attention kernels behind b200dnn_sdpa: softmax(Q K^T * scale + mask) V per (batch, head) without a score matrix in
+// memory (reference operator: lowoha_operators/sdpa/lowoha_sdpa.hpp:48-55; steps of its BMM backend:
+// bmm_sdpa/lowoha_sdpa_bmm.cpp).
+//
+// Both kernels keep the steps and roundings of that backend: f32 scores, f32 softmax with the FINAL row maximum and row sum,
+// probabilities rounded to bf16 after the division, products with V accumulated in f32.  A one-sweep (online) softmax would
+// round unnormalised probabilities instead and give other results; so the prompt kernel sweeps the keys twice: the first
+// sweep takes row maximum and row sum, the second recomputes the scores and multiplies the normalised probabilities with V.
+// The extra Q K^T costs half as much again on the tensor pipe and saves every rescale of the accumulator.
+// The exponential is ex2.approx on an argument with log2(e) folded into the scale (and -log2 of the row sum into the bias):
+// its error, below 1e-6 of a probability, is far under the bf16 rounding that follows.
+#pragma once
+#include "common.cuh"
+#include "mbar.cuh"
+#include "tc_gemm.cuh"
+
+namespace b200 {
+
+struct SdpaMask { const void *p; int32_t dt; int64_t mb, mh, mi; };   // element (b,h,i,j) at p + b*mb + h*mh + i*mi + j
+
+struct SdpaFlashArgs {
+  int S, KV, D, H;
+  int n_bh;                 // batch * heads
+  int n_qt;                 // query tiles of tiles * 128 rows
+  int tiles;                // 128-row tiles per CTA: 1 or 2
+  int bh_major;             // work order: all query tiles of a head first, else all heads of the longest query tile first
+  float scale_log2;         // scale * log2(e), > 0
+  int causal;
+  SdpaMask mask; int mask_vec;   // mask_vec: every mask row starts on a 16-byte boundary
+  int kb, kh, vb, vh;       // 0 where K / V are broadcast over the batch / the heads (stride 0), else 1
+  uint16_t *out; int64_t ob, oh, os;
+  int out_align;            // bytes every output row start is aligned to: 32, 16 or 2
+  int32_t *status;
+  int test_no_loads;
+};
+
+constexpr int kFlashSoftmaxWarps = 16;  // two 128-row tiles x two halves of a key block x four lane quadrants
+constexpr int kFlashThreads = 32 * (kFlashSoftmaxWarps + 2);
+constexpr int kFlashSlots = 4;          // K / V ring
+struct FlashTrue { static constexpr bool value = true; };
+struct FlashFalse { static constexpr bool value = false; };
+
+__device__ __forceinline__ float ex2f(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ uint64_t pk2(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ void upk2(uint64_t r, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(r)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+
+// 2^x for two arguments on the FMA pipe, to share the exponentials between the two pipes: x = n + f with n the nearest integer
+// (added and removed as 1.5 * 2^23), 2^f by a degree-5 polynomial in Horner form, n added to the exponent field.  The
+// coefficients are the minimax fit in relative error of 2^f on [-1/2, 1/2] (Remez exchange in double, rounded to f32):
+// 2.1e-7 in f32 arithmetic, as ex2.approx.  Arguments are clamped at -126 (there 2^x is 1e-38 where ex2.approx gives 0).
+__device__ __forceinline__ uint64_t ex2_poly2(uint64_t x2) {
+  float x0, x1;
+  upk2(x2, x0, x1);
+  x2 = pk2(fmaxf(x0, -126.0f), fmaxf(x1, -126.0f));
+  const uint64_t magic = pk2(12582912.0f, 12582912.0f), nmagic = pk2(-12582912.0f, -12582912.0f), neg1 = pk2(-1.0f, -1.0f);
+  const uint64_t t2 = add2(x2, magic);
+  const uint64_t f2 = fma2(add2(t2, nmagic), neg1, x2);
+  uint64_t r = fma2(f2, pk2(0.0013276472454890609f, 0.0013276472454890609f), pk2(0.009675540961325169f, 0.009675540961325169f));
+  r = fma2(r, f2, pk2(0.05550713092088699f, 0.05550713092088699f));
+  r = fma2(r, f2, pk2(0.24022120237350464f, 0.24022120237350464f));
+  r = fma2(r, f2, pk2(0.6931469440460205f, 0.6931469440460205f));
+  r = fma2(r, f2, pk2(1.0000001192092896f, 1.0000001192092896f));
+  float t0, t1, r0, r1;
+  upk2(t2, t0, t1); upk2(r, r0, r1);
+  return pk2(__uint_as_float(__float_as_uint(r0) + (__float_as_uint(t0) << 23)), __uint_as_float(__float_as_uint(r1) + (__float_as_uint(t1) << 23)));
+}
+// pairs of a 32-score chunk (of 16) that take the polynomial
+#ifndef B200_FLASH_POLY
+#define B200_FLASH_POLY 4
+#endif
+template <bool POLY>
+__device__ __forceinline__ uint64_t ex2_pair(uint64_t x2, int i) {
+  if (POLY && (i * B200_FLASH_POLY) % 16 < B200_FLASH_POLY) return ex2_poly2(x2);
+  float x0, x1;
+  upk2(x2, x0, x1);
+  return pk2(ex2f(x0), ex2f(x1));
+}
+
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, int w, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+               ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar) : "memory");
+}
+// A from tensor memory (bf16 pairs, one row per lane), B from shared memory
+__device__ __forceinline__ void tc_mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+               ::"r"(d_tmem), "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+                 "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// MN-major, SWIZZLE_128B operand: 128-byte rows of 64 elements along N, one row per k.  Eight k rows are one 1 KiB group
+// (stride byte offset 1024); the next 64 elements of N start `lead` bytes further (leading byte offset).
+__device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t saddr, uint32_t lead) {
+  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lead >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+
+// Prompt form: one CTA per (batch, head, 256 query rows), 320 threads.
+//   warps 0-3, 4-7  softmax of query rows 0-127 and 128-255: one thread per row, scores read from tensor memory
+//   warp 8          TMA producer: Q once; K blocks of 128 keys (sweep 1); K and V blocks in turn (sweep 2)
+//   warp 9          MMA issuer
+// Tensor memory (512 columns): S0 S1 O0 O1.  In sweep 1 the O columns are the second score buffer of their tile, so the
+// tensor pipe runs a block ahead; in sweep 2 the normalised probabilities replace the scores in place as bf16 pairs and are the
+// A operand of the product with V straight from tensor memory, and the two row tiles alternate: while one is in its
+// exponentials the other's products run.
+// Bound by the exponentials (two per score: 16 per clock and SM, 1024 clocks per 128 x 128 block and sweep) beside the tensor
+// pipe (three products of 512 clocks per block).  256 query rows per CTA, because K and V then pass the L2 half as often as with 128
+// (64 KB per two blocks: 6 TB/s over the device at that rate, against 12 TB/s).
+template <int DB, bool MASK>
+__global__ void __launch_bounds__(kFlashThreads, 1)
+sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                  const __grid_constant__ CUtensorMap map_v, const SdpaFlashArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t bars[32];
+  __shared__ float2 stats[2][2][128];                  // row maximum and row sum of each half
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ volatile int s_err;
+  constexpr uint32_t kBox = 128 * 128;                 // [128 rows][64 elements]
+  constexpr uint32_t kTile = DB * kBox;                // 128 rows of Q, K or V
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (the same in every lane, and known to be)
+  const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t ring0 = smem0 + (uint32_t)a.tiles * kTile;
+  const uint32_t bar0 = smem_u32(bars);
+  const uint32_t q_full = bar0;
+  auto kv_full = [&](int s) { return bar0 + 8u * (1 + s); };
+  auto kv_empty = [&](int s) { return bar0 + 8u * (1 + kFlashSlots + s); };
+  auto s_full = [&](int t, int b) { return bar0 + 8u * (1 + 2 * kFlashSlots + 2 * t + b); };
+  auto s_free = [&](int t, int b) { return bar0 + 8u * (5 + 2 * kFlashSlots + 2 * t + b); };
+  auto p_ready = [&](int t, int half) { return bar0 + 8u * (9 + 2 * kFlashSlots + 2 * t + half); };
+  auto o_done = [&](int t) { return bar0 + 8u * (13 + 2 * kFlashSlots + t); };
+
+  if (threadIdx.x == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
+    mbar_init(q_full, 1);
+    for (int s = 0; s < kFlashSlots; ++s) { mbar_init(kv_full(s), 1); mbar_init(kv_empty(s), 1); }
+    for (int t = 0; t < 2; ++t) {
+      for (int b = 0; b < 2; ++b) { mbar_init(s_full(t, b), 1); mbar_init(s_free(t, b), 8); mbar_init(p_ready(t, b), 4); }
+      mbar_init(o_done(t), 1);
+    }
+    s_err = 0;
+    mbar_fence_init();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == kFlashSoftmaxWarps + 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_base_slot;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  // this CTA's work item
+  int bh, qt;
+  if (a.bh_major) { bh = blockIdx.x / a.n_qt; qt = a.n_qt - 1 - (blockIdx.x - bh * a.n_qt); }
+  else { const int r = blockIdx.x / a.n_bh; bh = blockIdx.x - r * a.n_bh; qt = a.n_qt - 1 - r; }
+  const int b = bh / a.H, h = bh - b * a.H;
+  const int q0 = qt * a.tiles * 128;
+  // key blocks that row tile t meets
+  auto n_blocks = [&](int t) {
+    const int r0 = q0 + t * 128;
+    if (t >= a.tiles || r0 >= a.S) return 0;
+    return (min(a.KV, a.causal ? r0 + 128 : a.KV) + 127) >> 7;
+  };
+  const int nb0 = n_blocks(0), nb1 = n_blocks(1), nmax = max(nb0, nb1);
+
+  if (warp == kFlashSoftmaxWarps) {
+    // ------------------------------------------------------------------ producer
+    if (lane == 0 && !a.test_no_loads) {
+      const int active = nb1 > 0 ? 2 : 1;
+      mbar_expect_tx(q_full, (uint32_t)active * kTile);
+      for (int t = 0; t < active; ++t)
+        for (int d = 0; d < DB; ++d)
+          tma_load_4d(smem0 + (uint32_t)t * kTile + (uint32_t)d * kBox, &map_q, d * 64, q0 + t * 128, h, b, q_full);
+      const int total = 3 * nmax;
+      for (int u = 0; u < total; ++u) {
+        const int slot = u % kFlashSlots;
+        if (!mbar_wait(kv_empty(slot), ((uint32_t)(u / kFlashSlots) & 1u) ^ 1u)) { s_err = 1; report_status(a.status, 21); break; }
+        const int w = u - nmax;
+        const bool is_v = w >= 0 && (w & 1);
+        const int blk = w < 0 ? u : (w >> 1);
+        mbar_expect_tx(kv_full(slot), kTile);
+        const CUtensorMap *m = is_v ? &map_v : &map_k;
+        const int hh = is_v ? h * a.vh : h * a.kh, bb = is_v ? b * a.vb : b * a.kb;
+        for (int d = 0; d < DB; ++d)
+          tma_load_4d(ring0 + (uint32_t)slot * kTile + (uint32_t)d * kBox, m, d * 64, blk * 128, hh, bb, kv_full(slot));
+      }
+    }
+  } else if (warp == kFlashSoftmaxWarps + 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    // The whole warp walks the schedule and one elected lane issues: control flow and operands stay warp-uniform, so the
+    // descriptors live in uniform registers.  (Inside a lane == 0 branch every MMA first moved its operands there, about 100
+    // clocks each: the issue, not the tensor pipe, was the bound -- 1.2 us for two 128 x 128 x 128 products instead of 0.6.)
+    const uint32_t idesc_s = make_idesc_bf16(128);
+    const uint32_t idesc_o = make_idesc_bf16((a.D + 15) & ~15) | (1u << 16);           // B (V) is N-major
+    const int ksteps = (a.D + 15) >> 4;
+    const uint64_t q_desc = make_smem_desc(smem0), k_desc = make_smem_desc(ring0), v_desc = make_smem_desc_mn(ring0, kBox);
+    constexpr uint64_t kTileD = kTile >> 4, kBoxD = kBox >> 4;
+    auto qk = [&](int t, uint32_t d_tmem, int slot, uint32_t bar) {
+      const uint64_t qa = q_desc + (uint64_t)t * kTileD, ka = k_desc + (uint64_t)slot * kTileD;
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < 4 * DB; ++k)
+          if (k < ksteps) tc_mma_bf16(d_tmem, qa + (k >> 2) * kBoxD + (k & 3) * 2, ka + (k >> 2) * kBoxD + (k & 3) * 2, idesc_s, k ? 1u : 0u);
+        tc_commit(bar);
+      }
+      __syncwarp();
+    };
+    auto pv = [&](int t, int slot, bool first, int k0) {       // 64 keys: k0 = 0 or 4
+      const uint64_t va = v_desc + (uint64_t)slot * kTileD + (uint64_t)(k0 * 128);
+      const uint32_t pa = tmem + (uint32_t)t * 128u + (k0 ? 64u : 0u), od = tmem + 256u + (uint32_t)t * 128u;
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) tc_mma_bf16_ts(od, pa + (uint32_t)k * 8u, va + k * 128, idesc_o, (first && k0 + k == 0) ? 0u : 1u);
+      }
+      __syncwarp();
+    };
+    auto commit = [&](uint32_t bar) { if (elect_one()) tc_commit(bar); __syncwarp(); };
+    auto wait = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0; };
+    bool ok = wait(q_full, 0);
+    int u = 0;
+    auto full = [&](int uu) { return wait(kv_full(uu % kFlashSlots), (uint32_t)(uu / kFlashSlots) & 1u); };
+    // sweep 1: scores only, two buffers per tile
+    for (int j = 0; ok && j < nmax; ++j, ++u) {
+      ok = full(u);
+      if (!ok) break;
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        if (!ok || j >= (t ? nb1 : nb0)) continue;
+        ok = wait(s_free(t, j & 1), ((uint32_t)(j >> 1) & 1u) ^ 1u);
+        if (!ok) break;
+        tc_fence_after();
+        qk(t, tmem + (uint32_t)t * 128u + ((j & 1) ? 256u : 0u), u % kFlashSlots, s_full(t, j & 1));
+      }
+      commit(kv_empty(u % kFlashSlots));
+    }
+    // sweep 2: first scores
+    if (ok) ok = full(u);
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const int nb = t ? nb1 : nb0;
+      if (!ok || nb == 0) continue;
+      ok = wait(s_free(t, 0), ((uint32_t)((nb + 1) >> 1) & 1u) ^ 1u);
+      if (!ok) break;
+      tc_fence_after();
+      qk(t, tmem + (uint32_t)t * 128u, u % kFlashSlots, s_full(t, 0));
+    }
+    if (ok) { commit(kv_empty(u % kFlashSlots)); ++u; }
+    for (int j = 0; ok && j < nmax; ++j, u += 2) {
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const int nb = t ? nb1 : nb0;
+        if (!ok || j >= nb) continue;
+        ok = wait(p_ready(t, 0), (uint32_t)j & 1u) && full(u);
+        if (!ok) break;
+        tc_fence_after();
+        pv(t, u % kFlashSlots, j == 0, 0);
+        ok = wait(p_ready(t, 1), (uint32_t)j & 1u);
+        if (!ok) break;
+        tc_fence_after();
+        pv(t, u % kFlashSlots, j == 0, 4);
+        if (j + 1 < nb) {
+          ok = full(u + 1);
+          if (!ok) break;
+          qk(t, tmem + (uint32_t)t * 128u, (u + 1) % kFlashSlots, s_full(t, 0));
+        } else commit(o_done(t));
+      }
+      commit(kv_empty(u % kFlashSlots));
+      if (j + 1 < nmax) commit(kv_empty((u + 1) % kFlashSlots));
+    }
+    if (!ok && lane == 0) { s_err = 1; report_status(a.status, 22); }
+  } else {
+    // ------------------------------------------------------------------ softmax
+    // thread: one row, one half (64 keys) of every block
+    const int t = warp >> 3, half = (warp >> 2) & 1, nb = t ? nb1 : nb0;
+    const int row_in_tile = (warp & 3) * 32 + lane, row = q0 + t * 128 + row_in_tile;
+    const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t ts0 = tmem + lane_off + (uint32_t)t * 128u + (uint32_t)half * 64u, to0 = ts0 + 256u;
+    const float ninf = __int_as_float(0xff800000), c = a.scale_log2;
+    const int n_keys = min(a.KV, a.causal ? row + 1 : a.KV);         // keys this row sees
+    const int64_t moff = MASK ? (int64_t)b * a.mask.mb + (int64_t)h * a.mask.mh + (int64_t)min(row, a.S - 1) * a.mask.mi : 0;
+    // a chunk of 32 scores in the log2 domain; with a mask, scale and mask are applied here (vector loads where the mask's rows
+    // allow it: all lanes read the same bytes when the mask does not depend on the query)
+    auto mask32 = [&](uint32_t (&s)[32], int j0) {
+      if constexpr (MASK) {
+        const float log2e = 1.44269504088896340736f;
+        auto put = [&](int i, float mv) { s[i] = __float_as_uint(__fmaf_rn(__uint_as_float(s[i]), c, __fmul_rn(mv, log2e))); };
+        const bool whole = j0 + 32 <= a.KV;
+        if (a.mask.dt == DT_F32) {
+          const float *mp = reinterpret_cast<const float *>(a.mask.p) + moff + j0;
+          if (a.mask_vec && whole) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              const float4 v = __ldg(reinterpret_cast<const float4 *>(mp + i));
+              put(i, v.x); put(i + 1, v.y); put(i + 2, v.z); put(i + 3, v.w);
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) put(i, j0 + i < a.KV ? __ldg(mp + i) : 0.f);
+          }
+        } else {
+          const uint16_t *mp = reinterpret_cast<const uint16_t *>(a.mask.p) + moff + j0;
+          if (a.mask_vec && whole) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) {
+              const uint4 v = __ldg(reinterpret_cast<const uint4 *>(mp + i));
+              const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) { put(i + 2 * e, __uint_as_float(w[e] << 16)); put(i + 2 * e + 1, __uint_as_float(w[e] & 0xffff0000u)); }
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) put(i, j0 + i < a.KV ? bf16_bits_to_f32(__ldg(mp + i)) : 0.f);
+          }
+        }
+      }
+    };
+    auto limit32 = [&](uint32_t (&s)[32], int j0) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) if (j0 + i >= n_keys) s[i] = __float_as_uint(ninf);
+    };
+    float m = ninf, l = 0.f;
+    bool ok = true;
+    uint32_t ph0 = 0, ph1 = 0;
+    const float cc = MASK ? 1.0f : c;
+    // this half of a block with the row maximum brought up to date (first block, blocks of rows that a mask has hidden so far, and the recovery below)
+    auto half_with_max = [&](uint32_t ta, int k0, bool last) {
+      float mx = ninf;
+#pragma unroll 1
+      for (int q = 0; q < 2; ++q) {
+        uint32_t s[32];
+        tc_ld32(ta + (uint32_t)q * 32u, s);
+        tc_wait_ld();
+        mask32(s, k0 + q * 32);
+        if (last) limit32(s, k0 + q * 32);
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(s[i]), __uint_as_float(s[i + 1])));
+      }
+      const float mn = fmaxf(m, mx), nmc = mn == ninf ? 0.f : -mn * cc;      // (no key so far: every term is 2^-inf)
+      const uint64_t c2 = pk2(cc, cc), b2 = pk2(nmc, nmc);
+      uint64_t acc = 0ull;
+#pragma unroll 1
+      for (int q = 0; q < 2; ++q) {
+        uint32_t s[32];
+        tc_ld32(ta + (uint32_t)q * 32u, s);
+        tc_wait_ld();
+        mask32(s, k0 + q * 32);
+        if (last) limit32(s, k0 + q * 32);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc = add2(acc, ex2_pair<false>(fma2(pk2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), c2, b2), i));
+      }
+      float e0, e1;
+      upk2(acc, e0, e1);
+      l = __fmaf_rn(l, ex2f(__fmaf_rn(m, cc, nmc)), e0 + e1);
+      m = mn;
+    };
+    // ---- sweep 1: row maximum and row sum.  The reference m only has to keep the sum in range, so after the first block it stays as
+    // it is (the first block's maximum: the sum is at least 1) and a block's terms are added without a maximum of their own; a block
+    // whose sum leaves the comfortable range (scores 40 above the reference, in powers of two) is done again with its maximum.
+    auto sum_half = [&](uint32_t ta, int k0, auto poly, bool last) {
+      const uint64_t c2 = pk2(cc, cc), b2 = pk2(-m * cc, -m * cc);
+      uint64_t acc[2] = {0ull, 0ull};
+      uint32_t s[2][32];
+      tc_ld32(ta, s[0]);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        tc_wait_ld();
+        if (q < 1) tc_ld32(ta + 32u, s[1]);
+        mask32(s[q], k0 + q * 32);
+        if (last) limit32(s[q], k0 + q * 32);
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          acc[i & 1] = add2(acc[i & 1], ex2_pair<decltype(poly)::value>(fma2(pk2(__uint_as_float(s[q][2 * i]), __uint_as_float(s[q][2 * i + 1])), c2, b2), i));
+      }
+      float e0, e1;
+      upk2(add2(acc[0], acc[1]), e0, e1);
+      return e0 + e1;
+    };
+    for (int j = 0; ok && j < nb; ++j) {
+      const int bf = j & 1, k0 = j * 128 + half * 64;
+      ok = __all_sync(0xffffffffu, mbar_wait(s_full(t, bf), bf ? ph1 : ph0));      // one decision per warp: tensor-memory loads are warp-wide
+      if (!ok) break;
+      if (bf) ph1 ^= 1u; else ph0 ^= 1u;
+      tc_fence_after();
+      const uint32_t ta = bf ? to0 : ts0;
+      if (j == 0 || (MASK && !__all_sync(0xffffffffu, m > ninf))) half_with_max(ta, k0, j == nb - 1);
+      else {
+        // (the polynomial does not return 0 for the -inf of a masked key)
+        const float e = j == nb - 1 ? sum_half(ta, k0, FlashFalse{}, true) : (MASK ? sum_half(ta, k0, FlashFalse{}, false) : sum_half(ta, k0, FlashTrue{}, false));
+        if (__any_sync(0xffffffffu, !(e < 1.0995e12f))) half_with_max(ta, k0, j == nb - 1);
+        else l += e;
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(s_free(t, bf));
+    }
+    // ---- the two halves of a row together
+    stats[t][half][row_in_tile] = make_float2(m, l);
+    asm volatile("bar.sync %0, 256;" ::"r"(1 + t) : "memory");
+    {
+      const float2 o = stats[t][half ^ 1][row_in_tile];
+      const float mn = fmaxf(m, o.x), nmc = mn == ninf ? 0.f : -mn * cc;
+      l = l * ex2f(__fmaf_rn(m, cc, nmc)) + o.y * ex2f(__fmaf_rn(o.x, cc, nmc));
+      m = mn;
+    }
+    // ---- sweep 2: p = 2^(s * c - m * c - log2 l); a row that sees no key gives zeros
+    const float bias = l > 0.f ? -m * cc - __log2f(l) : ninf;
+    const uint64_t pc2 = pk2(cc, cc), pb2 = pk2(bias, bias);
+    auto p_half = [&](int k0, auto poly, bool last) {
+      uint32_t s[2][32];
+      tc_ld32(ts0, s[0]);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        tc_wait_ld();
+        if (q < 1) tc_ld32(ts0 + 32u, s[1]);
+        mask32(s[q], k0 + q * 32);
+        if (last) limit32(s[q], k0 + q * 32);
+        uint32_t p[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          float x0, x1;
+          upk2(ex2_pair<decltype(poly)::value>(fma2(pk2(__uint_as_float(s[q][2 * i]), __uint_as_float(s[q][2 * i + 1])), pc2, pb2), i), x0, x1);
+          p[i] = pack_bf16x2(x0, x1);
+        }
+        tc_st16(ts0 + (uint32_t)q * 16u, p);      // (over scores of this half that have been read)
+      }
+      tc_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_ready(t, half));
+    };
+    for (int j = 0; ok && j < nb; ++j) {
+      ok = __all_sync(0xffffffffu, mbar_wait(s_full(t, 0), ph0));
+      if (!ok) break;
+      ph0 ^= 1u;
+      tc_fence_after();
+      if (MASK || j == nb - 1) p_half(j * 128 + half * 64, FlashFalse{}, j == nb - 1); else p_half(j * 128 + half * 64, FlashTrue{}, false);
+    }
+    if (ok && nb > 0) ok = __all_sync(0xffffffffu, mbar_wait(o_done(t), 0));
+    if (ok && nb > 0) {
+      tc_fence_after();
+      uint16_t *o = a.out + (int64_t)b * a.ob + (int64_t)h * a.oh + (int64_t)row * a.os;
+      const int units = (a.D + 15) >> 4, u0 = half ? (units + 1) >> 1 : 0, u1 = half ? units : (units + 1) >> 1;     // the halves share the columns
+      const uint32_t od = tmem + lane_off + 256u + (uint32_t)t * 128u;
+      for (int d0 = u0 * 16; d0 < u1 * 16; d0 += 16) {
+        uint32_t r[16], pk[8];
+        tc_ld16(od + (uint32_t)d0, r);
+        tc_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) pk[i] = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+        if (row < a.S) {
+          if (a.out_align == 32 && d0 + 16 <= a.D) st_global_v8(o + d0, pk);
+          else if (a.out_align >= 16) {
+            *reinterpret_cast<uint4 *>(o + d0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            if (d0 + 16 <= a.D) *reinterpret_cast<uint4 *>(o + d0 + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) if (d0 + i < a.D) o[d0 + i] = (uint16_t)(pk[i >> 1] >> ((i & 1) * 16));
+          }
+        }
+        __syncwarp();
+      }
+    }
+    if (!ok && lane == 0) { s_err = 1; report_status(a.status, 23); }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (s_err) {
+    for (int i = 0; i < 64; ++i) __nanosleep(20000);     // copies still in flight land before shared memory is released
+    __syncthreads();
+  }
+  if (warp == kFlashSoftmaxWarps + 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+}
+
+// ---- few query rows (S <= 16) against many keys: bound by reading K and V once -----------------------------------------
+// A cluster of C CTAs per (batch, head), each with a contiguous share of the keys; eight consumer warps and a producer warp.
+//   0. the producer streams the share's K blocks and then its V blocks (128 keys each) through one shared-memory ring with TMA: the
+//      first V blocks are on their way while the row maxima and sums of step 2 are exchanged, so HBM does not pause there, and the
+//      bytes in flight per SM are the ring's (two CTAs of three slots), not a register budget.
+//   1. scores: warp w takes keys 16 w .. 16 w + 15 of a block with mma.m16n8k16 (A: the query rows, in registers for the whole
+//      call; B: eight keys).  K rows sit in 64-byte pieces ([128 keys][32 elements], no swizzle): a lane's fragment of key g is the
+//      16 bytes at 8 t of a piece, the same assignment of d to fragment positions on both operands, so a quarter warp reads
+//      128 contiguous bytes.  f32 scores (log2 domain, mask applied) stay in shared memory.
+//   2. final row maximum and row sum over the cluster through distributed shared memory, p = bf16(e / sum).
+//   3. p V: keys are the k dimension; V sits in 128-byte swizzled rows, a lane reads 16 bytes (8 columns) of four key rows (a
+//      quarter warp: eight different bank groups) and pairs them with byte permutes.  Up to eight query rows: V^T p^T, columns
+//      of V as the 16 MMA rows; more: p V with the query rows as MMA rows.
+//   4. f32 partial outputs are added over warps and CTAs in a fixed order.
+struct SdpaDecodeArgs {
+  const uint16_t *q; uint16_t *out;
+  int64_t qb, qh, qs, ob, oh, os;
+  int kb, kh, vb, vh;      // 0 where K / V are broadcast over the batch / the heads, else 1
+  int S, KV, D, H;
+  int chunk;               // keys per CTA, a multiple of 128
+  int sc_stride;           // f32 per score row in shared memory
+  float scale_log2;
+  int causal;
+  SdpaMask mask;
+  int32_t *status;
+};
+constexpr int kSdpaDecodeWarps = 8, kSdpaDecodeThreads = 32 * (kSdpaDecodeWarps + 1), kSdpaDecodeSlots = 3;
+
+__device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t caddr) { float v; asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(caddr) : "memory"); return v; }
+
+// shared memory: [ring][scores, later the partial outputs]
+__host__ __device__ inline size_t sdpa_decode_ring_bytes(int db) { return (size_t)kSdpaDecodeSlots * db * 16384; }
+
+// DB: 64-element blocks of the head dimension (1: D <= 64, 2: D <= 128); HI: more than eight query rows
+template <int DB, bool HI>
+__global__ void __launch_bounds__(kSdpaDecodeThreads, 2)
+sdpa_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const SdpaDecodeArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t bars[2 * kSdpaDecodeSlots];
+  __shared__ float wred[kSdpaDecodeWarps][16], cmax[16], csum[16], row_m[16], row_inv[16];
+  __shared__ volatile int s_err;
+  constexpr int NP = 2 * DB;                       // 32-element pieces of a key row
+  constexpr uint32_t kSlot = DB * 16384;           // 128 keys
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  uint32_t csize, crank;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(csize));
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u, bar0 = smem_u32(bars);
+  float *sc = reinterpret_cast<float *>(smem_raw + (ring - smem_u32(smem_raw)) + sdpa_decode_ring_bytes(DB));
+  auto full = [&](int s) { return bar0 + 8u * (uint32_t)s; };
+  auto empty = [&](int s) { return bar0 + 8u * (uint32_t)(kSdpaDecodeSlots + s); };
+  if (tid == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
+    for (int s = 0; s < kSdpaDecodeSlots; ++s) { mbar_init(full(s), 1); mbar_init(empty(s), kSdpaDecodeWarps); }
+    s_err = 0;
+    mbar_fence_init();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  __syncthreads();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int bh = blockIdx.x / csize, b = bh / a.H, h = bh - b * a.H;
+  const int k0 = (int)crank * a.chunk, k1 = min(a.KV, k0 + a.chunk);     // this CTA's keys (k1 <= k0: none)
+  const int nblk = k1 > k0 ? (k1 - k0 + 127) >> 7 : 0;
+  const int S = a.S, D = a.D;
+  const float ninf = __int_as_float(0xff800000);
+  bool ok = true;
+
+  // The producer takes part in the barriers of step 2, so before them it may only wait for slots that the K blocks free: blocks up to
+  // nblk + slots - 1; the others follow in step 3.
+  auto produce = [&](int from, int to) {
+    if (lane != 0) return;
+    for (int u = from; u < to; ++u) {
+      const int slot = u % kSdpaDecodeSlots;
+      if (!mbar_wait(empty(slot), ((uint32_t)(u / kSdpaDecodeSlots) & 1u) ^ 1u)) { s_err = 1; report_status(a.status, 41); break; }
+      const bool is_v = u >= nblk;
+      const int key = k0 + (is_v ? u - nblk : u) * 128;
+      const uint32_t dst = ring + (uint32_t)slot * kSlot;
+      mbar_expect_tx(full(slot), kSlot);
+      if (is_v) { for (int d = 0; d < DB; ++d) tma_load_4d(dst + (uint32_t)d * 16384u, &map_v, d * 64, key, h * a.vh, b * a.vb, full(slot)); }
+      else { for (int i = 0; i < NP; ++i) tma_load_4d(dst + (uint32_t)i * 8192u, &map_k, i * 32, key, h * a.kh, b * a.kb, full(slot)); }
+    }
+  };
+  const int n_early = min(2 * nblk, nblk + kSdpaDecodeSlots);
+  if (warp == kSdpaDecodeWarps) { produce(0, n_early); __syncwarp(); }
+  // ---- query fragments
+  uint4 qlo[NP], qhi[HI ? NP : 1];
+  if (warp < kSdpaDecodeWarps) {
+    const uint16_t *qp = a.q + (int64_t)b * a.qb + (int64_t)h * a.qh;
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int d = i * 32 + t * 8;
+      qlo[i] = (g < S && d < D) ? __ldg(reinterpret_cast<const uint4 *>(qp + (int64_t)g * a.qs + d)) : make_uint4(0, 0, 0, 0);
+      if constexpr (HI) qhi[i] = (g + 8 < S && d < D) ? __ldg(reinterpret_cast<const uint4 *>(qp + (int64_t)(g + 8) * a.qs + d)) : make_uint4(0, 0, 0, 0);
+    }
+    // ---- 1. scores
+    float m_lo = ninf, m_hi = ninf;
+    const int64_t moff = (int64_t)b * a.mask.mb + (int64_t)h * a.mask.mh;
+    for (int u = 0; u < nblk; ++u) {
+      const int slot = u % kSdpaDecodeSlots;
+      // (one decision per warp; the other warps meet this one at the barriers below either way)
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(full(slot), (uint32_t)(u / kSdpaDecodeSlots) & 1u));
+      if (!ok) { if (lane == 0) { s_err = 1; report_status(a.status, 42); } break; }
+      const int kw = u * 128 + warp * 16;                    // this warp's first key, relative to k0
+      uint4 kr[2][NP];
+#pragma unroll
+      for (int v = 0; v < 2; ++v)
+#pragma unroll
+        for (int i = 0; i < NP; ++i) kr[v][i] = ld_shared_v4(ring + (uint32_t)slot * kSlot + (uint32_t)(i * 8192 + (warp * 16 + v * 8 + g) * 64 + t * 16));
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty(slot));
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+          uint4 hi = make_uint4(0, 0, 0, 0);
+          if constexpr (HI) hi = qhi[i];
+          mma_bf16_16816(acc, qlo[i].x, hi.x, qlo[i].y, hi.y, kr[v][i].x, kr[v][i].y);
+          mma_bf16_16816(acc, qlo[i].z, hi.z, qlo[i].w, hi.w, kr[v][i].z, kr[v][i].w);
+        }
+        const int key = kw + v * 8 + 2 * t;
+#pragma unroll
+        for (int hb = 0; hb < (HI ? 2 : 1); ++hb) {
+          const int row = g + 8 * hb;
+          if (row < S) {
+            float x[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int j = k0 + key + e;
+              float mv = 0.f;
+              if (a.mask.p && j < k1) mv = __fmul_rn(load_as_f32(a.mask.p, a.mask.dt, moff + (int64_t)row * a.mask.mi + j), 1.44269504088896340736f);
+              x[e] = (j < k1 && !(a.causal && j > row)) ? __fmaf_rn(acc[2 * hb + e], a.scale_log2, mv) : ninf;
+            }
+            *reinterpret_cast<float2 *>(sc + (size_t)row * a.sc_stride + key) = make_float2(x[0], x[1]);
+            if (hb) m_hi = fmaxf(m_hi, fmaxf(x[0], x[1])); else m_lo = fmaxf(m_lo, fmaxf(x[0], x[1]));
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) { m_lo = fmaxf(m_lo, __shfl_xor_sync(0xffffffffu, m_lo, o)); m_hi = fmaxf(m_hi, __shfl_xor_sync(0xffffffffu, m_hi, o)); }
+    if (t == 0) { wred[warp][g] = m_lo; wred[warp][g + 8] = m_hi; }
+  }
+  // ---- 2. row maximum and row sum over the cluster
+  auto csync = [&]() { if (csize > 1) cluster_sync_all(); else __syncthreads(); };
+  __syncthreads();
+  if (tid < 16) {
+    float v = wred[0][tid];
+    for (int w = 1; w < kSdpaDecodeWarps; ++w) v = fmaxf(v, wred[w][tid]);
+    cmax[tid] = v;
+  }
+  csync();
+  if (tid < 16) {
+    float v = cmax[tid];
+    for (uint32_t r = 0; r < csize; ++r) if (r != crank) v = fmaxf(v, ld_cluster_f32(cluster_map(smem_u32(&cmax[tid]), r)));
+    row_m[tid] = v == ninf ? 0.f : v;
+  }
+  __syncthreads();
+  const int nk = nblk * 128;                               // (scores of keys past the end are -inf)
+  if (warp < kSdpaDecodeWarps && ok) {
+    // the warps share the rows; with fewer rows than warps each row is cut into 8 / S' parts (S' = rows rounded up to a power of two)
+    const int parts = S >= 8 ? 1 : (S > 4 ? 1 : (S > 2 ? 2 : (S > 1 ? 4 : 8)));
+    for (int row = warp / parts; row < S; row += kSdpaDecodeWarps / parts) {
+      const float m = row_m[row];
+      float sum = 0.f;
+      float *sr = sc + (size_t)row * a.sc_stride;
+      for (int j = ((warp % parts) * 32 + lane) * 2; j < nk; j += 64 * parts) {
+        float2 x = *reinterpret_cast<float2 *>(sr + j);
+        x.x = ex2f(x.x - m); x.y = ex2f(x.y - m);
+        sum += x.x + x.y;
+        *reinterpret_cast<float2 *>(sr + j) = x;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (lane == 0) wred[warp % parts][row] = sum;
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(kSdpaDecodeWarps * 32) : "memory");
+    if (tid < S) {
+      float v = wred[0][tid];
+      for (int q = 1; q < parts; ++q) v += wred[q][tid];
+      csum[tid] = v;
+    }
+  } else if (warp < kSdpaDecodeWarps) asm volatile("bar.sync 1, %0;" ::"n"(kSdpaDecodeWarps * 32) : "memory");
+  csync();
+  if (tid < 16) {
+    float v = 0.f;
+    if (tid < S) for (uint32_t r = 0; r < csize; ++r) v += csize > 1 ? ld_cluster_f32(cluster_map(smem_u32(&csum[tid]), r)) : csum[tid];
+    row_inv[tid] = v > 0.f ? __fdiv_rn(1.0f, v) : 0.f;
+  }
+  __syncthreads();
+  // ---- 3. p V
+  constexpr int NA = HI ? 8 : 4;                           // accumulator tiles per 64 columns
+  float acc[DB][NA][4];
+#pragma unroll
+  for (int s = 0; s < DB; ++s)
+#pragma unroll
+    for (int i = 0; i < NA; ++i) acc[s][i][0] = acc[s][i][1] = acc[s][i][2] = acc[s][i][3] = 0.f;
+  if (warp == kSdpaDecodeWarps) { produce(n_early, 2 * nblk); __syncwarp(); }
+  else {
+    const float inv_lo = row_inv[g], inv_hi = row_inv[g + 8];
+    for (int n = 0; n < nblk; ++n) {
+      const int u = nblk + n, slot = u % kSdpaDecodeSlots;
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(full(slot), (uint32_t)(u / kSdpaDecodeSlots) & 1u));
+      if (!ok) { if (lane == 0) { s_err = 1; report_status(a.status, 43); } break; }
+      const int kw = n * 128 + warp * 16;
+      uint4 vr[4][DB];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int row = warp * 16 + 2 * t + (r & 1) + (r >> 1) * 8;
+#pragma unroll
+        for (int s = 0; s < DB; ++s) vr[r][s] = ld_shared_v4(ring + (uint32_t)slot * kSlot + (uint32_t)(s * 16384 + row * 128 + ((g ^ (row & 7)) << 4)));
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty(slot));
+      uint32_t p0 = 0, p1 = 0, p2 = 0, p3 = 0;             // probabilities of rows g (p0: keys 2t.., p2: 2t + 8..) and g + 8 (p1, p3)
+      if (g < S) {
+        const float *sr = sc + (size_t)g * a.sc_stride + kw + 2 * t;
+        const float2 x = *reinterpret_cast<const float2 *>(sr), y = *reinterpret_cast<const float2 *>(sr + 8);
+        p0 = pack_bf16x2(__fmul_rn(x.x, inv_lo), __fmul_rn(x.y, inv_lo)); p2 = pack_bf16x2(__fmul_rn(y.x, inv_lo), __fmul_rn(y.y, inv_lo));
+      }
+      if (HI && g + 8 < S) {
+        const float *sr = sc + (size_t)(g + 8) * a.sc_stride + kw + 2 * t;
+        const float2 x = *reinterpret_cast<const float2 *>(sr), y = *reinterpret_cast<const float2 *>(sr + 8);
+        p1 = pack_bf16x2(__fmul_rn(x.x, inv_hi), __fmul_rn(x.y, inv_hi)); p3 = pack_bf16x2(__fmul_rn(y.x, inv_hi), __fmul_rn(y.y, inv_hi));
+      }
+#pragma unroll
+      for (int s = 0; s < DB; ++s) {
+        const uint32_t w0[4] = {vr[0][s].x, vr[0][s].y, vr[0][s].z, vr[0][s].w}, w1[4] = {vr[1][s].x, vr[1][s].y, vr[1][s].z, vr[1][s].w};
+        const uint32_t w2[4] = {vr[2][s].x, vr[2][s].y, vr[2][s].z, vr[2][s].w}, w3[4] = {vr[3][s].x, vr[3][s].y, vr[3][s].z, vr[3][s].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          // columns 8 g + 2 i and 8 g + 2 i + 1 of this set, keys (2t, 2t + 1) and (2t + 8, 2t + 9)
+          const uint32_t e0 = __byte_perm(w0[i], w1[i], 0x5410u), o0 = __byte_perm(w0[i], w1[i], 0x7632u);
+          const uint32_t e1 = __byte_perm(w2[i], w3[i], 0x5410u), o1 = __byte_perm(w2[i], w3[i], 0x7632u);
+          if constexpr (HI) {
+            mma_bf16_16816(acc[s][(2 * i) % NA], p0, p1, p2, p3, e0, e1);
+            mma_bf16_16816(acc[s][(2 * i + 1) % NA], p0, p1, p2, p3, o0, o1);
+          } else mma_bf16_16816(acc[s][i], e0, o0, e1, o1, p0, p2);
+        }
+      }
+    }
+  }
+  __syncthreads();                    // every warp has read its scores: the space takes the partial outputs
+  // [8 warps][S][D] f32, then their sum in [0][S][D]
+  float *red = sc;
+  if (warp < kSdpaDecodeWarps) {
+#pragma unroll
+    for (int s = 0; s < DB; ++s)
+#pragma unroll
+      for (int i = 0; i < NA; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int row = HI ? g + 8 * (e >> 1) : 2 * t + (e & 1);
+          const int d = HI ? s * 64 + (2 * t + (e & 1)) * 8 + i : s * 64 + g * 8 + 2 * i + (e >> 1);
+          if (row < S && d < D) red[((size_t)warp * S + row) * D + d] = acc[s][i][e];
+        }
+  }
+  __syncthreads();
+  for (int i = tid; i < S * D; i += kSdpaDecodeThreads) {
+    float v = red[i];
+#pragma unroll
+    for (int w = 1; w < kSdpaDecodeWarps; ++w) v += red[(size_t)w * S * D + i];
+    red[i] = v;
+  }
+  csync();
+  // ---- 4. sum over the cluster; the CTAs share the elements
+  if (!s_err)
+    for (int i = (int)crank * kSdpaDecodeThreads + tid; i < S * D; i += (int)csize * kSdpaDecodeThreads) {
+      float v = 0.f;
+      if (csize > 1) { for (uint32_t r = 0; r < csize; ++r) v += ld_cluster_f32(cluster_map(smem_u32(red + i), r)); }
+      else v = red[i];
+      const int row = i / D, d = i - row * D;
+      a.out[(int64_t)b * a.ob + (int64_t)h * a.oh + (int64_t)row * a.os + d] = (uint16_t)(pack_bf16x2(v, 0.f) & 0xFFFFu);
+    }
+  if (csize > 1) cluster_sync_all();  // nobody leaves while a neighbour may still read its shared memory
+  if (s_err) { for (int i = 0; i < 64; ++i) __nanosleep(20000); }      // copies still in flight land before shared memory is released
+}
+
+}  // namespace b200
