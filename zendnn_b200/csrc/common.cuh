@@ -110,6 +110,25 @@ __device__ __forceinline__ int32_t load_zp(const EpiParams &e) {
   }
 }
 
+// Sixteen bytes at any address, of which the first `avail` exist (the rest come back as zero): five aligned words and funnel shifts.
+// Only aligned words that hold at least one existing byte are read.
+__device__ __forceinline__ uint4 ld16_any(const uint8_t *p, int avail) {
+  const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3);
+  const uint32_t *w = reinterpret_cast<const uint32_t *>(p - mis);
+  const int last = (int)mis + (avail < 16 ? avail : 16);      // existing bytes, counted from the first aligned word
+  uint32_t x[5];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) x[i] = 4 * i < last ? w[i] : 0u;
+  uint32_t o[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    o[i] = __funnelshift_r(x[i], x[i + 1], mis * 8);
+    const int left = avail - 4 * i;
+    if (left < 4) o[i] = left > 0 ? o[i] & (0xFFFFFFFFu >> (32 - 8 * left)) : 0u;
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 __device__ __forceinline__ bool finite_f32(float v) { return (__float_as_uint(v) & 0x7F800000u) != 0x7F800000u; }
 
 // Per-row / per-group view of the epilogue operands (the grouped GEMM swaps these per expert).

@@ -96,12 +96,8 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, 1) decode_gemm_kernel(Decod
         if (vec && k + 16 <= g.K) {
           asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem + (size_t)r * g.a_stride + k)), "l"(src) : "memory");
           continue;
-        } else {
-          uint8_t tmp[16];
-#pragma unroll
-          for (int b = 0; b < 16; ++b) tmp[b] = (k + b < g.K) ? src[b] : (uint8_t)0;
-          v = *reinterpret_cast<uint4 *>(tmp);
         }
+        v = ld16_any(src, g.K - k);
       }
       *reinterpret_cast<uint4 *>(smem + (size_t)r * g.a_stride + k) = v;
     }

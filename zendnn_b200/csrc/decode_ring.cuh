@@ -134,7 +134,8 @@ __global__ void __launch_bounds__((kRingWarps + 1) * 32, 1) decode_ring_kernel(D
         const uint32_t dst = smem_u32(smem + (size_t)r * g.a_stride);
         for (int k = tid * 16; k < kv; k += kConsumers * 16)
           asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)k), "l"(src + k) : "memory");
-        for (int k = kv + tid; k < g.K; k += kConsumers) smem[(size_t)r * g.a_stride + k] = src[k];
+        for (int k = kv + tid * 16; k < g.K; k += kConsumers * 16)      // (an unaligned row, or the tail: columns k >= K hold zero weights)
+          *reinterpret_cast<uint4 *>(smem + (size_t)r * g.a_stride + k) = ld16_any(src + k, g.K - k);
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
       decode_epi_stage(epi, es, g0 * 8, n_local * 8, g.N, g.M, tid, kConsumers);
