@@ -321,6 +321,58 @@ __device__ __forceinline__ void warp_store_rows64(uint8_t *sbuf, const uint4 (&v
   warp_store_rows32(sbuf, v[2], v[3], g_row0 + 32, pitch_bytes, rows_valid, lane);
 }
 
+// The same block for a destination without 16-byte alignment (an odd N or ldc): the rows pass through the staging block and leave
+// element by element, but along the rows -- an instruction writes 32 bytes of each of four (4-byte elements) or four (bf16, as
+// aligned words) rows instead of one element in each of 32.  M = 5000, N = 4097, K = 4096, bf16 out: 259 -> 111 us.
+// cols: how many of the block's columns exist.
+__device__ __forceinline__ void warp_stage_rows32(uint8_t *sbuf, const uint4 &v0, const uint4 &v1, int lane) {
+  const int sw = (lane >> 2) & 1;
+  *reinterpret_cast<uint4 *>(sbuf + lane * 32 + ((0 ^ sw) << 4)) = v0;
+  *reinterpret_cast<uint4 *>(sbuf + lane * 32 + ((1 ^ sw) << 4)) = v1;
+  __syncwarp();
+}
+__device__ __forceinline__ const uint8_t *warp_staged_byte(const uint8_t *sbuf, int row, int byte) {
+  return sbuf + row * 32 + ((((byte >> 4) ^ (row >> 2)) & 1) << 4) + (byte & 15);
+}
+// [32 rows x 8 four-byte elements]
+__device__ __forceinline__ void warp_store_any32(uint8_t *sbuf, const uint4 &v0, const uint4 &v1, uint8_t *g_row0, int64_t pitch_bytes, int rows_valid,
+                                                 int cols, int lane) {
+  warp_stage_rows32(sbuf, v0, v1, lane);
+  const int c = lane & 7;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int R = 4 * j + (lane >> 3);
+    const uint32_t val = *reinterpret_cast<const uint32_t *>(warp_staged_byte(sbuf, R, c * 4));
+    if (R < rows_valid && c < cols) *reinterpret_cast<uint32_t *>(g_row0 + (int64_t)R * pitch_bytes + c * 4) = val;
+  }
+  __syncwarp();
+}
+// [32 rows x 16 bf16]
+__device__ __forceinline__ void warp_store_any16(uint8_t *sbuf, const uint4 &v0, const uint4 &v1, uint8_t *g_row0, int64_t pitch_bytes, int rows_valid,
+                                                 int cols, int lane) {
+  warp_stage_rows32(sbuf, v0, v1, lane);
+  const int w = lane & 7;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int R = 4 * j + (lane >> 3);
+    uint8_t *g = g_row0 + (int64_t)R * pitch_bytes;
+    // the row's elements as words of the destination: elements (2w, 2w + 1), or, where the row starts in the middle of a word,
+    // (2w + 1, 2w + 2); the last lane of such a row takes elements 0 and 15
+    const bool odd = (reinterpret_cast<uintptr_t>(g) & 2) != 0;
+    const int e0 = odd ? 2 * w + 1 : 2 * w, e1 = (odd && w == 7) ? 0 : e0 + 1;
+    const uint32_t lo = *reinterpret_cast<const uint16_t *>(warp_staged_byte(sbuf, R, e0 * 2));
+    const uint32_t hi = *reinterpret_cast<const uint16_t *>(warp_staged_byte(sbuf, R, e1 * 2));
+    if (R < rows_valid) {
+      if (e1 == e0 + 1 && e1 < cols) *reinterpret_cast<uint32_t *>(g + e0 * 2) = lo | (hi << 16);
+      else {
+        if (e0 < cols) *reinterpret_cast<uint16_t *>(g + e0 * 2) = (uint16_t)lo;
+        if (e1 < cols) *reinterpret_cast<uint16_t *>(g + e1 * 2) = (uint16_t)hi;
+      }
+    }
+  }
+  __syncwarp();
+}
+
 // The same [32 rows x 32 bytes] block as one TMA store: the lanes write their rows to the staging block (plain row-major),
 // one lane hands it to the copy engine and waits until the engine has read it.  Keeps the result off the load/store path.
 __device__ __forceinline__ void warp_tma_store_rows32(uint8_t *sbuf, const uint4 &v0, const uint4 &v1, const CUtensorMap *map,
@@ -350,7 +402,7 @@ struct EpiStore {          // where this warp's rows of the current tile go
   int row_c;               // row coordinate of the warp's first row in map_c
 };
 
-// One 32-column chunk of one output row.  Results leave, in this order of preference, as 32-byte stores of the lane's own
+// Sixteen columns of one output row.  Results leave, in this order of preference, as 32-byte stores of the lane's own
 // row (destination 32-byte aligned), through the warp's staging block (16-byte aligned), or element by element.
 // accumulator -> f32 before bias: the dequantising chain of the INT8 forms, or the f32 sum of the bf16 form as it is
 template <bool F16>
@@ -359,50 +411,55 @@ __device__ __forceinline__ float tc_acc_f32(uint32_t r, int comp, float s_src, f
   else return __fmul_rn(__fmul_rn((float)((int32_t)r - comp), s_src), w);
 }
 
-template <int ACT, bool F16>
-__device__ __forceinline__ void tc_epi_chunk(const EpiParams &epi, const EpiCtx &cx, const uint32_t (&r)[32], const TileCols &tc,
-                                             int c0, int pc0, int N, int m_dst, bool has_bias, const EpiStore &es, int lane) {
+template <int ACT>
+__device__ __forceinline__ void tc_act16(const EpiParams &epi, float (&x)[16], int m, int n) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) x[i] = tc_act<ACT>(epi, x[i], m, n + i);
+}
+
+// (Only the activation depends on fast_act: the loads before it and the stores behind it exist once.  With the whole chunk
+// instantiated per activation the split form spilled hundreds of registers.)
+template <bool F16>
+__device__ __forceinline__ void tc_epi_half(int fast_act, const EpiParams &epi, const EpiCtx &cx, const uint32_t (&r)[16], const TileCols &tc,
+                                            int c0, int pc, int N, int m_dst, bool has_bias, const EpiStore &es, int lane) {
   const bool has_zp = !F16 && epi.has_zp != 0;
+  const bool full = pc + 16 <= N;
   if (!F16 && epi.dst_dt == DT_S32) {
-    int32_t y[32];
+    int32_t y[16];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) y[i] = has_zp ? (int32_t)r[i] - tc.comp[c0 + i] : (int32_t)r[i];
-    if (es.v8 && pc0 + 32 <= N) {
+    for (int i = 0; i < 16; ++i) y[i] = has_zp ? (int32_t)r[i] - tc.comp[c0 + i] : (int32_t)r[i];
+    if (es.v8 && full) {
       if (es.row_ok) {
-        uint8_t *o = reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc0) * 4;
+        uint8_t *o = reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4;
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
+        for (int p = 0; p < 2; ++p) {
           uint32_t v[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) v[i] = (uint32_t)y[8 * p + i];
           st_global_v8(o + 32 * p, v);
         }
       }
-    } else if (es.coalesce && pc0 + 32 <= N) {
+    } else if (es.coalesce && full) {
+      uint4 v[4];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint4 v[4];
+      for (int p = 0; p < 4; ++p) v[p] = make_uint4(y[4 * p], y[4 * p + 1], y[4 * p + 2], y[4 * p + 3]);
+      warp_store_rows64(es.sbuf, v, es.g_row0 + (size_t)pc * 4, es.pitch_bytes, es.rows_valid, lane);
+    } else {
 #pragma unroll
-        for (int p = 0; p < 4; ++p) v[p] = make_uint4(y[16 * h + 4 * p], y[16 * h + 4 * p + 1], y[16 * h + 4 * p + 2], y[16 * h + 4 * p + 3]);
-        warp_store_rows64(es.sbuf, v, es.g_row0 + (size_t)(pc0 + 16 * h) * 4, es.pitch_bytes, es.rows_valid, lane);
-      }
-    } else if (es.row_ok) {
-      int32_t *o = reinterpret_cast<int32_t *>(cx.dst) + (int64_t)m_dst * cx.ldc + pc0;
-#pragma unroll
-      for (int i = 0; i < 32; ++i)
-        if (pc0 + i < N) o[i] = y[i];
+      for (int p = 0; p < 2; ++p)
+        if (pc + 8 * p < N)
+          warp_store_any32(es.sbuf, make_uint4(y[8 * p], y[8 * p + 1], y[8 * p + 2], y[8 * p + 3]), make_uint4(y[8 * p + 4], y[8 * p + 5], y[8 * p + 6], y[8 * p + 7]),
+                           es.g_row0 + (size_t)(pc + 8 * p) * 4, es.pitch_bytes, es.rows_valid, N - (pc + 8 * p), lane);
     }
     return;
   }
-  // two halves of 16 columns: fewer values live at once
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  {
     float x[16];
 #pragma unroll
     for (int i = 0; i < 16; i += 4) {
       // shared memory is the busiest resource of this kernel (the tensor core reads its operands from it):
       // bias and compensation are fetched only when they exist
-      const int ci = c0 + 16 * h + i;
+      const int ci = c0 + i;
       float4 w4 = make_float4(1.f, 1.f, 1.f, 1.f);
       if constexpr (!F16) w4 = *reinterpret_cast<const float4 *>(&tc.ws[ci]);
       float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -413,13 +470,21 @@ __device__ __forceinline__ void tc_epi_chunk(const EpiParams &epi, const EpiCtx 
       const int kv[4] = {k4.x, k4.y, k4.z, k4.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        float v = tc_acc_f32<F16>(r[16 * h + i + j], kv[j], cx.s_src, wv[j]);
+        float v = tc_acc_f32<F16>(r[i + j], kv[j], cx.s_src, wv[j]);
         if (has_bias) v = __fadd_rn(v, bv[j]);
-        x[i + j] = tc_act<ACT>(epi, v, m_dst, pc0 + 16 * h + i + j);
+        x[i + j] = v;
       }
     }
-    const int pc = pc0 + 16 * h;          // first column of this half
-    const bool full = pc + 16 <= N;
+    switch (fast_act) {
+    case FA_NONE: break;
+    case FA_RELU: tc_act16<FA_RELU>(epi, x, m_dst, pc); break;
+    case FA_GELU_TANH: tc_act16<FA_GELU_TANH>(epi, x, m_dst, pc); break;
+    case FA_GELU_ERF: tc_act16<FA_GELU_ERF>(epi, x, m_dst, pc); break;
+    case FA_SIGMOID: tc_act16<FA_SIGMOID>(epi, x, m_dst, pc); break;
+    case FA_SWISH: tc_act16<FA_SWISH>(epi, x, m_dst, pc); break;
+    case FA_TANH: tc_act16<FA_TANH>(epi, x, m_dst, pc); break;
+    default: tc_act16<FA_GENERIC>(epi, x, m_dst, pc); break;
+    }
     if (epi.dst_dt == DT_BF16) {
       uint32_t pk[8];
 #pragma unroll
@@ -431,11 +496,9 @@ __device__ __forceinline__ void tc_epi_chunk(const EpiParams &epi, const EpiCtx 
       } else if (es.coalesce && full) {
         warp_store_rows32(es.sbuf, make_uint4(pk[0], pk[1], pk[2], pk[3]), make_uint4(pk[4], pk[5], pk[6], pk[7]),
                           es.g_row0 + (size_t)pc * 2, es.pitch_bytes, es.rows_valid, lane);
-      } else if (es.row_ok) {
-        uint16_t *o = reinterpret_cast<uint16_t *>(cx.dst) + (int64_t)m_dst * cx.ldc + pc;
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (pc + i < N) o[i] = (uint16_t)(pk[i >> 1] >> ((i & 1) * 16));
+      } else if (pc < N) {
+        warp_store_any16(es.sbuf, make_uint4(pk[0], pk[1], pk[2], pk[3]), make_uint4(pk[4], pk[5], pk[6], pk[7]), es.g_row0 + (size_t)pc * 2, es.pitch_bytes,
+                         es.rows_valid, N - pc, lane);
       }
     } else {
       if (es.v8 && full) {
@@ -455,29 +518,15 @@ __device__ __forceinline__ void tc_epi_chunk(const EpiParams &epi, const EpiCtx 
         for (int p = 0; p < 4; ++p)
           v[p] = make_uint4(__float_as_uint(x[4 * p]), __float_as_uint(x[4 * p + 1]), __float_as_uint(x[4 * p + 2]), __float_as_uint(x[4 * p + 3]));
         warp_store_rows64(es.sbuf, v, es.g_row0 + (size_t)pc * 4, es.pitch_bytes, es.rows_valid, lane);
-      } else if (es.row_ok) {
-        float *o = reinterpret_cast<float *>(cx.dst) + (int64_t)m_dst * cx.ldc + pc;
+      } else {
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (pc + i < N) o[i] = x[i];
+        for (int p = 0; p < 2; ++p)
+          if (pc + 8 * p < N)
+            warp_store_any32(es.sbuf, make_uint4(__float_as_uint(x[8 * p]), __float_as_uint(x[8 * p + 1]), __float_as_uint(x[8 * p + 2]), __float_as_uint(x[8 * p + 3])),
+                             make_uint4(__float_as_uint(x[8 * p + 4]), __float_as_uint(x[8 * p + 5]), __float_as_uint(x[8 * p + 6]), __float_as_uint(x[8 * p + 7])),
+                             es.g_row0 + (size_t)(pc + 8 * p) * 4, es.pitch_bytes, es.rows_valid, N - (pc + 8 * p), lane);
       }
     }
-  }
-}
-
-template <bool F16>
-__device__ __forceinline__ void tc_epi_dispatch(int fast_act, const EpiParams &epi, const EpiCtx &cx, const uint32_t (&r)[32],
-                                                const TileCols &tcols, int c0, int pc0, int N, int m_dst, bool has_bias,
-                                                const EpiStore &es, int lane) {
-  switch (fast_act) {
-  case FA_NONE: tc_epi_chunk<FA_NONE, F16>(epi, cx, r, tcols, c0, pc0, N, m_dst, has_bias, es, lane); break;
-  case FA_RELU: tc_epi_chunk<FA_RELU, F16>(epi, cx, r, tcols, c0, pc0, N, m_dst, has_bias, es, lane); break;
-  case FA_GELU_TANH: tc_epi_chunk<FA_GELU_TANH, F16>(epi, cx, r, tcols, c0, pc0, N, m_dst, has_bias, es, lane); break;
-  case FA_GELU_ERF: tc_epi_chunk<FA_GELU_ERF, F16>(epi, cx, r, tcols, c0, pc0, N, m_dst, has_bias, es, lane); break;
-  case FA_SIGMOID: tc_epi_chunk<FA_SIGMOID, F16>(epi, cx, r, tcols, c0, pc0, N, m_dst, has_bias, es, lane); break;
-  case FA_SWISH: tc_epi_chunk<FA_SWISH, F16>(epi, cx, r, tcols, c0, pc0, N, m_dst, has_bias, es, lane); break;
-  case FA_TANH: tc_epi_chunk<FA_TANH, F16>(epi, cx, r, tcols, c0, pc0, N, m_dst, has_bias, es, lane); break;
-  default: tc_epi_chunk<FA_GENERIC, F16>(epi, cx, r, tcols, c0, pc0, N, m_dst, has_bias, es, lane); break;
   }
 }
 
@@ -501,7 +550,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   // programmatic dependent launch: the next kernel of the stream may take this CTA's SM as soon as it is free; this
   // kernel touches global memory only after griddepcontrol.wait below (the set-up before it uses none)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (the same in every lane, and known to be)
   if (threadIdx.x == 0) TC_STAMP(0);
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   static_assert(!(SPLIT && PAIR), "the split form and the pair form are separate kernels");
@@ -595,34 +644,43 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && (!PAIR || crank == 0)) {      // pair form: the leader issues for both CTAs
+    // The whole warp walks the tiles and one elected lane issues, so that operands and control flow are warp-uniform: inside a
+    // single-lane branch every MMA first moves its descriptors to uniform registers (about 100 clocks an MMA, longer than the MMA itself
+    // for tiles up to 128 columns; the pair form gained too: 127 -> 113 us at M = 2048, K = 4096, N = 14336 with the epilogue below).
+    if (!PAIR || crank == 0) {      // pair form: the leader issues for both CTAs
       const uint32_t idesc = F16 ? make_idesc_bf16(a.BN, tile_m) : make_idesc_i8(a.a_unsigned, a.BN, tile_m);
       int stage = 0; uint32_t phase = 0; int acc = 0; uint32_t acc_phase = 0;
-      for (int tile = tile0; tile < total_tiles && !s_err; tile += tile_step) {
-        if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u)) { s_err = 2; report_status(a.status, 2); break; }
+      auto wait = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0; };
+      auto commit = [&](uint32_t bar) { if constexpr (PAIR) tc_commit_pair(bar); else tc_commit(bar); };
+      for (int tile = tile0; tile < total_tiles && __shfl_sync(0xffffffffu, s_err ? 0 : 1, 0); tile += tile_step) {
+        if (!wait(tempty_bar(acc), acc_phase ^ 1u)) { if (lane == 0) { s_err = 2; report_status(a.status, 2); } break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * a.BN);
+        // (the lanes compare notes once per tile, not per K block: after an expired wait the remaining blocks are issued on what the
+        // stages hold, and the tile is not published)
         bool ok = true;
         for (int kb = kb_begin; kb < kb_end; ++kb) {
-          if (!mbar_wait(full_bar(stage), phase)) { ok = false; break; }
-          if (kb == kb_begin && tile == tile0) TC_STAMP(2);
+          if (ok) ok = mbar_wait(full_bar(stage), phase);
+          if (lane == 0 && kb == kb_begin && tile == tile0) TC_STAMP(2);
           tc_fence_after();
           const uint32_t sa = smem0 + (uint32_t)stage * stage_bytes;
           const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + a_bytes);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < kTcBK / 32; ++k) {
-            const uint32_t accum = ((kb - kb_begin) | k) ? 1u : 0u;
-            if constexpr (PAIR && F16) tc_mma_bf16_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
-            else if constexpr (PAIR) tc_mma_i8_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
-            else if constexpr (F16) tc_mma_bf16(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
-            else tc_mma_i8(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
+            for (int k = 0; k < kTcBK / 32; ++k) {
+              const uint32_t accum = ((kb - kb_begin) | k) ? 1u : 0u;
+              if constexpr (PAIR && F16) tc_mma_bf16_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
+              else if constexpr (PAIR) tc_mma_i8_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
+              else if constexpr (F16) tc_mma_bf16(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
+              else tc_mma_i8(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
+            }
+            commit(empty_bar(stage));
           }
-          if constexpr (PAIR) tc_commit_pair(empty_bar(stage)); else tc_commit(empty_bar(stage));
           if (++stage == S) { stage = 0; phase ^= 1u; }
         }
-        if (!ok) { s_err = 3; report_status(a.status, 3); break; }
-        if constexpr (PAIR) tc_commit_pair(tfull_bar(acc)); else tc_commit(tfull_bar(acc));
-        if (tile == tile0) TC_STAMP(3);
+        if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) { s_err = 3; report_status(a.status, 3); } break; }
+        if (elect_one()) commit(tfull_bar(acc));
+        if (lane == 0 && tile == tile0) TC_STAMP(3);
         if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
     }
@@ -743,17 +801,19 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int per = (a.BN / 32 + kTcEpiParts - 1) / kTcEpiParts;
         const int c_begin = part * per, c_end = min(nc, c_begin + per);
         for (int c = c_begin; c < c_end; ++c) {
-          uint32_t r[32];
-          tc_ld32(taddr0 + (uint32_t)(c * 32), r);
-          tc_wait_ld();
-          const int pc0 = pc_tile + c * 32;
+#pragma unroll 1
+          for (int h = 0; h < 2; ++h) {             // sixteen columns at a time: fewer values live at once
+            uint32_t r[16];
+            tc_ld16(taddr0 + (uint32_t)(c * 32 + 16 * h), r);
+            tc_wait_ld();
 #ifdef B200DNN_TIMING_EXPERIMENTS
-          if (a.dbg == 2) { uint32_t x = 0;
+            if (a.dbg == 2) { uint32_t x = 0;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) x ^= r[i];
-            if (x == 0x12345678u) report_status(a.status, 99); continue; }
+              for (int i = 0; i < 16; ++i) x ^= r[i];
+              if (x == 0x12345678u) report_status(a.status, 99); continue; }
 #endif
-          tc_epi_dispatch<F16>(a.fast_act, epi, cx, r, tcols, c * 32, pc0, a.N, m_dst, has_bias, es, lane);
+            tc_epi_half<F16>(a.fast_act, epi, cx, r, tcols, c * 32 + 16 * h, pc_tile + c * 32 + 16 * h, a.N, m_dst, has_bias, es, lane);
+          }
         }
       } else {
         // gated: packed columns [g(32) u(32)] -> 32 outputs; dst is [rows, I] bf16.  Sixteen outputs at a time: their
@@ -895,14 +955,17 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       cluster_arrive_all();   // this warp reads no neighbour any more
       arrived = true;
       for (int c = (int)crank + a.k_splits * part; c < nc; c += a.k_splits * kTcEpiParts) {
-        uint32_t r[32];
         const uint32_t base = smem0 + (uint32_t)((c * kTcBM + row_in_tile) * 128);
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          uint32_t r[16];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const uint4 v = ld_shared_v4(base + (uint32_t)((u ^ (row_in_tile & 7)) << 4));
-          r[4 * u] = v.x; r[4 * u + 1] = v.y; r[4 * u + 2] = v.z; r[4 * u + 3] = v.w;
+          for (int u = 0; u < 4; ++u) {
+            const uint4 v = ld_shared_v4(base + (uint32_t)(((u + 4 * h) ^ (row_in_tile & 7)) << 4));
+            r[4 * u] = v.x; r[4 * u + 1] = v.y; r[4 * u + 2] = v.z; r[4 * u + 3] = v.w;
+          }
+          tc_epi_half<F16>(a.fast_act, epi, cx, r, tcols, c * 32 + 16 * h, pc_tile + c * 32 + 16 * h, a.N, m_dst, has_bias, es, lane);
         }
-        tc_epi_dispatch<F16>(a.fast_act, epi, cx, r, tcols, c * 32, pc_tile + c * 32, a.N, m_dst, has_bias, es, lane);
       }
     }
     // nobody leaves while a neighbour may still read its shared memory: arrive as soon as the own reads are done,
