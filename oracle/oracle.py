@@ -32,7 +32,8 @@ def build(force=False):
     ref_root = os.environ.get("ZENDNN_REFERENCE_ROOT", "/root/reference")
     ref = os.path.join(_HERE, "_ref", "libzendnn_ref.so")
     ref2 = os.path.join(_HERE, "_ref", "libzendnn_ref2.so")
-    if os.path.isdir(ref_root) and (force or not os.path.exists(ref) or not os.path.exists(ref2)):
+    # a mount point without a checkout in it counts as none
+    if os.path.isdir(os.path.join(ref_root, "zendnnl", "src")) and (force or not os.path.exists(ref) or not os.path.exists(ref2)):
         subprocess.check_call(["make", "-C", _HERE, "-s", "ref", "REF=" + ref_root])
 
 
