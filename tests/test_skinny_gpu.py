@@ -1,0 +1,60 @@
+"""The few-row tcgen05 kernel (weight as the MMA's 128 rows, shares of K added over a cluster) at the edges of its range: row
+counts beside multiples of 16, column tiles with a remainder, K with a remainder and with too few blocks to share, every result type."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def capi():
+    from zendnn_b200 import capi as c
+    assert c.lib.b200dnn_device_count() > 0, "no CUDA device"
+    return c
+
+
+@pytest.mark.parametrize("M,K,N", [(17, 128, 128), (17, 1100, 130), (33, 4096, 1000), (48, 2064, 513), (16, 8192, 3080), (31, 544, 4097)])
+@pytest.mark.parametrize("out", ["s32", "f32", "bf16"])
+def test_skinny_int8(capi, oracle, M, K, N, out):
+    rng = np.random.default_rng(M * 7 + N)
+    K16 = K + (-K) % 16                                     # rows at a pitch the copy engine takes
+    A = np.zeros((M, K16), dtype=np.uint8)
+    A[:, :K] = rng.integers(0, 256, (M, K))
+    W = rng.integers(-128, 128, (K, N), dtype=np.int8)
+    zp = np.array([131], dtype=np.int32)
+    acc = (A[:, :K].astype(np.int64) - 131) @ W.astype(np.int64)
+    kw = dict(lda=K16, src_dt=capi.DT["u8"], dst_dt=capi.DT[out], src_zp=zp, weights_const=False)
+    if out == "s32":
+        dst = np.zeros((M, N), dtype=np.int32)
+        capi.check(capi.matmul(capi.make_matmul(M, N, K, A, W, dst, **kw)))
+        assert (dst == acc).all()
+        return
+    ss, sw, bias = np.array([0.013], dtype=np.float32), rng.uniform(0.001, 0.01, N).astype(np.float32), rng.standard_normal(N).astype(np.float32)
+    dst = np.zeros((M, N), dtype=np.float32 if out == "f32" else np.uint16)
+    capi.check(capi.matmul(capi.make_matmul(M, N, K, A, W, dst, src_scale=ss, wei_scale=sw, bias=bias, postops=["relu"], **kw)))
+    ref = np.maximum((acc.astype(np.float32) * ss) * sw + bias, np.float32(0))      # one rounding per operation, as in the kernel
+    if out == "f32":
+        assert (dst == ref).all()
+    else:
+        assert (dst == oracle.f32_to_bf16(ref)).all()
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 64, 16), (1, 4096, 1000), (15, 1096, 257), (16, 8192, 384), (49, 2048, 1030), (64, 520, 4100)])
+@pytest.mark.parametrize("out", ["f32", "bf16"])
+def test_skinny_bf16(capi, oracle, M, K, N, out):
+    rng = np.random.default_rng(M * 5 + K)
+    A, W = (oracle.f32_to_bf16(rng.standard_normal(s).astype(np.float32)) for s in ((M, K), (K, N)))
+    bias = rng.standard_normal(N).astype(np.float32)
+    dst = np.zeros((M, N), dtype=np.float32 if out == "f32" else np.uint16)
+    d = capi.make_matmul(M, N, K, A, W, dst, src_dt=capi.DT["bf16"], wei_dt=capi.DT["bf16"], dst_dt=capi.DT[out], bias=bias, weights_const=True)
+    a, w = ((x.astype(np.uint32) << 16).view(np.float32).astype(np.float64) for x in (A, W))
+    ref = a @ w + bias
+    # f32 sums of K exact products: each of the K additions rounds by at most 2^-24 of a partial sum (2^-23 where the tensor core cuts
+    # instead), and a partial sum is at most sum |a||w|; bf16 rounds the result by 2^-9 of itself on top
+    tol = K * 2.0 ** -23 * (np.abs(a) @ np.abs(w) + np.abs(bias))
+    for _ in range(2):                                      # the second call finds the packed weight and reads it early
+        dst[:] = 0
+        capi.check(capi.matmul(d))
+        got = dst.astype(np.float64) if out == "f32" else (dst.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+        assert (np.abs(got - ref) <= tol + (0 if out == "f32" else 2.0 ** -8 * np.abs(ref))).all()
+    capi.lib.b200dnn_clear_caches()

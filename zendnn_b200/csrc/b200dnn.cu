@@ -15,6 +15,7 @@
 #include "decode_gemm.cuh"
 #include "decode_ring.cuh"
 #include "tc_gemm.cuh"
+#include "skinny_gemm.cuh"
 #include "moe_kernels.cuh"
 #include "sdpa_flash_api.cuh"
 
@@ -112,7 +113,8 @@ int32_t resolve_weight(const void *weight, int wei_format, int64_t K, int64_t N,
       *pw = it->second;
     } else {
       auto it = D.host_packed.find(weight);
-      if (it == D.host_packed.end()) {
+      const bool uploaded = it == D.host_packed.end();
+      if (uploaded) {
         PackHeader h; memcpy(&h, weight, sizeof h);
         B2_CHECK(h.magic == kPackMagic, B200DNN_FAILURE, "mem_format_b='r' but the weight buffer was not written by b200dnn_prepack");
         size_t bytes = pack_bytes(h.K, h.N);
@@ -125,6 +127,7 @@ int32_t resolve_weight(const void *weight, int wei_format, int64_t K, int64_t N,
       }
       B2_TRY(wait_ready(it->second, st));
       *pw = it->second;
+      pw->fresh = uploaded;
     }
     B2_CHECK(pw->K == K && pw->N == N && pw->gated == gated, B200DNN_FAILURE,
              "prepacked weight is K=%lld N=%lld gated=%d, call asks for K=%lld N=%lld gated=%d", (long long)pw->K,
@@ -148,6 +151,21 @@ int32_t resolve_weight(const void *weight, int wei_format, int64_t K, int64_t N,
   else { buf = rt().ws.alloc(pack_bytes(K, N)); B2_CHECK(buf, B200DNN_FAILURE, "workspace allocation failed"); }
   B2_TRY(pack_into(w_dev, K, N, ldb, transB, gated, buf, st, pw));
   if (cache) { pw->owned = buf; B2_TRY(mark_ready(*pw, st)); D.wcache.emplace(key, *pw); }
+  pw->fresh = true;
+  return B200DNN_SUCCESS;
+}
+
+// A launch that may overlap the end of the kernel in front of it on the stream (which must have triggered its dependents): only for
+// kernels that touch memory behind griddepcontrol.wait alone.
+template <typename... P, typename... V>
+int32_t launch_pdl(void (*kern)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, bool pdl, V... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = pdl && env_int("B200DNN_PDL", 1) != 0 ? 1 : 0;
+  B2_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
   return B200DNN_SUCCESS;
 }
 
@@ -174,8 +192,8 @@ int32_t launch_quant_rows_t(const RowQuantArgs &a, int32_t src_dt, int64_t rows,
     long long want = (rows * segs + 7) / 8;
     const unsigned grid = (unsigned)(want < rt().sm_count * 5 ? want : rt().sm_count * 5);
     // (eight loads in flight per lane measured slower: 110 against 92 us at configuration 4)
-    if (src_dt == B200DNN_BF16) quant_known_absmax_kernel<uint16_t, 4><<<grid, 256, 0, st>>>(a, (int)rows, segs, seg_len);
-    else quant_known_absmax_kernel<float, 4><<<grid, 256, 0, st>>>(a, (int)rows, segs, seg_len);
+    if (src_dt == B200DNN_BF16) B2_TRY(launch_pdl(quant_known_absmax_kernel<uint16_t, 4>, grid, 256, 0, st, !EP, a, (int)rows, segs, seg_len));
+    else B2_TRY(launch_pdl(quant_known_absmax_kernel<float, 4>, grid, 256, 0, st, !EP, a, (int)rows, segs, seg_len));
     B2_LAUNCHED();
     B2_CUDA(cudaGetLastError());
     return B200DNN_SUCCESS;
@@ -184,7 +202,7 @@ int32_t launch_quant_rows_t(const RowQuantArgs &a, int32_t src_dt, int64_t rows,
     const int nv = (a.K / E + 31) / 32;
     unsigned grid = (unsigned)((rows + 7) / 8);
     if (EP && a.n_rows_dev && grid > (unsigned)(rt().sm_count * 16)) grid = (unsigned)(rt().sm_count * 16);   // the warps stride over the rows
-#define B2_QW(T, NV) quant_per_token_warp_kernel<T, NV, EP><<<grid, 256, 0, st>>>(a, (int)rows)
+#define B2_QW(T, NV) B2_TRY((launch_pdl(quant_per_token_warp_kernel<T, NV, EP>, grid, 256, 0, st, !EP, a, (int)rows)))
     if (src_dt == B200DNN_BF16) { if (nv <= 2) B2_QW(uint16_t, 2); else if (nv <= 4) B2_QW(uint16_t, 4); else if (nv <= 8) B2_QW(uint16_t, 8); else B2_QW(uint16_t, 16); }
     else { if (nv <= 2) B2_QW(float, 2); else if (nv <= 4) B2_QW(float, 4); else if (nv <= 8) B2_QW(float, 8); else B2_QW(float, 16); }
 #undef B2_QW
@@ -192,16 +210,17 @@ int32_t launch_quant_rows_t(const RowQuantArgs &a, int32_t src_dt, int64_t rows,
     B2_CUDA(cudaGetLastError());
     return B200DNN_SUCCESS;
   }
-  const bool short_row = a.K / E <= 2 * kQuantThreads;     // the whole row fits two cached vectors per thread
+  const int nvec = a.K / E;
+  const bool short_row = nvec <= 2 * kQuantThreads;     // the whole row fits two cached vectors per thread
+  // few long rows (fewer than SMs): as many threads as keep a row in two vectors each, see quant_per_token_kernel
+  const bool wide = !short_row && rows <= rt().sm_count;
   unsigned grid_rows = (unsigned)rows;
   if (EP && a.n_rows_dev && grid_rows > (unsigned)(rt().sm_count * 32)) grid_rows = (unsigned)(rt().sm_count * 32);   // the CTAs stride over the rows
-  if (src_dt == B200DNN_BF16) {
-    if (short_row) quant_per_token_kernel<uint16_t, 2, EP><<<grid_rows, kQuantThreads, 0, st>>>(a);
-    else quant_per_token_kernel<uint16_t, kQuantRegVec, EP><<<grid_rows, kQuantThreads, 0, st>>>(a);
-  } else if (src_dt == B200DNN_F32) {
-    if (short_row) quant_per_token_kernel<float, 2, EP><<<grid_rows, kQuantThreads, 0, st>>>(a);
-    else quant_per_token_kernel<float, kQuantRegVec, EP><<<grid_rows, kQuantThreads, 0, st>>>(a);
-  } else return fail(B200DNN_UNIMPLEMENTED, "per-token quantisation takes f32 or bf16 input");
+#define B2_QR(T, NV, THR) B2_TRY((launch_pdl(quant_per_token_kernel<T, NV, EP, THR>, grid_rows, THR, 0, st, !EP, a)))
+  if (src_dt == B200DNN_BF16) { if (short_row) B2_QR(uint16_t, 2, kQuantThreads); else if (wide) B2_QR(uint16_t, 2, 1024); else B2_QR(uint16_t, kQuantRegVec, kQuantThreads); }
+  else if (src_dt == B200DNN_F32) { if (short_row) B2_QR(float, 2, kQuantThreads); else if (wide) B2_QR(float, 2, 1024); else B2_QR(float, kQuantRegVec, kQuantThreads); }
+  else return fail(B200DNN_UNIMPLEMENTED, "per-token quantisation takes f32 or bf16 input");
+#undef B2_QR
   B2_LAUNCHED();
   B2_CUDA(cudaGetLastError());
   return B200DNN_SUCCESS;
@@ -450,6 +469,21 @@ int tc_tile_rows(long long rows, int N) {
   return tiles >= 2LL * (rt().sm_count / 2) ? 2 * kTcBM : kTcBM;
 }
 
+// The epilogue's FA_* code of a post-op chain.
+int fast_act_code(const EpiParams &epi) {
+  if (epi.n_po == 0) return FA_NONE;
+  if (epi.n_po != 1) return FA_GENERIC;
+  switch (epi.po[0].type) {
+  case PO_RELU: return FA_RELU;
+  case PO_GELU_TANH: return FA_GELU_TANH;
+  case PO_GELU_ERF: return FA_GELU_ERF;
+  case PO_SIGMOID: return FA_SIGMOID;
+  case PO_SWISH: return FA_SWISH;
+  case PO_TANH: return FA_TANH;
+  default: return FA_GENERIC;
+  }
+}
+
 // Plain or grouped tcgen05 GEMM.  A: [M_total, lda] device, 16-byte aligned rows.  bf16 form (args.f16): K and lda count
 // bytes (two per element) and pw0 holds a bf16 pack.
 int32_t launch_tc(const uint8_t *A, int64_t lda, bool a_unsigned, int M_total, int N, int K, const PackedWeight &pw0,
@@ -459,19 +493,7 @@ int32_t launch_tc(const uint8_t *A, int64_t lda, bool a_unsigned, int M_total, i
   B2_TRY(make_map_2d(&map_a, A, (uint64_t)K, (uint64_t)M_total, (uint64_t)lda, kTcBM));
   args.M_total = M_total; args.N = N; args.k_blocks = (int)(pw0.Kp / 128);
   args.a_unsigned = a_unsigned ? 1 : 0; args.gated = pw0.gated; args.status = R.status;
-  args.fast_act = FA_GENERIC;
-  if (epi.n_po == 0) args.fast_act = FA_NONE;
-  else if (epi.n_po == 1) {
-    switch (epi.po[0].type) {
-    case PO_RELU: args.fast_act = FA_RELU; break;
-    case PO_GELU_TANH: args.fast_act = FA_GELU_TANH; break;
-    case PO_GELU_ERF: args.fast_act = FA_GELU_ERF; break;
-    case PO_SIGMOID: args.fast_act = FA_SIGMOID; break;
-    case PO_SWISH: args.fast_act = FA_SWISH; break;
-    case PO_TANH: args.fast_act = FA_TANH; break;
-    default: break;
-    }
-  }
+  args.fast_act = fast_act_code(epi);
   args.test_no_loads = env_int("B200DNN_TEST_NO_LOADS", 0);   // see tc_gemm.cuh; off unless a test sets it
   args.stamps = nullptr;
 #ifdef B200DNN_TIMING_EXPERIMENTS
@@ -586,6 +608,88 @@ int32_t launch_tc(const uint8_t *A, int64_t lda, bool a_unsigned, int M_total, i
   }
   B2_LAUNCHED();
   B2_CUDA(cudaGetLastError());
+  return B200DNN_SUCCESS;
+}
+
+// CTAs of skinny_gemm_kernel that are resident at once when it is launched in clusters of s
+int skinny_room(int s) {
+  if (s == 1) return rt().sm_count;
+  int *cache = rt().shared->skinny_room;   // per device; two threads may both compute the same value
+  if (cache[s] == 0) {
+    cache[s] = -1;
+    if (ensure_max_smem((const void *)skinny_gemm_kernel<false>, kSkinnyRing + 1024) == B200DNN_SUCCESS) {
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3((unsigned)(s * 64)); cfg.blockDim = dim3(kSkinnyThreads); cfg.dynamicSmemBytes = kSkinnyRing + 1024;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)s; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr; cfg.numAttrs = 1;
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, skinny_gemm_kernel<false>, &cfg) == cudaSuccess && n > 0) cache[s] = n * s;
+      else cudaGetLastError();
+      if (env_int("B200DNN_DEBUG", 0)) fprintf(stderr, "b200dnn: skinny clusters of %d: %d resident CTAs\n", s, cache[s]);
+    }
+  }
+  return cache[s];
+}
+
+// Few rows (skinny_gemm.cuh).  A: [M, lda] device bytes, 16-byte aligned rows; K and lda count bytes; early: see SkinnyArgs.
+int32_t launch_skinny(const uint8_t *A, int64_t lda, bool a_unsigned, bool f16, int M, int N, int K, const PackedWeight &pw, const EpiParams &epi,
+                      int fast_act, bool early, cudaStream_t st) {
+  Runtime &R = rt();
+  SkinnyArgs g{};
+  g.M = M; g.N = N; g.k_blocks = (int)(pw.Kp / 128); g.MP = (M + 15) & ~15;
+  g.a_unsigned = a_unsigned ? 1 : 0; g.fast_act = fast_act; g.early = early ? 1 : 0; g.status = R.status;
+  g.test_no_loads = env_int("B200DNN_TEST_NO_LOADS", 0);
+  B2_CHECK(M >= 1 && g.MP <= kSkinnyMaxM, B200DNN_FAILURE, "skinny form: %d rows", M);
+  // Shares of K: the fewest microseconds by a model of the stream (6.5 TB/s over the device, at most 100 GB/s an SM) plus the additions through distributed shared memory, among the choices that are resident at once.
+  const int tiles = (N + 127) / 128;
+  int best = 1;
+  double best_us = 1e30;
+  const int forced = env_int("B200DNN_SKINNY_SPLIT", 0);
+  for (int s = 1; s <= kSkinnyMaxSplits; ++s) {
+    if (s > 1 && (g.k_blocks < 4 * s || (long long)tiles * s > skinny_room(s))) continue;
+    if (forced > 0 && s != forced) continue;
+    const long long ctas = (long long)tiles * s, room = R.sm_count;
+    const long long live = ctas < room ? ctas : room;
+    const double rate = std::min(6.5e6 / (double)live, 1.0e5);           // bytes per microsecond and CTA
+    const double us = (double)((g.k_blocks + s - 1) / s) * (128 * 128 + g.MP * 128) / rate * (double)((ctas + room - 1) / room) + 0.15 * s;
+    if (us < best_us) { best_us = us; best = s; }
+  }
+  g.splits = best;
+  const int stage_bytes = 128 * 128 + g.MP * 128;
+  int stages = kSkinnyRing / stage_bytes;
+  const int per = (g.k_blocks + best - 1) / best;
+  if (stages > kSkinnyMaxStages) stages = kSkinnyMaxStages;
+  if (stages > per) stages = per;
+  g.stages = stages;
+  size_t smem = (size_t)stages * stage_bytes;
+  if (smem < (size_t)g.MP * 512) smem = (size_t)g.MP * 512;      // the partial sums lie over the ring
+  smem += 1024;
+  CUtensorMap map_a, map_w;
+  B2_TRY(make_map_2d(&map_a, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, (uint32_t)g.MP));
+  B2_TRY(make_map_wt(&map_w, pw.wt, (uint64_t)pw.Kp, (uint64_t)pw.Np, 128));
+  auto kern = f16 ? skinny_gemm_kernel<true> : skinny_gemm_kernel<false>;
+  B2_TRY(ensure_max_smem((const void *)kern, kSkinnyRing + 1024));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(tiles * best)); cfg.blockDim = dim3(kSkinnyThreads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  // (a weight packed in this very call: a plain launch, so that the early reads of a LATER call, which follow this kernel's start, follow
+  // the end of the packing as well)
+  if (!pw.fresh && env_int("B200DNN_PDL", 1) != 0) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  if (best > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = (unsigned)best; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = 1;
+    ++na;
+  }
+  cfg.attrs = attr; cfg.numAttrs = na;
+  B2_CUDA(cudaLaunchKernelEx(&cfg, kern, map_a, map_w, g, epi));
+  B2_LAUNCHED();
   return B200DNN_SUCCESS;
 }
 
@@ -1086,14 +1190,27 @@ int32_t b200dnn_matmul(const b200dnn_matmul_t *d, void *stream) {
   const bool tc_ok = (lda % 16 == 0) && ((reinterpret_cast<uintptr_t>(A) & 15) == 0);
   int which = d->force_kernel;
   if (which == 0) which = (M <= 16 || !tc_ok) ? 1 : 2;
-  B2_CHECK(which == 1 || which == 3 || tc_ok, B200DNN_FAILURE, "tcgen05 kernel needs a 16-byte aligned source with lda %% 16 == 0");
-  if (which == 1 || which == 3) {
+  // the weight may be read before the kernel in front has finished: that kernel is this call's quantisation, which itself waited for
+  // everything before it, or the caller says that its weights are in place (and they were not packed or uploaded in this call)
+  const bool early = !pw.fresh && (dyn || (d->flags & B200DNN_FLAG_STABLE_WEIGHTS) != 0);
+  // Few rows on the tensor cores (skinny_gemm.cuh), us: M = 16, K = 4096, N = 11008 12.7 -> 12.0, K = 11008, N = 4096 with quantisation
+  // 19.5 -> 17.9, but K = N = 4096 7.2 -> 7.6 (its fixed cost is higher); M = 32, N = 11008 17.7 -> 13.5, N = 1024 9.4 -> 6.1; M = 64, K = N =
+  // 4096 10.4 -> 10.9 (every CTA reads all activation rows of its share of K).
+  const bool skinny = (M > 16 && M <= 48) || (M > 8 && M <= 16 && (long long)K * N >= (24ll << 20));
+  if (d->force_kernel == 0 && tc_ok && skinny) {
+    B2_TRY(launch_skinny(A, lda, a_unsigned, false, M, N, K, pw, epi, M <= 16 && epi.n_po > 0 ? FA_GENERIC : fast_act_code(epi), early, st));
+    which = 4;
+  }
+  B2_CHECK(which != 2 || tc_ok, B200DNN_FAILURE, "tcgen05 kernel needs a 16-byte aligned source with lda %% 16 == 0");
+  if (which == 4) {
+    // launched above
+  } else if (which == 1 || which == 3) {
     int32_t rc = B200DNN_UNIMPLEMENTED;
     // decode kernel: 0 tiled only, 1 register-batch form, 2 ring form, 3..5 ring with that many groups per stage;
     // default: ring for M <= 2 and weights of 24 MB or more (measured faster there: 10.9 against 11.5 us at 45 MB, but
     // 5.9 against 5.7 us at 16.8 MB), register-batch form otherwise
     const int dk = env_int("B200DNN_DECODE_KERNEL", (M <= 2 && (long long)K * N >= (24ll << 20)) ? 2 : 1);
-    const bool pdl = (d->flags & B200DNN_FLAG_STABLE_WEIGHTS) != 0 && env_int("B200DNN_PDL", 1) != 0;
+    const bool pdl = early && env_int("B200DNN_PDL", 1) != 0;
     if (which == 1 && M <= 16 && dk >= 2) {
       // groups per stage: split the CTA's groups into equal sets of at most five
       const int groups = (N + 7) / 8, grid = groups < rt().sm_count ? groups : rt().sm_count;

@@ -48,6 +48,7 @@ int32_t resolve_bf16_weight(const void *weight, int64_t K, int64_t N, int64_t ld
   *pw = PackedWeight{};
   pw->wt = (const int8_t *)buf; pw->K = K; pw->N = N; pw->Kp = Kp; pw->Np = Np; pw->gated = gated; pw->I = I;
   if (cache) { pw->owned = buf; B2_TRY(mark_ready(*pw, st)); D.wcache.emplace(key, *pw); }
+  pw->fresh = true;
   return B200DNN_SUCCESS;
 }
 
@@ -125,6 +126,12 @@ int32_t matmul_bf16_packed(const b200dnn_matmul_t *d, const PackedWeight &pw, cu
     B2_LAUNCHED();
     B2_CUDA(cudaGetLastError());
     A = (const uint8_t *)tmp; lda = ld2;
+  }
+  // few rows (skinny_gemm.cuh), us: K = 4096, N = 11008, M = 8 31.0 -> 19.8, M = 64 24.4 -> 23.9, but M = 96 24.7 -> 27.3
+  if (d->force_kernel == 0 && M <= 64) {
+    const bool early = (d->flags & B200DNN_FLAG_STABLE_WEIGHTS) != 0 && !pw.fresh;
+    B2_TRY(launch_skinny(A, lda * 2, false, true, M, N, 2 * K, pw, epi, fast_act_code(epi), early, st));
+    return finish_out({&o_dst}, st);
   }
   TcGemmArgs ta{};
   const int tile_rows = tc_tile_rows(M, N);

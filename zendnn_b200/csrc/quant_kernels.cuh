@@ -162,12 +162,17 @@ __device__ __forceinline__ float block_max(float v, float *sh) {
 // register budget of four or five CTAs per SM: left to its own choice the compiler took 32 registers and spilled the cache).
 // EP: the expert-parallel forms (row count known only on the device: the CTAs stride over the rows; scatter into other
 // GPUs' receive buffers).  They are a separate instantiation so that the plain form keeps its register budget.
-template <typename T, int NV, bool EP>
-__global__ void __launch_bounds__(kQuantThreads, NV > 2 ? (EP ? 4 : (sizeof(T) == 2 ? 5 : 4)) : 6) quant_per_token_kernel(RowQuantArgs a) {
-  __shared__ float sh[kQuantThreads / 32];
+// THR: threads of the CTA.  Few long rows leave most of the chip idle whatever is done, so their time is the chain load - reduce -
+// convert of one row: 1024 threads with at most two vectors each (one row of 11008 and the GEMM behind it: 22.6 -> 18.0 us, with the
+// overlapped launch).
+template <typename T, int NV, bool EP, int THR = kQuantThreads>
+__global__ void __launch_bounds__(THR, THR > kQuantThreads ? 1 : (NV > 2 ? (EP ? 4 : (sizeof(T) == 2 ? 5 : 4)) : 6)) quant_per_token_kernel(RowQuantArgs a) {
+  __shared__ float sh[THR / 32];
   constexpr int E = VecTraits<T>::kPer16B;
-  // a GEMM launched as a programmatic dependent may start its set-up while this grid drains (it waits for the whole
-  // grid before it reads anything)
+  // Programmatic dependent launch on both sides: this kernel's launch overlaps the one in front (it touches memory only after the
+  // wait), and a GEMM behind it may start early.  The trigger comes after the wait, so whatever such a GEMM reads before its own
+  // wait (its weight) was written by work that is complete.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int row_limit = (EP && a.n_rows_dev) ? *a.n_rows_dev : (int)gridDim.x;
   for (int r = blockIdx.x; r < row_limit; r += EP ? (int)gridDim.x : row_limit) {
@@ -199,7 +204,7 @@ __global__ void __launch_bounds__(kQuantThreads, NV > 2 ? (EP ? 4 : (sizeof(T) =
   if (vec) {
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
-      int v = threadIdx.x + j * kQuantThreads;
+      int v = threadIdx.x + j * THR;
       if (v < nvec) {
         cache[j] = reinterpret_cast<const uint4 *>(src)[v];
         if (need_amax) {
@@ -209,14 +214,14 @@ __global__ void __launch_bounds__(kQuantThreads, NV > 2 ? (EP ? 4 : (sizeof(T) =
         }
       }
     }
-    for (int v = threadIdx.x + NV * kQuantThreads; need_amax && v < nvec; v += kQuantThreads) {
+    for (int v = threadIdx.x + NV * THR; need_amax && v < nvec; v += THR) {
       uint4 q = reinterpret_cast<const uint4 *>(src)[v];
       const T *e = reinterpret_cast<const T *>(&q);
 #pragma unroll
       for (int i = 0; i < E; ++i) { float f = elem_to_f32<T>(e[i]); if (finite_f32(f)) amax = fmaxf(amax, fabsf(f)); }
     }
   } else {
-    for (int k = threadIdx.x; need_amax && k < K; k += kQuantThreads) {
+    for (int k = threadIdx.x; need_amax && k < K; k += THR) {
       float f = elem_to_f32<T>(src[k]); if (finite_f32(f)) amax = fmaxf(amax, fabsf(f));
     }
   }
@@ -253,13 +258,13 @@ __global__ void __launch_bounds__(kQuantThreads, NV > 2 ? (EP ? 4 : (sizeof(T) =
     };
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
-      int v = threadIdx.x + j * kQuantThreads;
+      int v = threadIdx.x + j * THR;
       if (v < nvec) emit(cache[j], v);
     }
-    for (int v = threadIdx.x + NV * kQuantThreads; v < nvec; v += kQuantThreads)
+    for (int v = threadIdx.x + NV * THR; v < nvec; v += THR)
       emit(reinterpret_cast<const uint4 *>(src)[v], v);
   } else {
-    for (int k = threadIdx.x; k < K; k += kQuantThreads) {
+    for (int k = threadIdx.x; k < K; k += THR) {
       const int8_t qv = quant_sym_r(elem_to_f32<T>(src[k]), scale, rinv);
       if (sp) {
         for (int j = 0; j < a.scatter_n; ++j) { const int d = sc[j]; if (d >= 0 && d < a.scatter_cap) a.peer_dst[sp[j]][(int64_t)d * a.dst_ld + k] = qv; }
@@ -319,6 +324,7 @@ __global__ void __launch_bounds__(kQuantThreads) quant_per_token_asym_kernel(con
 template <typename T, int U>
 __global__ void __launch_bounds__(256) quant_known_absmax_kernel(RowQuantArgs a, int rows, int segs, int seg_len) {
   constexpr int E = VecTraits<T>::kPer16B;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int lane = threadIdx.x & 31;
   const int row_limit = a.n_rows_dev ? min(rows, *a.n_rows_dev) : rows;
@@ -364,6 +370,7 @@ __global__ void __launch_bounds__(256) quant_known_absmax_kernel(RowQuantArgs a,
 template <typename T, int NV, bool EP>
 __global__ void __launch_bounds__(256) quant_per_token_warp_kernel(RowQuantArgs a, int rows) {
   constexpr int E = VecTraits<T>::kPer16B;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int lane = threadIdx.x & 31;
   const int row_limit = (EP && a.n_rows_dev) ? min(rows, *a.n_rows_dev) : rows;

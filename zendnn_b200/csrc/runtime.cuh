@@ -95,6 +95,7 @@ struct PackedWeight {
   // cache-owned buffers are packed on the stream of the call that first saw the weight; calls on other streams wait
   // for this event until it has been seen complete once
   cudaEvent_t ready = nullptr; cudaStream_t ready_stream = nullptr; bool complete = true;
+  bool fresh = false;      // written by work that this very call has put on the stream
 };
 
 // Small host inputs of one call (activations of a decode step, scales, zero point, bias, descriptor tables) are
@@ -151,6 +152,7 @@ struct DeviceShared {
   std::mutex attr_mu;
   std::map<const void *, int> smem_limit;                 // kernels whose dynamic shared-memory limit was raised
   int split_room[5] = {0, 0, 0, 0, 0};
+  int skinny_room[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
 };
 
 // Descriptor tables that depend only on the caller's weight pointers (per-expert epilogue pointers, tensor maps) are

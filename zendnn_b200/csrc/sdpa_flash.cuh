@@ -123,7 +123,6 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   __shared__ volatile int s_err;
   constexpr uint32_t kBox = 128 * 128;                 // [128 rows][64 elements]
   constexpr uint32_t kTile = DB * kBox;                // 128 rows of Q, K or V
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (the same in every lane, and known to be)
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t ring0 = smem0 + (uint32_t)a.tiles * kTile;
@@ -158,6 +157,8 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_slot;
+  // (behind the allocation: a dependent's CTA on this SM can then not take tensor memory that this one still waits for)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   // this CTA's work item

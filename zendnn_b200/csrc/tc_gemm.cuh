@@ -547,9 +547,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile int s_err;
 
-  // programmatic dependent launch: the next kernel of the stream may take this CTA's SM as soon as it is free; this
-  // kernel touches global memory only after griddepcontrol.wait below (the set-up before it uses none)
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (the same in every lane, and known to be)
   if (threadIdx.x == 0) TC_STAMP(0);
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -596,6 +593,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if constexpr (PAIR) cluster_sync_all();   // the partner's barriers exist before anything of this CTA signals them
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
+  // programmatic dependent launch: the next kernel of the stream may take this CTA's SM as soon as it is free (not before this CTA has
+  // its tensor memory, or a dependent's CTA could hold the columns that this one waits for); this kernel touches global memory
+  // only after griddepcontrol.wait (the set-up before it uses none)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");   // everything before this launch in the stream is complete and visible
   if (threadIdx.x == 0) TC_STAMP(1);
 

@@ -124,6 +124,7 @@ int32_t resolve_woq_weight(const b200dnn_matmul_t *d, int64_t group, cudaStream_
   *pw = PackedWeight{};
   pw->wt = (const int8_t *)buf; pw->K = K; pw->N = N; pw->Kp = a.Kp; pw->Np = Np;
   if (cache) { pw->owned = buf; B2_TRY(mark_ready(*pw, st)); D.woq_cache.emplace(key, *pw); }
+  pw->fresh = true;
   return B200DNN_SUCCESS;
 }
 
