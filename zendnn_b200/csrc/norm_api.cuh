@@ -127,174 +127,201 @@ __global__ void __launch_bounds__(kNormThreads) norm_rows_kernel(const NormArgs 
   }
 }
 
+__device__ __forceinline__ float norm_lo(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float norm_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
+// four parameters (f32 or bf16, 16-byte aligned array), group i4
+__device__ __forceinline__ void norm_load4(const void *p, int32_t dt, int i4, float (&g)[4]) {
+  if (dt == B200DNN_F32) {
+    const float4 v = reinterpret_cast<const float4 *>(p)[i4];
+    g[0] = v.x; g[1] = v.y; g[2] = v.z; g[3] = v.w;
+  } else {
+    const uint2 v = reinterpret_cast<const uint2 *>(p)[i4];
+    g[0] = norm_lo(v.x); g[1] = norm_hi(v.x); g[2] = norm_lo(v.y); g[3] = norm_hi(v.y);
+  }
+}
+
+// One row of the full-width form, held by the CTA as the bf16 pairs it came in: v = input, r = residual (fused add).  red: a buffer per
+// reduction, used by one row in two (so one barrier each).  Same arithmetic as the generic kernel.
+template <int NV>
+__device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, uint32_t (&v)[NV][4], const uint32_t (&r)[NV][4], float (*red)[kNormThreads / 32]) {
+  const int nvec = (int)(a.n >> 3);
+  auto lo = norm_lo; auto hi = norm_hi;
+  const int64_t off = b * a.n;
+  uint4 *rv = a.residual ? reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(a.residual) + off) : nullptr;
+  auto sum = [](float x, float *sh) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
+    __syncthreads();
+    float t = 0.f;
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += sh[i];
+    return t;
+  };
+  auto largest = [](float x, float *sh) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
+    __syncthreads();
+    float t = 0.f;
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t = fmaxf(t, sh[i]);
+    return t;
+  };
+  float s1 = 0.f;
+  if (a.type == NORM_FUSED_ADD_RMS) {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int i = threadIdx.x + j * blockDim.x;
+      if (i < nvec) {
+        const uint32_t (&rw)[4] = r[j];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float s_lo = __fadd_rn(lo(rw[e]), lo(v[j][e])), s_hi = __fadd_rn(hi(rw[e]), hi(v[j][e]));
+          s1 = __fmaf_rn(s_lo, s_lo, s1); s1 = __fmaf_rn(s_hi, s_hi, s1);
+          v[j][e] = pack_bf16x2(s_lo, s_hi);
+        }
+        rv[i] = make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]);
+      }
+    }
+  } else if (a.type == NORM_RMS) {
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { s1 = __fmaf_rn(lo(v[j][e]), lo(v[j][e]), s1); s1 = __fmaf_rn(hi(v[j][e]), hi(v[j][e]), s1); }
+  } else {
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { s1 = __fadd_rn(s1, lo(v[j][e])); s1 = __fadd_rn(s1, hi(v[j][e])); }
+  }
+  s1 = sum(s1, red[0]);
+  float mean = 0.f, inv;
+  if (a.type == NORM_LAYER) {
+    mean = __fdiv_rn(s1, (float)a.n);
+    float s2 = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if (threadIdx.x + j * blockDim.x < nvec) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float d0 = __fadd_rn(lo(v[j][e]), -mean), d1 = __fadd_rn(hi(v[j][e]), -mean);
+          s2 = __fmaf_rn(d0, d0, s2); s2 = __fmaf_rn(d1, d1, s2);
+        }
+      }
+    s2 = sum(s2, red[1]);
+    inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(s2, (float)a.n), a.eps)));
+  } else inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(s1, (float)a.n), a.eps)));
+  float amax = 0.f;
+  const bool layer = a.type == NORM_LAYER, shift = a.use_shift && layer;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int i = threadIdx.x + j * blockDim.x;
+    if (i < nvec) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {          // two halves of four elements
+        float g[4] = {1.f, 1.f, 1.f, 1.f};
+        if (a.use_scale) norm_load4(a.gamma, a.gamma_dt, 2 * i + h, g);
+        float bt[4] = {0.f, 0.f, 0.f, 0.f};
+        if (shift) norm_load4(a.beta, a.beta_dt, 2 * i + h, bt);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const uint32_t w = v[j][2 * h + e];
+          float y0 = lo(w), y1 = hi(w);
+          if (layer) { y0 = __fadd_rn(y0, -mean); y1 = __fadd_rn(y1, -mean); }
+          y0 = __fmul_rn(y0, inv); y1 = __fmul_rn(y1, inv);
+          if (a.use_scale) { y0 = __fmul_rn(y0, g[2 * e]); y1 = __fmul_rn(y1, g[2 * e + 1]); }
+          if (shift) { y0 = __fadd_rn(y0, bt[2 * e]); y1 = __fadd_rn(y1, bt[2 * e + 1]); }
+          const uint32_t o = pack_bf16x2(y0, y1);
+          v[j][2 * h + e] = o;
+          // rounding to bf16 is monotonic: the largest rounded magnitude is the rounded largest magnitude (a NaN does not
+          // enter fmaxf; an infinity does and is dealt with after the loop)
+          if (a.q) amax = fmaxf(amax, fmaxf(fabsf(y0), fabsf(y1)));
+        }
+      }
+      if (a.y) reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(a.y) + off)[i] = make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]);
+    }
+  }
+  if (a.q) {
+    amax = largest(amax, red[2]);
+    amax = __uint_as_float(pack_bf16x2(amax, 0.0f) << 16);
+    if (!finite_f32(amax)) {
+      // an infinite element (it quantises to 0): take the maximum over the finite rounded values instead
+      uint32_t mb = 0u;
+#pragma unroll
+      for (int j = 0; j < NV; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t m0 = (v[j][e] << 16) & 0x7FFFFFFFu, m1 = v[j][e] & 0x7FFF0000u;
+          mb = max(mb, m0 < 0x7F800000u ? m0 : 0u);
+          mb = max(mb, m1 < 0x7F800000u ? m1 : 0u);
+        }
+      amax = largest(__uint_as_float(mb), red[3]);
+    }
+    const float scale = scale_from_absmax(amax);
+    const float rinv = __frcp_rn(scale);
+    // q = rne(v / scale) without a division: m = v * rinv + 1.5 * 2^23 holds the integer nearest to the product in its low
+    // byte; d = v * rinv - that integer is the product's distance from it, and whenever |d| < 0.4999 (d^2 < 0.2499, one
+    // fused operation whose sign bit is and-ed over the vector) the product and the exact quotient round alike: rinv is
+    // the correctly rounded reciprocal, so v * rinv is within 127.5 * 2^-24 < 1e-5 of v / scale.  An element that fails
+    // the test, through a near-tie or because it is not finite, takes the exact division.
+    const float magic = 12582912.0f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int i = threadIdx.x + j * blockDim.x;
+      if (i < nvec) {
+        uint32_t mbits[8], ok = 0x80000000u;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float v0 = lo(v[j][e]), v1 = hi(v[j][e]);
+          const float m0 = __fmaf_rn(v0, rinv, magic), m1 = __fmaf_rn(v1, rinv, magic);
+          const float d0 = __fmaf_rn(v0, rinv, __fsub_rn(magic, m0)), d1 = __fmaf_rn(v1, rinv, __fsub_rn(magic, m1));
+          const uint32_t c0 = __float_as_uint(__fmaf_rn(d0, d0, -0.2499f)), c1 = __float_as_uint(__fmaf_rn(d1, d1, -0.2499f));
+          ok &= c0 & c1;
+          mbits[2 * e] = __float_as_uint(m0); mbits[2 * e + 1] = __float_as_uint(m1);
+        }
+        if (!ok) {
+          // only the elements that failed take the division (about two in ten thousand)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float ve = (e & 1) ? hi(v[j][e >> 1]) : lo(v[j][e >> 1]);
+            const float de = __fmaf_rn(ve, rinv, __fsub_rn(magic, __uint_as_float(mbits[e])));
+            if (!(__fmaf_rn(de, de, -0.2499f) < 0.0f)) mbits[e] = (uint32_t)(uint8_t)quant_sym(ve, scale);
+          }
+        }
+        *reinterpret_cast<uint2 *>(a.q + b * a.q_ld + (int64_t)i * 8) =
+            make_uint2(low_bytes4(mbits[0], mbits[1], mbits[2], mbits[3]), low_bytes4(mbits[4], mbits[5], mbits[6], mbits[7]));
+      }
+    }
+    if (threadIdx.x == 0) a.q_scale[b] = scale;
+  }
+}
+
 // The decoder-layer case at full width: bf16 rows of at most NV * 8 * blockDim elements, 16-byte aligned, bf16 out.  One
 // CTA per row; a thread keeps its NV vectors of eight elements in registers (as the bf16 pairs they are at every stage that
 // is kept) between the passes, so the row is read once and every access is a 16-byte vector (8 bytes for the s8 codes).
-// Same arithmetic as the generic kernel.
+// HBM-bound, with the resident CTAs covering each other's reductions: all loads of a row (input and residual) are in flight before the first
+// store, each reduction costs one barrier, and the launch overlaps the kernel in front.  4096 rows of 4096 with residual add and s8 codes
+// (151 MB): 36.9 -> 30.5 us (4.9 TB/s); a ring of rows filled by bulk copies ahead of persistent CTAs took 35.7 us (four CTAs per SM where
+// there are six here).
 template <int NV>
 __global__ void __launch_bounds__(kNormThreads, NV <= 2 ? 6 : (NV <= 4 ? 4 : 2)) norm_rows_vec_kernel(const NormArgs a) {
-  __shared__ float sh[kNormThreads / 32];
+  __shared__ float red[2][4][kNormThreads / 32];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int nvec = (int)(a.n >> 3);
-  auto lo = [](uint32_t w) { return __uint_as_float(w << 16); };
-  auto hi = [](uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); };
-  for (int64_t b = blockIdx.x; b < a.batch; b += gridDim.x) {
-    const int64_t off = b * a.n;
-    const uint4 *xv = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(a.x) + off);
-    uint4 *rv = a.residual ? reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(a.residual) + off) : nullptr;
-    uint32_t v[NV][4];
-    float s1 = 0.f;
+  int parity = 0;
+  for (int64_t b = blockIdx.x; b < a.batch; b += gridDim.x, parity ^= 1) {
+    const uint4 *xv = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(a.x) + b * a.n);
+    const uint4 *rv = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(a.residual) + b * a.n);
+    uint32_t v[NV][4], r[NV][4];
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
       const int i = threadIdx.x + j * blockDim.x;
-      v[j][0] = v[j][1] = v[j][2] = v[j][3] = 0u;
-      if (i < nvec) {
-        const uint4 q = xv[i];
-        v[j][0] = q.x; v[j][1] = q.y; v[j][2] = q.z; v[j][3] = q.w;
-      }
+      const uint4 q = i < nvec ? xv[i] : make_uint4(0u, 0u, 0u, 0u);
+      v[j][0] = q.x; v[j][1] = q.y; v[j][2] = q.z; v[j][3] = q.w;
+      const uint4 s = (a.type == NORM_FUSED_ADD_RMS && i < nvec) ? rv[i] : make_uint4(0u, 0u, 0u, 0u);
+      r[j][0] = s.x; r[j][1] = s.y; r[j][2] = s.z; r[j][3] = s.w;
     }
-    if (a.type == NORM_FUSED_ADD_RMS) {
-#pragma unroll
-      for (int j = 0; j < NV; ++j) {
-        const int i = threadIdx.x + j * blockDim.x;
-        if (i < nvec) {
-          const uint4 r = rv[i];
-          const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float s_lo = __fadd_rn(lo(rw[e]), lo(v[j][e])), s_hi = __fadd_rn(hi(rw[e]), hi(v[j][e]));
-            s1 = __fmaf_rn(s_lo, s_lo, s1); s1 = __fmaf_rn(s_hi, s_hi, s1);
-            v[j][e] = pack_bf16x2(s_lo, s_hi);
-          }
-          rv[i] = make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]);
-        }
-      }
-    } else if (a.type == NORM_RMS) {
-#pragma unroll
-      for (int j = 0; j < NV; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { s1 = __fmaf_rn(lo(v[j][e]), lo(v[j][e]), s1); s1 = __fmaf_rn(hi(v[j][e]), hi(v[j][e]), s1); }
-    } else {
-#pragma unroll
-      for (int j = 0; j < NV; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { s1 = __fadd_rn(s1, lo(v[j][e])); s1 = __fadd_rn(s1, hi(v[j][e])); }
-    }
-    s1 = norm_block_sum(s1, sh);
-    float mean = 0.f, inv;
-    if (a.type == NORM_LAYER) {
-      mean = __fdiv_rn(s1, (float)a.n);
-      float s2 = 0.f;
-#pragma unroll
-      for (int j = 0; j < NV; ++j)
-        if (threadIdx.x + j * blockDim.x < nvec) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float d0 = __fadd_rn(lo(v[j][e]), -mean), d1 = __fadd_rn(hi(v[j][e]), -mean);
-            s2 = __fmaf_rn(d0, d0, s2); s2 = __fmaf_rn(d1, d1, s2);
-          }
-        }
-      s2 = norm_block_sum(s2, sh);
-      inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(s2, (float)a.n), a.eps)));
-    } else inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(s1, (float)a.n), a.eps)));
-    float amax = 0.f;
-    const bool layer = a.type == NORM_LAYER, shift = a.use_shift && layer;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      const int i = threadIdx.x + j * blockDim.x;
-      if (i < nvec) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {          // two halves of four elements
-          float g[4] = {1.f, 1.f, 1.f, 1.f};
-          if (a.use_scale) {
-            if (a.gamma_dt == B200DNN_F32) {
-              const float4 g4 = reinterpret_cast<const float4 *>(a.gamma)[2 * i + h];
-              g[0] = g4.x; g[1] = g4.y; g[2] = g4.z; g[3] = g4.w;
-            } else {
-              const uint2 gq = reinterpret_cast<const uint2 *>(a.gamma)[2 * i + h];
-              g[0] = lo(gq.x); g[1] = hi(gq.x); g[2] = lo(gq.y); g[3] = hi(gq.y);
-            }
-          }
-          float bt[4] = {0.f, 0.f, 0.f, 0.f};
-          if (shift) {
-            if (a.beta_dt == B200DNN_F32) {
-              const float4 b4 = reinterpret_cast<const float4 *>(a.beta)[2 * i + h];
-              bt[0] = b4.x; bt[1] = b4.y; bt[2] = b4.z; bt[3] = b4.w;
-            } else {
-              const uint2 bq = reinterpret_cast<const uint2 *>(a.beta)[2 * i + h];
-              bt[0] = lo(bq.x); bt[1] = hi(bq.x); bt[2] = lo(bq.y); bt[3] = hi(bq.y);
-            }
-          }
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const uint32_t w = v[j][2 * h + e];
-            float y0 = lo(w), y1 = hi(w);
-            if (layer) { y0 = __fadd_rn(y0, -mean); y1 = __fadd_rn(y1, -mean); }
-            y0 = __fmul_rn(y0, inv); y1 = __fmul_rn(y1, inv);
-            if (a.use_scale) { y0 = __fmul_rn(y0, g[2 * e]); y1 = __fmul_rn(y1, g[2 * e + 1]); }
-            if (shift) { y0 = __fadd_rn(y0, bt[2 * e]); y1 = __fadd_rn(y1, bt[2 * e + 1]); }
-            const uint32_t o = pack_bf16x2(y0, y1);
-            v[j][2 * h + e] = o;
-            // rounding to bf16 is monotonic: the largest rounded magnitude is the rounded largest magnitude (a NaN does not
-            // enter fmaxf; an infinity does and is dealt with after the loop)
-            if (a.q) amax = fmaxf(amax, fmaxf(fabsf(y0), fabsf(y1)));
-          }
-        }
-        if (a.y) reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(a.y) + off)[i] = make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]);
-      }
-    }
-    if (a.q) {
-      amax = norm_block_max(amax, sh);
-      amax = __uint_as_float(pack_bf16x2(amax, 0.0f) << 16);
-      if (!finite_f32(amax)) {
-        // an infinite element (it quantises to 0): take the maximum over the finite rounded values instead
-        uint32_t mb = 0u;
-#pragma unroll
-        for (int j = 0; j < NV; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const uint32_t m0 = (v[j][e] << 16) & 0x7FFFFFFFu, m1 = v[j][e] & 0x7FFF0000u;
-            mb = max(mb, m0 < 0x7F800000u ? m0 : 0u);
-            mb = max(mb, m1 < 0x7F800000u ? m1 : 0u);
-          }
-        amax = norm_block_max(__uint_as_float(mb), sh);
-      }
-      const float scale = scale_from_absmax(amax);
-      const float rinv = __frcp_rn(scale);
-      // q = rne(v / scale) without a division: m = v * rinv + 1.5 * 2^23 holds the integer nearest to the product in its low
-      // byte; d = v * rinv - that integer is the product's distance from it, and whenever |d| < 0.4999 (d^2 < 0.2499, one
-      // fused operation whose sign bit is and-ed over the vector) the product and the exact quotient round alike: rinv is
-      // the correctly rounded reciprocal, so v * rinv is within 127.5 * 2^-24 < 1e-5 of v / scale.  An element that fails
-      // the test, through a near-tie or because it is not finite, takes the exact division.
-      const float magic = 12582912.0f;
-#pragma unroll
-      for (int j = 0; j < NV; ++j) {
-        const int i = threadIdx.x + j * blockDim.x;
-        if (i < nvec) {
-          uint32_t mbits[8], ok = 0x80000000u;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float v0 = lo(v[j][e]), v1 = hi(v[j][e]);
-            const float m0 = __fmaf_rn(v0, rinv, magic), m1 = __fmaf_rn(v1, rinv, magic);
-            const float d0 = __fmaf_rn(v0, rinv, __fsub_rn(magic, m0)), d1 = __fmaf_rn(v1, rinv, __fsub_rn(magic, m1));
-            const uint32_t c0 = __float_as_uint(__fmaf_rn(d0, d0, -0.2499f)), c1 = __float_as_uint(__fmaf_rn(d1, d1, -0.2499f));
-            ok &= c0 & c1;
-            mbits[2 * e] = __float_as_uint(m0); mbits[2 * e + 1] = __float_as_uint(m1);
-          }
-          if (!ok) {
-            // only the elements that failed take the division (about two in ten thousand)
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const float ve = (e & 1) ? hi(v[j][e >> 1]) : lo(v[j][e >> 1]);
-              const float de = __fmaf_rn(ve, rinv, __fsub_rn(magic, __uint_as_float(mbits[e])));
-              if (!(__fmaf_rn(de, de, -0.2499f) < 0.0f)) mbits[e] = (uint32_t)(uint8_t)quant_sym(ve, scale);
-            }
-          }
-          *reinterpret_cast<uint2 *>(a.q + b * a.q_ld + (int64_t)i * 8) =
-              make_uint2(low_bytes4(mbits[0], mbits[1], mbits[2], mbits[3]), low_bytes4(mbits[4], mbits[5], mbits[6], mbits[7]));
-        }
-      }
-      if (threadIdx.x == 0) a.q_scale[b] = scale;
-    }
+    norm_row_vec<NV>(a, b, v, r, red[parity]);
   }
 }
 
@@ -402,10 +429,11 @@ extern "C" int32_t b200dnn_normalization(const b200dnn_norm_t *d, void *stream) 
       const int nv = (nvec + threads - 1) / threads;
       const long long cap = (long long)R.sm_count * 64;
       const unsigned grid = (unsigned)(batch < cap ? batch : cap);
-      if (nv <= 1) norm_rows_vec_kernel<1><<<grid, threads, 0, st>>>(a);
-      else if (nv <= 2) norm_rows_vec_kernel<2><<<grid, threads, 0, st>>>(a);
-      else if (nv <= 4) norm_rows_vec_kernel<4><<<grid, threads, 0, st>>>(a);
-      else norm_rows_vec_kernel<8><<<grid, threads, 0, st>>>(a);
+      const int nvt = nv <= 1 ? 1 : (nv <= 2 ? 2 : (nv <= 4 ? 4 : 8));
+      if (nvt == 1) B2_TRY(launch_pdl(norm_rows_vec_kernel<1>, grid, (unsigned)threads, 0, st, true, a));
+      else if (nvt == 2) B2_TRY(launch_pdl(norm_rows_vec_kernel<2>, grid, (unsigned)threads, 0, st, true, a));
+      else if (nvt == 4) B2_TRY(launch_pdl(norm_rows_vec_kernel<4>, grid, (unsigned)threads, 0, st, true, a));
+      else B2_TRY(launch_pdl(norm_rows_vec_kernel<8>, grid, (unsigned)threads, 0, st, true, a));
       B2_LAUNCHED();
       B2_CUDA(cudaGetLastError());
       return finish_out({&o_y, &o_res, &o_q, &o_s}, st);
