@@ -132,16 +132,16 @@ int32_t launch_gs_t(const GsGemmArgs &a, const EpiParams &epi, cudaStream_t st) 
 template <int CH, bool W4, int R>
 int32_t launch_gs_decode_r(const GsDecodeArgs &da, const EpiParams &epi, size_t smem, int grid, cudaStream_t st) {
   B2_TRY(ensure_max_smem((const void *)gs_decode_kernel<CH, W4, R>, (int)smem));
-  gs_decode_kernel<CH, W4, R><<<grid, kGsWarps * 32, smem, st>>>(da, epi);
+  B2_TRY(launch_pdl(gs_decode_kernel<CH, W4, R>, (unsigned)grid, kGsWarps * 32u, smem, st, da.early != 0, da, epi));
   B2_LAUNCHED();
   B2_CUDA(cudaGetLastError());
   return B200DNN_SUCCESS;
 }
 template <int CH, bool W4>
-int32_t launch_gs_decode_t(const GsGemmArgs &a, const EpiParams &epi, cudaStream_t st, bool *done) {
+int32_t launch_gs_decode_t(const GsGemmArgs &a, const EpiParams &epi, bool early, cudaStream_t st, bool *done) {
   *done = false;
   GsDecodeArgs da{};
-  da.g = a;
+  da.g = a; da.early = early ? 1 : 0;
   da.rows_staged = a.M;
   // row stride of the staged activations: the lanes of a quarter warp (16-byte loads) or half warp (8-byte loads) read
   // distinct bank groups when the stride is 64 (32) bytes off a multiple of 128
@@ -299,8 +299,10 @@ int32_t matmul_group_scaled(const b200dnn_matmul_t *d, cudaStream_t st) {
     bool done = false;
     int32_t rcd;
     const bool ch128 = p.gs % 128 == 0 && env_int("B200DNN_GS_CH128", 1) != 0;     // fewer, larger items per group
-    if (p.w4) rcd = ch128 ? launch_gs_decode_t<128, true>(a, epi, st, &done) : ch64 ? launch_gs_decode_t<64, true>(a, epi, st, &done) : launch_gs_decode_t<32, true>(a, epi, st, &done);
-    else rcd = ch128 ? launch_gs_decode_t<128, false>(a, epi, st, &done) : ch64 ? launch_gs_decode_t<64, false>(a, epi, st, &done) : launch_gs_decode_t<32, false>(a, epi, st, &done);
+    // (directly behind the per-token quantisation, which waited for everything in front of it)
+    const bool early = p.dyn && p.src_cols == 1 && !p.src_per_tensor;
+    if (p.w4) rcd = ch128 ? launch_gs_decode_t<128, true>(a, epi, early, st, &done) : ch64 ? launch_gs_decode_t<64, true>(a, epi, early, st, &done) : launch_gs_decode_t<32, true>(a, epi, early, st, &done);
+    else rcd = ch128 ? launch_gs_decode_t<128, false>(a, epi, early, st, &done) : ch64 ? launch_gs_decode_t<64, false>(a, epi, early, st, &done) : launch_gs_decode_t<32, false>(a, epi, early, st, &done);
     B2_TRY(rcd);
     if (done) return finish_out({&o_dst, &o_scale}, st);
   } else B2_TRY(prepare_source());
