@@ -170,7 +170,7 @@ int32_t moe_core(int G, const std::vector<ExpertWeightsIn> &ew, int K, int I, in
                  RowQuantArgs qa, int32_t src_dt, int R, const int32_t *row_off_dev, const int32_t *tile_prefix_dev,
                  int m_tiles_bound, const std::vector<void *> *dst_down_dev, const std::vector<int64_t> *ldc_down,
                  void **O_out, int64_t *ldO_out, cudaStream_t st, void *O_given = nullptr, int tile_rows = kTcBM,
-                 const uint16_t **Z_out = nullptr) {
+                 const uint16_t **Z_out = nullptr, uint32_t *zmax = nullptr /* row maxima already set to zero, or null */) {
   Runtime &Rt = rt();
   B2_CHECK(act >= 1 && act <= 3, B200DNN_UNIMPLEMENTED, "fused MoE needs a gated activation (got %d)", act);
   B2_CHECK(I % kGateGranule == 0, B200DNN_UNIMPLEMENTED, "expert FFN width must be a multiple of %d", kGateGranule);
@@ -216,11 +216,12 @@ int32_t moe_core(int G, const std::vector<ExpertWeightsIn> &ew, int K, int I, in
   int8_t *A1 = (int8_t *)Rt.ws.alloc((size_t)R * Kq);
   float *s1 = (float *)Rt.ws.alloc((size_t)R * 4);
   uint16_t *Z = (uint16_t *)Rt.ws.alloc((size_t)R * I * 2);
-  uint32_t *zmax = (uint32_t *)Rt.ws.alloc((size_t)R * 4);
+  const bool zero_max = zmax == nullptr;
+  if (zero_max) zmax = (uint32_t *)Rt.ws.alloc((size_t)R * 4);
   int8_t *A2 = (int8_t *)Rt.ws.alloc((size_t)R * Iq);
   float *s2v = (float *)Rt.ws.alloc((size_t)R * 4);
   B2_CHECK(A1 && s1 && Z && zmax && A2 && s2v, B200DNN_FAILURE, "workspace allocation failed");
-  B2_CUDA(cudaMemsetAsync(zmax, 0, (size_t)R * 4, st));
+  if (zero_max) B2_CUDA(cudaMemsetAsync(zmax, 0, (size_t)R * 4, st));
 
   // 1. quantise the gathered rows (src_dt == s8: the caller hands over rows that are already quantised,
   //    qa.src = s8 [R, qa.src_ld], qa.scale = their f32 scales -- the expert-parallel path after dispatch)
@@ -420,13 +421,23 @@ extern "C" int32_t b200dnn_moe_layer(const void *x, int64_t ldx, const float *lo
   int32_t *row_token = (int32_t *)Rt.ws.alloc((size_t)R * 4);
   B2_CHECK(ids && w && rank && cnt && row_off && tile_prefix && slot_rows && slot_w && row_token, B200DNN_FAILURE, "workspace allocation failed");
   rt().mark(-1);
-  B2_TRY(launch_route_topk((const float *)l_dev, T, E, topk, 1, ids, w, st));
-  B2_TRY(launch_expert_rank(ids, T * topk, E, rank, cnt, st));
   const int tile_rows = tc_tile_rows(R, H < 2 * I ? H : 2 * I);
-  expert_offsets_kernel<<<1, 32, 0, st>>>(cnt, E, S, T, row_off, tile_prefix, tile_rows);
-  B2_LAUNCHED();
-  build_maps_kernel<<<(unsigned)((R + 255) / 256), 256, 0, st>>>(ids, rank, w, row_off, T, topk, E, S, slot_rows, slot_w, row_token);
-  B2_LAUNCHED();
+  uint32_t *zmax = nullptr;
+  if (T <= kRouteSmallT && T * topk <= kRouteSmallSlots && G <= kRouteSmallGroups) {
+    zmax = (uint32_t *)Rt.ws.alloc((size_t)R * 4);
+    B2_CHECK(zmax, B200DNN_FAILURE, "workspace allocation failed");
+#define B2_RS(PER) launch_pdl(route_small_kernel<PER>, 1u, 1024u, 0, st, true, (const float *)l_dev, T, E, topk, S, tile_rows, row_off, tile_prefix, slot_rows, slot_w, row_token, zmax)
+    B2_TRY(E <= 32 ? B2_RS(1) : E <= 64 ? B2_RS(2) : E <= 128 ? B2_RS(4) : B2_RS(8));
+#undef B2_RS
+    B2_LAUNCHED();
+  } else {
+    B2_TRY(launch_route_topk((const float *)l_dev, T, E, topk, 1, ids, w, st));
+    B2_TRY(launch_expert_rank(ids, T * topk, E, rank, cnt, st));
+    expert_offsets_kernel<<<1, 32, 0, st>>>(cnt, E, S, T, row_off, tile_prefix, tile_rows);
+    B2_LAUNCHED();
+    build_maps_kernel<<<(unsigned)((R + 255) / 256), 256, 0, st>>>(ids, rank, w, row_off, T, topk, E, S, slot_rows, slot_w, row_token);
+    B2_LAUNCHED();
+  }
   B2_CUDA(cudaGetLastError());
   rt().mark(0);
 
@@ -440,14 +451,14 @@ extern "C" int32_t b200dnn_moe_layer(const void *x, int64_t ldx, const float *lo
   void *O = nullptr; int64_t ldO = 0;
   const int m_tiles_bound = (R + tile_rows - 1) / tile_rows + G;
   B2_TRY(moe_core(G, ew, K, I, H, transB, act, 1, qa, B200DNN_BF16, R, row_off, tile_prefix, m_tiles_bound, nullptr, nullptr, &O, &ldO, st,
-                  nullptr, tile_rows));
+                  nullptr, tile_rows, nullptr, zmax));
 
   Staged o_out;
   B2_TRY(stage_out(out, span_bytes(T, H, ld_out, B200DNN_BF16), st, &o_out, ld_out != H));
   ReduceArgs ra{};
   ra.base = O; ra.ld = ldO; ra.slot_rows = slot_rows; ra.w = slot_w; ra.nslots = ns; ra.D = H; ra.dt = B200DNN_BF16;
   ra.out = o_out.dev; ra.ld_out = ld_out;
-  moe_reduce_kernel<<<(unsigned)T, 256, (sizeof(void *) + 4) * ns, st>>>(ra);
+  B2_TRY(launch_pdl(moe_reduce_kernel, (unsigned)T, 256u, (sizeof(void *) + 4) * ns, st, true, ra));
   B2_LAUNCHED();
   B2_CUDA(cudaGetLastError());
   rt().mark(8);
