@@ -49,7 +49,8 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t d; a
 // 2^x for two arguments on the FMA pipe, to share the exponentials between the two pipes: x = n + f with n the nearest integer
 // (added and removed as 1.5 * 2^23), 2^f by a degree-5 polynomial in Horner form, n added to the exponent field.  The
 // coefficients are the minimax fit in relative error of 2^f on [-1/2, 1/2] (Remez exchange in double, rounded to f32):
-// 2.1e-7 in f32 arithmetic, as ex2.approx.  Arguments are clamped at -126 (there 2^x is 1e-38 where ex2.approx gives 0).
+// 2.1e-7 in f32 arithmetic, as ex2.approx.  Arguments are clamped at -126 (there 2^x is 1e-38 where ex2.approx gives 0) and must be
+// less than 128 (n is added to the exponent field as it is): both sweeps pass arguments of at most about 0.
 __device__ __forceinline__ uint64_t ex2_poly2(uint64_t x2) {
   float x0, x1;
   upk2(x2, x0, x1);
@@ -334,43 +335,9 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     bool ok = true;
     uint32_t ph0 = 0, ph1 = 0;
     const float cc = MASK ? 1.0f : c;
-    // this half of a block with the row maximum brought up to date (first block, blocks of rows that a mask has hidden so far, and the recovery below)
-    auto half_with_max = [&](uint32_t ta, int k0, bool last) {
-      float mx = ninf;
-#pragma unroll 1
-      for (int q = 0; q < 2; ++q) {
-        uint32_t s[32];
-        tc_ld32(ta + (uint32_t)q * 32u, s);
-        tc_wait_ld();
-        mask32(s, k0 + q * 32);
-        if (last) limit32(s, k0 + q * 32);
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(s[i]), __uint_as_float(s[i + 1])));
-      }
-      const float mn = fmaxf(m, mx), nmc = mn == ninf ? 0.f : -mn * cc;      // (no key so far: every term is 2^-inf)
-      const uint64_t c2 = pk2(cc, cc), b2 = pk2(nmc, nmc);
-      uint64_t acc = 0ull;
-#pragma unroll 1
-      for (int q = 0; q < 2; ++q) {
-        uint32_t s[32];
-        tc_ld32(ta + (uint32_t)q * 32u, s);
-        tc_wait_ld();
-        mask32(s, k0 + q * 32);
-        if (last) limit32(s, k0 + q * 32);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) acc = add2(acc, ex2_pair<false>(fma2(pk2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), c2, b2), i));
-      }
-      float e0, e1;
-      upk2(acc, e0, e1);
-      l = __fmaf_rn(l, ex2f(__fmaf_rn(m, cc, nmc)), e0 + e1);
-      m = mn;
-    };
-    // ---- sweep 1: row maximum and row sum.  The reference m only has to keep the sum in range, so after the first block it stays as
-    // it is (the first block's maximum: the sum is at least 1) and a block's terms are added without a maximum of their own; a block
-    // whose sum leaves the comfortable range (scores 40 above the reference, in powers of two) is done again with its maximum.
+    // ---- sweep 1: row maximum and row sum of this half, 32 scores at a time; the sum is kept relative to the largest score so far,
+    // so no term exceeds 1 (ex2_poly2 is only good up to there) and a single score far above all others is met wherever it lies
     auto sum_half = [&](uint32_t ta, int k0, auto poly, bool last) {
-      const uint64_t c2 = pk2(cc, cc), b2 = pk2(-m * cc, -m * cc);
-      uint64_t acc[2] = {0ull, 0ull};
       uint32_t s[2][32];
       tc_ld32(ta, s[0]);
 #pragma unroll
@@ -379,13 +346,20 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         if (q < 1) tc_ld32(ta + 32u, s[1]);
         mask32(s[q], k0 + q * 32);
         if (last) limit32(s[q], k0 + q * 32);
+        float mx = m;
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(s[q][i]), __uint_as_float(s[q][i + 1])));
+        const float nmc = mx == ninf ? 0.f : -mx * cc;      // (no key so far: every term is 2^-inf)
+        const uint64_t c2 = pk2(cc, cc), b2 = pk2(nmc, nmc);
+        uint64_t acc[2] = {0ull, 0ull};
 #pragma unroll
         for (int i = 0; i < 16; ++i)
           acc[i & 1] = add2(acc[i & 1], ex2_pair<decltype(poly)::value>(fma2(pk2(__uint_as_float(s[q][2 * i]), __uint_as_float(s[q][2 * i + 1])), c2, b2), i));
+        float e0, e1;
+        upk2(add2(acc[0], acc[1]), e0, e1);
+        l = __fmaf_rn(l, ex2f(__fmaf_rn(m, cc, nmc)), e0 + e1);
+        m = mx;
       }
-      float e0, e1;
-      upk2(add2(acc[0], acc[1]), e0, e1);
-      return e0 + e1;
     };
     for (int j = 0; ok && j < nb; ++j) {
       const int bf = j & 1, k0 = j * 128 + half * 64;
@@ -394,13 +368,8 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       if (bf) ph1 ^= 1u; else ph0 ^= 1u;
       tc_fence_after();
       const uint32_t ta = bf ? to0 : ts0;
-      if (j == 0 || (MASK && !__all_sync(0xffffffffu, m > ninf))) half_with_max(ta, k0, j == nb - 1);
-      else {
-        // (the polynomial does not return 0 for the -inf of a masked key)
-        const float e = j == nb - 1 ? sum_half(ta, k0, FlashFalse{}, true) : (MASK ? sum_half(ta, k0, FlashFalse{}, false) : sum_half(ta, k0, FlashTrue{}, false));
-        if (__any_sync(0xffffffffu, !(e < 1.0995e12f))) half_with_max(ta, k0, j == nb - 1);
-        else l += e;
-      }
+      // (the polynomial does not return 0 for the -inf of a masked key)
+      if (MASK || j == nb - 1) sum_half(ta, k0, FlashFalse{}, j == nb - 1); else sum_half(ta, k0, FlashTrue{}, false);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(s_free(t, bf));
