@@ -1,5 +1,7 @@
-"""Attention with the values that break a softmax: scores far above the others.  The few-query kernel (up to 16 rows), the prompt kernel
-and the three-step form (scores, softmax and product one after the other) have to agree with the oracle."""
+"""Attention with the values that break a softmax: one key whose score towers over the others, infinities
+and NaN.  The few-query kernel (up to 16 rows), the prompt kernel and the
+three-step form (scores, softmax and product one after the other) have to agree with the oracle, and with each other where the
+oracle is not defined."""
 import numpy as np
 import pytest
 
@@ -43,3 +45,36 @@ def test_one_dominating_key_causal(capi, oracle):
     st, out = run(capi, q, k, v, scale=1.0, causal=True)
     assert st == capi.SUCCESS, capi.last_error()
     close(oracle, out, oracle.sdpa(q, k, v, scale=1.0, causal=True), v, "causal")
+
+
+@pytest.mark.parametrize("S", [7, 150])
+@pytest.mark.parametrize("what", ["nan key", "inf key", "nan query", "inf query", "nan mask", "inf mask"])
+def test_non_finite_scores(capi, oracle, monkeypatch, S, what):
+    """A NaN or an infinite score reaches its row as it does in the three-step form, wherever the key lies."""
+    rng = np.random.default_rng(S)
+    B, H, KV, D = 40, 1, 384, 64
+    q, k, v = make(oracle, rng, B, H, S, KV, D)
+    mask = None
+    bad = {"nan": 0x7FC0, "inf": 0x7F80}[what[:3]]
+    keys = [(b if b < 32 else 16 * (b - 32)) + (0, 128, 256)[b % 3] for b in range(B)]
+    if what.endswith("key"):
+        for b in range(B):
+            k[b, 0, keys[b], 5] = bad
+    elif what.endswith("query"):
+        q[:, 0, S // 2, 5] = bad
+        q[1:4, 0, S // 2, :] = bad
+    else:
+        mask = np.zeros((B, 1, S, KV), dtype=np.float32)
+        for b in range(B):
+            mask[b, 0, :, keys[b]] = np.nan if what[:3] == "nan" else np.inf
+        mask[5, 0, 2] = np.nan
+    got = {}
+    for fused in ("0", "1"):
+        monkeypatch.setenv("B200DNN_SDPA_FUSED", fused)
+        st, out = run(capi, q, k, v, mask=mask)
+        assert st == capi.SUCCESS, capi.last_error()
+        got[fused] = oracle.bf16_to_f32(out)
+    a, b = got["0"], got["1"]
+    assert (np.isnan(a) == np.isnan(b)).all(), (what, int(np.isnan(a).sum()), int(np.isnan(b).sum()))
+    ok = ~np.isnan(a)
+    assert (np.abs(a - b)[ok] <= 2.0 ** -7 * np.abs(a[ok]) + 1e-3 * np.abs(oracle.bf16_to_f32(v)).max()).all()

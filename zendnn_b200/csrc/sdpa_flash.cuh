@@ -37,8 +37,6 @@ struct SdpaFlashArgs {
 constexpr int kFlashSoftmaxWarps = 16;  // two 128-row tiles x two halves of a key block x four lane quadrants
 constexpr int kFlashThreads = 32 * (kFlashSoftmaxWarps + 2);
 constexpr int kFlashSlots = 4;          // K / V ring
-struct FlashTrue { static constexpr bool value = true; };
-struct FlashFalse { static constexpr bool value = false; };
 
 __device__ __forceinline__ float ex2f(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ uint64_t pk2(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
@@ -46,34 +44,7 @@ __device__ __forceinline__ void upk2(uint64_t r, float &lo, float &hi) { asm("mo
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 
-// 2^x for two arguments on the FMA pipe, to share the exponentials between the two pipes: x = n + f with n the nearest integer
-// (added and removed as 1.5 * 2^23), 2^f by a degree-5 polynomial in Horner form, n added to the exponent field.  The
-// coefficients are the minimax fit in relative error of 2^f on [-1/2, 1/2] (Remez exchange in double, rounded to f32):
-// 2.1e-7 in f32 arithmetic, as ex2.approx.  Arguments are clamped at -126 (there 2^x is 1e-38 where ex2.approx gives 0) and must be
-// less than 128 (n is added to the exponent field as it is): both sweeps pass arguments of at most about 0.
-__device__ __forceinline__ uint64_t ex2_poly2(uint64_t x2) {
-  float x0, x1;
-  upk2(x2, x0, x1);
-  x2 = pk2(fmaxf(x0, -126.0f), fmaxf(x1, -126.0f));
-  const uint64_t magic = pk2(12582912.0f, 12582912.0f), nmagic = pk2(-12582912.0f, -12582912.0f), neg1 = pk2(-1.0f, -1.0f);
-  const uint64_t t2 = add2(x2, magic);
-  const uint64_t f2 = fma2(add2(t2, nmagic), neg1, x2);
-  uint64_t r = fma2(f2, pk2(0.0013276472454890609f, 0.0013276472454890609f), pk2(0.009675540961325169f, 0.009675540961325169f));
-  r = fma2(r, f2, pk2(0.05550713092088699f, 0.05550713092088699f));
-  r = fma2(r, f2, pk2(0.24022120237350464f, 0.24022120237350464f));
-  r = fma2(r, f2, pk2(0.6931469440460205f, 0.6931469440460205f));
-  r = fma2(r, f2, pk2(1.0000001192092896f, 1.0000001192092896f));
-  float t0, t1, r0, r1;
-  upk2(t2, t0, t1); upk2(r, r0, r1);
-  return pk2(__uint_as_float(__float_as_uint(r0) + (__float_as_uint(t0) << 23)), __uint_as_float(__float_as_uint(r1) + (__float_as_uint(t1) << 23)));
-}
-// pairs of a 32-score chunk (of 16) that take the polynomial
-#ifndef B200_FLASH_POLY
-#define B200_FLASH_POLY 4
-#endif
-template <bool POLY>
-__device__ __forceinline__ uint64_t ex2_pair(uint64_t x2, int i) {
-  if (POLY && (i * B200_FLASH_POLY) % 16 < B200_FLASH_POLY) return ex2_poly2(x2);
+__device__ __forceinline__ uint64_t ex2_pair(uint64_t x2) {
   float x0, x1;
   upk2(x2, x0, x1);
   return pk2(ex2f(x0), ex2f(x1));
@@ -327,17 +298,18 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         }
       }
     };
+    int n_vis = n_keys;
     auto limit32 = [&](uint32_t (&s)[32], int j0) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) if (j0 + i >= n_keys) s[i] = __float_as_uint(ninf);
+      for (int i = 0; i < 32; ++i) if (j0 + i >= n_vis) s[i] = __float_as_uint(ninf);
     };
     float m = ninf, l = 0.f;
     bool ok = true;
     uint32_t ph0 = 0, ph1 = 0;
     const float cc = MASK ? 1.0f : c;
     // ---- sweep 1: row maximum and row sum of this half, 32 scores at a time; the sum is kept relative to the largest score so far,
-    // so no term exceeds 1 (ex2_poly2 is only good up to there) and a single score far above all others is met wherever it lies
-    auto sum_half = [&](uint32_t ta, int k0, auto poly, bool last) {
+    // so a single score far above all others is met wherever it lies.  (fmaxf passes over a NaN; the sum does not)
+    auto sum_half = [&](uint32_t ta, int k0, bool last) {
       uint32_t s[2][32];
       tc_ld32(ta, s[0]);
 #pragma unroll
@@ -354,7 +326,7 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         uint64_t acc[2] = {0ull, 0ull};
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          acc[i & 1] = add2(acc[i & 1], ex2_pair<decltype(poly)::value>(fma2(pk2(__uint_as_float(s[q][2 * i]), __uint_as_float(s[q][2 * i + 1])), c2, b2), i));
+          acc[i & 1] = add2(acc[i & 1], ex2_pair(fma2(pk2(__uint_as_float(s[q][2 * i]), __uint_as_float(s[q][2 * i + 1])), c2, b2)));
         float e0, e1;
         upk2(add2(acc[0], acc[1]), e0, e1);
         l = __fmaf_rn(l, ex2f(__fmaf_rn(m, cc, nmc)), e0 + e1);
@@ -368,8 +340,7 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       if (bf) ph1 ^= 1u; else ph0 ^= 1u;
       tc_fence_after();
       const uint32_t ta = bf ? to0 : ts0;
-      // (the polynomial does not return 0 for the -inf of a masked key)
-      if (MASK || j == nb - 1) sum_half(ta, k0, FlashFalse{}, j == nb - 1); else sum_half(ta, k0, FlashTrue{}, false);
+      if (j == nb - 1) sum_half(ta, k0, true); else sum_half(ta, k0, false);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(s_free(t, bf));
@@ -383,10 +354,14 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       l = l * ex2f(__fmaf_rn(m, cc, nmc)) + o.y * ex2f(__fmaf_rn(o.x, cc, nmc));
       m = mn;
     }
-    // ---- sweep 2: p = 2^(s * c - m * c - log2 l); a row that sees no key gives zeros
-    const float bias = l > 0.f ? -m * cc - __log2f(l) : ninf;
+    // ---- sweep 2: p = 2^(s * c - m * c - log2 l).  A row without a score above -inf gives zeros (all its scores count as masked); a NaN
+    // in the sum makes the whole row NaN
+    const bool dead = m == ninf;
+    if (dead) n_vis = 0;
+    const bool any_dead = __any_sync(0xffffffffu, dead) != 0;
+    const float bias = dead ? ninf : -m * cc - __log2f(l);
     const uint64_t pc2 = pk2(cc, cc), pb2 = pk2(bias, bias);
-    auto p_half = [&](int k0, auto poly, bool last) {
+    auto p_half = [&](int k0, bool last) {
       uint32_t s[2][32];
       tc_ld32(ts0, s[0]);
 #pragma unroll
@@ -399,7 +374,7 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           float x0, x1;
-          upk2(ex2_pair<decltype(poly)::value>(fma2(pk2(__uint_as_float(s[q][2 * i]), __uint_as_float(s[q][2 * i + 1])), pc2, pb2), i), x0, x1);
+          upk2(ex2_pair(fma2(pk2(__uint_as_float(s[q][2 * i]), __uint_as_float(s[q][2 * i + 1])), pc2, pb2)), x0, x1);
           p[i] = pack_bf16x2(x0, x1);
         }
         tc_st16(ts0 + (uint32_t)q * 16u, p);      // (over scores of this half that have been read)
@@ -414,7 +389,7 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       if (!ok) break;
       ph0 ^= 1u;
       tc_fence_after();
-      if (MASK || j == nb - 1) p_half(j * 128 + half * 64, FlashFalse{}, j == nb - 1); else p_half(j * 128 + half * 64, FlashTrue{}, false);
+      if (j == nb - 1 || any_dead) p_half(j * 128 + half * 64, true); else p_half(j * 128 + half * 64, false);
     }
     if (ok && nb > 0) ok = __all_sync(0xffffffffu, mbar_wait(o_done(t), 0));
     if (ok && nb > 0) {
@@ -617,7 +592,7 @@ sdpa_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
   if (tid < 16) {
     float v = cmax[tid];
     for (uint32_t r = 0; r < csize; ++r) if (r != crank) v = fmaxf(v, ld_cluster_f32(cluster_map(smem_u32(&cmax[tid]), r)));
-    row_m[tid] = v == ninf ? 0.f : v;
+    row_m[tid] = v;
   }
   __syncthreads();
   const int nk = nblk * 128;                               // (scores of keys past the end are -inf)
@@ -630,7 +605,7 @@ sdpa_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
       float *sr = sc + (size_t)row * a.sc_stride;
       for (int j = ((warp % parts) * 32 + lane) * 2; j < nk; j += 64 * parts) {
         float2 x = *reinterpret_cast<float2 *>(sr + j);
-        x.x = ex2f(x.x - m); x.y = ex2f(x.y - m);
+        x.x = m == ninf ? 0.f : ex2f(x.x - m); x.y = m == ninf ? 0.f : ex2f(x.y - m);      // (no score above -inf: zeros)
         sum += x.x + x.y;
         *reinterpret_cast<float2 *>(sr + j) = x;
       }
