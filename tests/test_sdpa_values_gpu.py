@@ -1,5 +1,5 @@
-"""Attention with the values that break a softmax: one key whose score towers over the others, infinities
-and NaN.  The few-query kernel (up to 16 rows), the prompt kernel and the
+"""Attention with the values that break a softmax: one key whose score towers over the others, masks of the type's lowest finite
+value, masks of any size on every key of a row, infinities and NaN.  The few-query kernel (up to 16 rows), the prompt kernel and the
 three-step form (scores, softmax and product one after the other) have to agree with the oracle, and with each other where the
 oracle is not defined."""
 import numpy as np
@@ -10,6 +10,7 @@ from test_sdpa_gpu import capi, close, make, run  # noqa: F401  (capi: fixture)
 pytestmark = pytest.mark.gpu
 
 GAPS = (60.0, 89.0, 100.0, 150.0, 200.0, 400.0)
+FORMS = {"few queries": (7, "1"), "prompt": (150, "1"), "three steps": (150, "0")}
 
 
 def one_large_key(oracle, rng, B, S, KV, D, keys):
@@ -45,6 +46,30 @@ def test_one_dominating_key_causal(capi, oracle):
     st, out = run(capi, q, k, v, scale=1.0, causal=True)
     assert st == capi.SUCCESS, capi.last_error()
     close(oracle, out, oracle.sdpa(q, k, v, scale=1.0, causal=True), v, "causal")
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("value", ["lowest", -1e9, -1e4, 1e4])
+@pytest.mark.parametrize("causal", [False, True])
+def test_rows_that_carry_one_finite_mask_value(capi, oracle, monkeypatch, form, bf16, value, causal):
+    """Padding is usually written as the lowest finite value.  A row whose keys all carry it is a softmax over what is left of the
+    scores after the addition (equal ones for the lowest value), not a row without keys."""
+    S, fused = FORMS[form]
+    monkeypatch.setenv("B200DNN_SDPA_FUSED", fused)
+    lowest = np.float32(-3.3895313892515355e38) if bf16 else np.finfo(np.float32).min
+    low = lowest if value == "lowest" else np.float32(value)
+    rng = np.random.default_rng(S)
+    B, H, KV, D = 2, 2, 300, 64
+    q, k, v = make(oracle, rng, B, H, S, KV, D)
+    m = np.zeros((B, 1, S, KV), dtype=np.float32)
+    m[0, :, :, :140] = low                              # left padding: under the causal mask the first rows see nothing else
+    m[1, :, S // 2] = low                               # a padding query
+    m[1, :, :, 200:] = low
+    mask = oracle.f32_to_bf16(m) if bf16 else m
+    st, out = run(capi, q, k, v, mask=mask, causal=causal)
+    assert st == capi.SUCCESS, capi.last_error()
+    close(oracle, out, oracle.sdpa(q, k, v, oracle.bf16_to_f32(mask) if bf16 else m, causal=causal), v, (form, bf16, value, causal))
 
 
 @pytest.mark.parametrize("S", [7, 150])

@@ -51,7 +51,7 @@ int32_t launch_sdpa_decode(const SdpaCall &c, cudaStream_t st) {
   a.qb = c.qs[0]; a.qh = c.qs[1]; a.qs = c.qs[2]; a.ob = c.os[0]; a.oh = c.os[1]; a.os = c.os[2];
   a.kb = walks(c.ks[0], c.B); a.kh = walks(c.ks[1], c.H); a.vb = walks(c.vs[0], c.B); a.vh = walks(c.vs[1], c.H);
   a.S = (int)c.S; a.KV = (int)c.KV; a.D = (int)c.D; a.H = (int)c.H;
-  a.scale_log2 = c.scale * 1.44269504088896340736f; a.causal = c.causal;
+  a.scale = c.scale; a.causal = c.causal;
   a.mask = SdpaMask{c.mask, c.mask_dt, c.mb, c.mh, c.mi};
   a.status = rt().status;
   const int64_t heads = c.B * c.H;
@@ -99,7 +99,7 @@ int32_t launch_sdpa_flash(const SdpaCall &c, cudaStream_t st) {
   // Longest query tiles of all heads first (under a causal mask their lengths differ by the sequence length) while every head's K
   // and V stay in the L2 together; head after head otherwise.
   a.bh_major = !c.causal || 4 * heads * c.KV * c.D > (64ll << 20);
-  a.scale_log2 = c.scale * 1.44269504088896340736f; a.causal = c.causal;
+  a.scale = c.scale; a.causal = c.causal;
   a.mask = SdpaMask{c.mask, c.mask_dt, c.mb, c.mh, c.mi};
   const int64_t mstep = c.mask_dt == B200DNN_F32 ? 4 : 8;
   a.mask_vec = (reinterpret_cast<uintptr_t>(c.mask) & 15) == 0 && c.mb % mstep == 0 && c.mh % mstep == 0 && c.mi % mstep == 0;

@@ -24,7 +24,7 @@ struct SdpaFlashArgs {
   int n_qt;                 // query tiles of tiles * 128 rows
   int tiles;                // 128-row tiles per CTA: 1 or 2
   int bh_major;             // work order: all query tiles of a head first, else all heads of the longest query tile first
-  float scale_log2;         // scale * log2(e), > 0
+  float scale;              // > 0
   int causal;
   SdpaMask mask; int mask_vec;   // mask_vec: every mask row starts on a 16-byte boundary
   int kb, kh, vb, vh;       // 0 where K / V are broadcast over the batch / the heads (stride 0), else 1
@@ -42,6 +42,7 @@ __device__ __forceinline__ float ex2f(float x) { float r; asm("ex2.approx.ftz.f3
 __device__ __forceinline__ uint64_t pk2(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
 __device__ __forceinline__ void upk2(uint64_t r, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(r)); }
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 
 __device__ __forceinline__ uint64_t ex2_pair(uint64_t x2) {
@@ -259,15 +260,15 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const int row_in_tile = (warp & 3) * 32 + lane, row = q0 + t * 128 + row_in_tile;
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t ts0 = tmem + lane_off + (uint32_t)t * 128u + (uint32_t)half * 64u, to0 = ts0 + 256u;
-    const float ninf = __int_as_float(0xff800000), c = a.scale_log2;
+    const float ninf = __int_as_float(0xff800000), c = a.scale * 1.44269504088896340736f;
     const int n_keys = min(a.KV, a.causal ? row + 1 : a.KV);         // keys this row sees
     const int64_t moff = MASK ? (int64_t)b * a.mask.mb + (int64_t)h * a.mask.mh + (int64_t)min(row, a.S - 1) * a.mask.mi : 0;
-    // a chunk of 32 scores in the log2 domain; with a mask, scale and mask are applied here (vector loads where the mask's rows
-    // allow it: all lanes read the same bytes when the mask does not depend on the query)
+    // a chunk of 32 scores; with a mask, scale and mask are applied here (vector loads where the mask's rows allow it: all lanes read the
+    // same bytes when the mask does not depend on the query).  The mask is added as it is: the type's lowest finite value times log2(e)
+    // would be an infinity, and a row that carries it throughout is a softmax over equal scores, not a row without keys
     auto mask32 = [&](uint32_t (&s)[32], int j0) {
       if constexpr (MASK) {
-        const float log2e = 1.44269504088896340736f;
-        auto put = [&](int i, float mv) { s[i] = __float_as_uint(__fmaf_rn(__uint_as_float(s[i]), c, __fmul_rn(mv, log2e))); };
+        auto put = [&](int i, float mv) { s[i] = __float_as_uint(__fadd_rn(__fmul_rn(__uint_as_float(s[i]), a.scale), mv)); };
         const bool whole = j0 + 32 <= a.KV;
         if (a.mask.dt == DT_F32) {
           const float *mp = reinterpret_cast<const float *>(a.mask.p) + moff + j0;
@@ -306,7 +307,14 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     float m = ninf, l = 0.f;
     bool ok = true;
     uint32_t ph0 = 0, ph1 = 0;
-    const float cc = MASK ? 1.0f : c;
+    // a score's distance from the row maximum m as a power of two: (s - m) * log2(e) with a mask, where m may be as large as the type
+    // goes, and s * c - m * c in one operation without
+    const float log2e = 1.44269504088896340736f, cc = MASK ? 1.0f : c;
+    auto arg = [&](const uint32_t (&s)[32], int i, float nmc) {
+      const uint64_t s2 = pk2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), b2 = pk2(nmc, nmc);
+      if constexpr (MASK) return mul2(add2(s2, b2), pk2(log2e, log2e)); else return fma2(s2, pk2(cc, cc), b2);
+    };
+    auto arg1 = [&](float x, float nmc) { if constexpr (MASK) return (x + nmc) * log2e; else return __fmaf_rn(x, cc, nmc); };
     // ---- sweep 1: row maximum and row sum of this half, 32 scores at a time; the sum is kept relative to the largest score so far,
     // so a single score far above all others is met wherever it lies.  (fmaxf passes over a NaN; the sum does not)
     auto sum_half = [&](uint32_t ta, int k0, bool last) {
@@ -322,14 +330,13 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
         for (int i = 0; i < 32; i += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(s[q][i]), __uint_as_float(s[q][i + 1])));
         const float nmc = mx == ninf ? 0.f : -mx * cc;      // (no key so far: every term is 2^-inf)
-        const uint64_t c2 = pk2(cc, cc), b2 = pk2(nmc, nmc);
         uint64_t acc[2] = {0ull, 0ull};
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          acc[i & 1] = add2(acc[i & 1], ex2_pair(fma2(pk2(__uint_as_float(s[q][2 * i]), __uint_as_float(s[q][2 * i + 1])), c2, b2)));
+          acc[i & 1] = add2(acc[i & 1], ex2_pair(arg(s[q], i, nmc)));
         float e0, e1;
         upk2(add2(acc[0], acc[1]), e0, e1);
-        l = __fmaf_rn(l, ex2f(__fmaf_rn(m, cc, nmc)), e0 + e1);
+        l = __fmaf_rn(l, ex2f(arg1(m, nmc)), e0 + e1);
         m = mx;
       }
     };
@@ -351,16 +358,15 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     {
       const float2 o = stats[t][half ^ 1][row_in_tile];
       const float mn = fmaxf(m, o.x), nmc = mn == ninf ? 0.f : -mn * cc;
-      l = l * ex2f(__fmaf_rn(m, cc, nmc)) + o.y * ex2f(__fmaf_rn(o.x, cc, nmc));
+      l = l * ex2f(arg1(m, nmc)) + o.y * ex2f(arg1(o.x, nmc));
       m = mn;
     }
-    // ---- sweep 2: p = 2^(s * c - m * c - log2 l).  A row without a score above -inf gives zeros (all its scores count as masked); a NaN
+    // ---- sweep 2: p = 2^(distance - log2 l).  A row without a score above -inf gives zeros (all its scores count as masked); a NaN
     // in the sum makes the whole row NaN
     const bool dead = m == ninf;
     if (dead) n_vis = 0;
     const bool any_dead = __any_sync(0xffffffffu, dead) != 0;
-    const float bias = dead ? ninf : -m * cc - __log2f(l);
-    const uint64_t pc2 = pk2(cc, cc), pb2 = pk2(bias, bias);
+    const float nll = dead ? ninf : -__log2f(l), nmc = dead ? 0.f : -m * cc;
     auto p_half = [&](int k0, bool last) {
       uint32_t s[2][32];
       tc_ld32(ts0, s[0]);
@@ -374,7 +380,7 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           float x0, x1;
-          upk2(ex2_pair(fma2(pk2(__uint_as_float(s[q][2 * i]), __uint_as_float(s[q][2 * i + 1])), pc2, pb2)), x0, x1);
+          upk2(ex2_pair(add2(arg(s[q], i, nmc), pk2(nll, nll))), x0, x1);
           p[i] = pack_bf16x2(x0, x1);
         }
         tc_st16(ts0 + (uint32_t)q * 16u, p);      // (over scores of this half that have been read)
@@ -439,7 +445,7 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 //   1. scores: warp w takes keys 16 w .. 16 w + 15 of a block with mma.m16n8k16 (A: the query rows, in registers for the whole
 //      call; B: eight keys).  K rows sit in 64-byte pieces ([128 keys][32 elements], no swizzle): a lane's fragment of key g is the
 //      16 bytes at 8 t of a piece, the same assignment of d to fragment positions on both operands, so a quarter warp reads
-//      128 contiguous bytes.  f32 scores (log2 domain, mask applied) stay in shared memory.
+//      128 contiguous bytes.  f32 scores (scaled, mask applied) stay in shared memory.
 //   2. final row maximum and row sum over the cluster through distributed shared memory, p = bf16(e / sum).
 //   3. p V: keys are the k dimension; V sits in 128-byte swizzled rows, a lane reads 16 bytes (8 columns) of four key rows (a
 //      quarter warp: eight different bank groups) and pairs them with byte permutes.  Up to eight query rows: V^T p^T, columns
@@ -452,7 +458,7 @@ struct SdpaDecodeArgs {
   int S, KV, D, H;
   int chunk;               // keys per CTA, a multiple of 128
   int sc_stride;           // f32 per score row in shared memory
-  float scale_log2;
+  float scale;
   int causal;
   SdpaMask mask;
   int32_t *status;
@@ -566,9 +572,9 @@ sdpa_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
               const int j = k0 + key + e;
-              float mv = 0.f;
-              if (a.mask.p && j < k1) mv = __fmul_rn(load_as_f32(a.mask.p, a.mask.dt, moff + (int64_t)row * a.mask.mi + j), 1.44269504088896340736f);
-              x[e] = (j < k1 && !(a.causal && j > row)) ? __fmaf_rn(acc[2 * hb + e], a.scale_log2, mv) : ninf;
+              float y = __fmul_rn(acc[2 * hb + e], a.scale);
+              if (a.mask.p && j < k1) y = __fadd_rn(y, load_as_f32(a.mask.p, a.mask.dt, moff + (int64_t)row * a.mask.mi + j));
+              x[e] = (j < k1 && !(a.causal && j > row)) ? y : ninf;
             }
             *reinterpret_cast<float2 *>(sc + (size_t)row * a.sc_stride + key) = make_float2(x[0], x[1]);
             if (hb) m_hi = fmaxf(m_hi, fmaxf(x[0], x[1])); else m_lo = fmaxf(m_lo, fmaxf(x[0], x[1]));
@@ -605,7 +611,7 @@ sdpa_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
       float *sr = sc + (size_t)row * a.sc_stride;
       for (int j = ((warp % parts) * 32 + lane) * 2; j < nk; j += 64 * parts) {
         float2 x = *reinterpret_cast<float2 *>(sr + j);
-        x.x = m == ninf ? 0.f : ex2f(x.x - m); x.y = m == ninf ? 0.f : ex2f(x.y - m);      // (no score above -inf: zeros)
+        x.x = m == ninf ? 0.f : ex2f((x.x - m) * 1.44269504088896340736f); x.y = m == ninf ? 0.f : ex2f((x.y - m) * 1.44269504088896340736f);      // (no score above -inf: zeros)
         sum += x.x + x.y;
         *reinterpret_cast<float2 *>(sr + j) = x;
       }
