@@ -103,3 +103,21 @@ def test_non_finite_scores(capi, oracle, monkeypatch, S, what):
     assert (np.isnan(a) == np.isnan(b)).all(), (what, int(np.isnan(a).sum()), int(np.isnan(b).sum()))
     ok = ~np.isnan(a)
     assert (np.abs(a - b)[ok] <= 2.0 ** -7 * np.abs(a[ok]) + 1e-3 * np.abs(oracle.bf16_to_f32(v)).max()).all()
+
+
+@pytest.mark.parametrize("S", [7, 150])
+@pytest.mark.parametrize("base", [2.0 ** 10, 2.0 ** 16, -2.0 ** 16])
+def test_scores_with_a_large_common_part(capi, oracle, S, base):
+    """Scores of one size far from 0: what counts is their distance from the row maximum, which f32 holds exactly here (the products of
+    the common part are powers of two, the rest small integers over 16), so probabilities keep their precision at any size."""
+    rng = np.random.default_rng(S)
+    B, H, KV, D = 1, 2, 300, 64
+    q, k = np.zeros((B, H, S, D), np.float32), np.zeros((B, H, KV, D), np.float32)
+    q[..., 0], k[..., 0] = 2.0 ** 5, base / 2.0 ** 5
+    q[..., 1:5] = rng.integers(-8, 9, (B, H, S, 4)) / 4.0
+    k[..., 1:5] = rng.integers(-8, 9, (B, H, KV, 4)) / 4.0
+    v = rng.standard_normal((B, H, KV, D)).astype(np.float32)
+    q, k, v = (oracle.f32_to_bf16(a) for a in (q, k, v))
+    st, out = run(capi, q, k, v, scale=1.0)
+    assert st == capi.SUCCESS, capi.last_error()
+    close(oracle, out, oracle.sdpa(q, k, v, scale=1.0), v, (S, base))

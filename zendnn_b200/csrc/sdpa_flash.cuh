@@ -7,8 +7,12 @@
 // round unnormalised probabilities instead and give other results; so the prompt kernel sweeps the keys twice: the first
 // sweep takes row maximum and row sum, the second recomputes the scores and multiplies the normalised probabilities with V.
 // The extra Q K^T costs half as much again on the tensor pipe and saves every rescale of the accumulator.
-// The exponential is ex2.approx on an argument with log2(e) folded into the scale (and -log2 of the row sum into the bias):
-// its error, below 1e-6 of a probability, is far under the bf16 rounding that follows.
+// Score, mask, distance from the row maximum and quotient by the row sum are formed in natural units with the operations of the
+// three-step form (the distance with one rounding less).  Error of the f32 probabilities against double, mean / mean weighted by the
+// probability / largest, for 2048 keys with scores of spread 1, 4 and 10 at scale 2^-3.5 (head_dim 128), in units of 1e-7:
+//   three-step form   0.94 / 0.79 / 5.3    3.5 / 1.9 / 24    9.4 / 2.4 / 62
+//   here              0.91 / 0.76 / 4.8    3.1 / 0.80 / 17   7.5 / 0.65 / 40
+// and 1.2 / 1.0 / 9 on both sides with a mask of spread 1, 150 / 150 / 330 with one of -1000.
 #pragma once
 #include "common.cuh"
 #include "mbar.cuh"
@@ -45,10 +49,24 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { u
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 
+// exp(-u) of two arguments u >= 0 (infinities included), as 2^(u * -log2 e).  The plain form rounds the product; it serves the row sum, where
+// the roundings of hundreds of terms average out.  The corrected form multiplies by 1 + (exact product - rounded product) * ln 2, with
+// log2 e in two parts, so that what remains is the error of ex2.approx (and of u).
+constexpr float kLog2e = 1.44269504088896340736f, kLog2eLo = (float)(1.44269504088896340736 - (double)kLog2e), kLn2 = 0.693147180559945309417f;
 __device__ __forceinline__ uint64_t ex2_pair(uint64_t x2) {
   float x0, x1;
   upk2(x2, x0, x1);
   return pk2(ex2f(x0), ex2f(x1));
+}
+__device__ __forceinline__ uint64_t exp_neg2_plain(uint64_t u2) { return ex2_pair(mul2(u2, pk2(-kLog2e, -kLog2e))); }
+__device__ __forceinline__ uint64_t exp_neg2(uint64_t u2) {
+  float u0, u1;
+  upk2(u2, u0, u1);
+  u2 = pk2(fminf(u0, 1e4f), fminf(u1, 1e4f));      // (already 0; an infinity would meet itself below)
+  const uint64_t x2 = mul2(u2, pk2(-kLog2e, -kLog2e));
+  const uint64_t r2 = fma2(u2, pk2(kLog2eLo, kLog2eLo), fma2(u2, pk2(kLog2e, kLog2e), x2));      // what rounding the product dropped
+  const uint64_t e2 = ex2_pair(x2);
+  return fma2(mul2(e2, pk2(-kLn2, -kLn2)), r2, e2);
 }
 
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, int w, uint32_t bar) {
@@ -260,7 +278,7 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const int row_in_tile = (warp & 3) * 32 + lane, row = q0 + t * 128 + row_in_tile;
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t ts0 = tmem + lane_off + (uint32_t)t * 128u + (uint32_t)half * 64u, to0 = ts0 + 256u;
-    const float ninf = __int_as_float(0xff800000), c = a.scale * 1.44269504088896340736f;
+    const float ninf = __int_as_float(0xff800000);
     const int n_keys = min(a.KV, a.causal ? row + 1 : a.KV);         // keys this row sees
     const int64_t moff = MASK ? (int64_t)b * a.mask.mb + (int64_t)h * a.mask.mh + (int64_t)min(row, a.S - 1) * a.mask.mi : 0;
     // a chunk of 32 scores; with a mask, scale and mask are applied here (vector loads where the mask's rows allow it: all lanes read the
@@ -268,7 +286,12 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     // would be an infinity, and a row that carries it throughout is a softmax over equal scores, not a row without keys
     auto mask32 = [&](uint32_t (&s)[32], int j0) {
       if constexpr (MASK) {
-        auto put = [&](int i, float mv) { s[i] = __float_as_uint(__fadd_rn(__fmul_rn(__uint_as_float(s[i]), a.scale), mv)); };
+        const uint64_t sc2 = pk2(a.scale, a.scale);
+        auto put = [&](int i, float m0, float m1) {
+          float y0, y1;
+          upk2(add2(mul2(pk2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), sc2), pk2(m0, m1)), y0, y1);
+          s[i] = __float_as_uint(y0); s[i + 1] = __float_as_uint(y1);
+        };
         const bool whole = j0 + 32 <= a.KV;
         if (a.mask.dt == DT_F32) {
           const float *mp = reinterpret_cast<const float *>(a.mask.p) + moff + j0;
@@ -276,11 +299,11 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
             for (int i = 0; i < 32; i += 4) {
               const float4 v = __ldg(reinterpret_cast<const float4 *>(mp + i));
-              put(i, v.x); put(i + 1, v.y); put(i + 2, v.z); put(i + 3, v.w);
+              put(i, v.x, v.y); put(i + 2, v.z, v.w);
             }
           } else {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) put(i, j0 + i < a.KV ? __ldg(mp + i) : 0.f);
+            for (int i = 0; i < 32; i += 2) put(i, j0 + i < a.KV ? __ldg(mp + i) : 0.f, j0 + i + 1 < a.KV ? __ldg(mp + i + 1) : 0.f);
           }
         } else {
           const uint16_t *mp = reinterpret_cast<const uint16_t *>(a.mask.p) + moff + j0;
@@ -290,11 +313,11 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
               const uint4 v = __ldg(reinterpret_cast<const uint4 *>(mp + i));
               const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-              for (int e = 0; e < 4; ++e) { put(i + 2 * e, __uint_as_float(w[e] << 16)); put(i + 2 * e + 1, __uint_as_float(w[e] & 0xffff0000u)); }
+              for (int e = 0; e < 4; ++e) put(i + 2 * e, __uint_as_float(w[e] << 16), __uint_as_float(w[e] & 0xffff0000u));
             }
           } else {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) put(i, j0 + i < a.KV ? bf16_bits_to_f32(__ldg(mp + i)) : 0.f);
+            for (int i = 0; i < 32; i += 2) put(i, j0 + i < a.KV ? bf16_bits_to_f32(__ldg(mp + i)) : 0.f, j0 + i + 1 < a.KV ? bf16_bits_to_f32(__ldg(mp + i + 1)) : 0.f);
           }
         }
       }
@@ -307,14 +330,11 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     float m = ninf, l = 0.f;
     bool ok = true;
     uint32_t ph0 = 0, ph1 = 0;
-    // a score's distance from the row maximum m as a power of two: (s - m) * log2(e) with a mask, where m may be as large as the type
-    // goes, and s * c - m * c in one operation without
-    const float log2e = 1.44269504088896340736f, cc = MASK ? 1.0f : c;
-    auto arg = [&](const uint32_t (&s)[32], int i, float nmc) {
-      const uint64_t s2 = pk2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), b2 = pk2(nmc, nmc);
-      if constexpr (MASK) return mul2(add2(s2, b2), pk2(log2e, log2e)); else return fma2(s2, pk2(cc, cc), b2);
+    // u = m - s * scale, the distance of two scores from the row maximum m (natural units; with a mask the scale is in s already)
+    const float sc = MASK ? 1.0f : a.scale;
+    auto below = [&](const uint32_t (&s)[32], int i, float m_ref) {
+      return fma2(pk2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), pk2(-sc, -sc), pk2(m_ref, m_ref));
     };
-    auto arg1 = [&](float x, float nmc) { if constexpr (MASK) return (x + nmc) * log2e; else return __fmaf_rn(x, cc, nmc); };
     // ---- sweep 1: row maximum and row sum of this half, 32 scores at a time; the sum is kept relative to the largest score so far,
     // so a single score far above all others is met wherever it lies.  (fmaxf passes over a NaN; the sum does not)
     auto sum_half = [&](uint32_t ta, int k0, bool last) {
@@ -326,17 +346,18 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         if (q < 1) tc_ld32(ta + 32u, s[1]);
         mask32(s[q], k0 + q * 32);
         if (last) limit32(s[q], k0 + q * 32);
-        float mx = m;
+        float mx = ninf;
 #pragma unroll
         for (int i = 0; i < 32; i += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(s[q][i]), __uint_as_float(s[q][i + 1])));
-        const float nmc = mx == ninf ? 0.f : -mx * cc;      // (no key so far: every term is 2^-inf)
+        mx = fmaxf(m, __fmul_rn(mx, sc));
+        const float ref = mx == ninf ? 0.f : mx;            // (no key so far: every term is exp(-inf))
         uint64_t acc[2] = {0ull, 0ull};
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          acc[i & 1] = add2(acc[i & 1], ex2_pair(arg(s[q], i, nmc)));
+          acc[i & 1] = add2(acc[i & 1], exp_neg2_plain(below(s[q], i, ref)));
         float e0, e1;
         upk2(add2(acc[0], acc[1]), e0, e1);
-        l = __fmaf_rn(l, ex2f(arg1(m, nmc)), e0 + e1);
+        l = __fmaf_rn(l, expf(m - ref), e0 + e1);
         m = mx;
       }
     };
@@ -357,16 +378,16 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     asm volatile("bar.sync %0, 256;" ::"r"(1 + t) : "memory");
     {
       const float2 o = stats[t][half ^ 1][row_in_tile];
-      const float mn = fmaxf(m, o.x), nmc = mn == ninf ? 0.f : -mn * cc;
-      l = l * ex2f(arg1(m, nmc)) + o.y * ex2f(arg1(o.x, nmc));
+      const float mn = fmaxf(m, o.x), ref = mn == ninf ? 0.f : mn;
+      l = l * expf(m - ref) + o.y * expf(o.x - ref);
       m = mn;
     }
-    // ---- sweep 2: p = 2^(distance - log2 l).  A row without a score above -inf gives zeros (all its scores count as masked); a NaN
+    // ---- sweep 2: p = exp(s - m) / l.  A row without a score above -inf gives zeros (all its scores count as masked); a NaN
     // in the sum makes the whole row NaN
     const bool dead = m == ninf;
     if (dead) n_vis = 0;
     const bool any_dead = __any_sync(0xffffffffu, dead) != 0;
-    const float nll = dead ? ninf : -__log2f(l), nmc = dead ? 0.f : -m * cc;
+    const float inv = dead ? 0.f : __fdiv_rn(1.0f, l), ref = dead ? 0.f : m;
     auto p_half = [&](int k0, bool last) {
       uint32_t s[2][32];
       tc_ld32(ts0, s[0]);
@@ -380,7 +401,7 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           float x0, x1;
-          upk2(ex2_pair(add2(arg(s[q], i, nmc), pk2(nll, nll))), x0, x1);
+          upk2(mul2(exp_neg2(below(s[q], i, ref)), pk2(inv, inv)), x0, x1);
           p[i] = pack_bf16x2(x0, x1);
         }
         tc_st16(ts0 + (uint32_t)q * 16u, p);      // (over scores of this half that have been read)
@@ -611,7 +632,7 @@ sdpa_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
       float *sr = sc + (size_t)row * a.sc_stride;
       for (int j = ((warp % parts) * 32 + lane) * 2; j < nk; j += 64 * parts) {
         float2 x = *reinterpret_cast<float2 *>(sr + j);
-        x.x = m == ninf ? 0.f : ex2f((x.x - m) * 1.44269504088896340736f); x.y = m == ninf ? 0.f : ex2f((x.y - m) * 1.44269504088896340736f);      // (no score above -inf: zeros)
+        x.x = m == ninf ? 0.f : expf(x.x - m); x.y = m == ninf ? 0.f : expf(x.y - m);      // (no score above -inf: zeros)
         sum += x.x + x.y;
         *reinterpret_cast<float2 *>(sr + j) = x;
       }
