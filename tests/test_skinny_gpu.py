@@ -58,3 +58,18 @@ def test_skinny_bf16(capi, oracle, M, K, N, out):
         got = dst.astype(np.float64) if out == "f32" else (dst.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
         assert (np.abs(got - ref) <= tol + (0 if out == "f32" else 2.0 ** -8 * np.abs(ref))).all()
     capi.lib.b200dnn_clear_caches()
+
+
+@pytest.mark.parametrize("kernel", [4, 5, -1])
+def test_other_kernel_numbers_stay_with_the_tile_kernel(capi, oracle, kernel):
+    """force_kernel names the kernels 1 to 3; any other number runs the tcgen05 tile kernel, which refuses rows that the copy engine
+    cannot read."""
+    rng = np.random.default_rng(kernel + 1)
+    for M, K in ((5, 64), (20, 160)):
+        A, W = rng.integers(-128, 128, (M, K), dtype=np.int8), rng.integers(-128, 128, (K, 72), dtype=np.int8)
+        dst = np.zeros((M, 72), dtype=np.int32)
+        capi.check(capi.matmul(capi.make_matmul(M, 72, K, A, W, dst, src_dt=capi.DT["s8"], dst_dt=capi.DT["s32"], weights_const=False, force_kernel=kernel)))
+        assert (dst == A.astype(np.int32) @ W.astype(np.int32)).all()
+    A, dst = rng.integers(-128, 128, (20, 33), dtype=np.int8), np.zeros((20, 72), dtype=np.int32)
+    d = capi.make_matmul(20, 72, 33, A, W, dst, src_dt=capi.DT["s8"], dst_dt=capi.DT["s32"], weights_const=False, force_kernel=kernel)
+    assert capi.matmul(d) == capi.FAILURE and "16-byte aligned" in capi.last_error()

@@ -1197,13 +1197,10 @@ int32_t b200dnn_matmul(const b200dnn_matmul_t *d, void *stream) {
   // 19.5 -> 17.9, but K = N = 4096 7.2 -> 7.6 (its fixed cost is higher); M = 32, N = 11008 17.7 -> 13.5, N = 1024 9.4 -> 6.1; M = 64, K = N =
   // 4096 10.4 -> 10.9 (every CTA reads all activation rows of its share of K).
   const bool skinny = (M > 16 && M <= 48) || (M > 8 && M <= 16 && (long long)K * N >= (24ll << 20));
-  if (d->force_kernel == 0 && tc_ok && skinny) {
+  const bool few_rows = d->force_kernel == 0 && tc_ok && skinny;
+  B2_CHECK(few_rows || which == 1 || which == 3 || tc_ok, B200DNN_FAILURE, "tcgen05 kernel needs a 16-byte aligned source with lda %% 16 == 0");
+  if (few_rows) {
     B2_TRY(launch_skinny(A, lda, a_unsigned, false, M, N, K, pw, epi, M <= 16 && epi.n_po > 0 ? FA_GENERIC : fast_act_code(epi), early, st));
-    which = 4;
-  }
-  B2_CHECK(which != 2 || tc_ok, B200DNN_FAILURE, "tcgen05 kernel needs a 16-byte aligned source with lda %% 16 == 0");
-  if (which == 4) {
-    // launched above
   } else if (which == 1 || which == 3) {
     int32_t rc = B200DNN_UNIMPLEMENTED;
     // decode kernel: 0 tiled only, 1 register-batch form, 2 ring form, 3..5 ring with that many groups per stage;
