@@ -25,24 +25,6 @@ namespace {
 
 cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
-// Tuning and test knobs.  The environment is read once per knob (a lookup walks the whole environment, a microsecond
-// per call on a box with a few hundred variables, and a call asks for several); with B200DNN_ENV_DYNAMIC=1, which the
-// tests set, every call reads it afresh.  name must be a string literal (the cache is keyed by its address).
-int env_int(const char *name, int dflt) {
-  static const bool dynamic = [] { const char *e = getenv("B200DNN_ENV_DYNAMIC"); return e && atoi(e) != 0; }();
-  if (dynamic) { const char *e = getenv(name); return e ? atoi(e) : dflt; }
-  struct Slot { const char *name; bool set; int value; };
-  static Slot slots[64];
-  static int n_slots = 0;
-  static std::mutex mu;
-  std::lock_guard<std::mutex> lk(mu);
-  for (int i = 0; i < n_slots; ++i)
-    if (slots[i].name == name) return slots[i].set ? slots[i].value : dflt;
-  const char *e = getenv(name);
-  if (n_slots < 64) { slots[n_slots].name = name; slots[n_slots].set = e != nullptr; slots[n_slots].value = e ? atoi(e) : 0; ++n_slots; }
-  return e ? atoi(e) : dflt;
-}
-
 // ------------------------------------------------------------------------------------ prepack
 int32_t pack_into(const void *w_dev, int64_t K, int64_t N, int64_t ldb, int transB, int gated, void *dst_dev,
                   cudaStream_t st, PackedWeight *out) {
@@ -152,20 +134,6 @@ int32_t resolve_weight(const void *weight, int wei_format, int64_t K, int64_t N,
   B2_TRY(pack_into(w_dev, K, N, ldb, transB, gated, buf, st, pw));
   if (cache) { pw->owned = buf; B2_TRY(mark_ready(*pw, st)); D.wcache.emplace(key, *pw); }
   pw->fresh = true;
-  return B200DNN_SUCCESS;
-}
-
-// A launch that may overlap the end of the kernel in front of it on the stream (which must have triggered its dependents): only for
-// kernels that touch memory behind griddepcontrol.wait alone.
-template <typename... P, typename... V>
-int32_t launch_pdl(void (*kern)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, bool pdl, V... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = pdl && env_int("B200DNN_PDL", 1) != 0 ? 1 : 0;
-  B2_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
   return B200DNN_SUCCESS;
 }
 

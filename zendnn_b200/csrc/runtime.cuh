@@ -41,6 +41,24 @@ inline int32_t fail(int32_t code, const char *fmt, ...) {
 inline std::atomic<int64_t> &launch_counter() { static std::atomic<int64_t> c{0}; return c; }
 #define B2_LAUNCHED() (++b200::launch_counter())
 
+// Tuning and test knobs.  The environment is read once per knob (a lookup walks the whole environment, a microsecond
+// per call on a box with a few hundred variables, and a call asks for several); with B200DNN_ENV_DYNAMIC=1, which the
+// tests set, every call reads it afresh.  name must be a string literal (the cache is keyed by its address).
+inline int env_int(const char *name, int dflt) {
+  static const bool dynamic = [] { const char *e = getenv("B200DNN_ENV_DYNAMIC"); return e && atoi(e) != 0; }();
+  if (dynamic) { const char *e = getenv(name); return e ? atoi(e) : dflt; }
+  struct Slot { const char *name; bool set; int value; };
+  static Slot slots[64];
+  static int n_slots = 0;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
+  for (int i = 0; i < n_slots; ++i)
+    if (slots[i].name == name) return slots[i].set ? slots[i].value : dflt;
+  const char *e = getenv(name);
+  if (n_slots < 64) { slots[n_slots].name = name; slots[n_slots].set = e != nullptr; slots[n_slots].value = e ? atoi(e) : 0; ++n_slots; }
+  return e ? atoi(e) : dflt;
+}
+
 inline int device_count() {
   static int n = [] { int c = 0; if (cudaGetDeviceCount(&c) != cudaSuccess) { cudaGetLastError(); c = 0; } return c; }();
   return n;
@@ -277,6 +295,33 @@ inline int32_t ensure_max_smem(const void *fn, int bytes = 227 * 1024) {
     have = bytes;
   }
   return B200DNN_SUCCESS;
+}
+
+// A launch that may overlap the end of the kernel in front of it on the stream (which must have triggered its dependents): only for
+// kernels that touch memory behind griddepcontrol.wait alone.  pdl false, or B200DNN_PDL=0: a plain launch.  cluster: CTAs per cluster.
+template <typename... P, typename... V>
+inline int32_t launch_pdl_cluster(void (*kern)(P...), unsigned grid, unsigned threads, size_t smem, unsigned cluster, cudaStream_t st, bool pdl, const V &...args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if (pdl && env_int("B200DNN_PDL", 1) != 0) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  if (cluster > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = cluster; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = 1;
+    ++na;
+  }
+  cfg.attrs = attr; cfg.numAttrs = na;
+  B2_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+  return B200DNN_SUCCESS;
+}
+template <typename... P, typename... V>
+inline int32_t launch_pdl(void (*kern)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, bool pdl, const V &...args) {
+  return launch_pdl_cluster(kern, grid, threads, smem, 1, st, pdl, args...);
 }
 
 // Entered at the top of every C-ABI entry point: finds (or creates) the context of (current device, stream), takes its

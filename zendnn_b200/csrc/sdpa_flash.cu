@@ -24,22 +24,10 @@ int32_t make_map_heads(CUtensorMap *m, const void *base, int64_t D, int64_t rows
 
 int walks(int64_t stride, int64_t n) { return n > 1 && stride != 0 ? 1 : 0; }     // 0: broadcast
 
-template <typename K, typename... Args>
-int32_t launch_pdl(K kern, unsigned grid, unsigned threads, size_t smem, unsigned cluster, cudaStream_t st, const Args &...args) {
+template <typename... P>
+int32_t launch(void (*kern)(P...), unsigned grid, unsigned threads, size_t smem, unsigned cluster, cudaStream_t st, const P &...args) {
   B2_TRY(ensure_max_smem((const void *)kern, (int)smem));
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.numAttrs = 1;
-  if (cluster > 1) {
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
-    cfg.numAttrs = 2;
-  }
-  cfg.attrs = attr;
-  B2_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+  B2_TRY(launch_pdl_cluster(kern, grid, threads, smem, cluster, st, true, args...));
   B2_LAUNCHED();
   return B200DNN_SUCCESS;
 }
@@ -80,11 +68,11 @@ int32_t launch_sdpa_decode(const SdpaCall &c, cudaStream_t st) {
   B2_TRY(make_map_heads(&mv, c.v, c.D, c.KV, a.vh ? c.H : 1, a.vb ? c.B : 1, c.vs[2], c.vs[1], c.vs[0], 64));
   const unsigned grid = (unsigned)(heads * split);
   if (db == 1) {
-    if (c.S <= 8) return launch_pdl(sdpa_decode_kernel<1, false>, grid, kSdpaDecodeThreads, smem, split, st, mk, mv, a);
-    return launch_pdl(sdpa_decode_kernel<1, true>, grid, kSdpaDecodeThreads, smem, split, st, mk, mv, a);
+    if (c.S <= 8) return launch(sdpa_decode_kernel<1, false>, grid, kSdpaDecodeThreads, smem, split, st, mk, mv, a);
+    return launch(sdpa_decode_kernel<1, true>, grid, kSdpaDecodeThreads, smem, split, st, mk, mv, a);
   }
-  if (c.S <= 8) return launch_pdl(sdpa_decode_kernel<2, false>, grid, kSdpaDecodeThreads, smem, split, st, mk, mv, a);
-  return launch_pdl(sdpa_decode_kernel<2, true>, grid, kSdpaDecodeThreads, smem, split, st, mk, mv, a);
+  if (c.S <= 8) return launch(sdpa_decode_kernel<2, false>, grid, kSdpaDecodeThreads, smem, split, st, mk, mv, a);
+  return launch(sdpa_decode_kernel<2, true>, grid, kSdpaDecodeThreads, smem, split, st, mk, mv, a);
 }
 
 int32_t launch_sdpa_flash(const SdpaCall &c, cudaStream_t st) {
@@ -116,11 +104,11 @@ int32_t launch_sdpa_flash(const SdpaCall &c, cudaStream_t st) {
   const size_t smem = (size_t)(a.tiles + kFlashSlots) * db * 16384 + 1024;
   const unsigned grid = (unsigned)(heads * a.n_qt);
   if (db == 1) {
-    if (c.mask) return launch_pdl(sdpa_flash_kernel<1, true>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
-    return launch_pdl(sdpa_flash_kernel<1, false>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
+    if (c.mask) return launch(sdpa_flash_kernel<1, true>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
+    return launch(sdpa_flash_kernel<1, false>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
   }
-  if (c.mask) return launch_pdl(sdpa_flash_kernel<2, true>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
-  return launch_pdl(sdpa_flash_kernel<2, false>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
+  if (c.mask) return launch(sdpa_flash_kernel<2, true>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
+  return launch(sdpa_flash_kernel<2, false>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
 }
 
 }  // namespace
