@@ -46,13 +46,14 @@ def test_skinny_bf16(capi, oracle, M, K, N, out):
     A, W = (oracle.f32_to_bf16(rng.standard_normal(s).astype(np.float32)) for s in ((M, K), (K, N)))
     bias = rng.standard_normal(N).astype(np.float32)
     dst = np.zeros((M, N), dtype=np.float32 if out == "f32" else np.uint16)
-    d = capi.make_matmul(M, N, K, A, W, dst, src_dt=capi.DT["bf16"], wei_dt=capi.DT["bf16"], dst_dt=capi.DT[out], bias=bias, weights_const=True)
+    d = capi.make_matmul(M, N, K, A, W, dst, src_dt=capi.DT["bf16"], wei_dt=capi.DT["bf16"], dst_dt=capi.DT[out], bias=bias, weights_const=True,
+                         flags=capi.FLAG_STABLE_WEIGHTS)
     a, w = ((x.astype(np.uint32) << 16).view(np.float32).astype(np.float64) for x in (A, W))
     ref = a @ w + bias
     # f32 sums of K exact products: each of the K additions rounds by at most 2^-24 of a partial sum (2^-23 where the tensor core cuts
     # instead), and a partial sum is at most sum |a||w|; bf16 rounds the result by 2^-9 of itself on top
     tol = K * 2.0 ** -23 * (np.abs(a) @ np.abs(w) + np.abs(bias))
-    for _ in range(2):                                      # the second call finds the packed weight and reads it early
+    for _ in range(2):                                      # the second call finds the packed weight, complete, and reads it early
         dst[:] = 0
         capi.check(capi.matmul(d))
         got = dst.astype(np.float64) if out == "f32" else (dst.astype(np.uint32) << 16).view(np.float32).astype(np.float64)

@@ -57,22 +57,29 @@ PackedWeight view_of(const void *dev_base, const PackHeader &h) {
   return pw;
 }
 
-// A cache-owned packed weight was written on the stream of the call that first saw it: a call on another stream waits
-// for that work (until it has been seen complete once).  Callers hold the cache mutex.
-int32_t wait_ready(PackedWeight &pw, cudaStream_t st) {
-  if (pw.complete || !pw.ready || st == pw.ready_stream) return B200DNN_SUCCESS;
-  {
-    RelaxedCapture relaxed;      // an event query is not a capturable call: allowed while this thread captures a graph
-    if (cudaEventQuery(pw.ready) == cudaSuccess) { pw.complete = true; return B200DNN_SUCCESS; }
+// A cache-owned packed weight was written on the stream of the call that first saw it: a call on another stream waits for that work.
+// Until the work has been seen complete once the weight is `fresh` for every call: no kernel may read it ahead of its own
+// griddepcontrol.wait.  (The order of the stream is no help there: a kernel that triggers its dependents before its own wait, as the
+// GEMM kernels do, lets them start while the packing in front of it may still be on its way to memory.)  An event recorded during a
+// stream capture cannot be asked, and each replay packs again: such a weight stays fresh.  Callers hold the cache mutex.
+int32_t take_cached(PackedWeight &entry, cudaStream_t st, PackedWeight *pw) {
+  if (!entry.complete && entry.ready) {
+    if (!entry.captured) {
+      RelaxedCapture relaxed;      // an event query is not a capturable call: allowed while this thread captures a graph
+      if (cudaEventQuery(entry.ready) == cudaSuccess) entry.complete = true; else cudaGetLastError();
+    }
+    if (!entry.complete && st != entry.ready_stream) B2_CUDA(cudaStreamWaitEvent(st, entry.ready, 0));
   }
-  cudaGetLastError();
-  B2_CUDA(cudaStreamWaitEvent(st, pw.ready, 0));
+  *pw = entry;
+  pw->fresh = !entry.complete;
   return B200DNN_SUCCESS;
 }
 int32_t mark_ready(PackedWeight &pw, cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
   B2_CUDA(cudaEventCreateWithFlags(&pw.ready, cudaEventDisableTiming));
   B2_CUDA(cudaEventRecord(pw.ready, st));
-  pw.ready_stream = st; pw.complete = false;
+  pw.ready_stream = st; pw.complete = false; pw.captured = cap != cudaStreamCaptureStatusNone;
   return B200DNN_SUCCESS;
 }
 
@@ -95,8 +102,7 @@ int32_t resolve_weight(const void *weight, int wei_format, int64_t K, int64_t N,
       *pw = it->second;
     } else {
       auto it = D.host_packed.find(weight);
-      const bool uploaded = it == D.host_packed.end();
-      if (uploaded) {
+      if (it == D.host_packed.end()) {
         PackHeader h; memcpy(&h, weight, sizeof h);
         B2_CHECK(h.magic == kPackMagic, B200DNN_FAILURE, "mem_format_b='r' but the weight buffer was not written by b200dnn_prepack");
         size_t bytes = pack_bytes(h.K, h.N);
@@ -107,9 +113,7 @@ int32_t resolve_weight(const void *weight, int wei_format, int64_t K, int64_t N,
         B2_TRY(mark_ready(v, st));
         it = D.host_packed.emplace(weight, v).first;
       }
-      B2_TRY(wait_ready(it->second, st));
-      *pw = it->second;
-      pw->fresh = uploaded;
+      B2_TRY(take_cached(it->second, st, pw));
     }
     B2_CHECK(pw->K == K && pw->N == N && pw->gated == gated, B200DNN_FAILURE,
              "prepacked weight is K=%lld N=%lld gated=%d, call asks for K=%lld N=%lld gated=%d", (long long)pw->K,
@@ -123,7 +127,7 @@ int32_t resolve_weight(const void *weight, int wei_format, int64_t K, int64_t N,
   if (cache) {
     lk.lock();
     auto it = D.wcache.find(key);
-    if (it != D.wcache.end()) { B2_TRY(wait_ready(it->second, st)); *pw = it->second; return B200DNN_SUCCESS; }
+    if (it != D.wcache.end()) return take_cached(it->second, st, pw);
   }
   const int64_t wrows = transB ? N : K, wcols = transB ? K : N;
   const void *w_dev = nullptr;
@@ -643,9 +647,7 @@ int32_t launch_skinny(const uint8_t *A, int64_t lda, bool a_unsigned, bool f16, 
   cfg.gridDim = dim3((unsigned)(tiles * best)); cfg.blockDim = dim3(kSkinnyThreads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr[2];
   int na = 0;
-  // (a weight packed in this very call: a plain launch, so that the early reads of a LATER call, which follow this kernel's start, follow
-  // the end of the packing as well)
-  if (!pw.fresh && env_int("B200DNN_PDL", 1) != 0) {
+  if (env_int("B200DNN_PDL", 1) != 0) {
     attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
@@ -1159,7 +1161,7 @@ int32_t b200dnn_matmul(const b200dnn_matmul_t *d, void *stream) {
   int which = d->force_kernel;
   if (which == 0) which = (M <= 16 || !tc_ok) ? 1 : 2;
   // the weight may be read before the kernel in front has finished: that kernel is this call's quantisation, which itself waited for
-  // everything before it, or the caller says that its weights are in place (and they were not packed or uploaded in this call)
+  // everything before it, or the caller says that its weights are in place (and the library's own copy of them is: see take_cached)
   const bool early = !pw.fresh && (dyn || (d->flags & B200DNN_FLAG_STABLE_WEIGHTS) != 0);
   // Few rows on the tensor cores (skinny_gemm.cuh), us: M = 16, K = 4096, N = 11008 12.7 -> 12.0, K = 11008, N = 4096 with quantisation
   // 19.5 -> 17.9, but K = N = 4096 7.2 -> 7.6 (its fixed cost is higher); M = 32, N = 11008 17.7 -> 13.5, N = 1024 9.4 -> 6.1; M = 64, K = N =

@@ -29,7 +29,7 @@ int32_t resolve_bf16_weight(const void *weight, int64_t K, int64_t N, int64_t ld
   if (cache) {
     lk.lock();
     auto it = D.wcache.find(key);
-    if (it != D.wcache.end()) { B2_TRY(wait_ready(it->second, st)); *pw = it->second; return B200DNN_SUCCESS; }
+    if (it != D.wcache.end()) return take_cached(it->second, st, pw);
   }
   const int64_t I = gated ? N / 2 : 0;
   if (gated) B2_CHECK(N % 2 == 0 && I % kGateGranule == 0, B200DNN_UNIMPLEMENTED,

@@ -90,7 +90,7 @@ int32_t resolve_gs_weight(const b200dnn_matmul_t *d, bool w4, int64_t Kp, cudaSt
   if (cache) {
     lk.lock();
     auto it = D.wcache.find(key);
-    if (it != D.wcache.end()) { B2_TRY(wait_ready(it->second, st)); *pw = it->second; return B200DNN_SUCCESS; }
+    if (it != D.wcache.end()) return take_cached(it->second, st, pw);
   }
   const int64_t wrows = d->transB ? N : K, wcols = d->transB ? K : N;
   const size_t src_bytes = w4 ? (size_t)(((wrows - 1) * d->ldb + wcols + 1) / 2) : span_bytes(wrows, wcols, d->ldb, B200DNN_S8);
@@ -108,6 +108,7 @@ int32_t resolve_gs_weight(const b200dnn_matmul_t *d, bool w4, int64_t Kp, cudaSt
   *pw = PackedWeight{};
   pw->wt = (const int8_t *)buf; pw->K = K; pw->N = N; pw->Kp = Kp; pw->Np = N; pw->gated = w4 ? kGsLayoutS4 : kGsLayoutS8;
   if (cache) { pw->owned = buf; B2_TRY(mark_ready(*pw, st)); D.wcache.emplace(key, *pw); }
+  pw->fresh = true;
   return B200DNN_SUCCESS;
 }
 

@@ -112,8 +112,8 @@ struct PackedWeight {
   void *owned = nullptr;   // cache-owned device buffer
   // cache-owned buffers are packed on the stream of the call that first saw the weight; calls on other streams wait
   // for this event until it has been seen complete once
-  cudaEvent_t ready = nullptr; cudaStream_t ready_stream = nullptr; bool complete = true;
-  bool fresh = false;      // written by work that this very call has put on the stream
+  cudaEvent_t ready = nullptr; cudaStream_t ready_stream = nullptr; bool complete = true, captured = false;
+  bool fresh = false;      // of one call's copy: the work that writes the buffer has not been seen complete, so it may not be read early
 };
 
 // Small host inputs of one call (activations of a decode step, scales, zero point, bias, descriptor tables) are

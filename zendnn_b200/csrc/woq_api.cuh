@@ -99,7 +99,7 @@ int32_t resolve_woq_weight(const b200dnn_matmul_t *d, int64_t group, cudaStream_
   if (cache) {
     lk.lock();
     auto it = D.woq_cache.find(key);
-    if (it != D.woq_cache.end()) { B2_TRY(wait_ready(it->second, st)); *pw = it->second; return B200DNN_SUCCESS; }
+    if (it != D.woq_cache.end()) return take_cached(it->second, st, pw);
   }
   const int64_t wrows = d->transB ? N : K, wcols = d->transB ? K : N;
   WoqPackArgs a{};
