@@ -263,6 +263,10 @@ inline int32_t device_shared(DeviceShared **out) {
   int dev = 0;
   B2_CUDA(cudaGetDevice(&dev));
   B2_CHECK(dev >= 0 && dev < 64, B200DNN_FAILURE, "device ordinal %d out of range", dev);
+  // A thread that has not used CUDA yet has no current context, and the tensor-map encoder, a driver call that may be the first of a
+  // call on device buffers, refuses to work without one (the runtime's calls bind it themselves, but not all of them do).
+  static thread_local int bound = -1;
+  if (bound != dev) { B2_CUDA(cudaSetDevice(dev)); bound = dev; }
   std::lock_guard<std::mutex> lk(devices_mu());
   DeviceShared *&slot = device_slot(dev);
   if (!slot) {
