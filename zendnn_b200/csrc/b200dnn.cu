@@ -373,26 +373,30 @@ extern "C" __attribute__((visibility("default"))) int32_t b200dnn_debug_stamps(u
 }
 #endif
 
-// CTAs that are resident at once when the split form is launched in clusters of s (clusters do not tile the GPCs perfectly)
-int split_room(int s) {
-  int *cache = rt().shared->split_room;   // per device; two threads may both compute the same value
-  if (cache[s] == 0) {
-    cache[s] = -1;
-    if (ensure_max_smem((const void *)tc_gemm_kernel<true>, kTcSmemBudget + 1024) == B200DNN_SUCCESS) {
-      cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3((unsigned)(s * 64)); cfg.blockDim = dim3(kTcThreads); cfg.dynamicSmemBytes = kTcSmemBudget + 1024;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = (unsigned)s; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr; cfg.numAttrs = 1;
-      int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, tc_gemm_kernel<true>, &cfg) == cudaSuccess && n > 0) cache[s] = n * s;
-      else cudaGetLastError();
-      if (env_int("B200DNN_DEBUG", 0)) fprintf(stderr, "b200dnn: clusters of %d: %d resident CTAs\n", s, cache[s]);
-    }
+// CTAs of a kernel that are resident at once when it is launched in clusters of s (clusters do not tile the GPCs perfectly); -1: none.
+// Kept per device in *cache (0: not asked yet).  Several threads may ask at once: each stores the answer only when it has it, because a
+// caller that met something else would split K another way, and f32 sums with it.
+template <typename K>
+int cluster_room(K kern, int threads, int smem, int s, std::atomic<int> *cache) {
+  int room = cache->load(std::memory_order_relaxed);
+  if (room != 0) return room;
+  room = -1;
+  if (ensure_max_smem((const void *)kern, smem) == B200DNN_SUCCESS) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(s * 64)); cfg.blockDim = dim3((unsigned)threads); cfg.dynamicSmemBytes = (size_t)smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)s; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0) room = n * s;
+    else cudaGetLastError();
+    if (env_int("B200DNN_DEBUG", 0)) fprintf(stderr, "b200dnn: clusters of %d (%d threads): %d resident CTAs\n", s, threads, room);
   }
-  return cache[s];
+  cache->store(room, std::memory_order_relaxed);
+  return room;
 }
+int split_room(int s) { return cluster_room(tc_gemm_kernel<true>, kTcThreads, kTcSmemBudget + 1024, s, &rt().shared->split_room[s]); }
 
 void pick_split(int m_tiles, int N, int k_blocks, int *bn, int *splits) {
   const int forced = env_int("B200DNN_TC_KSPLIT", 0);   // 0 choose, 1 never, 2..4 that many
@@ -583,27 +587,7 @@ int32_t launch_tc(const uint8_t *A, int64_t lda, bool a_unsigned, int M_total, i
   return B200DNN_SUCCESS;
 }
 
-// CTAs of skinny_gemm_kernel that are resident at once when it is launched in clusters of s
-int skinny_room(int s) {
-  if (s == 1) return rt().sm_count;
-  int *cache = rt().shared->skinny_room;   // per device; two threads may both compute the same value
-  if (cache[s] == 0) {
-    cache[s] = -1;
-    if (ensure_max_smem((const void *)skinny_gemm_kernel<false>, kSkinnyRing + 1024) == B200DNN_SUCCESS) {
-      cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3((unsigned)(s * 64)); cfg.blockDim = dim3(kSkinnyThreads); cfg.dynamicSmemBytes = kSkinnyRing + 1024;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = (unsigned)s; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr; cfg.numAttrs = 1;
-      int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, skinny_gemm_kernel<false>, &cfg) == cudaSuccess && n > 0) cache[s] = n * s;
-      else cudaGetLastError();
-      if (env_int("B200DNN_DEBUG", 0)) fprintf(stderr, "b200dnn: skinny clusters of %d: %d resident CTAs\n", s, cache[s]);
-    }
-  }
-  return cache[s];
-}
+int skinny_room(int s) { return cluster_room(skinny_gemm_kernel<false>, kSkinnyThreads, kSkinnyRing + 1024, s, &rt().shared->skinny_room[s]); }
 
 // Few rows (skinny_gemm.cuh).  A: [M, lda] device bytes, 16-byte aligned rows; K and lda count bytes; early: see SkinnyArgs.
 int32_t launch_skinny(const uint8_t *A, int64_t lda, bool a_unsigned, bool f16, int M, int N, int K, const PackedWeight &pw, const EpiParams &epi,

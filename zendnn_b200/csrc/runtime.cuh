@@ -169,8 +169,7 @@ struct DeviceShared {
   std::map<cudaStream_t, Runtime *> ctxs;
   std::mutex attr_mu;
   std::map<const void *, int> smem_limit;                 // kernels whose dynamic shared-memory limit was raised
-  int split_room[5] = {0, 0, 0, 0, 0};
-  int skinny_room[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  std::atomic<int> split_room[5] = {}, skinny_room[9] = {};   // by cluster size: see cluster_room
 };
 
 // Descriptor tables that depend only on the caller's weight pointers (per-expert epilogue pointers, tensor maps) are
