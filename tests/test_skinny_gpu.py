@@ -74,3 +74,30 @@ def test_other_kernel_numbers_stay_with_the_tile_kernel(capi, oracle, kernel):
     A, dst = rng.integers(-128, 128, (20, 33), dtype=np.int8), np.zeros((20, 72), dtype=np.int32)
     d = capi.make_matmul(20, 72, 33, A, W, dst, src_dt=capi.DT["s8"], dst_dt=capi.DT["s32"], weights_const=False, force_kernel=kernel)
     assert capi.matmul(d) == capi.FAILURE and "16-byte aligned" in capi.last_error()
+
+
+# both sides of the lines that the choice of kernel draws: rows against bytes of a column, one wave of column tiles (148 x 128 columns) and
+# how full the last one is, rows of 16 x K that the decode kernel has no room for
+@pytest.mark.parametrize("M,K,N", [(24, 512, 300), (25, 1008, 300), (25, 1024, 300), (33, 1536, 300), (33, 1520, 300), (48, 1024, 18944), (9, 2048, 18945),
+                                   (17, 3072, 18945), (24, 3072, 37889), (25, 512, 25600), (24, 512, 18945), (16, 14336, 18960), (9, 8192, 18944)])
+def test_lines_of_the_choice_int8(capi, M, K, N):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    A, W = (torch.randint(-128, 128, s, dtype=torch.int8, device="cuda", generator=g) for s in ((M, K), (K, N)))
+    dst = torch.full((M, N), 7, dtype=torch.int32, device="cuda")
+    capi.check(capi.matmul(capi.make_matmul(M, N, K, A, W, dst, src_dt=capi.DT["s8"], dst_dt=capi.DT["s32"], weights_const=False),
+                           torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(dst, (A.double() @ W.double()).int())
+
+
+@pytest.mark.parametrize("M,K,N", [(64, 1024, 300), (64, 1016, 300), (48, 768, 300), (48, 760, 300), (8, 512, 18944), (8, 512, 18945), (8, 512, 25300),
+                                   (9, 1536, 25300), (24, 1536, 25300), (24, 1528, 25300), (25, 1536, 25300)])
+def test_lines_of_the_choice_bf16(capi, M, K, N):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    A, W = (torch.randn(s, device="cuda", generator=g).bfloat16() for s in ((M, K), (K, N)))
+    dst = torch.zeros(M, N, device="cuda")
+    capi.check(capi.matmul(capi.make_matmul(M, N, K, A, W, dst, src_dt=capi.DT["bf16"], wei_dt=capi.DT["bf16"], dst_dt=capi.DT["f32"], weights_const=False),
+                           torch.cuda.current_stream().cuda_stream))
+    a, w = A.double(), W.double()
+    assert ((dst - a @ w).abs() <= K * 2.0 ** -23 * (a.abs() @ w.abs())).all()      # see test_skinny_bf16

@@ -248,6 +248,11 @@ int32_t launch_stream(const uint8_t *A, int64_t lda, bool a_unsigned, int M, int
   return B200DNN_SUCCESS;
 }
 
+// Shared memory of decode_gemm_kernel: staged rows, sums and epilogue operands of the CTA's column groups.
+size_t decode_smem(int M, int N, int64_t Kp) {
+  const int groups = (N + 7) / 8, grid = groups < rt().sm_count ? groups : rt().sm_count, local = (groups + grid - 1) / grid;
+  return (size_t)(M > 8 ? 16 : 8) * (size_t)(Kp + 16) + (size_t)local * 512 + decode_epi_bytes(local);
+}
 // Decode-shape kernel (M <= 16): persistent, evenly split over all warps of the device.
 // Returns unimplemented when the shape does not fit it (the caller then uses the tiled streaming kernel).
 int32_t launch_decode(const uint8_t *A, int64_t lda, bool a_unsigned, int M, int N, int K, const PackedWeight &pw,
@@ -261,7 +266,7 @@ int32_t launch_decode(const uint8_t *A, int64_t lda, bool a_unsigned, int M, int
   const int grid = g.groups < R.sm_count ? g.groups : R.sm_count;
   g.max_local_groups = (g.groups + grid - 1) / grid;
   g.tune = env_int("B200DNN_DECODE_TUNE", 0);
-  const size_t smem = (size_t)g.rows_staged * g.a_stride + (size_t)g.max_local_groups * 512 + decode_epi_bytes(g.max_local_groups);
+  const size_t smem = decode_smem(M, N, pw.Kp);
   if (M > 16 || smem > 220 * 1024) return B200DNN_UNIMPLEMENTED;
   void (*kern)(DecodeGemmArgs, EpiParams) = a_unsigned ? decode_gemm_kernel<true> : decode_gemm_kernel<false>;
   B2_TRY(ensure_max_smem((const void *)kern));
@@ -648,6 +653,21 @@ int32_t launch_skinny(const uint8_t *A, int64_t lda, bool a_unsigned, bool f16, 
   B2_CUDA(cudaLaunchKernelEx(&cfg, kern, map_a, map_w, g, epi));
   B2_LAUNCHED();
   return B200DNN_SUCCESS;
+}
+
+// Does the few-row kernel beat the tile kernel?  col_bytes: bytes of a weight column.  Over 1400 shapes (M 1 to 64, K 512 to 14336, N 512 to
+// 50176, bf16 and INT8) the choice is 0.7 % off the better of the two on average.
+//   - Column tiles for at most one wave of CTAs: always up to 24 rows (bf16, K = 4096, N = 1024, M = 16: 6.6 us against 12.5); with more rows the
+//     fixed cost of handling them (about 0.04 us a row) must be less than what the tile kernel loses by not sharing K (about 0.9 us a KiB
+//     of column): bf16, M = 64, N = 4096: K = 512 7.5 against 6.2, K = 2048 9.6 against 10.2.
+//   - More column tiles than SMs: the kernel is not persistent, so its last wave must be well filled (K = 8192, N = 20480 is 160 tiles: 71
+//     against 60 us for 8 rows; N = 50176 is 392 and K = 4096: 69 against 107), and every tile pays for its rows again (K = 4096, N = 28672:
+//     8 rows 44 against 56, 32 rows 48 against 45).  Columns of at most 512 bytes are one short burst each: 12.9 against 17.1 (N = 50176).
+bool few_rows_pay(int M, int N, int64_t col_bytes) {
+  const long long tiles = (N + 127) / 128, sms = rt().sm_count, waves = (tiles + sms - 1) / sms;
+  if (waves == 1) return M <= 24 || col_bytes >= 32ll * ((M + 15) & ~15);
+  if (M <= 24 && col_bytes <= 512) return true;
+  return 3 * tiles >= 2 * waves * sms && (M <= 8 || (M <= 24 && col_bytes >= 3072));
 }
 
 // the stream has been drained: report a kernel that gave up on one of its bounded waits
@@ -1150,10 +1170,11 @@ int32_t b200dnn_matmul(const b200dnn_matmul_t *d, void *stream) {
   // the weight may be read before the kernel in front has finished: that kernel is this call's quantisation, which itself waited for
   // everything before it, or the caller says that its weights are in place (and the library's own copy of them is: see take_cached)
   const bool early = !pw.fresh && (dyn || (d->flags & B200DNN_FLAG_STABLE_WEIGHTS) != 0);
-  // Few rows on the tensor cores (skinny_gemm.cuh), us: M = 16, K = 4096, N = 11008 12.7 -> 12.0, K = 11008, N = 4096 with quantisation
-  // 19.5 -> 17.9, but K = N = 4096 7.2 -> 7.6 (its fixed cost is higher); M = 32, N = 11008 17.7 -> 13.5, N = 1024 9.4 -> 6.1; M = 64, K = N =
-  // 4096 10.4 -> 10.9 (every CTA reads all activation rows of its share of K).
-  const bool skinny = (M > 16 && M <= 48) || (M > 8 && M <= 16 && (long long)K * N >= (24ll << 20));
+  // Few rows on the tensor cores (skinny_gemm.cuh).  Up to 16 rows against the decode kernel, us: K = 4096, N = 11008 12.7 -> 12.2, K = 14336,
+  // N = 4096 31.0 -> 16.0, but K = N = 4096 7.2 -> 7.6 (its fixed cost is higher), and with more column tiles than SMs K = 4096, N = 50176
+  // 37.3 -> 41.0: there only rows that the decode kernel has no room for.  Above 48 rows the tile kernel (M = 64, K = N = 4096: 10.4 -> 10.9).
+  const bool skinny = M <= 16 ? M > 8 && (long long)K * N >= (24ll << 20) && ((N + 127) / 128 <= rt().sm_count || decode_smem(M, N, pw.Kp) > 220 * 1024)
+                              : M <= 48 && few_rows_pay(M, N, K);
   const bool few_rows = d->force_kernel == 0 && tc_ok && skinny;
   B2_CHECK(few_rows || which == 1 || which == 3 || tc_ok, B200DNN_FAILURE, "tcgen05 kernel needs a 16-byte aligned source with lda %% 16 == 0");
   if (few_rows) {

@@ -127,8 +127,8 @@ int32_t matmul_bf16_packed(const b200dnn_matmul_t *d, const PackedWeight &pw, cu
     B2_CUDA(cudaGetLastError());
     A = (const uint8_t *)tmp; lda = ld2;
   }
-  // few rows (skinny_gemm.cuh), us: K = 4096, N = 11008, M = 8 31.0 -> 19.8, M = 64 24.4 -> 23.9, but M = 96 24.7 -> 27.3
-  if (d->force_kernel == 0 && M <= 64) {
+  // few rows (skinny_gemm.cuh); M = 96, K = 4096, N = 11008: 24.7 us in the tile kernel, 27.3 there
+  if (d->force_kernel == 0 && M <= 64 && few_rows_pay(M, N, 2ll * K)) {
     const bool early = (d->flags & B200DNN_FLAG_STABLE_WEIGHTS) != 0 && !pw.fresh;
     B2_TRY(launch_skinny(A, lda * 2, false, true, M, N, 2 * K, pw, epi, fast_act_code(epi), early, st));
     return finish_out({&o_dst}, st);
