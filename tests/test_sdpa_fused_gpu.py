@@ -73,3 +73,62 @@ def test_keys_and_values_shared_by_all_heads(capi, oracle, S):
     torch.cuda.synchronize()
     rep = lambda x: np.ascontiguousarray(np.repeat(x, H, axis=1))  # noqa: E731
     close(oracle, out.cpu().numpy().view(np.uint16), oracle.sdpa(q, rep(k), rep(v)), v, S)
+
+
+@pytest.mark.parametrize("S", [16, 20])
+@pytest.mark.parametrize("masked", [False, True])
+def test_few_heads_with_many_keys(capi, oracle, S, masked):
+    """One head against 16384 keys: the three-step form where it can take all heads at once, the prompt kernel for another storage order."""
+    rng = np.random.default_rng(S)
+    B, H, KV, D = 1, 2, 16384, 128
+    q, k, v = make(oracle, rng, B, H, S, KV, D)
+    mask = None
+    if masked:
+        mask = np.zeros((1, 1, S, KV), dtype=np.float32)
+        mask[..., KV - 700:] = np.finfo(np.float32).min
+        mask[0, 0, 3] = -np.inf
+    ref = oracle.sdpa(q, k, v, mask)
+    st, out = run(capi, q, k, v, mask=mask)
+    assert st == capi.SUCCESS, capi.last_error()
+    close(oracle, out, ref, v, "one pitch")
+    qs = np.ascontiguousarray(q.transpose(0, 2, 1, 3)).transpose(0, 2, 1, 3)      # [batch, seq, head, dim] storage
+    st, out = run(capi, qs, k, v, mask=mask)
+    assert st == capi.SUCCESS, capi.last_error()
+    close(oracle, out, ref, v, "rows of the heads interleaved")
+
+
+def test_few_heads_with_many_keys_in_a_graph(capi, oracle):
+    """The same call captured and replayed on new inputs, with other calls on the stream in between."""
+    import torch
+    S, KV, D = 20, 16384, 128
+    rng = np.random.default_rng(1)
+    sets = [make(oracle, rng, 1, 1, S, KV, D) for _ in range(3)]
+    dev = [torch.from_numpy(x.view(np.int16)).cuda() for x in sets[0]]
+    out = torch.zeros((1, 1, S, D), dtype=torch.int16, device="cuda")
+
+    def desc(q, k, v, o):
+        d = capi.SdpaDesc()
+        d.batch, d.num_heads, d.seq_len, d.kv_seq_len, d.head_dim = 1, 1, S, KV, D
+        for name, x in (("q_stride", q), ("k_stride", k), ("v_stride", v), ("o_stride", o)):
+            setattr(d, name, (C.c_int64 * 4)(*x.stride()))
+        d.qkv_dt = d.out_dt = capi.DT["bf16"]
+        d.query, d.key, d.value, d.output = (x.data_ptr() for x in (q, k, v, o))
+        return d
+    d = desc(*dev, out)
+    stream = torch.cuda.Stream()
+    other = [torch.from_numpy(x.view(np.int16)).cuda() for x in sets[2]]
+    d_other = desc(*other, torch.zeros_like(out))
+    with torch.cuda.stream(stream):
+        capi.check(capi.lib.b200dnn_sdpa(C.byref(d), stream.cuda_stream))
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            capi.check(capi.lib.b200dnn_sdpa(C.byref(d), stream.cuda_stream))
+        for s in sets[:2]:
+            for t, x in zip(dev, s):
+                t.copy_(torch.from_numpy(x.view(np.int16)))
+            capi.check(capi.lib.b200dnn_sdpa(C.byref(d_other), stream.cuda_stream))
+            out.zero_()
+            g.replay()
+            torch.cuda.synchronize()
+            close(oracle, out.cpu().numpy().view(np.uint16), oracle.sdpa(*s), s[2], "replay")

@@ -125,7 +125,11 @@ struct SmallBatch {
   size_t used = 0, sent = 0;
   cudaEvent_t ev = nullptr; bool in_flight = false;   // the last copy may still be reading `pinned`
   void begin() {
-    if (in_flight) { cudaEventSynchronize(ev); in_flight = false; }
+    if (in_flight) {
+      RelaxedCapture relaxed;      // (a call that is being captured, behind one that was not)
+      cudaEventSynchronize(ev);
+      in_flight = false;
+    }
     used = sent = 0;
   }
   // returns the device address the bytes will have after flush(), or nullptr when they do not fit
@@ -294,6 +298,7 @@ inline int32_t ensure_max_smem(const void *fn, int bytes = 227 * 1024) {
   std::lock_guard<std::mutex> lk(D.attr_mu);
   int &have = D.smem_limit[fn];
   if (have < bytes) {
+    RelaxedCapture relaxed;     // the kernel may be loaded here for the first time, which a capture in its strict modes does not allow
     B2_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     have = bytes;
   }

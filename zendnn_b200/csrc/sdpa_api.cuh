@@ -5,9 +5,10 @@
 //   P           = softmax(S * scale + mask) over kv, f32, rounded to bf16; causal: key j > query i is masked
 //   O_bh        = P V_bh               bf16 x bf16 -> out_dt
 // scale == 0 means 1 / sqrt(head_dim) (bmm_sdpa/lowoha_sdpa_utils.cpp:25-27).  A row whose keys are all masked gives zeros.
-// One fused kernel (sdpa_flash.cuh) takes rows of 16-byte vectors with a head dimension of up to 128, in any storage order.  Measured
-// against the three-step form below: 32 heads x 2048 causal, head_dim 128: 62 us for 636; 256 heads x 1 query x 3000 keys: 64 us
-// for 569 (6.1 TB/s); [batch, seq, head, dim] storage, which went head by head: 61 us for 8.6 ms at 1280 heads x 4 queries.
+// Fused kernels (sdpa_flash.cuh) take rows of 16-byte vectors with a head dimension of up to 128, in any storage order.  Measured
+// against the three-step form below: 32 heads x 2048 causal, head_dim 128: 61 us for 636; 256 heads x 1 query x 3000 keys: 64 us
+// for 569 (6.1 TB/s); [batch, seq, head, dim] storage, which went head by head: 61 us for 8.6 ms at 1280 heads x 4 queries.  Prompts of a
+// few heads against many keys stay with the three-step form (the rule is in sdpa_flash.cu).
 // Everything else runs the steps one after the other on the tcgen05 GEMM's bf16 form, the scores making a round trip through HBM
 // (seq * kv * 6 bytes per head): tensors whose query rows follow each other at one pitch over all heads in five launches for all
 // heads (K and V of every head into the tile layout, two grouped products, one softmax), other layouts head by head.
@@ -113,6 +114,10 @@ extern "C" int32_t b200dnn_sdpa(const b200dnn_sdpa_t *d, void *stream) {
   const float scale = d->scale == 0.0 ? 1.0f / std::sqrt((float)D) : (float)d->scale;
   const int64_t mb = msz[0] > 1 ? mst[0] : 0, mh = msz[1] > 1 ? mst[1] : 0, mi = msz[2] > 1 ? mst[2] : 0;
 
+  // the query rows of all heads follow each other at one pitch: the three-step form can take all heads at once
+  const bool rows_regular = d->q_stride[1] == S * d->q_stride[2] && (B == 1 || d->q_stride[0] == H * d->q_stride[1]) &&
+                            d->q_stride[2] % 8 == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0 && B * H * S < (1ll << 30);
+
   // ---- one fused kernel where it fits (B200DNN_SDPA_GROUPED=0 keeps the head-by-head form, B200DNN_SDPA_FUSED=0 the BMM forms)
   if (env_int("B200DNN_SDPA_GROUPED", 1) != 0 && env_int("B200DNN_SDPA_FUSED", 1) != 0) {
     SdpaCall c{};
@@ -122,16 +127,15 @@ extern "C" int32_t b200dnn_sdpa(const b200dnn_sdpa_t *d, void *stream) {
     c.scale = scale; c.causal = d->is_causal ? 1 : 0;
     c.mask = mk; c.mask_dt = d->mask_dt; c.mb = mb; c.mh = mh; c.mi = mi;
     c.test_no_loads = env_int("B200DNN_TEST_NO_LOADS", 0);
+    c.grouped = rows_regular && !c.test_no_loads ? 1 : 0;
     const int32_t rc = sdpa_fused(c, st);
     if (rc == B200DNN_SUCCESS) return finish_out({&o_out}, st);
     if (rc != B200DNN_UNIMPLEMENTED) return rc;
   }
 
-  // ---- all heads at once: when the query rows of all heads follow each other at one pitch, the two products are grouped
+  // ---- all heads at once: the two products are grouped
   // launches (one group per head, the head's K or V as its weight) and the softmax is one launch; several rounds when the
   // scores of all heads would not fit 1.5 GB
-  const bool rows_regular = d->q_stride[1] == S * d->q_stride[2] && (B == 1 || d->q_stride[0] == H * d->q_stride[1]) &&
-                            d->q_stride[2] % 8 == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0 && B * H * S < (1ll << 30);
   if (rows_regular && env_int("B200DNN_SDPA_GROUPED", 1) != 0) {
     const int64_t G = B * H;
     int64_t per_round = (int64_t)((1536ll << 20) / (S * (KV * 4 + kvp * 2)));

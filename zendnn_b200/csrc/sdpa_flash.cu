@@ -84,6 +84,21 @@ int32_t launch_sdpa_flash(const SdpaCall &c, cudaStream_t st) {
   a.tiles = (c.S <= 128 || heads * ((c.S + 255) / 256) < sms) ? 1 : 2;
   a.n_qt = (int)((c.S + a.tiles * 128 - 1) / (a.tiles * 128));
   if (heads * a.n_qt >= (1ll << 31)) return B200DNN_UNIMPLEMENTED;
+  // A CTA walks all keys of its rows, so a few heads with many keys leave most SMs idle (1 head x 17 queries x 16384 keys: 469 us with a mask),
+  // where the three-step form spreads the keys over the device (122 us).  Both in microseconds, fitted to 1676 calls (1 to 32 heads, 4 to
+  // 4096 queries, 512 to 131072 keys, with and without a mask): a wave of CTAs takes so much per 128 keys, the three-step form has its five
+  // launches, K and V to pack and the scores to write and read.  The choice is 0.2 % off the better form on average, 26 % at worst; this
+  // kernel always, 36 %.
+  if (c.grouped) {
+    const bool wide = c.D > 64, mask = c.mask != nullptr;
+    const double blocks = (double)(((c.causal && c.S < c.KV ? c.S : c.KV) + 127) / 128), waves = (double)((heads * a.n_qt + sms - 1) / sms);
+    const double block_us = a.tiles == 2 ? (mask ? 4.6 : 3.5) : (mask ? (wide ? 3.8 : 3.4) : (wide ? 2.3 : 2.0));
+    const double h = (double)heads, s = (double)c.S, kv = (double)c.KV;
+    const bool slower = 6.0 + waves * blocks * block_us > 31.0 + kv * (0.005 + h * (wide ? 0.0006 : 0.0004)) + 5e-6 * h * s * kv + (mask ? 0.002 : 0.001) * h * s;
+    // (the three-step form sends tables from the call's pinned block, which a captured graph would read again when it is replayed)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+    if (slower && cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) return B200DNN_UNIMPLEMENTED;
+  }
   // Longest query tiles of all heads first (under a causal mask their lengths differ by the sequence length) while every head's K
   // and V stay in the L2 together; head after head otherwise.
   a.bh_major = !c.causal || 4 * heads * c.KV * c.D > (64ll << 20);

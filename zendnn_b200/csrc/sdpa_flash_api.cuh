@@ -12,6 +12,7 @@ struct SdpaCall {
   float scale; int causal;
   const void *mask; int32_t mask_dt; int64_t mb, mh, mi;   // element (b,h,i,j) at b*mb + h*mh + i*mi + j; null: none
   int test_no_loads;
+  int grouped;             // the caller has the three-step form for all heads at once: it may be the faster one (see sdpa_fused)
 };
 
 // Enqueues one kernel, or returns unimplemented when the call does not fit (the caller then takes the BMM form).
