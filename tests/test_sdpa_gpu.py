@@ -71,20 +71,40 @@ def test_plain_and_causal(capi, oracle, shape, causal):
 
 
 def test_head_by_head_form_on_contiguous_tensors(capi, oracle, monkeypatch):
-    """Contiguous [batch, head, seq, dim] tensors take the grouped launches; the head-by-head form must give the same answer
-    (to the tolerance), here with a 4-D mask and the causal mask together."""
-    monkeypatch.setenv("B200DNN_SDPA_GROUPED", "0")
+    """Contiguous [batch, head, seq, dim] tensors take a fused kernel; the head-by-head and the grouped three-step form must give the
+    same answer (to the tolerance), here with a 4-D mask and the causal mask together."""
     rng = np.random.default_rng(8)
     B, H, S, KV, D = 2, 2, 130, 130, 64
     q, k, v = make(oracle, rng, B, H, S, KV, D)
     m4 = rng.standard_normal((B, H, S, KV)).astype(np.float32)
-    st, out = run(capi, q, k, v, mask=m4, causal=True)
-    assert st == capi.SUCCESS, capi.last_error()
-    close(oracle, out, oracle.sdpa(q, k, v, m4, causal=True), v, "head by head")
-    monkeypatch.setenv("B200DNN_SDPA_GROUPED", "1")
-    st, out2 = run(capi, q, k, v, mask=m4, causal=True)
-    assert st == capi.SUCCESS, capi.last_error()
-    close(oracle, out2, oracle.sdpa(q, k, v, m4, causal=True), v, "grouped")
+    for form, grouped, fused in (("head by head", "0", "1"), ("grouped", "1", "0"), ("fused", "1", "1")):
+        monkeypatch.setenv("B200DNN_SDPA_GROUPED", grouped)
+        monkeypatch.setenv("B200DNN_SDPA_FUSED", fused)
+        st, out = run(capi, q, k, v, mask=m4, causal=True)
+        assert st == capi.SUCCESS, capi.last_error()
+        close(oracle, out, oracle.sdpa(q, k, v, m4, causal=True), v, form)
+
+
+@pytest.mark.parametrize("D", [136, 192, 256, 20, 33])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("layout", ["bhsd", "bshd"])
+def test_head_dimensions_of_the_three_step_forms(capi, oracle, D, causal, layout):
+    """Head dimensions above 128 or not a multiple of 8 are not the fused kernels': grouped launches where the query rows of all heads
+    follow each other at one pitch of 16-byte vectors, head by head otherwise."""
+    rng = np.random.default_rng(D)
+    B, H = 2, 3
+    for S, KV in ((70, 70), (5, 131)):
+        q, k, v = make(oracle, rng, B, H, S, KV, D)
+        m = np.zeros((B, 1, S, KV), dtype=np.float32)
+        m[0, :, :, KV - 30:] = np.finfo(np.float32).min
+        m[1, :, 2] = np.finfo(np.float32).min
+        m[1, :, 4] = -np.inf
+        ref = oracle.sdpa(q, k, v, m, causal=causal)
+        if layout == "bshd":
+            q, k, v = (np.ascontiguousarray(x.transpose(0, 2, 1, 3)).transpose(0, 2, 1, 3) for x in (q, k, v))
+        st, out = run(capi, q, k, v, mask=m, causal=causal)
+        assert st == capi.SUCCESS, capi.last_error()
+        close(oracle, np.ascontiguousarray(out), ref, np.ascontiguousarray(v), (S, KV, D, causal, layout))
 
 
 def test_masks_scale_and_strides(capi, oracle):

@@ -41,7 +41,7 @@ int32_t launch_sdpa_decode(const SdpaCall &c, cudaStream_t st) {
   a.S = (int)c.S; a.KV = (int)c.KV; a.D = (int)c.D; a.H = (int)c.H;
   a.scale = c.scale; a.causal = c.causal;
   a.mask = SdpaMask{c.mask, c.mask_dt, c.mb, c.mh, c.mi};
-  a.status = rt().status;
+  a.status = rt().status; a.test_no_loads = c.test_no_loads;
   const int64_t heads = c.B * c.H;
   const int db = c.D <= 64 ? 1 : 2;
   // CTAs per head: the busiest SM's keys, plus about 300 keys' worth of time (3 us) for the start and the exchange of each round of
@@ -139,7 +139,7 @@ int32_t sdpa_fused(const SdpaCall &c, cudaStream_t st) {
   };
   if (!ok(c.q, c.qs, c.B, c.H, false) || !ok(c.k, c.ks, c.B, c.H, true) || !ok(c.v, c.vs, c.B, c.H, true)) return B200DNN_UNIMPLEMENTED;
   if (c.B * c.H > (1ll << 28)) return B200DNN_UNIMPLEMENTED;
-  if (c.S <= 16 && !c.test_no_loads) {
+  if (c.S <= 16) {
     const int32_t rc = launch_sdpa_decode(c, st);
     if (rc != B200DNN_UNIMPLEMENTED) return rc;
   }

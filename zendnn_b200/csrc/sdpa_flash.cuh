@@ -35,7 +35,7 @@ struct SdpaFlashArgs {
   uint16_t *out; int64_t ob, oh, os;
   int out_align;            // bytes every output row start is aligned to: 32, 16 or 2
   int32_t *status;
-  int test_no_loads;
+  int test_no_loads;        // test hook, as in SdpaDecodeArgs
 };
 
 constexpr int kFlashSoftmaxWarps = 16;  // two 128-row tiles x two halves of a key block x four lane quadrants
@@ -92,16 +92,18 @@ __device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t saddr, uint32_t l
   return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lead >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 
-// Prompt form: one CTA per (batch, head, 256 query rows), 320 threads.
-//   warps 0-3, 4-7  softmax of query rows 0-127 and 128-255: one thread per row, scores read from tensor memory
-//   warp 8          TMA producer: Q once; K blocks of 128 keys (sweep 1); K and V blocks in turn (sweep 2)
-//   warp 9          MMA issuer
+// Prompt form: one CTA per (batch, head, 256 query rows), 576 threads.
+//   warps 0-15      softmax: eight per 128-row tile, of which four take keys 0-63 of a block and four keys 64-127 (two threads per row), scores
+//                   read from tensor memory
+//   warp 16         TMA producer: Q once; K blocks of 128 keys (sweep 1); K and V blocks in turn (sweep 2)
+//   warp 17         MMA issuer
 // Tensor memory (512 columns): S0 S1 O0 O1.  In sweep 1 the O columns are the second score buffer of their tile, so the
 // tensor pipe runs a block ahead; in sweep 2 the normalised probabilities replace the scores in place as bf16 pairs and are the
 // A operand of the product with V straight from tensor memory, and the two row tiles alternate: while one is in its
 // exponentials the other's products run.
-// Bound by the exponentials (two per score: 16 per clock and SM, 1024 clocks per 128 x 128 block and sweep) beside the tensor
-// pipe (three products of 512 clocks per block).  256 query rows per CTA, because K and V then pass the L2 half as often as with 128
+// Bounds, per pair of 128 x 128 blocks (both row tiles, both sweeps): 4096 clocks of exponentials (two per score, 16 a clock) and 3072 of
+// the tensor pipe (three products a block); it takes about 6900 (32 heads x 2048 without a mask, head_dim 128: 116 us in two waves of CTAs).
+// 256 query rows per CTA, because K and V then pass the L2 half as often as with 128
 // (64 KB per two blocks: 6 TB/s over the device at that rate, against 12 TB/s).
 template <int DB, bool MASK>
 __global__ void __launch_bounds__(kFlashThreads, 1)
@@ -483,6 +485,7 @@ struct SdpaDecodeArgs {
   int causal;
   SdpaMask mask;
   int32_t *status;
+  int test_no_loads;       // test hook: the producer issues no copies, so the waits expire
 };
 constexpr int kSdpaDecodeWarps = 8, kSdpaDecodeThreads = 32 * (kSdpaDecodeWarps + 1), kSdpaDecodeSlots = 3;
 
@@ -534,7 +537,7 @@ sdpa_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
   // The producer takes part in the barriers of step 2, so before them it may only wait for slots that the K blocks free: blocks up to
   // nblk + slots - 1; the others follow in step 3.
   auto produce = [&](int from, int to) {
-    if (lane != 0) return;
+    if (lane != 0 || a.test_no_loads) return;
     for (int u = from; u < to; ++u) {
       const int slot = u % kSdpaDecodeSlots;
       if (!mbar_wait(empty(slot), ((uint32_t)(u / kSdpaDecodeSlots) & 1u) ^ 1u)) { s_err = 1; report_status(a.status, 41); break; }
