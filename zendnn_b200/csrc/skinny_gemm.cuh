@@ -24,7 +24,7 @@ namespace b200 {
 
 constexpr int kSkinnyThreads = 320;
 constexpr int kSkinnyMaxStages = 12;
-constexpr int kSkinnyMaxM = 128;
+constexpr int kSkinnyMaxM = 64;               // rows: tensor-memory columns of the accumulator, and the largest launch
 constexpr int kSkinnyMaxSplits = 8;              // CTAs per cluster (the portable limit)
 constexpr int kSkinnyRing = 216 * 1024;
 

@@ -5,7 +5,7 @@
   python -m zendnn_b200.run_case gs <w4a8|s8> M K N --gs G [--copies C] [--reps R]
   python -m zendnn_b200.run_case bf16 M K N [--copies C] [--reps R] [--act gelu_tanh] [--bias]
   python -m zendnn_b200.run_case norm <rms|fused_add_rms|layer> ROWS COLS [--quant] [--no-output] [--reps R]
-  python -m zendnn_b200.run_case sdpa BATCH HEADS SEQ DIM [--causal] [--reps R]
+  python -m zendnn_b200.run_case sdpa BATCH HEADS SEQ DIM [--kv KEYS] [--causal] [--reps R]
 
 matmul: s8 per-token activations x s8 per-channel prepacked weight -> bf16; `--copies` distinct prepacked
 weights are used in turn (pick copies * K * N above the L2 size to keep the weight stream in HBM);
@@ -143,12 +143,13 @@ def _sdpa(args):
     st = torch.cuda.current_stream().cuda_stream
     B, H, S, D = args.batch, args.heads, args.seq, args.dim
     g = torch.Generator(device=dev).manual_seed(0)
-    q, k, v = (torch.randn(B, H, S, D, generator=g, device=dev).to(torch.bfloat16) for _ in range(3))
+    KV = args.kv or S
+    q, k, v = (torch.randn(B, H, n, D, generator=g, device=dev).to(torch.bfloat16) for n in (S, KV, KV))
     o = torch.empty_like(q)
     d = capi.SdpaDesc()
-    d.batch, d.num_heads, d.seq_len, d.kv_seq_len, d.head_dim = B, H, S, S, D
-    for name in ("q_stride", "k_stride", "v_stride", "o_stride"):
-        setattr(d, name, (C.c_int64 * 4)(H * S * D, S * D, D, 1))
+    d.batch, d.num_heads, d.seq_len, d.kv_seq_len, d.head_dim = B, H, S, KV, D
+    for name, n in (("q_stride", S), ("k_stride", KV), ("v_stride", KV), ("o_stride", S)):
+        setattr(d, name, (C.c_int64 * 4)(H * n * D, n * D, D, 1))
     d.qkv_dt = d.out_dt = capi.DT["bf16"]
     d.is_causal = int(args.causal)
     d.query, d.key, d.value, d.output = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr()
@@ -162,9 +163,9 @@ def _sdpa(args):
     e1.record()
     torch.cuda.synchronize()
     us = e0.elapsed_time(e1) * 1e3 / args.reps
-    flops = 4.0 * B * H * S * S * D
-    print("sdpa B%d H%d S%d D%d%s: %.1f us per call, %.0f TFLOP/s of 4*B*H*S*S*D (BMM form: the scores pass through HBM)" %
-          (B, H, S, D, " causal" if args.causal else "", us, flops / us / 1e6))
+    flops = 4.0 * B * H * S * KV * D
+    print("sdpa B%d H%d S%d KV%d D%d%s: %.1f us per call, %.0f TFLOP/s of 4*B*H*S*KV*D, %.0f GB/s of Q, K, V and O" %
+          (B, H, S, KV, D, " causal" if args.causal else "", us, flops / us / 1e6, 4e-3 * B * H * (S + KV) * D / us))
 
 
 def _gs(args):
@@ -338,6 +339,7 @@ def main():
     nm.add_argument("--reps", type=int, default=5)
     sd = sub.add_parser("sdpa")
     sd.add_argument("batch", type=int); sd.add_argument("heads", type=int); sd.add_argument("seq", type=int); sd.add_argument("dim", type=int)
+    sd.add_argument("--kv", type=int, default=0, help="keys (default: as many as queries)")
     sd.add_argument("--causal", action="store_true")
     sd.add_argument("--reps", type=int, default=3)
     e = sub.add_parser("moe")
