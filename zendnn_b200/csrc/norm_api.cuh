@@ -298,8 +298,8 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, uint3
 // The decoder-layer case at full width: bf16 rows of at most NV * 8 * blockDim elements, 16-byte aligned, bf16 out.  One
 // CTA per row; a thread keeps its NV vectors of eight elements in registers (as the bf16 pairs they are at every stage that
 // is kept) between the passes, so the row is read once and every access is a 16-byte vector (8 bytes for the s8 codes).
-// HBM-bound, with the resident CTAs covering each other's reductions: all loads of a row (input and residual) are in flight before the first
-// store, each reduction costs one barrier, and the launch overlaps the kernel in front.  4096 rows of 4096 with residual add and s8 codes
+// Bound by HBM without the quantised output and by instruction issue with it (3.15 of 4 instructions a cycle): all loads of a row (input and
+// residual) are in flight before the first store, each reduction costs one barrier, and the launch overlaps the kernel in front.  4096 rows of 4096 with residual add and s8 codes
 // (151 MB): 36.9 -> 30.5 us (4.9 TB/s); a ring of rows filled by bulk copies ahead of persistent CTAs took 35.7 us (four CTAs per SM where
 // there are six here).
 template <int NV>
