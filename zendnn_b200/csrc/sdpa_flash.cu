@@ -96,8 +96,11 @@ int32_t launch_sdpa_flash(const SdpaCall &c, cudaStream_t st) {
     const double h = (double)heads, s = (double)c.S, kv = (double)c.KV;
     const bool slower = 6.0 + waves * blocks * block_us > 31.0 + kv * (0.005 + h * (wide ? 0.0006 : 0.0004)) + 5e-6 * h * s * kv + (mask ? 0.002 : 0.001) * h * s;
     // (the three-step form sends tables from the call's pinned block, which a captured graph would read again when it is replayed)
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
-    if (slower && cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) return B200DNN_UNIMPLEMENTED;
+    if (slower) {
+      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+      if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+      else if (cap == cudaStreamCaptureStatusNone) return B200DNN_UNIMPLEMENTED;
+    }
   }
   // Longest query tiles of all heads first (under a causal mask their lengths differ by the sequence length) while every head's K
   // and V stay in the L2 together; head after head otherwise.
