@@ -11,8 +11,9 @@
 // three-step form (the distance with one rounding less).  Error of the f32 probabilities against double, mean / mean weighted by the
 // probability / largest, for 2048 keys with scores of spread 1, 4 and 10 at scale 2^-3.5 (head_dim 128), in units of 1e-7:
 //   three-step form   0.94 / 0.79 / 5.3    3.5 / 1.9 / 24    9.4 / 2.4 / 62
-//   here              0.91 / 0.76 / 4.8    3.1 / 0.80 / 17   7.5 / 0.65 / 40
-// and 1.2 / 1.0 / 9 on both sides with a mask of spread 1, 150 / 150 / 330 with one of -1000.
+//   here              0.92 / 0.76 / 4.8    3.1 / 0.81 / 17    7.5 / 0.65 / 40
+// and 1.2 / 1.0 / 9 on both sides with a mask of spread 1, 150 / 150 / 330 with one of -1000; head_dim 64 without a mask 0.92 / 0.74 / 5.1 and
+// 0.93 / 0.75 / 4.9.
 #pragma once
 #include "common.cuh"
 #include "mbar.cuh"
@@ -49,16 +50,18 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { u
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 
-// exp(-u) of two arguments u >= 0 (infinities included), as 2^(u * -log2 e).  The plain form rounds the product; it serves the row sum, where
-// the roundings of hundreds of terms average out.  The corrected form multiplies by 1 + (exact product - rounded product) * ln 2, with
-// log2 e in two parts, so that what remains is the error of ex2.approx (and of u).
+// exp(-u) of two arguments u >= 0 (infinities included), as 2^(u * -log2 e) with log2 e in two parts.  The plain form rounds the product; it serves
+// the row sum, where the roundings of hundreds of terms average out.  The corrected form multiplies by 1 + (exact product - rounded
+// product) * ln 2, so that what remains is the error of ex2.approx (and of u), of which the part that has one sign is in the sum as well.
 constexpr float kLog2e = 1.44269504088896340736f, kLog2eLo = (float)(1.44269504088896340736 - (double)kLog2e), kLn2 = 0.693147180559945309417f;
 __device__ __forceinline__ uint64_t ex2_pair(uint64_t x2) {
   float x0, x1;
   upk2(x2, x0, x1);
   return pk2(ex2f(x0), ex2f(x1));
 }
-__device__ __forceinline__ uint64_t exp_neg2_plain(uint64_t u2) { return ex2_pair(mul2(u2, pk2(-kLog2e, -kLog2e))); }
+__device__ __forceinline__ uint64_t exp_neg2_plain(uint64_t u2) {
+  return ex2_pair(fma2(u2, pk2(-kLog2e, -kLog2e), mul2(u2, pk2(-kLog2eLo, -kLog2eLo))));
+}
 __device__ __forceinline__ uint64_t exp_neg2(uint64_t u2) {
   float u0, u1;
   upk2(u2, u0, u1);
