@@ -145,7 +145,8 @@ int32_t resolve_weight(const void *weight, int wei_format, int64_t K, int64_t N,
 template <bool EP>
 int32_t launch_quant_rows_t(const RowQuantArgs &a, int32_t src_dt, int64_t rows, cudaStream_t st) {
   if (rows <= 0) return B200DNN_SUCCESS;
-  // short, aligned, non-grouped rows: one warp per row
+  // aligned, non-grouped rows of up to 16 vectors a lane (bf16: 4096 elements): one warp per row.  Against a CTA per row, us, bf16: 8192 x 4096 19.8
+  // and 23.8, 5092 x 2688 11.5 and 13.8, 512 x 4096 5.0 and 7.5.
   const int E = src_dt == B200DNN_BF16 ? 8 : 4;
   const bool aligned = a.n_groups == 0 && a.K % E == 0 && (reinterpret_cast<uintptr_t>(a.src) & 15) == 0 &&
                        (a.src_ld * (src_dt == B200DNN_BF16 ? 2 : 4)) % 16 == 0 &&
@@ -170,7 +171,7 @@ int32_t launch_quant_rows_t(const RowQuantArgs &a, int32_t src_dt, int64_t rows,
     B2_CUDA(cudaGetLastError());
     return B200DNN_SUCCESS;
   }
-  if (aligned && rows >= 64 && a.K / E <= 32 * 8 && (src_dt == B200DNN_BF16 || src_dt == B200DNN_F32)) {
+  if (aligned && rows >= 64 && a.K / E <= 32 * 16 && (src_dt == B200DNN_BF16 || src_dt == B200DNN_F32)) {
     const int nv = (a.K / E + 31) / 32;
     unsigned grid = (unsigned)((rows + 7) / 8);
     if (EP && a.n_rows_dev && grid > (unsigned)(rt().sm_count * 16)) grid = (unsigned)(rt().sm_count * 16);   // the warps stride over the rows

@@ -258,38 +258,12 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, uint3
     }
     const float scale = scale_from_absmax(amax);
     const float rinv = __frcp_rn(scale);
-    // q = rne(v / scale) without a division: m = v * rinv + 1.5 * 2^23 holds the integer nearest to the product in its low
-    // byte; d = v * rinv - that integer is the product's distance from it, and whenever |d| < 0.4999 (d^2 < 0.2499, one
-    // fused operation whose sign bit is and-ed over the vector) the product and the exact quotient round alike: rinv is
-    // the correctly rounded reciprocal, so v * rinv is within 127.5 * 2^-24 < 1e-5 of v / scale.  An element that fails
-    // the test, through a near-tie or because it is not finite, takes the exact division.
-    const float magic = 12582912.0f;
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
       const int i = threadIdx.x + j * blockDim.x;
-      if (i < nvec) {
-        uint32_t mbits[8], ok = 0x80000000u;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float v0 = lo(v[j][e]), v1 = hi(v[j][e]);
-          const float m0 = __fmaf_rn(v0, rinv, magic), m1 = __fmaf_rn(v1, rinv, magic);
-          const float d0 = __fmaf_rn(v0, rinv, __fsub_rn(magic, m0)), d1 = __fmaf_rn(v1, rinv, __fsub_rn(magic, m1));
-          const uint32_t c0 = __float_as_uint(__fmaf_rn(d0, d0, -0.2499f)), c1 = __float_as_uint(__fmaf_rn(d1, d1, -0.2499f));
-          ok &= c0 & c1;
-          mbits[2 * e] = __float_as_uint(m0); mbits[2 * e + 1] = __float_as_uint(m1);
-        }
-        if (!ok) {
-          // only the elements that failed take the division (about two in ten thousand)
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float ve = (e & 1) ? hi(v[j][e >> 1]) : lo(v[j][e >> 1]);
-            const float de = __fmaf_rn(ve, rinv, __fsub_rn(magic, __uint_as_float(mbits[e])));
-            if (!(__fmaf_rn(de, de, -0.2499f) < 0.0f)) mbits[e] = (uint32_t)(uint8_t)quant_sym(ve, scale);
-          }
-        }
+      if (i < nvec)
         *reinterpret_cast<uint2 *>(a.q + b * a.q_ld + (int64_t)i * 8) =
-            make_uint2(low_bytes4(mbits[0], mbits[1], mbits[2], mbits[3]), low_bytes4(mbits[4], mbits[5], mbits[6], mbits[7]));
-      }
+            quant_vec<uint16_t>(make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]), scale, rinv);
     }
     if (threadIdx.x == 0) a.q_scale[b] = scale;
   }

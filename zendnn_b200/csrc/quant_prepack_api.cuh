@@ -56,9 +56,9 @@ __device__ __forceinline__ int8_t quant_channel(float v, float s) {
   return (int8_t)max(-128, min(127, q));
 }
 
-// The same code without a division in the common case (the argument of quant_sym_r: the scale comes from the abs-max of
-// the channel itself, so every finite |v/s| <= 127 up to rounding, and away from a near-tie v*rinv rounds to the integer
-// the rounded quotient rounds to).  Near-ties and non-finite inputs take the division.
+// The same code without a division in the common case.  The scale comes from the abs-max of the channel itself, so every finite |v/s| <= 127
+// up to rounding; v*rinv, its rounding and the rounded quotient lie within 3 * 127.5 * 2^-24 < 2.3e-5 of v/s and, 1e-4 away from a half
+// integer, round to the same integer.  Near-ties and non-finite inputs take the division.
 __device__ __forceinline__ int8_t quant_channel_r(float v, float s, float rinv) {
   const float magic = 12582912.0f;
   const float qa = v * rinv, m = qa + magic, t = m - magic;
