@@ -3,6 +3,7 @@
 // of gs_gemm_kernel.  Included by b200dnn.cu in front of the C ABI.
 #pragma once
 #include "gs_gemm.cuh"
+#include "gs_tc.cuh"
 
 namespace {
 
@@ -183,6 +184,74 @@ int32_t launch_gs_decode_t(const GsGemmArgs &a, const EpiParams &epi, bool early
   return B200DNN_SUCCESS;
 }
 
+// The tensor-core form (gs_tc.cuh).
+int gs_tc_room(int s) {
+  return cluster_room(gs_tc_kernel<128, 1>, GsTcShape<128, 1>::kThreads, 220 * 1024, s, &rt().shared->gs_tc_room[s]);
+}
+template <int BM, int GPB>
+int32_t launch_gs_tc_t(const GsGemmArgs &g, GsTcArgs a, const CUtensorMap &map_w, const EpiParams &epi, cudaStream_t st) {
+  using Sh = GsTcShape<BM, GPB>;
+  CUtensorMap map_a;
+  B2_TRY(make_map_2d(&map_a, g.A, (uint64_t)g.Kp, (uint64_t)g.M, (uint64_t)g.lda, BM));
+  a.m_tiles = (g.M + BM - 1) / BM;
+  const int tiles = a.n_tiles * a.m_tiles;
+  int stages = (227 * 1024 - 6 * 1024 - Sh::kTail) / Sh::kStage;      // (barriers, row scales and alignment: less than 6 KiB)
+  if (stages > kGsTcMaxStages) stages = kGsTcMaxStages;
+  a.stages = stages;
+  const size_t smem = (size_t)stages * Sh::kStage + Sh::kTail + 1024;
+  B2_TRY(ensure_max_smem((const void *)gs_tc_kernel<BM, GPB>, (int)smem));
+  const unsigned grid = a.splits > 1 ? (unsigned)(tiles * a.splits) : (unsigned)(tiles < rt().sm_count ? tiles : rt().sm_count);
+  B2_TRY(launch_pdl_cluster(gs_tc_kernel<BM, GPB>, grid, (unsigned)Sh::kThreads, smem, (unsigned)a.splits, st, a.early != 0, map_w, map_a, a, epi));
+  B2_LAUNCHED();
+  return B200DNN_SUCCESS;
+}
+
+// Calls the tensor-core form takes: s4 codes, per-token rows, f32 weight scales, groups of 32, 64 or a multiple of 128 k.  Up to 16 rows it has the higher
+// fixed cost (7.2 us against 5 to 6, quantisation included) and the decode form the higher cost per column and k, the more so with more rows and shorter
+// groups: 121 measured shapes (K 1024 to 14336, N 512 to 14336) cross where K * (M + 8) passes 20, 40 and 80 thousand for groups of 32, 64 and
+// 128; the choice is 1.0, 1.3 and 1.5 % off the better form on average, the decode form always 22, 15 and 4 % (K = 11008, N = 4096, M = 16, us: 24.6 and 14.6;
+// K = N = 4096, M = 1: 7.2 and 9.4).  Above 16 rows it is at least twice as fast as the general form (M = 64, K = 4096, N = 11008: 92 -> 21).
+inline bool gs_tc_pays(const GsPlan &p, int32_t ws_dt, int M, int K) {
+  if (!p.w4 || p.src_cols != 1 || ws_dt != B200DNN_F32 || !(p.gs == 32 || p.gs == 64 || p.gs % 128 == 0)) return false;
+  const int mode = env_int("B200DNN_GS_TC", -1);
+  if (mode >= 0) return mode != 0;
+  return M > 16 || (long long)K * (M + 8) >= (p.gs == 32 ? 20000 : p.gs == 64 ? 40000 : 80000);
+}
+int32_t launch_gs_tc(const GsGemmArgs &g, const EpiParams &epi, bool early, cudaStream_t st) {
+  GsTcArgs a{};
+  a.M = g.M; a.N = g.N; a.k_blocks = (g.K + 127) / 128; a.group_blocks = g.gs > 128 ? g.gs / 128 : 1; a.G = g.G;
+  a.n_tiles = (g.N + 127) / 128;
+  a.sa = g.sa; a.sw = (const float *)g.sw; a.early = early ? 1 : 0; a.status = rt().status;
+  a.test_no_loads = env_int("B200DNN_TEST_NO_LOADS", 0);
+  CUtensorMap map_w;
+  B2_TRY(make_map_s4(&map_w, g.W, (uint64_t)(g.Kp >> 6), (uint64_t)((g.N + 7) / 8)));
+  // Rows per tile and shares of the groups: fewest microseconds by blocks of 128 k per CTA times the measured cost of one.  Splitting costs nothing
+  // that shows beside it; a cluster's CTAs are resident at once.
+  static const double block_us[4][3] = {{0.42, 0.29, 0.30}, {0.70, 0.33, 0.34}, {1.01, 0.51, 0.42}, {1.66, 0.98, 0.55}};      // [16, 32, 64, 128 rows][groups of 32, 64, 128]
+  const int cls = g.gs == 32 ? 0 : g.gs == 64 ? 1 : 2, units = a.k_blocks / a.group_blocks, sms = rt().sm_count;
+  const int forced_bm = env_int("B200DNN_GS_TC_BM", 0), forced = env_int("B200DNN_GS_TC_SPLIT", 0);
+  int bm = 0;
+  double best = 0.0;
+  for (int i = 0; i < 4; ++i) {
+    const int rows = 16 << i, tiles = a.n_tiles * ((g.M + rows - 1) / rows);
+    if (forced_bm ? rows != forced_bm : (i > 0 && rows / 2 >= g.M) || (rows < 64 && rows < g.M)) continue;      // (never more than half empty, never many small tiles)
+    for (int s = 1; s <= kGsTcMaxSplits; ++s) {
+      if (s > 1 && (units < 2 * s || tiles * s > gs_tc_room(s))) continue;
+      if (forced > 0 && s != forced && s != 1) continue;
+      const int blocks = s > 1 ? (units + s - 1) / s * a.group_blocks : (tiles + sms - 1) / sms * a.k_blocks;
+      const double us = blocks * block_us[i][cls];
+      if (bm == 0 || us < best || (forced > 1 && s == forced)) { best = us; bm = rows; a.splits = s; }
+    }
+  }
+#define B2_GS_TC(BM) \
+  return g.gs == 32 ? launch_gs_tc_t<BM, 4>(g, a, map_w, epi, st) : g.gs == 64 ? launch_gs_tc_t<BM, 2>(g, a, map_w, epi, st) : launch_gs_tc_t<BM, 1>(g, a, map_w, epi, st)
+  if (bm == 16) B2_GS_TC(16);
+  if (bm == 32) B2_GS_TC(32);
+  if (bm == 64) B2_GS_TC(64);
+  B2_GS_TC(128);
+#undef B2_GS_TC
+}
+
 // The whole call; the caller holds the call guard (B2_ENTER) and has checked is_group_scaled().
 int32_t matmul_group_scaled(const b200dnn_matmul_t *d, cudaStream_t st) {
   Runtime &R = rt();
@@ -292,6 +361,12 @@ int32_t matmul_group_scaled(const b200dnn_matmul_t *d, cudaStream_t st) {
     return B200DNN_SUCCESS;
   };
 
+  const bool early = p.dyn && p.src_cols == 1 && !p.src_per_tensor;      // (directly behind the per-token quantisation, which waited for everything in front of it)
+  if (gs_tc_pays(p, d->wei_scale.dt, M, K)) {
+    B2_TRY(prepare_source());
+    B2_TRY(launch_gs_tc(a, epi, early, st));
+    return finish_out({&o_dst, &o_scale}, st);
+  }
   // (the decode form addresses the weight and the scales with 32-bit offsets)
   if (M <= 16 && p.G >= kGsWarps && p.gs % 32 == 0 && d->wei_scale.dt == B200DNN_F32 && N % 2 == 0 &&
       (int64_t)(N + 8) * Kp < (int64_t)1 << 32 && (int64_t)p.G * N < (int64_t)1 << 30 &&
@@ -300,8 +375,6 @@ int32_t matmul_group_scaled(const b200dnn_matmul_t *d, cudaStream_t st) {
     bool done = false;
     int32_t rcd;
     const bool ch128 = p.gs % 128 == 0 && env_int("B200DNN_GS_CH128", 1) != 0;     // fewer, larger items per group
-    // (directly behind the per-token quantisation, which waited for everything in front of it)
-    const bool early = p.dyn && p.src_cols == 1 && !p.src_per_tensor;
     if (p.w4) rcd = ch128 ? launch_gs_decode_t<128, true>(a, epi, early, st, &done) : ch64 ? launch_gs_decode_t<64, true>(a, epi, early, st, &done) : launch_gs_decode_t<32, true>(a, epi, early, st, &done);
     else rcd = ch128 ? launch_gs_decode_t<128, false>(a, epi, early, st, &done) : ch64 ? launch_gs_decode_t<64, false>(a, epi, early, st, &done) : launch_gs_decode_t<32, false>(a, epi, early, st, &done);
     B2_TRY(rcd);

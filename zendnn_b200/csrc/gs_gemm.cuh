@@ -6,7 +6,7 @@
 // Integer sums per group are exact; the f32 sum over the groups runs in group order inside a warp.
 //
 // Layout: the weight is blocked as [N/8][Kp/64][8 columns][64 k], s8 (64 bytes per column and block) or s4 (32 bytes: two
-// codes per byte, even k in the low nibble), zero padded -- 4-bit weights stay 4-bit in HBM, which halves the bytes a
+// codes per byte, k in the low nibble and k + 4 in the high one), zero padded -- 4-bit weights stay 4-bit in HBM, which halves the bytes a
 // decode-shaped call streams, and the eight columns x 64 k that one warp-level load instruction fetches are one
 // contiguous 512-byte (256-byte) block, with the next k block of the same columns right behind it.  A is s8 [M][Kp]
 // (rows zero-padded to Kp, a multiple of 64).
@@ -16,9 +16,8 @@
 // k0 + 16 t of a 64-byte chunk (8 bytes at k0 + 8 t of a 32-byte chunk when the group size is not a multiple of 64) --
 // for the activation rows g and g + 8 and for weight column g of every column tile; both operands use the same
 // assignment of k to fragment positions, so each MMA adds products of matching k and a chunk is covered exactly once.
-// s4 codes are not sign-extended: the even and odd nibbles of a word are masked into the HIGH nibbles of two registers
-// (16 * w, exact), the activation bytes are permuted to the same even / odd order with two byte permutes per row, and
-// the group sum is shifted right by four (exact: it is a multiple of 16).
+// s4 codes are not sign-extended: the low and high nibbles of a word, k .. k + 3 and k + 4 .. k + 7 of its eight, are masked into the HIGH nibbles of
+// two registers (16 * w, exact), and the group sum is shifted right by four (exact: it is a multiple of 16).
 // Group sizes 4, 8 and 16 run the MMA of a 32-byte chunk once per group with the activation registers of the other
 // groups zeroed.
 // The warps that share a row tile add their f32 partial sums through shared memory in a fixed order.
@@ -78,8 +77,7 @@ __device__ __forceinline__ void gs_ld_a(const int8_t *arow, int k_piece, uint32_
   if (CH == 64) { const uint4 v = *reinterpret_cast<const uint4 *>(arow + k_piece); r[0] = v.x; r[1] = v.y; r[CH > 32 ? 2 : 0] = v.z; r[CH > 32 ? 3 : 0] = v.w; }
   else { const uint2 v = *reinterpret_cast<const uint2 *>(arow + k_piece); r[0] = v.x; r[1] = v.y; }
 }
-// MMA B registers {b0, b1} per 32 k: s8 pieces are used as they are, an s4 word becomes (even nibbles << 4, odd nibbles
-// in place)
+// MMA B registers {b0, b1} per 32 k: s8 pieces are used as they are, an s4 word becomes (low nibbles << 4, high nibbles in place)
 template <int CH, bool W4>
 __device__ __forceinline__ void gs_expand_b(const uint32_t (&r)[GsRaw<CH, W4>::RW], uint32_t (&b)[CH / 16]) {
 #pragma unroll
@@ -88,17 +86,6 @@ __device__ __forceinline__ void gs_expand_b(const uint32_t (&r)[GsRaw<CH, W4>::R
     else { b[2 * i] = r[(2 * i) % GsRaw<CH, W4>::RW]; b[2 * i + 1] = r[(2 * i + 1) % GsRaw<CH, W4>::RW]; }
   }
 }
-// The activation piece in the same order: unchanged for s8 weights; for s4 weights the bytes of each 8-byte half are split
-// into (even k, odd k)
-template <int CH, bool W4>
-__device__ __forceinline__ void gs_expand_a(const uint32_t (&r)[CH / 16], uint32_t (&a)[CH / 16]) {
-#pragma unroll
-  for (int i = 0; i < CH / 16; i += 2) {
-    if (W4) { a[i] = __byte_perm(r[i], r[i + 1], 0x6420); a[i + 1] = __byte_perm(r[i], r[i + 1], 0x7531); }
-    else { a[i] = r[i]; a[i + 1] = r[i + 1]; }
-  }
-}
-
 template <int NT, int CH, bool W4>
 __global__ void __launch_bounds__(kGsWarps * 32) gs_gemm_kernel(GsGemmArgs g, EpiParams epi) {
   __shared__ float red[kGsWarps][16][NT * 8 + 1];
@@ -173,9 +160,7 @@ __global__ void __launch_bounds__(kGsWarps * 32) gs_gemm_kernel(GsGemmArgs g, Ep
       for (int d = 0; d < D; ++d) {
         if (i0 + d < n_items) {
           if (cc == 0) zero_acc();
-          uint32_t al[NR], ah[NR];
-          gs_expand_a<CH, W4>(ral[d], al);
-          gs_expand_a<CH, W4>(rah[d], ah);
+          const uint32_t (&al)[NR] = ral[d], (&ah)[NR] = rah[d];
 #pragma unroll
           for (int j = 0; j < NT; ++j) {
             uint32_t b[NR];
@@ -193,11 +178,9 @@ __global__ void __launch_bounds__(kGsWarps * 32) gs_gemm_kernel(GsGemmArgs g, Ep
     const int n_chunks = (g.K + CH - 1) / CH;
     for (int ch = wk; ch < n_chunks; ch += KS) {
       const int kp = ch * CH + lt * PIECE;
-      uint32_t ral[NR], rah[NR], al[NR], ah[NR];
-      gs_ld_a<CH>(a_lo, kp, ral);
-      gs_ld_a<CH>(a_hi, kp, rah);
-      gs_expand_a<CH, W4>(ral, al);
-      gs_expand_a<CH, W4>(rah, ah);
+      uint32_t al[NR], ah[NR];
+      gs_ld_a<CH>(a_lo, kp, al);
+      gs_ld_a<CH>(a_hi, kp, ah);
       uint32_t b[NT][NR];
 #pragma unroll
       for (int j = 0; j < NT; ++j) {
@@ -208,16 +191,8 @@ __global__ void __launch_bounds__(kGsWarps * 32) gs_gemm_kernel(GsGemmArgs g, Ep
       for (int sub = 0; sub < nsub; ++sub) {
         const int grp = ch * nsub + sub;
         if (grp >= g.G) break;
-        // which of this lane's activation bytes belong to the group: s8 registers hold k = 8t + 4i .. + 3; s4 registers hold
-        // the even (odd) k of 8t .. 8t + 7, two per 4-element group
-        uint32_t m0k, m1k;
-        if (W4) {
-          if (g.gs == 4) m0k = m1k = (sub == 2 * lt) ? 0x0000FFFFu : (sub == 2 * lt + 1 ? 0xFFFF0000u : 0u);
-          else m0k = m1k = ((lt * 8) / g.gs == sub) ? 0xFFFFFFFFu : 0u;
-        } else {
-          m0k = ((lt * 8) / g.gs == sub) ? 0xFFFFFFFFu : 0u;
-          m1k = ((lt * 8 + 4) / g.gs == sub) ? 0xFFFFFFFFu : 0u;
-        }
+        // which of this lane's activation bytes belong to the group: the registers hold k = 8t + 4i .. + 3
+        const uint32_t m0k = ((lt * 8) / g.gs == sub) ? 0xFFFFFFFFu : 0u, m1k = ((lt * 8 + 4) / g.gs == sub) ? 0xFFFFFFFFu : 0u;
         zero_acc();
 #pragma unroll
         for (int j = 0; j < NT; ++j) mma_m16n8k32<false>(acc[j], al[0] & m0k, ah[0] & m0k, al[1] & m1k, ah[1] & m1k, b[j][0], b[j][1]);
@@ -409,15 +384,13 @@ __global__ void __launch_bounds__(kGsWarps * 32, 2) gs_decode_kernel(GsDecodeArg
         const uint32_t sw_ = ring_w + (uint32_t)c_slot * SLOTW;
         c_slot = c_slot + 1 == R ? 0 : c_slot + 1;
         const uint32_t kb = (uint32_t)(grp * g.gs + c * CH);
-        uint32_t ral[NR], rah[NR], al[NR], ah[NR];
-        lds_words<NR>(a_lo + kb, 16u, ral);
-        if (hi_rows) lds_words<NR>(a_hi + kb, 16u, rah);
+        uint32_t al[NR], ah[NR];
+        lds_words<NR>(a_lo + kb, 16u, al);
+        if (hi_rows) lds_words<NR>(a_hi + kb, 16u, ah);
         else {
 #pragma unroll
-          for (int i = 0; i < NR; ++i) rah[i] = 0;
+          for (int i = 0; i < NR; ++i) ah[i] = 0;
         }
-        gs_expand_a<CH, W4>(ral, al);
-        gs_expand_a<CH, W4>(rah, ah);
 #pragma unroll
         for (int j = 0; j < NT; ++j) {
           uint32_t rb[RW], b[NR];
@@ -477,7 +450,7 @@ __global__ void gs_pack_weight_kernel(const uint8_t *src, int64_t ldb, int trans
   const int64_t pairs = Kp / 2, np8 = (N + 7) / 8 * 8;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= pairs * np8) return;
-  const int n = (int)(i / pairs), k = (int)(i - (int64_t)n * pairs) * 2;
+  const int n = (int)(i / pairs), p = (int)(i - (int64_t)n * pairs);
   auto elem = [&](int kk) -> int {
     if (kk >= K || n >= N) return 0;
     const int64_t idx = transB ? (int64_t)n * ldb + kk : (int64_t)kk * ldb + n;
@@ -485,8 +458,9 @@ __global__ void gs_pack_weight_kernel(const uint8_t *src, int64_t ldb, int trans
     return (int)reinterpret_cast<const int8_t *>(src)[idx];
   };
   const int64_t nblk = Kp >> 6;
+  const int k = src_s4 ? (p >> 2) * 8 + (p & 3) : 2 * p;                       // s4: the byte holds k (low nibble) and k + 4
   const int64_t blk = ((int64_t)(n >> 3) * nblk + (k >> 6)) * 8 + (n & 7);     // (column tile, k block, column)
-  if (src_s4) dst[blk * 32 + ((k & 63) >> 1)] = (uint8_t)(elem(k) | (elem(k + 1) << 4));
+  if (src_s4) dst[blk * 32 + (p & 31)] = (uint8_t)(elem(k) | (elem(k + 4) << 4));
   else { dst[blk * 64 + (k & 63)] = (uint8_t)elem(k); dst[blk * 64 + (k & 63) + 1] = (uint8_t)elem(k + 1); }
 }
 

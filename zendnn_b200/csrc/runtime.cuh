@@ -173,7 +173,7 @@ struct DeviceShared {
   std::map<cudaStream_t, Runtime *> ctxs;
   std::mutex attr_mu;
   std::map<const void *, int> smem_limit;                 // kernels whose dynamic shared-memory limit was raised
-  std::atomic<int> split_room[5] = {}, skinny_room[9] = {};   // by cluster size: see cluster_room
+  std::atomic<int> split_room[5] = {}, skinny_room[9] = {}, gs_tc_room[9] = {};   // by cluster size: see cluster_room
 };
 
 // Descriptor tables that depend only on the caller's weight pointers (per-expert epilogue pointers, tensor maps) are
@@ -456,6 +456,20 @@ inline int32_t make_map_wt(CUtensorMap *m, const void *wt, uint64_t Kp, uint64_t
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   B2_CHECK(r == CUDA_SUCCESS, B200DNN_FAILURE, "cuTensorMapEncodeTiled (weight) failed with %d", (int)r);
+  return B200DNN_SUCCESS;
+}
+
+// 2-D map over s4 codes blocked as [col_tiles][k_blocks64][8][32 B] (gs_gemm.cuh): rows of k_blocks64 * 256 bytes, counted in words; the box, 512 bytes
+// (128 k of eight columns) x 16, lands as it lies in memory (8 KiB, no swizzle), zeros past the edges.
+inline int32_t make_map_s4(CUtensorMap *m, const void *codes, uint64_t k_blocks64, uint64_t col_tiles) {
+  B2_CHECK((reinterpret_cast<uintptr_t>(codes) & 15) == 0, B200DNN_FAILURE, "blocked codes are not laid out for TMA");
+  cuuint64_t dims[2] = {k_blocks64 * 64, col_tiles};
+  cuuint64_t strides[1] = {k_blocks64 * 256};
+  cuuint32_t box[2] = {128, 16};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = rt().encode(m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void *>(codes), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  B2_CHECK(r == CUDA_SUCCESS, B200DNN_FAILURE, "cuTensorMapEncodeTiled (codes) failed with %d", (int)r);
   return B200DNN_SUCCESS;
 }
 

@@ -194,6 +194,7 @@ __device__ __forceinline__ void st_shared_v4(uint32_t saddr, uint32_t x, uint32_
   asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // bf16 x bf16 -> f32, M x N x 16 (32 bytes of K per instruction, as kind::i8)
 __device__ __forceinline__ void tc_mma_bf16_pair(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
