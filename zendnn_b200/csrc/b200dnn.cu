@@ -322,50 +322,6 @@ int32_t launch_decode_ring(const uint8_t *A, int64_t lda, bool a_unsigned, int M
   return B200DNN_SUCCESS;
 }
 
-// Tile width.  With at least one tile per SM the candidates are the multiples of 32 from 256 down to 128 (multiples of
-// 64 in the gated form) and the cost of a candidate is its number of waves over the SMs times (width + 16): the last,
-// partly filled wave of a persistent grid can cost more than a narrower tile does (M=2048, N=14336: 896 tiles of 256
-// columns are 7 waves on 148 SMs, 1024 tiles of 224 columns are 7 waves as well and each is an eighth shorter).
-// Smaller problems take the widest tile that still gives every SM one.
-int pick_bn(int m_tiles, int N, int sm_count, int gated, int pair = 0) {
-  int forced = env_int("B200DNN_TC_BN", 0);
-  if (forced > 0) return forced;
-  if (pair) {
-    // pair form: m_tiles counts 256-row tiles, one per CTA pair; each CTA's half of the tile must hold whole
-    // 64-column gate/up blocks in the gated form (and whole 8-row weight groups always)
-    const int pairs = sm_count / 2, pstep = gated ? 128 : 32;
-    int best = 256; long long best_cost = -1;
-    for (int bn = 256; bn >= 128; bn -= pstep) {
-      const long long tiles = (long long)m_tiles * ((N + bn - 1) / bn);
-      const long long cost = ((tiles + pairs - 1) / pairs) * (bn + 16);
-      if (best_cost < 0 || cost < best_cost) { best = bn; best_cost = cost; }
-    }
-    return best;
-  }
-  const int step = gated ? 64 : 32;
-  if ((long long)m_tiles * ((N + 127) / 128) >= sm_count) {
-    int best = 256; long long best_cost = -1;
-    for (int bn = 256; bn >= 128; bn -= step) {
-      const long long tiles = (long long)m_tiles * ((N + bn - 1) / bn);
-      const long long cost = ((tiles + sm_count - 1) / sm_count) * (bn + 16);
-      if (best_cost < 0 || cost < best_cost) { best = bn; best_cost = cost; }
-    }
-    return best;
-  }
-  const int cands[3] = {128, 64, 32};
-  for (int i = 0; i < 3; ++i) {
-    int bn = cands[i];
-    if (gated && bn < 64) break;
-    if ((long long)m_tiles * ((N + bn - 1) / bn) >= sm_count || i == 2 || (gated && bn == 64)) return bn;
-  }
-  return gated ? 64 : 32;
-}
-
-// Split form for small plain GEMMs.  With fewer tiles than SMs the persistent kernel leaves SMs idle and, worse, too few
-// weight bytes in flight (stages x BN x 128 B per CTA) to cover the HBM latency: M = 128, N = K = 4096 streamed its weight
-// at 1.2 TB/s.  Clusters of 2 to 4 CTAs share one tile, each taking a share of the K blocks; the int32 partial sums are
-// added through distributed shared memory, so the result is the same bit for bit.  Chooses the (tile width, splits)
-// pair that puts the most CTAs on the device in one wave.
 #ifdef B200DNN_TIMING_EXPERIMENTS
 constexpr size_t kStampCtas = 4096;
 unsigned long long *stamp_buffer() {
@@ -404,44 +360,82 @@ int cluster_room(K kern, int threads, int smem, int s, std::atomic<int> *cache) 
 }
 int split_room(int s) { return cluster_room(tc_gemm_kernel<true>, kTcThreads, kTcSmemBudget + 1024, s, &rt().shared->split_room[s]); }
 
-void pick_split(int m_tiles, int N, int k_blocks, int *bn, int *splits) {
-  const int forced = env_int("B200DNN_TC_KSPLIT", 0);   // 0 choose, 1 never, 2..4 that many
-  if (forced == 1) return;
-  const int sm = rt().sm_count;
-  const int room[5] = {0, 0, split_room(2), split_room(3), split_room(4)};
-  // Cost model fitted to measurements (microseconds, without the fixed cost of a launch): the stage ring is filled
-  // from L2 at about 100 GB/s per SM and 9.5 TB/s over the device (every CTA re-reads its rows of A, so wide tiles
-  // move fewer bytes); adding the partial sums costs about 1.6 us per extra CTA of the cluster and 128 columns of tile.
-  auto stream_us = [&](long long ctas, int b, int kb_per_cta, int waves) {
-    const double per_cta = (double)(kTcBM + b) * kTcBK * kb_per_cta;
-    const double dev = per_cta * (double)ctas / 9.5e6, one = per_cta * waves / 1.0e5;
-    return dev > one ? dev : one;
-  };
-  const long long tiles0 = (long long)m_tiles * ((N + *bn - 1) / *bn);
-  const double unsplit = stream_us(tiles0, *bn, k_blocks, (int)((tiles0 + sm - 1) / sm));
-  double best = forced >= 2 ? 1e30 : unsplit - 0.5;
-  int best_bn = 0, best_s = 1;
-  const int widths[3] = {256, 128, 64};
-  const int forced_bn = env_int("B200DNN_TC_BN", 0);
-  for (int w = 0; w < 3; ++w) {
-    const int b = forced_bn > 0 ? forced_bn : widths[w];
-    if (b % 32 != 0 || b < 32 || b > 256) continue;
-    const long long tiles = (long long)m_tiles * ((N + b - 1) / b);
-    for (int s = 2; s <= 4; ++s) {
-      if (forced >= 2 && s != forced) continue;
-      const int per = (k_blocks + s - 1) / s;
-      if (per * (s - 1) >= k_blocks || per < 2) continue;          // every CTA needs K blocks of its own
-      if ((b / 32) < s) continue;                                   // and at least one 32-column chunk to finish
-      if (forced < 2 && (room[s] <= 0 || tiles * s > room[s])) continue;   // one wave of resident clusters
-      const double cost = stream_us(tiles * s, b, per, 1) + 1.6 * (s - 1) * b / 128.0;
-      if (cost < best) { best = cost; best_bn = b; best_s = s; }
-    }
-  }
-  if (best_s > 1) { *bn = best_bn; *splits = best_s; }
+// ---- form and tile of a tcgen05 GEMM ------------------------------------------------------------------------------------------
+// Microseconds of one launch, fitted to 375 plain GEMMs (M 65 to 8192, K and N 512 to 14336, INT8 and bf16) in every form and width, 23 times
+// each: within 10 % (standard deviation).  A wave of tiles costs a part that grows with the width (the epilogue that nothing hides) and, per 128-byte block
+// of K, the slower of a floor (the MMAs, or what a block costs beside them: barriers, issue) and its operands' way from L2 to shared memory at the
+// measured 20.4 (17.5 in the pair form) TB/s; the last wave only what its tiles ask for.  Operands and result also have to pass DRAM.
+// bf16: wide pair tiles keep the tensor pipe so busy that the clock gives way.  Choosing by it is 0.8 % off the best form and width on average;
+// the rules before (waves times width + 16; pairs from two tiles per pair of SMs; a split model of its own) 9.5 %.  Largest differences, us: M = 3615,
+// K = 5824, N = 576 in bf16 43.0 -> 28.4; M = 825, K = 1280, N = 10752 in INT8 22.9 -> 14.6; M = 4096, K = 14336, N = 4096 201 -> 161.
+double tc_cost_us(bool pair, int bn, int splits, long long tiles, int k_blocks, double dram_bytes, bool f16) {
+  static const double floor1[8] = {0.195, 0.20, 0.20, 0.20, 0.225, 0.24, 0.295, 0.315};      // widths 32, 64 ... 256: one CTA a tile
+  static const double floor2[8] = {0.205, 0.205, 0.206, 0.208, 0.217, 0.222, 0.26, 0.29};      // a pair
+  const int i = bn / 32 - 1, kb = (k_blocks + splits - 1) / splits;
+  const long long conc = pair ? rt().sm_count / 2 : rt().sm_count, ctas = tiles * splits, full = ctas / conc, last = ctas % conc;
+  double per_kb = (pair ? floor2 : floor1)[i];
+  if (pair && f16 && bn >= 224 && tiles > conc) per_kb *= 1.08;
+  const double bytes = (double)((pair ? 256 : 128) + bn) * 128.0 / (pair ? 17.5e6 : 20.4e6);       // us per block and tile in flight
+  const double wave = (pair ? 0.63 + 1.9 * bn / 256.0 : 0.32 + 1.7 * bn / 256.0);
+  double t = pair ? 5.3 : 4.55;
+  if (splits > 1) t += 1.6 + 0.77 * (splits - 1) * bn / 128.0;
+  t += (double)full * (wave + kb * std::max(per_kb, bytes * (double)conc));
+  if (last) t += wave + kb * std::max(per_kb, bytes * (double)last);
+  const double d = 4.0 + dram_bytes / 4.15e6;
+  return std::max(t, d) + 0.15 * std::min(t, d);
 }
 
-// Rows of a row tile for a GEMM over about `rows` rows: 256 (pair form, two CTAs per tile) for large problems, else 128.
-// B200DNN_TC_PAIR: -1 (default) by size, 0 never, 1 whenever the shape allows.
+struct TcChoice { int pair, bn, splits; };
+
+// Knobs: B200DNN_TC_PAIR -1 (default) by cost, 0 never, 1 whenever the shape allows; B200DNN_TC_BN, B200DNN_TC_KSPLIT (1 never, 2 to 4 that many).
+TcChoice tc_choose(long long M, int N, int k_blocks, bool f16) {
+  const int mode = env_int("B200DNN_TC_PAIR", -1), forced_bn = env_int("B200DNN_TC_BN", 0), forced = env_int("B200DNN_TC_KSPLIT", 0);
+  const double bytes = (double)k_blocks * 128.0 * (double)(M + N) + 2.0 * (double)M * N;
+  TcChoice best{0, forced_bn > 0 ? forced_bn : 128, 1};
+  double best_us = 1e30;
+  auto consider = [&](int pair, int bn, int s) {
+    const long long tiles = ((M + (pair ? 255 : 127)) / (pair ? 256 : 128)) * ((N + bn - 1) / bn);
+    const double us = tc_cost_us(pair != 0, bn, s, tiles, k_blocks, bytes, f16);
+    if (us < best_us) { best_us = us; best = {pair, bn, s}; }
+  };
+  const bool pair_ok = N >= 128 && mode != 0 && forced < 2, single_ok = !(mode == 1 && N >= 128) || forced >= 2;
+  for (int bn = 256; bn >= 32; bn -= 32) {
+    const bool width = forced_bn > 0 ? bn == forced_bn : true;
+    if (!width) continue;
+    if (pair_ok && bn >= 64) consider(1, bn, 1);
+    if (!single_ok) continue;
+    if (forced < 2) consider(0, bn, 1);
+    if (forced == 1 || (forced_bn <= 0 && bn != 64 && bn != 128 && bn != 256)) continue;
+    // clusters of 2 to 4 CTAs share a tile, each with K blocks of its own and at least one 32-column chunk to finish; the int32 partial sums are added
+    // through distributed shared memory, so the result is the same bit for bit.  All clusters are resident at once.
+    const long long tiles = ((M + 127) / 128) * ((N + bn - 1) / bn);
+    for (int s = 2; s <= 4; ++s) {
+      const int per = (k_blocks + s - 1) / s;
+      if ((forced >= 2 && s != forced) || per * (s - 1) >= k_blocks || per < 2 || bn / 32 < s) continue;
+      if (forced < 2 && (split_room(s) <= 0 || tiles * s > split_room(s))) continue;
+      consider(0, bn, s);
+    }
+  }
+  if (best_us > 1e29 && forced_bn <= 0) consider(0, 128, 1);        // (a knob that fits no form)
+  return best;
+}
+
+// Tile width of a grouped GEMM whose row tiles (128 rows, or 256 in the pair form) are counted already.  Gated: whole 64-column gate/up blocks in every
+// CTA's part of a tile.
+int pick_bn(int m_tiles, int N, int k_blocks, int gated, int pair, bool f16) {
+  const int forced = env_int("B200DNN_TC_BN", 0);
+  if (forced > 0) return forced;
+  const int step = gated ? (pair ? 128 : 64) : 32;
+  int best = 0;
+  double best_us = 0.0;
+  for (int bn = 256; bn >= (gated ? step : 64); bn -= step) {
+    const double us = tc_cost_us(pair != 0, bn, 1, (long long)m_tiles * ((N + bn - 1) / bn), k_blocks, 0.0, f16);
+    if (best == 0 || us < best_us) { best = bn; best_us = us; }
+  }
+  return best;
+}
+
+// Rows of a row tile of a grouped GEMM over about `rows` rows: 256 (pair form, two CTAs per tile) for large problems, else 128.
 int tc_tile_rows(long long rows, int N) {
   const int mode = env_int("B200DNN_TC_PAIR", -1);
   if (mode == 0 || N < 128) return kTcBM;
@@ -466,7 +460,8 @@ int fast_act_code(const EpiParams &epi) {
   }
 }
 
-// Plain or grouped tcgen05 GEMM.  A: [M_total, lda] device, 16-byte aligned rows.  bf16 form (args.f16): K and lda count
+// Plain or grouped tcgen05 GEMM (plain: form and tile are chosen here; grouped: args.pair and m_tiles_hint, its bound on row tiles, are given).
+// A: [M_total, lda] device, 16-byte aligned rows.  bf16 form (args.f16): K and lda count
 // bytes (two per element) and pw0 holds a bf16 pack.
 int32_t launch_tc(const uint8_t *A, int64_t lda, bool a_unsigned, int M_total, int N, int K, const PackedWeight &pw0,
                   TcGemmArgs args, const EpiParams &epi, int m_tiles_hint, cudaStream_t st) {
@@ -484,9 +479,13 @@ int32_t launch_tc(const uint8_t *A, int64_t lda, bool a_unsigned, int M_total, i
 #else
   args.dbg = 0;
 #endif
-  args.BN = pick_bn(m_tiles_hint, N, R.sm_count, pw0.gated, args.pair);
+  const bool plain = args.n_groups <= 1 && !args.maps_b && !args.groups && !args.tile_prefix && !pw0.gated;
   args.k_splits = 1;
-  if (!args.pair && args.n_groups <= 1 && !args.maps_b && !args.groups && !args.tile_prefix && !pw0.gated) pick_split(m_tiles_hint, N, args.k_blocks, &args.BN, &args.k_splits);
+  if (plain) {
+    const TcChoice c = tc_choose(M_total, N, args.k_blocks, args.f16 != 0);
+    args.pair = c.pair; args.BN = c.bn; args.k_splits = c.splits;
+    args.n_groups = 1; args.m_tiles_plain = m_tiles_hint = (M_total + (c.pair ? 255 : 127)) / (c.pair ? 256 : 128);
+  } else args.BN = pick_bn(m_tiles_hint, N, args.k_blocks, pw0.gated, args.pair, args.f16 != 0);
   B2_CHECK(args.BN % 32 == 0 && args.BN >= 32 && args.BN <= 256 && (!pw0.gated || args.BN % 64 == 0), B200DNN_FAILURE,
            "bad tile width %d", args.BN);
   B2_CHECK(!args.pair || (args.BN % 32 == 0 && args.BN >= 64 && (!pw0.gated || args.BN % 128 == 0)), B200DNN_FAILURE,
@@ -1202,10 +1201,8 @@ int32_t b200dnn_matmul(const b200dnn_matmul_t *d, void *stream) {
     B2_TRY(rc);
   } else {
     TcGemmArgs ta{};
-    const int tile_rows = tc_tile_rows(M, N);
-    ta.pair = tile_rows > kTcBM ? 1 : 0;
-    ta.n_groups = 1; ta.m_tiles_plain = (M + tile_rows - 1) / tile_rows; ta.shared_dst = 1;
-    B2_TRY(launch_tc(A, lda, a_unsigned, M, N, K, pw, ta, epi, ta.m_tiles_plain, st));
+    ta.shared_dst = 1;
+    B2_TRY(launch_tc(A, lda, a_unsigned, M, N, K, pw, ta, epi, 0, st));
   }
   if (requant) {
     const int64_t n = (int64_t)M * N;

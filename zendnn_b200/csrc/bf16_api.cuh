@@ -134,11 +134,8 @@ int32_t matmul_bf16_packed(const b200dnn_matmul_t *d, const PackedWeight &pw, cu
     return finish_out({&o_dst}, st);
   }
   TcGemmArgs ta{};
-  const int tile_rows = tc_tile_rows(M, N);
-  ta.pair = tile_rows > kTcBM ? 1 : 0;
-  ta.f16 = 1;
-  ta.n_groups = 1; ta.m_tiles_plain = (M + tile_rows - 1) / tile_rows; ta.shared_dst = 1;
-  B2_TRY(launch_tc(A, lda * 2, false, M, N, 2 * K, pw, ta, epi, ta.m_tiles_plain, st));
+  ta.f16 = 1; ta.shared_dst = 1;
+  B2_TRY(launch_tc(A, lda * 2, false, M, N, 2 * K, pw, ta, epi, 0, st));
   return finish_out({&o_dst}, st);
 }
 

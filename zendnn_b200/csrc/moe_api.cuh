@@ -26,7 +26,7 @@ int32_t grouped_gemm(const uint8_t *A, int64_t lda, int R, int N, int K, const s
   ta.n_groups = G; ta.row_off = row_off_dev; ta.tile_prefix = tile_prefix_dev; ta.groups = groups_dev;
   // one tensor map per expert, in device memory
   const PackedWeight &p0 = pws[0];
-  const int BN = pick_bn(m_tiles_bound, N, Rt.sm_count, p0.gated, ta.pair);
+  const int BN = pick_bn(m_tiles_bound, N, (int)(p0.Kp / 128), p0.gated, ta.pair, f16);
   std::vector<CUtensorMap> maps(G);
   for (int g = 0; g < G; ++g) {
     B2_CHECK(pws[g].Kp == p0.Kp && pws[g].Np == p0.Np && pws[g].gated == p0.gated, B200DNN_UNIMPLEMENTED,
