@@ -263,7 +263,13 @@ enum : int { FA_GENERIC = -1, FA_NONE = 0, FA_RELU, FA_GELU_TANH, FA_GELU_ERF, F
 
 // sigmoid-family activations through one exp and one reciprocal.  gelu_tanh uses the identity
 // 0.5*x*(1+tanh(u)) = x / (1 + exp(-2u)), which has no cancellation for very negative u.
-__device__ __forceinline__ float fast_sigmoid_mul(float x, float arg) { return __fdividef(x, 1.0f + __expf(-arg)); }
+// exp(-a) = 2^(-a log2 e); x / (1 + e) = x * rcp(1 + e): an infinite e gives 0 times x.
+constexpr float kTcNegLog2e = -1.44269504088896340736f;
+__device__ __forceinline__ float tc_ex2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float tc_rcp(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float fast_sigmoid_mul(float x, float arg) {
+  return __fmul_rn(x, tc_rcp(__fadd_rn(1.0f, tc_ex2(__fmul_rn(arg, kTcNegLog2e)))));
+}
 
 template <int ACT>
 __device__ __forceinline__ float tc_act(const EpiParams &epi, float x, int m, int n) {
@@ -271,7 +277,7 @@ __device__ __forceinline__ float tc_act(const EpiParams &epi, float x, int m, in
   if (ACT == FA_RELU) return fmaxf(x, 0.0f);
   if (ACT == FA_GELU_TANH) {
     const float c = 0.79788458347320556640625f, f = 0.044715f;
-    const float inner = (c * x) * (1.0f + (f * x) * x);
+    const float inner = __fmul_rn(__fmul_rn(c, x), __fadd_rn(1.0f, __fmul_rn(__fmul_rn(f, x), x)));
     return fast_sigmoid_mul(x, 2.0f * inner);
   }
   if (ACT == FA_GELU_ERF) return po_gelu_erf(x);
@@ -289,6 +295,27 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return d;
 }
 
+// two f32 operations per instruction, each rounded as the scalar one
+__device__ __forceinline__ uint64_t tc_pack2(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ void tc_unpack2(uint64_t r, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(r)); }
+__device__ __forceinline__ uint64_t tc_mul2(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ uint64_t tc_add2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+
+// x / (1 + exp(-arg)) of two elements, arg2 already times -log2(e): the operations of fast_sigmoid_mul
+__device__ __forceinline__ uint64_t tc_sigmoid_mul2(uint64_t x2, uint64_t arg2) {
+  float a0, a1, b0, b1;
+  tc_unpack2(arg2, a0, a1);
+  tc_unpack2(tc_add2(tc_pack2(1.0f, 1.0f), tc_pack2(tc_ex2(a0), tc_ex2(a1))), b0, b1);
+  return tc_mul2(x2, tc_pack2(tc_rcp(b0), tc_rcp(b1)));
+}
+// gelu_tanh as in tc_act: the factor 2 of its argument is in the constant (exact)
+__device__ __forceinline__ uint64_t tc_gelu_tanh2(uint64_t x2) {
+  const uint64_t c2 = tc_pack2(0.79788458347320556640625f, 0.79788458347320556640625f), f2 = tc_pack2(0.044715f, 0.044715f);
+  const uint64_t inner = tc_mul2(tc_mul2(c2, x2), tc_add2(tc_pack2(1.0f, 1.0f), tc_mul2(tc_mul2(f2, x2), x2)));
+  return tc_sigmoid_mul2(x2, tc_mul2(inner, tc_pack2(2.0f * kTcNegLog2e, 2.0f * kTcNegLog2e)));
+}
+__device__ __forceinline__ uint64_t tc_swish2(uint64_t x2) { return tc_sigmoid_mul2(x2, tc_mul2(x2, tc_pack2(kTcNegLog2e, kTcNegLog2e))); }
+
 struct TileCols {          // per-tile column operands staged in shared memory
   float ws[256];
   float bias[256];
@@ -301,8 +328,13 @@ struct TileCols {          // per-tile column operands staged in shared memory
 // as two instructions that each write 16 rows x 32 contiguous bytes (whole sectors), instead of 32
 // scattered 16-byte pieces per instruction.
 // g_row0: address of the block's first row; rows_valid: how many of the 32 rows exist.
+__device__ __forceinline__ void tc_staging_free(int lane) {
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  __syncwarp();
+}
 __device__ __forceinline__ void warp_store_rows32(uint8_t *sbuf, const uint4 &v0, const uint4 &v1, uint8_t *g_row0, int64_t pitch_bytes,
                                                   int rows_valid, int lane) {
+  tc_staging_free(lane);
   const int sw = (lane >> 2) & 1;
   *reinterpret_cast<uint4 *>(sbuf + lane * 32 + ((0 ^ sw) << 4)) = v0;
   *reinterpret_cast<uint4 *>(sbuf + lane * 32 + ((1 ^ sw) << 4)) = v1;
@@ -327,6 +359,7 @@ __device__ __forceinline__ void warp_store_rows64(uint8_t *sbuf, const uint4 (&v
 // aligned words) rows instead of one element in each of 32.  M = 5000, N = 4097, K = 4096, bf16 out: 259 -> 111 us.
 // cols: how many of the block's columns exist.
 __device__ __forceinline__ void warp_stage_rows32(uint8_t *sbuf, const uint4 &v0, const uint4 &v1, int lane) {
+  tc_staging_free(lane);
   const int sw = (lane >> 2) & 1;
   *reinterpret_cast<uint4 *>(sbuf + lane * 32 + ((0 ^ sw) << 4)) = v0;
   *reinterpret_cast<uint4 *>(sbuf + lane * 32 + ((1 ^ sw) << 4)) = v1;
@@ -374,10 +407,12 @@ __device__ __forceinline__ void warp_store_any16(uint8_t *sbuf, const uint4 &v0,
   __syncwarp();
 }
 
-// The same [32 rows x 32 bytes] block as one TMA store: the lanes write their rows to the staging block (plain row-major),
-// one lane hands it to the copy engine and waits until the engine has read it.  Keeps the result off the load/store path.
+// The same [32 rows x 32 bytes] block as one TMA store: the lanes write their rows to the staging block (plain row-major) and one lane hands it
+// to the copy engine.  Keeps the result off the load/store path.  The engine reads the block while the warp works on the next one: every
+// use of the block waits for that first (tc_staging_free).
 __device__ __forceinline__ void warp_tma_store_rows32(uint8_t *sbuf, const uint4 &v0, const uint4 &v1, const CUtensorMap *map,
                                                       int x_bytes, int row, int lane) {
+  tc_staging_free(lane);
   *reinterpret_cast<uint4 *>(sbuf + lane * 32) = v0;
   *reinterpret_cast<uint4 *>(sbuf + lane * 32 + 16) = v1;
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -386,9 +421,7 @@ __device__ __forceinline__ void warp_tma_store_rows32(uint8_t *sbuf, const uint4
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
                  ::"l"(map), "r"(x_bytes), "r"(row), "r"(smem_u32(sbuf)) : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
   }
-  __syncwarp();
 }
 
 struct EpiStore {          // where this warp's rows of the current tile go
@@ -410,6 +443,12 @@ template <bool F16>
 __device__ __forceinline__ float tc_acc_f32(uint32_t r, int comp, float s_src, float w) {
   if constexpr (F16) return __uint_as_float(r);
   else return __fmul_rn(__fmul_rn((float)((int32_t)r - comp), s_src), w);
+}
+
+template <bool F16>
+__device__ __forceinline__ float tc_acc_to_f32(uint32_t r) {
+  if constexpr (F16) return __uint_as_float(r);
+  else return (float)(int32_t)r;
 }
 
 template <int ACT>
@@ -455,34 +494,53 @@ __device__ __forceinline__ void tc_epi_half(int fast_act, const EpiParams &epi, 
     return;
   }
   {
-    float x[16];
+    // accumulator -> f32: compensation, x source scale, x weight scale, + bias, one rounding per operation, two columns per instruction.  (Scalar
+    // arithmetic with selects for the operands that may be missing, 15.6 instructions an element in all, and a division per sigmoid: tiles of less than
+    // 4096 bytes of K waited for them.  9472 x 8192 with bias and GELU, K = 2048: 139 -> 123 us, K = 4096: 213 -> 197; f32 out, K = 2048: 178 -> 147.)
+    uint64_t x2[8];
+    if (has_zp) {
 #pragma unroll
-    for (int i = 0; i < 16; i += 4) {
-      // shared memory is the busiest resource of this kernel (the tensor core reads its operands from it):
-      // bias and compensation are fetched only when they exist
-      const int ci = c0 + i;
-      float4 w4 = make_float4(1.f, 1.f, 1.f, 1.f);
-      if constexpr (!F16) w4 = *reinterpret_cast<const float4 *>(&tc.ws[ci]);
-      float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
-      int4 k4 = make_int4(0, 0, 0, 0);
-      if (has_bias) b4 = *reinterpret_cast<const float4 *>(&tc.bias[ci]);
-      if (has_zp) k4 = *reinterpret_cast<const int4 *>(&tc.comp[ci]);
-      const float wv[4] = {w4.x, w4.y, w4.z, w4.w}, bv[4] = {b4.x, b4.y, b4.z, b4.w};
-      const int kv[4] = {k4.x, k4.y, k4.z, k4.w};
+      for (int i = 0; i < 16; i += 4) {
+        const int4 k4 = *reinterpret_cast<const int4 *>(&tc.comp[c0 + i]);
+        x2[i / 2] = tc_pack2((float)((int32_t)r[i] - k4.x), (float)((int32_t)r[i + 1] - k4.y));
+        x2[i / 2 + 1] = tc_pack2((float)((int32_t)r[i + 2] - k4.z), (float)((int32_t)r[i + 3] - k4.w));
+      }
+    } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float v = tc_acc_f32<F16>(r[i + j], kv[j], cx.s_src, wv[j]);
-        if (has_bias) v = __fadd_rn(v, bv[j]);
-        x[i + j] = v;
+      for (int i = 0; i < 8; ++i) x2[i] = tc_pack2(tc_acc_to_f32<F16>(r[2 * i]), tc_acc_to_f32<F16>(r[2 * i + 1]));
+    }
+    if constexpr (!F16) {
+      const uint64_t s2 = tc_pack2(cx.s_src, cx.s_src);
+#pragma unroll
+      for (int i = 0; i < 16; i += 4) {
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(&tc.ws[c0 + i]);
+        x2[i / 2] = tc_mul2(tc_mul2(x2[i / 2], s2), w.x);
+        x2[i / 2 + 1] = tc_mul2(tc_mul2(x2[i / 2 + 1], s2), w.y);
       }
     }
+    if (has_bias) {
+#pragma unroll
+      for (int i = 0; i < 16; i += 4) {
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(&tc.bias[c0 + i]);
+        x2[i / 2] = tc_add2(x2[i / 2], w.x);
+        x2[i / 2 + 1] = tc_add2(x2[i / 2 + 1], w.y);
+      }
+    }
+    if (fast_act == FA_GELU_TANH) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x2[i] = tc_gelu_tanh2(x2[i]);
+    } else if (fast_act == FA_SWISH) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x2[i] = tc_swish2(x2[i]);
+    }
+    float x[16];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) tc_unpack2(x2[i], x[2 * i], x[2 * i + 1]);
     switch (fast_act) {
-    case FA_NONE: break;
+    case FA_NONE: case FA_GELU_TANH: case FA_SWISH: break;
     case FA_RELU: tc_act16<FA_RELU>(epi, x, m_dst, pc); break;
-    case FA_GELU_TANH: tc_act16<FA_GELU_TANH>(epi, x, m_dst, pc); break;
     case FA_GELU_ERF: tc_act16<FA_GELU_ERF>(epi, x, m_dst, pc); break;
     case FA_SIGMOID: tc_act16<FA_SIGMOID>(epi, x, m_dst, pc); break;
-    case FA_SWISH: tc_act16<FA_SWISH>(epi, x, m_dst, pc); break;
     case FA_TANH: tc_act16<FA_TANH>(epi, x, m_dst, pc); break;
     default: tc_act16<FA_GENERIC>(epi, x, m_dst, pc); break;
     }
@@ -701,23 +759,45 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (gd.dst) { dst = gd.dst; ldc = gd.ldc; m_dst0 = t.m_local0; }   // else: shared dst, global row index
       }
       const int pc_tile = t.nt * a.BN;
-      float cw[8], cbv[8]; int32_t ck[8];
+      // All loads of a tile in flight at once: the types are decided outside the loops (decided inside, each load waited for the one before it and a
+      // tile took 5800 clocks here, 3000 without scales -- the bound of every tile with less than 2048 bytes of K)
+      float cw[8], cbv[8]; int32_t ck[8]; int n[8]; bool in[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        cw[j] = 1.0f; cbv[j] = 0.0f; ck[j] = 0;
         const int pc = pc_tile + lane + 32 * j;
-        if (lane + 32 * j < a.BN && pc < a.N) {
-          const int n = (int)packed_to_logical(pc, a.gated, epi.gated_I);
-          if (epi.wei_scale_n) cw[j] = load_as_f32(wsp, epi.wei_scale_dt, epi.wei_scale_n > 1 ? n : 0);
-          if (bp) cbv[j] = load_as_f32(bp, epi.bias_dt, n);
-          if (zp) ck[j] = zp * csp[pc];
-        }
+        in[j] = lane + 32 * j < a.BN && pc < a.N;
+        n[j] = in[j] ? (int)packed_to_logical(pc, a.gated, epi.gated_I) : 0;
+        cw[j] = 1.0f; cbv[j] = 0.0f; ck[j] = 0;
       }
-      float rs[4];
+      auto load8 = [&](const void *p, int32_t dt, bool one, float (&v)[8]) {
+        if (dt == DT_F32) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int r = lane + 32 * j;
-        rs[j] = (epi.src_scale_n && r < t.rows) ? load_as_f32(epi.src_scale, epi.src_scale_dt, epi.src_scale_n > 1 ? t.row0 + r : 0) : 1.0f;
+          for (int j = 0; j < 8; ++j) if (in[j]) v[j] = reinterpret_cast<const float *>(p)[one ? 0 : n[j]];
+        } else {
+          uint16_t b[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) b[j] = in[j] ? reinterpret_cast<const uint16_t *>(p)[one ? 0 : n[j]] : (uint16_t)0;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) if (in[j]) v[j] = bf16_bits_to_f32(b[j]);
+        }
+      };
+      if (epi.wei_scale_n) load8(wsp, epi.wei_scale_dt, epi.wei_scale_n == 1, cw);
+      if (bp) load8(bp, epi.bias_dt, false, cbv);
+      if (zp) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) if (in[j]) ck[j] = csp[pc_tile + lane + 32 * j];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ck[j] *= zp;
+      }
+      float rs[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+      if (epi.src_scale_n) {
+        if (epi.src_scale_dt == DT_F32) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) if (lane + 32 * j < t.rows) rs[j] = reinterpret_cast<const float *>(epi.src_scale)[epi.src_scale_n > 1 ? t.row0 + lane + 32 * j : 0];
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) if (lane + 32 * j < t.rows) rs[j] = load_as_f32(epi.src_scale, epi.src_scale_dt, epi.src_scale_n > 1 ? t.row0 + lane + 32 * j : 0);
+        }
       }
       // the buffer is free when the epilogue warps have left the tile that used it two tiles ago
       if (!__all_sync(0xffffffffu, mbar_wait(cempty_bar(cb), cphase ^ 1u))) { if (lane == 0) { s_err = 6; report_status(a.status, 6); } break; }
@@ -833,37 +913,50 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             tc_ld16(taddr0 + (uint32_t)(c * 64 + 32 + 16 * h), ru);
             tc_wait_ld();
             const int cg = c * 64 + 16 * h, cu = cg + 32;
-            uint32_t pk[8];
+            const uint64_t s2 = tc_pack2(cx.s_src, cx.s_src);
+            uint32_t pk[8], mag = 0u;
 #pragma unroll
             for (int i = 0; i < 16; i += 4) {
-              const float4 wg4 = *reinterpret_cast<const float4 *>(&tcols.ws[cg + i]);
-              const float4 wu4 = *reinterpret_cast<const float4 *>(&tcols.ws[cu + i]);
-              const float wg[4] = {wg4.x, wg4.y, wg4.z, wg4.w}, wu[4] = {wu4.x, wu4.y, wu4.z, wu4.w};
-              float bg[4] = {0.f, 0.f, 0.f, 0.f}, bu[4] = {0.f, 0.f, 0.f, 0.f};
+              uint64_t g2[2], u2[2];
+#pragma unroll
+              for (int j = 0; j < 2; ++j) {
+                g2[j] = tc_pack2(tc_acc_to_f32<F16>(rg[i + 2 * j]), tc_acc_to_f32<F16>(rg[i + 2 * j + 1]));
+                u2[j] = tc_pack2(tc_acc_to_f32<F16>(ru[i + 2 * j]), tc_acc_to_f32<F16>(ru[i + 2 * j + 1]));
+              }
+              if constexpr (!F16) {
+                const ulonglong2 wg = *reinterpret_cast<const ulonglong2 *>(&tcols.ws[cg + i]), wu = *reinterpret_cast<const ulonglong2 *>(&tcols.ws[cu + i]);
+                g2[0] = tc_mul2(tc_mul2(g2[0], s2), wg.x); g2[1] = tc_mul2(tc_mul2(g2[1], s2), wg.y);
+                u2[0] = tc_mul2(tc_mul2(u2[0], s2), wu.x); u2[1] = tc_mul2(tc_mul2(u2[1], s2), wu.y);
+              }
               if (has_bias) {
-                const float4 bg4 = *reinterpret_cast<const float4 *>(&tcols.bias[cg + i]);
-                const float4 bu4 = *reinterpret_cast<const float4 *>(&tcols.bias[cu + i]);
-                bg[0] = bg4.x; bg[1] = bg4.y; bg[2] = bg4.z; bg[3] = bg4.w;
-                bu[0] = bu4.x; bu[1] = bu4.y; bu[2] = bu4.z; bu[3] = bu4.w;
+                const ulonglong2 bg = *reinterpret_cast<const ulonglong2 *>(&tcols.bias[cg + i]), bu = *reinterpret_cast<const ulonglong2 *>(&tcols.bias[cu + i]);
+                g2[0] = tc_add2(g2[0], bg.x); g2[1] = tc_add2(g2[1], bg.y);
+                u2[0] = tc_add2(u2[0], bu.x); u2[1] = tc_add2(u2[1], bu.y);
               }
-              float z[4];
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                float gv = tc_acc_f32<F16>(rg[i + j], 0, cx.s_src, wg[j]);
-                float uv = tc_acc_f32<F16>(ru[i + j], 0, cx.s_src, wu[j]);
-                if (has_bias) { gv = __fadd_rn(gv, bg[j]); uv = __fadd_rn(uv, bu[j]); }
-                if (epi.gated_act == ACT_SILU_MUL) z[j] = __fmul_rn(fast_sigmoid_mul(gv, gv), uv);
-                else z[j] = gated_f32(epi.gated_act, gv, uv);
-              }
-              pk[i >> 1] = pack_bf16x2(z[0], z[1]);
-              pk[(i >> 1) + 1] = pack_bf16x2(z[2], z[3]);
+              for (int j = 0; j < 2; ++j) {
+                float z[2];
+                if (epi.gated_act == ACT_SILU_MUL) tc_unpack2(tc_mul2(tc_swish2(g2[j]), u2[j]), z[0], z[1]);
+                else {
+                  float gv[2], uv[2];
+                  tc_unpack2(g2[j], gv[0], gv[1]);
+                  tc_unpack2(u2[j], uv[0], uv[1]);
 #pragma unroll
-              for (int q2 = 0; q2 < 2; ++q2) {
-                uint32_t mag = pk[(i >> 1) + q2] & 0x7FFF7FFFu;
-                mag &= ~__vcmpgeu2(mag, 0x7F807F80u);          // infinities and NaNs do not enter the maximum
-                amax2 = __vmaxu2(amax2, mag);
+                  for (int e = 0; e < 2; ++e) z[e] = gated_f32(epi.gated_act, gv[e], uv[e]);
+                }
+                pk[(i >> 1) + j] = pack_bf16x2(z[0], z[1]);
+                mag = __vmaxu2(mag, pk[(i >> 1) + j] & 0x7FFF7FFFu);
               }
             }
+            if (max(mag & 0xFFFFu, mag >> 16) >= 0x7F80u) {      // infinities and NaNs do not enter the maximum
+              mag = 0u;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const uint32_t m = pk[i] & 0x7FFF7FFFu;
+                mag = __vmaxu2(mag, m & ~__vcmpgeu2(m, 0x7F807F80u));
+              }
+            }
+            amax2 = __vmaxu2(amax2, mag);
             const int jc = j0 + 16 * h;
             if (es.map_c && es.rows_valid == 32) {
               warp_tma_store_rows32(es.sbuf, make_uint4(pk[0], pk[1], pk[2], pk[3]), make_uint4(pk[4], pk[5], pk[6], pk[7]), es.map_c,
