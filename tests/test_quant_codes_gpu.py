@@ -45,3 +45,29 @@ def test_f32_beside_the_middle_of_two_codes(oracle, K, rows):
         x[r, 5] = absmax
     x[0, 9], x[0, 10] = np.nan, np.inf
     _check(oracle, x, "f32", K)
+
+
+# a warp and a CTA per row, one and two vectors past a multiple, the longest rows of a warp, rows beyond a CTA's registers
+@pytest.mark.parametrize("dt", ["bf16", "f32"])
+@pytest.mark.parametrize("rows,K", [(70, 1), (70, 17), (64, 1999), (64, 2047), (5, 1001), (5, 4097), (64, 16385 + 8)])
+def test_rows_of_any_alignment(oracle, dt, rows, K):
+    """Source rows that start and end anywhere, into rows of codes that start on a vector: the bytes behind a row of codes stay as they were."""
+    import torch
+    from zendnn_b200 import capi
+    rng = np.random.default_rng(K)
+    ld, dld = K + 3, (K + 15) // 16 * 16 + 16
+    full = rng.normal(size=(rows, ld)).astype(np.float32)
+    full[rows // 2, K - 1], full[0, 0] = 50.0, np.inf if K > 1 else 3.0
+    if dt == "bf16":
+        full = oracle.f32_to_bf16(full)
+    x = np.concatenate([full[:1].ravel()[:1], full.ravel()])           # one element in front: no row is aligned to more than an element
+    dev = torch.from_numpy(x.view(np.int16 if dt == "bf16" else np.int32)).cuda()
+    q = torch.full((rows, dld), 99, dtype=torch.int8, device="cuda")
+    s = torch.zeros(rows, device="cuda")
+    es = 2 if dt == "bf16" else 4
+    capi.check(capi.lib.b200dnn_quant_per_token(dev.data_ptr() + es, capi.DT[dt], rows, K, ld, q.data_ptr(), dld, s.data_ptr(), capi.DT["f32"],
+                                                torch.cuda.current_stream().cuda_stream))
+    q_ref, s_ref = oracle.quant_per_token(np.ascontiguousarray(full[:, :K]))
+    assert (s.cpu().numpy() == s_ref).all()
+    got = q.cpu().numpy()
+    assert (got[:, :K] == q_ref).all() and (got[:, K:] == 99).all()

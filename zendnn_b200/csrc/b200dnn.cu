@@ -171,11 +171,14 @@ int32_t launch_quant_rows_t(const RowQuantArgs &a, int32_t src_dt, int64_t rows,
     B2_CUDA(cudaGetLastError());
     return B200DNN_SUCCESS;
   }
-  if (aligned && rows >= 64 && a.K / E <= 32 * 16 && (src_dt == B200DNN_BF16 || src_dt == B200DNN_F32)) {
-    const int nv = (a.K / E + 31) / 32;
+  // rows of any alignment (an odd K, say): vectors put together from words instead of element by element
+  const bool any = !EP && !aligned && a.n_groups == 0 && !a.scatter && !a.absmax_bits && (!a.dst || (reinterpret_cast<uintptr_t>(a.dst) % E == 0 && a.dst_ld % E == 0));
+  if ((aligned || any) && rows >= 64 && a.K <= 32 * 16 * E && (src_dt == B200DNN_BF16 || src_dt == B200DNN_F32)) {
+    const int nv = (a.K + 32 * E - 1) / (32 * E);
     unsigned grid = (unsigned)((rows + 7) / 8);
     if (EP && a.n_rows_dev && grid > (unsigned)(rt().sm_count * 16)) grid = (unsigned)(rt().sm_count * 16);   // the warps stride over the rows
-#define B2_QW(T, NV) B2_TRY((launch_pdl(quant_per_token_warp_kernel<T, NV, EP>, grid, 256, 0, st, !EP, a, (int)rows)))
+#define B2_QW(T, NV) do { if (any) B2_TRY((launch_pdl(quant_per_token_warp_kernel<T, NV, false, true>, grid, 256, 0, st, true, a, (int)rows))); \
+                          else B2_TRY((launch_pdl(quant_per_token_warp_kernel<T, NV, EP>, grid, 256, 0, st, !EP, a, (int)rows))); } while (0)
     if (src_dt == B200DNN_BF16) { if (nv <= 2) B2_QW(uint16_t, 2); else if (nv <= 4) B2_QW(uint16_t, 4); else if (nv <= 8) B2_QW(uint16_t, 8); else B2_QW(uint16_t, 16); }
     else { if (nv <= 2) B2_QW(float, 2); else if (nv <= 4) B2_QW(float, 4); else if (nv <= 8) B2_QW(float, 8); else B2_QW(float, 16); }
 #undef B2_QW
@@ -183,7 +186,7 @@ int32_t launch_quant_rows_t(const RowQuantArgs &a, int32_t src_dt, int64_t rows,
     B2_CUDA(cudaGetLastError());
     return B200DNN_SUCCESS;
   }
-  const int nvec = a.K / E;
+  const int nvec = (a.K + E - 1) / E;
   const bool short_row = nvec <= 2 * kQuantThreads;     // the whole row fits two cached vectors per thread
   // few long rows (fewer than SMs): as many threads as keep a row in two vectors each, see quant_per_token_kernel
   const bool wide = !short_row && rows <= rt().sm_count;
@@ -704,14 +707,27 @@ __global__ void transpose_src_kernel(const T *src, int64_t lda, int M, int K, T 
   }
 }
 
-// INT8 rows that are not 16-byte aligned, copied to a pitch the copy engine takes (16-byte multiple, zero-padded): 16 bytes per thread
-__global__ void __launch_bounds__(256) repitch_rows_u8_kernel(const uint8_t *src, int64_t src_ld, uint8_t *dst, int pitch, int rows, int cols) {
+// Rows that are not 16-byte aligned, copied to a pitch the copy engine takes (16-byte multiple, zero-padded): 16 bytes per thread, counted in bytes.
+// Launched with overlap: the launch hides behind the kernel in front, and the GEMM behind it may start early (the trigger comes after the wait, so
+// whatever such a GEMM reads before its own wait was written by work that is complete).
+__global__ void __launch_bounds__(256) repitch_rows_kernel(const uint8_t *src, int64_t src_ld, uint8_t *dst, int pitch, int rows, int cols) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int segs = pitch >> 4;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)rows * segs) return;
   const int r = (int)(i / segs), k = (int)(i - (int64_t)r * segs) * 16;
   *reinterpret_cast<uint4 *>(dst + (int64_t)r * pitch + k) = ld16_any(src + (int64_t)r * src_ld + k, cols - k);
+}
+// rows of `cols` bytes, `ld` apart -> workspace rows, *pitch apart
+int32_t repitch_rows(const uint8_t *src, int64_t ld, int rows, int cols, cudaStream_t st, const uint8_t **out, int64_t *pitch) {
+  *pitch = round_up(cols, 16);
+  uint8_t *tmp = (uint8_t *)rt().ws.alloc((size_t)rows * *pitch);
+  B2_CHECK(tmp, B200DNN_FAILURE, "workspace allocation failed");
+  B2_TRY(launch_pdl(repitch_rows_kernel, (unsigned)(((int64_t)rows * (*pitch / 16) + 255) / 256), 256u, 0, st, true, src, ld, tmp, (int)*pitch, rows, cols));
+  B2_LAUNCHED();
+  *out = tmp;
+  return B200DNN_SUCCESS;
 }
 
 int32_t untranspose_source(const b200dnn_matmul_t *d, b200dnn_matmul_t *t, cudaStream_t st) {
@@ -1156,13 +1172,7 @@ int32_t b200dnn_matmul(const b200dnn_matmul_t *d, void *stream) {
   // Rows that the copy engine cannot read in place (K or lda not a multiple of 16) are copied to such a pitch first: one pass over the
   // activations, against a weight stream per 16 rows in the tiled streaming kernel (M = 500, K = 1999, N = 3001: 86 us with it).
   if (d->force_kernel == 0 && M > 16 && ((lda % 16 != 0) || (reinterpret_cast<uintptr_t>(A) & 15) != 0)) {
-    const int64_t pitch = round_up(K, 16);
-    uint8_t *tmp = (uint8_t *)R.ws.alloc((size_t)M * pitch);
-    B2_CHECK(tmp, B200DNN_FAILURE, "workspace allocation failed");
-    repitch_rows_u8_kernel<<<(unsigned)(((int64_t)M * (pitch / 16) + 255) / 256), 256, 0, st>>>(A, lda, tmp, (int)pitch, M, K);
-    B2_LAUNCHED();
-    B2_CUDA(cudaGetLastError());
-    A = tmp; lda = pitch;
+    B2_TRY(repitch_rows(A, lda, M, K, st, &A, &lda));
   }
   const bool tc_ok = (lda % 16 == 0) && ((reinterpret_cast<uintptr_t>(A) & 15) == 0);
   int which = d->force_kernel;

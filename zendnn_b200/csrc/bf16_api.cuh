@@ -52,14 +52,6 @@ int32_t resolve_bf16_weight(const void *weight, int64_t K, int64_t N, int64_t ld
   return B200DNN_SUCCESS;
 }
 
-// rows of 2-byte elements copied to a pitch the copy engine accepts (16-byte multiple, 16-byte aligned base)
-__global__ void repitch_rows_u16_kernel(const uint16_t *src, int64_t src_ld, uint16_t *dst, int64_t dst_ld, int64_t rows, int64_t cols) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * dst_ld) return;
-  const int64_t r = i / dst_ld, c = i - r * dst_ld;
-  dst[i] = c < cols ? src[r * src_ld + c] : (uint16_t)0;
-}
-
 int32_t validate_bf16_matmul(const b200dnn_matmul_t *d) {
   const int M = d->M, N = d->N, K = d->K;
   B2_CHECK(d->src && d->weight && d->dst, B200DNN_FAILURE, "null src, weight or dst");
@@ -118,14 +110,8 @@ int32_t matmul_bf16_packed(const b200dnn_matmul_t *d, const PackedWeight &pw, cu
   const uint8_t *A = (const uint8_t *)src_dev;
   int64_t lda = d->lda;
   if ((reinterpret_cast<uintptr_t>(A) & 15) != 0 || (lda * 2) % 16 != 0) {
-    const int64_t ld2 = round_up(K, 8);
-    uint16_t *tmp = (uint16_t *)R.ws.alloc((size_t)M * ld2 * 2);
-    B2_CHECK(tmp, B200DNN_FAILURE, "workspace allocation failed");
-    const int64_t n = (int64_t)M * ld2;
-    repitch_rows_u16_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>((const uint16_t *)src_dev, d->lda, tmp, ld2, M, K);
-    B2_LAUNCHED();
-    B2_CUDA(cudaGetLastError());
-    A = (const uint8_t *)tmp; lda = ld2;
+    B2_TRY(repitch_rows(A, lda * 2, M, 2 * K, st, &A, &lda));
+    lda /= 2;
   }
   // few rows (skinny_gemm.cuh); M = 96, K = 4096, N = 11008: 24.7 us in the tile kernel, 27.3 there
   if (d->force_kernel == 0 && M <= 64 && few_rows_pay(M, N, 2ll * K)) {

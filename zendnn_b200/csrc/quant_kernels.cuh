@@ -106,6 +106,15 @@ __device__ __forceinline__ typename VecTraits<T>::Codes quant_vec(const uint4 &q
   }
 }
 
+// the first n codes of a vector
+template <typename T>
+__device__ __forceinline__ void put_codes_tail(int8_t *p, typename VecTraits<T>::Codes o, int n) {
+  uint32_t w[2];
+  if constexpr (sizeof(T) == 2) { w[0] = o.x; w[1] = o.y; } else { w[0] = o; w[1] = 0u; }
+#pragma unroll
+  for (int i = 0; i < VecTraits<T>::kPer16B - 1; ++i) if (i < n) p[i] = (int8_t)(w[i >> 2] >> (8 * (i & 3)));
+}
+
 // Abs-max over the finite elements, on the bit patterns (magnitudes order like integers; bf16: two per instruction).  add() takes every
 // element; when the maximum turns out not to be finite, the caller goes over its elements again with add_finite().
 template <typename T> struct AbsMax {
@@ -216,9 +225,14 @@ __global__ void __launch_bounds__(THR, THR > kQuantThreads ? 1 : (NV > 2 ? (EP ?
   const int32_t *sp = (EP && sc && a.scatter_peer) ? a.scatter_peer + (int64_t)r * a.scatter_n : nullptr;
   if (sc) dst = sp ? a.peer_dst[0] : a.dst;     // row offsets (and the peer's base) are applied per destination
   const int K = a.K;
-  const bool vec = ((reinterpret_cast<uintptr_t>(src) & 15) == 0) && (K % E == 0) &&
-                   (!dst || (reinterpret_cast<uintptr_t>(dst) % E) == 0);
-  const int nvec = vec ? K / E : 0;
+  // whole vectors of the destination; the source's rows may lie anywhere (their vectors are then put together from words, the last one with zeros)
+  const bool src_vec = ((reinterpret_cast<uintptr_t>(src) & 15) == 0) && (K % E == 0);
+  const bool vec = (src_vec || (!EP && !sc)) && (!dst || (reinterpret_cast<uintptr_t>(dst) % E) == 0);
+  const int nvec = vec ? (K + E - 1) / E : 0;
+  auto load_vec = [&](int v) {
+    if (src_vec) return reinterpret_cast<const uint4 *>(src)[v];
+    return ld16_any(reinterpret_cast<const uint8_t *>(src) + (int64_t)v * 16, (K - v * E) * (int)sizeof(T));
+  };
   uint4 cache[NV];
   AbsMax<T> amax;
   const bool need_amax = a.absmax_bits == nullptr;   // the row maximum may be given
@@ -226,17 +240,17 @@ __global__ void __launch_bounds__(THR, THR > kQuantThreads ? 1 : (NV > 2 ? (EP ?
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
       const int v = threadIdx.x + j * THR;
-      cache[j] = v < nvec ? reinterpret_cast<const uint4 *>(src)[v] : make_uint4(0u, 0u, 0u, 0u);
+      cache[j] = v < nvec ? load_vec(v) : make_uint4(0u, 0u, 0u, 0u);
     }
     if (need_amax) {
 #pragma unroll
       for (int j = 0; j < NV; ++j) amax.add(cache[j]);
-      for (int v = threadIdx.x + NV * THR; v < nvec; v += THR) amax.add(reinterpret_cast<const uint4 *>(src)[v]);
+      for (int v = threadIdx.x + NV * THR; v < nvec; v += THR) amax.add(load_vec(v));
       if (!amax.finite()) {
         amax.m = 0u;
 #pragma unroll
         for (int j = 0; j < NV; ++j) amax.add_finite(cache[j]);
-        for (int v = threadIdx.x + NV * THR; v < nvec; v += THR) amax.add_finite(reinterpret_cast<const uint4 *>(src)[v]);
+        for (int v = threadIdx.x + NV * THR; v < nvec; v += THR) amax.add_finite(load_vec(v));
       }
     }
   } else {
@@ -281,7 +295,8 @@ __global__ void __launch_bounds__(THR, THR > kQuantThreads ? 1 : (NV > 2 ? (EP ?
         for (int j = 0; j < a.scatter_n; ++j) { const int d = sc[j]; if (d >= 0 && d < a.scatter_cap) put(a.peer_dst[sp[j]] + (int64_t)d * a.dst_ld, o, v); }
       } else if (sc) {
         for (int j = 0; j < a.scatter_n; ++j) { const int d = sc[j]; if (d >= 0) put(dst + (int64_t)d * a.dst_ld, o, v); }
-      } else put(dst, o, v);
+      } else if ((v + 1) * E <= K) put(dst, o, v);
+      else put_codes_tail<T>(dst + v * E, o, K - v * E);
     };
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
@@ -289,7 +304,7 @@ __global__ void __launch_bounds__(THR, THR > kQuantThreads ? 1 : (NV > 2 ? (EP ?
       if (v < nvec) emit(cache[j], v);
     }
     for (int v = threadIdx.x + NV * THR; v < nvec; v += THR)
-      emit(reinterpret_cast<const uint4 *>(src)[v], v);
+      emit(load_vec(v), v);
   } else {
     for (int k = threadIdx.x; k < K; k += THR) {
       const int8_t qv = quant_sym_r<T>(elem_to_f32<T>(src[k]), scale, rinv);
@@ -391,8 +406,9 @@ __global__ void __launch_bounds__(256) quant_known_absmax_kernel(RowQuantArgs a,
 // One warp per row, for rows of at most 32 * NV vectors: the row lives in the lanes' registers (all its loads in flight), the abs-max is one warp
 // reduction, no shared memory and no CTA barrier.  Bound by HBM: 8192 x 4096 bf16 19.8 us, 16384 x 2048 17.3 us (5.1 and 5.8 TB/s of the
 // 3 bytes an element; 41.1 and 37.7 us with float maxima, tie tests and divisions).
-// Requires 16-byte aligned rows and K a multiple of the vector width (the launcher checks).
-template <typename T, int NV, bool EP>
+// Destination rows start on a vector of codes.  ANY: source rows of any alignment and length (no scatter): vectors are put together from aligned words;
+// otherwise 16-byte aligned rows and K a multiple of the vector width (the launcher checks).
+template <typename T, int NV, bool EP, bool ANY = false>
 __global__ void __launch_bounds__(256) quant_per_token_warp_kernel(RowQuantArgs a, int rows) {
   constexpr int E = VecTraits<T>::kPer16B;
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -406,12 +422,13 @@ __global__ void __launch_bounds__(256) quant_per_token_warp_kernel(RowQuantArgs 
   const int32_t *sc = a.scatter ? a.scatter + (int64_t)r * a.scatter_n : nullptr;
   const int32_t *sp = (EP && sc && a.scatter_peer) ? a.scatter_peer + (int64_t)r * a.scatter_n : nullptr;
   int8_t *dst = sp ? a.peer_dst[0] : (a.dst ? (sc ? a.dst : a.dst + (int64_t)r * a.dst_ld) : nullptr);
-  const int nvec = a.K / E;
+  const int nvec = ANY ? (a.K + E - 1) / E : a.K / E;
   uint4 cache[NV];
 #pragma unroll
   for (int j = 0; j < NV; ++j) {
     const int v = lane + j * 32;
-    cache[j] = v < nvec ? reinterpret_cast<const uint4 *>(src)[v] : make_uint4(0, 0, 0, 0);
+    if constexpr (ANY) cache[j] = v < nvec ? ld16_any(reinterpret_cast<const uint8_t *>(src) + (int64_t)v * 16, (a.K - v * E) * (int)sizeof(T)) : make_uint4(0, 0, 0, 0);
+    else cache[j] = v < nvec ? reinterpret_cast<const uint4 *>(src)[v] : make_uint4(0, 0, 0, 0);
   }
   float scale;
   if (a.absmax_bits) scale = scale_from_absmax(__uint_as_float(a.absmax_bits[r]));
@@ -459,8 +476,13 @@ __global__ void __launch_bounds__(256) quant_per_token_warp_kernel(RowQuantArgs 
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < NV; ++j)
-      if (lane + j * 32 < nvec) reinterpret_cast<Codes *>(dst)[lane + j * 32] = quant_vec<T>(cache[j], scale, rinv);
+    for (int j = 0; j < NV; ++j) {
+      const int v = lane + j * 32;
+      if (v >= nvec) continue;
+      const Codes o = quant_vec<T>(cache[j], scale, rinv);
+      if (!ANY || (v + 1) * E <= a.K) reinterpret_cast<Codes *>(dst)[v] = o;
+      else put_codes_tail<T>(dst + v * E, o, a.K - v * E);
+    }
   }
   }   // rows of this warp
 }
