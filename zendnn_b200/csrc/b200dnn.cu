@@ -145,8 +145,7 @@ int32_t resolve_weight(const void *weight, int wei_format, int64_t K, int64_t N,
 template <bool EP>
 int32_t launch_quant_rows_t(const RowQuantArgs &a, int32_t src_dt, int64_t rows, cudaStream_t st) {
   if (rows <= 0) return B200DNN_SUCCESS;
-  // aligned, non-grouped rows of up to 16 vectors a lane (bf16: 4096 elements): one warp per row.  Against a CTA per row, us, bf16: 8192 x 4096 19.8
-  // and 23.8, 5092 x 2688 11.5 and 13.8, 512 x 4096 5.0 and 7.5.
+  // a warp per row takes aligned, non-grouped rows of up to 16 vectors a lane (bf16: 4096 elements)
   const int E = src_dt == B200DNN_BF16 ? 8 : 4;
   const bool aligned = a.n_groups == 0 && a.K % E == 0 && (reinterpret_cast<uintptr_t>(a.src) & 15) == 0 &&
                        (a.src_ld * (src_dt == B200DNN_BF16 ? 2 : 4)) % 16 == 0 &&
@@ -171,16 +170,28 @@ int32_t launch_quant_rows_t(const RowQuantArgs &a, int32_t src_dt, int64_t rows,
     B2_CUDA(cudaGetLastError());
     return B200DNN_SUCCESS;
   }
+  B2_CHECK(src_dt == B200DNN_BF16 || (!EP && src_dt == B200DNN_F32), B200DNN_UNIMPLEMENTED, "per-token quantisation takes f32 or bf16 input");
   // rows of any alignment (an odd K, say): vectors put together from words instead of element by element
   const bool any = !EP && !aligned && a.n_groups == 0 && !a.scatter && !a.absmax_bits && (!a.dst || (reinterpret_cast<uintptr_t>(a.dst) % E == 0 && a.dst_ld % E == 0));
-  if ((aligned || any) && rows >= 64 && a.K <= 32 * 16 * E && (src_dt == B200DNN_BF16 || src_dt == B200DNN_F32)) {
-    const int nv = (a.K + 32 * E - 1) / (32 * E);
+  // A warp per row or a CTA per row.  A warp's chain is the longer one; it pays where the CTAs of two launches, which overlap, no longer fit the chip at
+  // once (three a SM and launch), with nine to sixteen vectors a lane where those of one do not.  Device time, us, CTA and warp, bf16: K = 1024 400 rows
+  // 1.8 and 1.9, 448 rows 2.3 and 1.9; K = 2048 128 rows 1.6 and 2.4, 512 rows 2.6 and 2.4, 4096 rows 8.3 and 4.5; K = 4096 128 rows 1.8 and 3.5, 1024
+  // rows 3.6 and 3.8, 4096 rows 10.6 and 8.8; scattered to two places, K = 4096, 880 rows 4.0 and 4.7, 900 rows 4.8 and 4.7.  Vectors put together from words take a
+  // warp longer still: K = 1021 640 rows 2.7 and 2.9, 4096 rows 8.5 and 6.4; K = 2045 1024 rows 3.9 and 5.2, K = 4093 4096 rows 15 and 25.
+  // B200DNN_QUANT_WARP: -1 by these lines, 0 never, 1 whenever the row fits.
+  const int nv = (a.K + 32 * E - 1) / (32 * E), qw = env_int("B200DNN_QUANT_WARP", -1), sms = rt().sm_count;      // nv: vectors a lane
+  const long long line = any ? (nv <= 2 ? 3 : 7) * sms : nv <= 2 ? 64 : (nv <= 8 ? 3 : a.scatter ? 6 : 7) * sms;
+  if ((aligned ? nv <= 16 : any && nv <= 4) && (qw < 0 ? rows >= line : qw != 0)) {
     unsigned grid = (unsigned)((rows + 7) / 8);
-    if (EP && a.n_rows_dev && grid > (unsigned)(rt().sm_count * 16)) grid = (unsigned)(rt().sm_count * 16);   // the warps stride over the rows
-#define B2_QW(T, NV) do { if (any) B2_TRY((launch_pdl(quant_per_token_warp_kernel<T, NV, false, true>, grid, 256, 0, st, true, a, (int)rows))); \
-                          else B2_TRY((launch_pdl(quant_per_token_warp_kernel<T, NV, EP>, grid, 256, 0, st, !EP, a, (int)rows))); } while (0)
-    if (src_dt == B200DNN_BF16) { if (nv <= 2) B2_QW(uint16_t, 2); else if (nv <= 4) B2_QW(uint16_t, 4); else if (nv <= 8) B2_QW(uint16_t, 8); else B2_QW(uint16_t, 16); }
-    else { if (nv <= 2) B2_QW(float, 2); else if (nv <= 4) B2_QW(float, 4); else if (nv <= 8) B2_QW(float, 8); else B2_QW(float, 16); }
+    if (EP && a.n_rows_dev && grid > (unsigned)(sms * 16)) grid = (unsigned)(sms * 16);   // the warps stride over the rows
+#define B2_QW(T, NV) B2_TRY((launch_pdl(quant_per_token_warp_kernel<T, NV, EP>, grid, 256, 0, st, !EP, a, (int)rows)))
+#define B2_QWA(T, NV) B2_TRY((launch_pdl(quant_per_token_warp_kernel<T, NV, false, true>, grid, 256, 0, st, true, a, (int)rows)))
+    if (any) {      // (not in the expert-parallel forms)
+      if (src_dt == B200DNN_BF16) { if (nv <= 2) B2_QWA(uint16_t, 2); else B2_QWA(uint16_t, 4); }
+      else { if (nv <= 2) B2_QWA(float, 2); else B2_QWA(float, 4); }
+    } else if (src_dt == B200DNN_BF16) { if (nv <= 2) B2_QW(uint16_t, 2); else if (nv <= 4) B2_QW(uint16_t, 4); else if (nv <= 8) B2_QW(uint16_t, 8); else B2_QW(uint16_t, 16); }
+    else if constexpr (!EP) { if (nv <= 2) B2_QW(float, 2); else if (nv <= 4) B2_QW(float, 4); else if (nv <= 8) B2_QW(float, 8); else B2_QW(float, 16); }
+#undef B2_QWA
 #undef B2_QW
     B2_LAUNCHED();
     B2_CUDA(cudaGetLastError());
@@ -189,13 +200,21 @@ int32_t launch_quant_rows_t(const RowQuantArgs &a, int32_t src_dt, int64_t rows,
   const int nvec = (a.K + E - 1) / E;
   const bool short_row = nvec <= 2 * kQuantThreads;     // the whole row fits two cached vectors per thread
   // few long rows (fewer than SMs): as many threads as keep a row in two vectors each, see quant_per_token_kernel
-  const bool wide = !short_row && rows <= rt().sm_count;
+  const bool wide = !short_row && rows <= sms;
   unsigned grid_rows = (unsigned)rows;
-  if (EP && a.n_rows_dev && grid_rows > (unsigned)(rt().sm_count * 32)) grid_rows = (unsigned)(rt().sm_count * 32);   // the CTAs stride over the rows
-#define B2_QR(T, NV, THR) B2_TRY((launch_pdl(quant_per_token_kernel<T, NV, EP, THR>, grid_rows, THR, 0, st, !EP, a)))
-  if (src_dt == B200DNN_BF16) { if (short_row) B2_QR(uint16_t, 2, kQuantThreads); else if (wide) B2_QR(uint16_t, 2, 1024); else B2_QR(uint16_t, kQuantRegVec, kQuantThreads); }
-  else if (src_dt == B200DNN_F32) { if (short_row) B2_QR(float, 2, kQuantThreads); else if (wide) B2_QR(float, 2, 1024); else B2_QR(float, kQuantRegVec, kQuantThreads); }
-  else return fail(B200DNN_UNIMPLEMENTED, "per-token quantisation takes f32 or bf16 input");
+  if (EP && a.n_rows_dev && grid_rows > (unsigned)(sms * 32)) grid_rows = (unsigned)(sms * 32);   // the CTAs stride over the rows
+  // rows that do not all start on 16 bytes, or whose length is no multiple of a vector
+  const bool src_any = !EP && !a.scatter && (a.K % E != 0 || (a.n_groups > 0 ? a.g_any != 0 : ((reinterpret_cast<uintptr_t>(a.src) | (uintptr_t)(a.src_ld * (16 / E))) & 15) != 0));
+#define B2_QR(T, NV, FORM, THR, ANY) B2_TRY((launch_pdl(quant_per_token_kernel<T, NV, FORM, THR, ANY>, grid_rows, THR, 0, st, !EP, a)))
+#define B2_QRF(T, NV, THR) do { \
+    if constexpr (EP) B2_QR(T, NV, kRowsPeers, THR, false); \
+    else if (a.n_groups > 0) { if (src_any) B2_QR(T, NV, kRowsGroups, THR, true); else B2_QR(T, NV, kRowsGroups, THR, false); } \
+    else if (a.scatter) B2_QR(T, NV, kRowsScatter, THR, false); \
+    else if (src_any) B2_QR(T, NV, kRowsPlain, THR, true); \
+    else B2_QR(T, NV, kRowsPlain, THR, false); } while (0)
+  if (src_dt == B200DNN_BF16) { if (short_row) B2_QRF(uint16_t, 2, kQuantThreads); else if (wide) B2_QRF(uint16_t, 2, 1024); else B2_QRF(uint16_t, kQuantRegVec, kQuantThreads); }
+  else if constexpr (!EP) { if (short_row) B2_QRF(float, 2, kQuantThreads); else if (wide) B2_QRF(float, 2, 1024); else B2_QRF(float, kQuantRegVec, kQuantThreads); }
+#undef B2_QRF
 #undef B2_QR
   B2_LAUNCHED();
   B2_CUDA(cudaGetLastError());
@@ -876,6 +895,8 @@ int32_t b200dnn_group_quant_per_token(int32_t num_groups, const void *const *src
     a.g_src = (const void *const *)tab; a.g_dst = (void *const *)(tab + tb); a.g_scale = (void *const *)(tab + 2 * tb);
     a.g_src_ld = (const int64_t *)(tab + 3 * tb); a.g_dst_ld = (const int64_t *)(tab + 3 * tb + sizeof(int64_t) * num_groups);
     a.row_off = (const int32_t *)(tab + 3 * tb + 2 * sizeof(int64_t) * num_groups);
+    for (int g = 0; g < num_groups; ++g)
+      if (row_off[g + 1] > row_off[g] && ((reinterpret_cast<uintptr_t>(s_dev[g]) | (uintptr_t)(src_ld[g] * dt_size(src_dt))) & 15) != 0) a.g_any = 1;
     B2_TRY(launch_quant_rows(a, src_dt, row_off[num_groups], st));
   }
   bool any = false;

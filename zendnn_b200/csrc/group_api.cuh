@@ -116,6 +116,8 @@ int32_t group_matmul_grouped(int G, const b200dnn_matmul_t *d, void *stream) {
     a.g_src = (const void *const *)t; a.g_dst = (void *const *)(t + tb); a.g_scale = (void *const *)(t + 2 * tb);
     a.g_src_ld = (const int64_t *)(t + 3 * tb); a.g_dst_ld = (const int64_t *)(t + 3 * tb + sizeof(int64_t) * G);
     a.row_off = (const int32_t *)(t + 3 * tb + 2 * sizeof(int64_t) * G);
+    for (int g = 0; g < G; ++g)
+      if (d[g].M > 0 && ((reinterpret_cast<uintptr_t>(src_dev[g]) | (uintptr_t)(sld[g] * dt_size(f->src_dt))) & 15) != 0) a.g_any = 1;
     B2_TRY(launch_quant_rows(a, f->src_dt, R, st));
   } else {
     for (int g = 0; g < G; ++g) {

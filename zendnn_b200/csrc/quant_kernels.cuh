@@ -167,6 +167,7 @@ struct RowQuantArgs {
   void *const *g_dst; const int64_t *g_dst_ld;
   void *const *g_scale;
   const int32_t *row_off;
+  int32_t g_any;                        // some group's rows do not start on 16 bytes
 };
 
 constexpr int kQuantThreads = 256;
@@ -187,16 +188,23 @@ __device__ __forceinline__ float block_max(float v, float *sh) {
   return r;
 }
 
+// What a launch's rows are: one strided (or gathered) matrix, several matrices, rows that go to several places, or the expert-parallel forms (the row count
+// known only on the device: the CTAs stride over the rows; destinations in other GPUs' receive buffers).
+enum : int { kRowsPlain = 0, kRowsGroups, kRowsScatter, kRowsPeers };
+
 // One CTA per row.  T = uint16_t (bf16 bits) or float; NV = 16-byte vectors of the row that a thread keeps in registers
-// between the two passes (2 for rows up to 512 vectors: few registers, six CTAs per SM; 8 for long rows, with the
-// register budget of four or five CTAs per SM: left to its own choice the compiler took 32 registers and spilled the cache).
-// EP: the expert-parallel forms (row count known only on the device: the CTAs stride over the rows; scatter into other
-// GPUs' receive buffers).  They are a separate instantiation so that the plain form keeps its register budget.
-// THR: threads of the CTA.  Few long rows leave most of the chip idle whatever is done, so their time is the chain load - reduce -
+// between the two passes (2 for rows up to 512 vectors: few registers, six CTAs per SM; 8 for long rows, with the register budget of three or four
+// CTAs per SM).  THR: threads of the CTA.  Few long rows leave most of the chip idle whatever is done, so their time is the chain load - reduce -
 // convert of one row: 1024 threads with at most two vectors each (one row of 11008 and the GEMM behind it: 22.6 -> 18.0 us, with the
 // overlapped launch).
-template <typename T, int NV, bool EP, int THR = kQuantThreads>
-__global__ void __launch_bounds__(THR, THR > kQuantThreads ? 1 : (NV > 2 ? (EP ? 4 : (sizeof(T) == 2 ? 5 : 4)) : 6)) quant_per_token_kernel(RowQuantArgs a) {
+// ANY: source rows of any alignment and length, their vectors put together from words, the last one with zeros.
+// FORM and ANY are instantiations of their own: as choices at run time they cost the long rows their registers (f32, eight vectors: 100 bytes spilled, none
+// now; 4096 rows of 2304 f32 17.9 -> 14.5 us, of 14336 71.7 -> 54.2, of 14336 bf16 38.0 -> 28.1).
+template <typename T, int NV, int FORM, int THR = kQuantThreads, bool ANY = false>
+__global__ void __launch_bounds__(THR, THR > kQuantThreads ? 1 : (NV > 2 ? (sizeof(T) == 4 && FORM != kRowsPlain ? 3 : 4) : 6))
+quant_per_token_kernel(RowQuantArgs a) {
+  constexpr bool EP = FORM == kRowsPeers, SCATTER = FORM == kRowsScatter || EP;
+  static_assert(!ANY || !SCATTER, "scattered rows are aligned");
   __shared__ uint32_t sh[THR / 32];
   constexpr int E = VecTraits<T>::kPer16B;
   // Programmatic dependent launch on both sides: this kernel's launch overlaps the one in front (it touches memory only after the
@@ -205,9 +213,11 @@ __global__ void __launch_bounds__(THR, THR > kQuantThreads ? 1 : (NV > 2 ? (EP ?
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int row_limit = (EP && a.n_rows_dev) ? *a.n_rows_dev : (int)gridDim.x;
-  for (int r = blockIdx.x; r < row_limit; r += EP ? (int)gridDim.x : row_limit) {
+  int r = (int)blockIdx.x;
+  if (EP && r >= row_limit) return;
+  do {
   const T *src; int8_t *dst; void *scale_out; int64_t scale_idx;
-  if (a.n_groups > 0) {
+  if constexpr (FORM == kRowsGroups) {
     int g = 0;
     while (g + 1 < a.n_groups && r >= a.row_off[g + 1]) ++g;
     const int lr = r - a.row_off[g];
@@ -221,17 +231,16 @@ __global__ void __launch_bounds__(THR, THR > kQuantThreads ? 1 : (NV > 2 ? (EP ?
     dst = a.dst ? a.dst + (int64_t)r * a.dst_ld : nullptr;
     scale_out = a.scale; scale_idx = r;
   }
-  const int32_t *sc = (a.scatter && a.n_groups == 0) ? a.scatter + (int64_t)r * a.scatter_n : nullptr;
-  const int32_t *sp = (EP && sc && a.scatter_peer) ? a.scatter_peer + (int64_t)r * a.scatter_n : nullptr;
+  const int32_t *sc = SCATTER && a.scatter ? a.scatter + (int64_t)r * a.scatter_n : nullptr;
+  const int32_t *sp = EP && sc && a.scatter_peer ? a.scatter_peer + (int64_t)r * a.scatter_n : nullptr;
   if (sc) dst = sp ? a.peer_dst[0] : a.dst;     // row offsets (and the peer's base) are applied per destination
   const int K = a.K;
-  // whole vectors of the destination; the source's rows may lie anywhere (their vectors are then put together from words, the last one with zeros)
-  const bool src_vec = ((reinterpret_cast<uintptr_t>(src) & 15) == 0) && (K % E == 0);
-  const bool vec = (src_vec || (!EP && !sc)) && (!dst || (reinterpret_cast<uintptr_t>(dst) % E) == 0);
-  const int nvec = vec ? (K + E - 1) / E : 0;
+  const bool vec = (ANY || (((reinterpret_cast<uintptr_t>(src) & 15) == 0) && (K % E == 0))) &&
+                   (!dst || (reinterpret_cast<uintptr_t>(dst) % E) == 0);
+  const int nvec = vec ? (ANY ? (K + E - 1) / E : K / E) : 0;
   auto load_vec = [&](int v) {
-    if (src_vec) return reinterpret_cast<const uint4 *>(src)[v];
-    return ld16_any(reinterpret_cast<const uint8_t *>(src) + (int64_t)v * 16, (K - v * E) * (int)sizeof(T));
+    if constexpr (ANY) return ld16_any(reinterpret_cast<const uint8_t *>(src) + (int64_t)v * 16, (K - v * E) * (int)sizeof(T));
+    else return reinterpret_cast<const uint4 *>(src)[v];
   };
   uint4 cache[NV];
   AbsMax<T> amax;
@@ -295,7 +304,7 @@ __global__ void __launch_bounds__(THR, THR > kQuantThreads ? 1 : (NV > 2 ? (EP ?
         for (int j = 0; j < a.scatter_n; ++j) { const int d = sc[j]; if (d >= 0 && d < a.scatter_cap) put(a.peer_dst[sp[j]] + (int64_t)d * a.dst_ld, o, v); }
       } else if (sc) {
         for (int j = 0; j < a.scatter_n; ++j) { const int d = sc[j]; if (d >= 0) put(dst + (int64_t)d * a.dst_ld, o, v); }
-      } else if ((v + 1) * E <= K) put(dst, o, v);
+      } else if (!ANY || (v + 1) * E <= K) put(dst, o, v);
       else put_codes_tail<T>(dst + v * E, o, K - v * E);
     };
 #pragma unroll
@@ -315,7 +324,7 @@ __global__ void __launch_bounds__(THR, THR > kQuantThreads ? 1 : (NV > 2 ? (EP ?
       } else dst[k] = qv;
     }
   }
-  }   // rows of this CTA
+  } while (EP && (r += (int)gridDim.x) < row_limit);   // rows of this CTA
 }
 
 // Per-token ASYMMETRIC dynamic quantisation to u8 (one f32 scale and one s32 zero point per row):
