@@ -53,6 +53,17 @@ def test_more_tiles_than_sms(oracle, monkeypatch, gs, bm):
     assert_bf16_close(out, ref, 1, "bm=%d gs=%d" % (bm, gs), atol=1e-5)
 
 
+@pytest.mark.parametrize("bm", [1, 48, 256, -16])
+@pytest.mark.parametrize("M", [4, 150])
+def test_tile_rows_that_do_not_exist(oracle, monkeypatch, M, bm):
+    """Refused on the host (the kernel divides by the number of shares, which nothing would have set)."""
+    monkeypatch.setenv("B200DNN_GS_TC", "1")
+    monkeypatch.setenv("B200DNN_GS_TC_BM", str(bm))
+    capi, d, out, _, _, _, keep = _case(oracle, M, 256, 136, 32)
+    assert capi.matmul(d) == capi.FAILURE and "bad tile rows %d" % bm in capi.last_error()
+    assert (out == 0).all()
+
+
 @pytest.mark.parametrize("M", [4, 200])
 def test_waits_run_out(monkeypatch, M):
     import torch

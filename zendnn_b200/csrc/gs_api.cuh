@@ -243,6 +243,7 @@ int32_t launch_gs_tc(const GsGemmArgs &g, const EpiParams &epi, bool early, cuda
       if (bm == 0 || us < best || (forced > 1 && s == forced)) { best = us; bm = rows; a.splits = s; }
     }
   }
+  B2_CHECK(bm != 0 && a.splits >= 1, B200DNN_FAILURE, "bad tile rows %d", forced_bm);      // (B200DNN_GS_TC_BM names no tile)
 #define B2_GS_TC(BM) \
   return g.gs == 32 ? launch_gs_tc_t<BM, 4>(g, a, map_w, epi, st) : g.gs == 64 ? launch_gs_tc_t<BM, 2>(g, a, map_w, epi, st) : launch_gs_tc_t<BM, 1>(g, a, map_w, epi, st)
   if (bm == 16) B2_GS_TC(16);
