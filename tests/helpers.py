@@ -1,6 +1,37 @@
 """Shared helpers for the GPU parity tests: seeded inputs shaped like the benchmark configs and
 comparison rules.  bf16 tensors are numpy uint16 bit patterns on the host."""
+import ctypes
+
 import numpy as np
+
+
+class _KernelNodeParams(ctypes.Structure):      # cudaKernelNodeParams
+    _fields_ = [("func", ctypes.c_void_p), ("grid", ctypes.c_uint * 3), ("block", ctypes.c_uint * 3), ("smem", ctypes.c_uint),
+                ("params", ctypes.c_void_p), ("extra", ctypes.c_void_p)]
+
+
+def kernel_grids(call):
+    """(CTAs, threads of one) of every kernel that call(stream) launches, from a captured graph; called twice before, so that weights are packed."""
+    import torch
+    rt = ctypes.CDLL("libcudart.so.12")
+    side = torch.cuda.Stream()
+    for _ in range(2):
+        call(side.cuda_stream)
+        torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g, stream=side):
+        call(side.cuda_stream)
+    raw, n = ctypes.c_void_p(g.raw_cuda_graph()), ctypes.c_size_t(0)
+    assert rt.cudaGraphGetNodes(raw, None, ctypes.byref(n)) == 0
+    nodes, out = (ctypes.c_void_p * n.value)(), []
+    assert rt.cudaGraphGetNodes(raw, nodes, ctypes.byref(n)) == 0
+    for node in nodes:
+        kind, p = ctypes.c_int(-1), _KernelNodeParams()
+        assert rt.cudaGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)) == 0
+        if kind.value == 0:                     # cudaGraphNodeTypeKernel
+            assert rt.cudaGraphKernelNodeGetParams(ctypes.c_void_p(node), ctypes.byref(p)) == 0
+            out.append((p.grid[0] * p.grid[1] * p.grid[2], p.block[0] * p.block[1] * p.block[2]))
+    return out
 
 
 def bf16_ulp_diff(a_bits, b_bits):

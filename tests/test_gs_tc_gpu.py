@@ -5,7 +5,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from helpers import assert_bf16_close
+from helpers import assert_bf16_close, kernel_grids
 
 pytestmark = pytest.mark.gpu
 
@@ -40,6 +40,51 @@ def test_edges(oracle, monkeypatch, M, N, gs, split):
     capi.check(capi.matmul(d))
     assert (sc == sa).all()
     assert_bf16_close(out, ref, 1, "M=%d K=%d N=%d gs=%d split=%d" % (M, K, N, gs, split), atol=1e-5)
+
+
+def _device_case(oracle, M, K, N, gs):
+    """The same on device memory, with a stream to call on: the call, what it launches per grid and block, its result and the oracle's."""
+    import torch
+    capi, d, out, ref, _, _, keep = _case(oracle, M, K, N, gs)
+    X, W, sw, b, packed = (torch.from_numpy(np.ascontiguousarray(x).view(np.int16) if x.dtype == np.uint16 else np.ascontiguousarray(x)).cuda() for x in keep)
+    o = torch.zeros((M, N), dtype=torch.int16, device="cuda")
+    d = capi.make_matmul(M, N, K, X, packed, o, src_dt=capi.DT["bf16"], dst_dt=capi.DT["bf16"], bias=b, src_scale=capi.quant(None, count=M),
+                         wei_scale=capi.quant(sw, K // gs * N, capi.DT["f32"]), dynamic_quant=True, wei_dt=capi.DT["s4"], postops=("swish",))
+    launched = kernel_grids(lambda st: capi.check(capi.matmul(d, st)))
+    o.zero_()
+    capi.check(capi.matmul(d, torch.cuda.current_stream().cuda_stream))
+    got = o.cpu().numpy().view(np.uint16)
+    capi.lib.b200dnn_clear_caches()
+    return launched, got, ref
+
+
+GS_TC_THREADS = {16: 608, 32: 608, 64: 864, 128: 864}      # of a CTA, by its rows
+
+
+@pytest.mark.parametrize("split", [3, 5, 6, 7, 8])
+@pytest.mark.parametrize("gs", [32, 64, 128, 256])
+@pytest.mark.parametrize("bm,M", [(16, 11), (32, 27), (64, 70), (128, 100)])
+def test_shares(oracle, monkeypatch, bm, M, gs, split):
+    """Shares of the groups that do not come out even (17 over a cluster; with groups of 32 and 64 the last block of 128 k is a quarter or half full)."""
+    monkeypatch.setenv("B200DNN_GS_TC", "1")
+    monkeypatch.setenv("B200DNN_GS_TC_BM", str(bm))
+    monkeypatch.setenv("B200DNN_GS_TC_SPLIT", str(split))
+    K = 16 * 128 + gs if gs <= 128 else 17 * gs
+    N = 200
+    launched, got, ref = _device_case(oracle, M, K, N, gs)
+    assert (2 * -(-M // bm) * split, GS_TC_THREADS[bm]) in launched, launched
+    assert_bf16_close(got, ref, 1, "bm=%d gs=%d split=%d" % (bm, gs, split), atol=1e-5)
+
+
+# both sides of each line of the choice, up to 16 rows: K, rows, columns against the decode form; the group and the columns against the general
+# form (fewer than eight groups); odd columns and rows that the decode form has no room for
+@pytest.mark.parametrize("M,K,N,gs,tensor_cores", [(1, 2048, 512, 32, False), (1, 4096, 512, 32, True), (16, 4096, 512, 128, False), (16, 8192, 512, 128, True),
+                                                   (2, 1024, 256, 64, False), (16, 1024, 28672, 64, True), (1, 256, 512, 128, False), (1, 256, 4864, 128, True),
+                                                   (1, 1024, 512, 1024, True), (12, 14336, 128, 128, True), (3, 1024, 333, 128, True), (3, 1024, 334, 128, False)])
+def test_lines_of_the_choice(oracle, monkeypatch, M, K, N, gs, tensor_cores):
+    launched, got, ref = _device_case(oracle, M, K, N, gs)
+    assert any(threads == 608 for _, threads in launched) == tensor_cores, launched
+    assert_bf16_close(got, ref, 1, "M=%d K=%d N=%d gs=%d" % (M, K, N, gs), atol=1e-5)
 
 
 @pytest.mark.parametrize("gs", [32, 128])

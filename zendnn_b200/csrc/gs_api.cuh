@@ -206,16 +206,62 @@ int32_t launch_gs_tc_t(const GsGemmArgs &g, GsTcArgs a, const CUtensorMap &map_w
   return B200DNN_SUCCESS;
 }
 
-// Calls the tensor-core form takes: s4 codes, per-token rows, f32 weight scales, groups of 32, 64 or a multiple of 128 k.  Up to 16 rows it has the higher
-// fixed cost (7.2 us against 5 to 6, quantisation included) and the decode form the higher cost per column and k, the more so with more rows and shorter
-// groups: 121 measured shapes (K 1024 to 14336, N 512 to 14336) cross where K * (M + 8) passes 20, 40 and 80 thousand for groups of 32, 64 and
-// 128; the choice is 1.0, 1.3 and 1.5 % off the better form on average, the decode form always 22, 15 and 4 % (K = 11008, N = 4096, M = 16, us: 24.6 and 14.6;
-// K = N = 4096, M = 1: 7.2 and 9.4).  Above 16 rows it is at least twice as fast as the general form (M = 64, K = 4096, N = 11008: 92 -> 21).
-inline bool gs_tc_pays(const GsPlan &p, int32_t ws_dt, int M, int K) {
+// Rows of a tile and shares of the groups (a cluster's CTAs are resident at once): fewest microseconds by blocks of 128 k per CTA times the measured cost
+// of one.  Splitting costs nothing that shows beside it.  bm 0: B200DNN_GS_TC_BM names no tile.
+struct GsTcPlan { int bm, splits, blocks; };      // blocks of 128 k that a CTA walks
+inline int gs_tc_class(int gs) { return gs == 32 ? 0 : gs == 64 ? 1 : 2; }
+GsTcPlan gs_tc_plan(int gs, int M, int N, int K) {
+  static const double block_us[4][3] = {{0.42, 0.29, 0.30}, {0.70, 0.33, 0.34}, {1.01, 0.51, 0.42}, {1.66, 0.98, 0.55}};      // [16, 32, 64, 128 rows][groups of 32, 64, 128]
+  const int k_blocks = (K + 127) / 128, group_blocks = gs > 128 ? gs / 128 : 1, units = k_blocks / group_blocks, n_tiles = (N + 127) / 128, sms = rt().sm_count;
+  const int forced_bm = env_int("B200DNN_GS_TC_BM", 0), forced = env_int("B200DNN_GS_TC_SPLIT", 0);
+  GsTcPlan p{};
+  double best = 0.0;
+  for (int i = 0; i < 4; ++i) {
+    const int rows = 16 << i, tiles = n_tiles * ((M + rows - 1) / rows);
+    // (no tile of twice the rows there are; 16 and 32 rows only where one tile holds them all)
+    if (forced_bm ? rows != forced_bm : (i > 0 && rows / 2 >= M) || (rows < 64 && rows < M)) continue;
+    for (int s = 1; s <= kGsTcMaxSplits; ++s) {
+      if (s > 1 && (units < 2 * s || tiles * s > gs_tc_room(s))) continue;
+      if (forced > 0 && s != forced && s != 1) continue;
+      const int blocks = s > 1 ? (units + s - 1) / s * group_blocks : (tiles + sms - 1) / sms * k_blocks;
+      const double us = blocks * block_us[i][gs_tc_class(gs)];
+      if (p.bm == 0 || us < best || (forced > 1 && s == forced)) { best = us; p = {rows, s, blocks}; }
+    }
+  }
+  return p;
+}
+
+// Calls the tensor-core form takes: s4 codes, per-token rows, f32 weight scales, groups of 32, 64 or a multiple of 128 k; above 16 rows always (at least twice
+// as fast as the general form: M = 64, K = 4096, N = 11008: 92 -> 21 us).  Up to 16 rows by the time of either, device microseconds fitted to 3549 measured
+// calls (K 128 to 14336, N 512 to 28672, M 1 to 16, groups of 32 to 1024), within 5 to 7 % (tensor cores) and 7 to 10 % (decode form):
+//   tensor cores: a fixed cost, the blocks that a CTA walks, the weight through HBM, the rows
+//   decode form: a fixed cost, K times the 16-column tiles that an SM gets, one after the other
+//   general form (fewer than eight groups, which its warps take one each, and one wave of CTAs): the group
+// The tensor cores have to be 8 % faster by that: the choice is 0.7, 1.0 and 1.0 % off the better form on average for groups of 32, 64 and from 128, 31 % at
+// worst (K = 512, N = 18944, gs = 32, M = 2: 8.0, not 6.1), and in three calls more than 5 % slower than the older form (K = 8192, N = 18944, gs = 1024, M = 1:
+// 22.9, not 19.8, the worst).  A line at K * (M + 8), without N, was 6, 11 and 27 % off, in 120 calls slower than the older form, 46 % at worst.
+inline bool gs_tc_pays(const GsPlan &p, int32_t ws_dt, int M, int N, int K, bool decode_fits) {
   if (!p.w4 || p.src_cols != 1 || ws_dt != B200DNN_F32 || !(p.gs == 32 || p.gs == 64 || p.gs % 128 == 0)) return false;
   const int mode = env_int("B200DNN_GS_TC", -1);
   if (mode >= 0) return mode != 0;
-  return M > 16 || (long long)K * (M + 8) >= (p.gs == 32 ? 20000 : p.gs == 64 ? 40000 : 80000);
+  if (M > 16) return true;
+  static const double tc[3][4] = {{5.36, 0.289, 0.043, 0.114}, {5.46, 0.232, 0.029, 0.088}, {5.73, 0.202, 0.048, 0.075}};
+  static const double dec[3][5] = {{3.32, 0.134, 0.923, 0.184, 0.028}, {3.44, 0.056, 0.551, 0.095, 0.025}, {3.66, -0.007, 0.388, 0.076, 0.026}};
+  const int c = gs_tc_class(p.gs);
+  const double k = K * 1e-3;
+  double other;
+  if (p.G < kGsWarps) {
+    if (N > 32 * rt().sm_count) return true;
+    other = 5.25 + 0.0037 * p.gs + (M > 8 ? 0.65 : 0.0);
+  } else {
+    // the general form, several times slower here (rows that the decode form has no room for: K = 14336, N = 4096, M = 16: 26 to 59 us, 15 to 16)
+    if (!decode_fits || (long long)M * K > 150000) return true;
+    const int w = ((N + 15) / 16 + rt().sm_count - 1) / rt().sm_count;
+    other = dec[c][0] + k * (dec[c][1] + w * (dec[c][2] + (M > 8 ? dec[c][3] : 0.0)) + dec[c][4] * M);
+  }
+  const double us = tc[c][0] + tc[c][2] * k * N * 1e-3 + tc[c][3] * k * M * 0.1;
+  if (us + tc[c][1] * ((K + 127) / 128) / kGsTcMaxSplits >= 0.92 * other) return false;      // (the smallest calls are spared the search for shares)
+  return us + tc[c][1] * gs_tc_plan(p.gs, M, N, K).blocks < 0.92 * other;
 }
 int32_t launch_gs_tc(const GsGemmArgs &g, const EpiParams &epi, bool early, cudaStream_t st) {
   GsTcArgs a{};
@@ -225,30 +271,14 @@ int32_t launch_gs_tc(const GsGemmArgs &g, const EpiParams &epi, bool early, cuda
   a.test_no_loads = env_int("B200DNN_TEST_NO_LOADS", 0);
   CUtensorMap map_w;
   B2_TRY(make_map_s4(&map_w, g.W, (uint64_t)(g.Kp >> 6), (uint64_t)((g.N + 7) / 8)));
-  // Rows per tile and shares of the groups: fewest microseconds by blocks of 128 k per CTA times the measured cost of one.  Splitting costs nothing
-  // that shows beside it; a cluster's CTAs are resident at once.
-  static const double block_us[4][3] = {{0.42, 0.29, 0.30}, {0.70, 0.33, 0.34}, {1.01, 0.51, 0.42}, {1.66, 0.98, 0.55}};      // [16, 32, 64, 128 rows][groups of 32, 64, 128]
-  const int cls = g.gs == 32 ? 0 : g.gs == 64 ? 1 : 2, units = a.k_blocks / a.group_blocks, sms = rt().sm_count;
-  const int forced_bm = env_int("B200DNN_GS_TC_BM", 0), forced = env_int("B200DNN_GS_TC_SPLIT", 0);
-  int bm = 0;
-  double best = 0.0;
-  for (int i = 0; i < 4; ++i) {
-    const int rows = 16 << i, tiles = a.n_tiles * ((g.M + rows - 1) / rows);
-    if (forced_bm ? rows != forced_bm : (i > 0 && rows / 2 >= g.M) || (rows < 64 && rows < g.M)) continue;      // (never more than half empty, never many small tiles)
-    for (int s = 1; s <= kGsTcMaxSplits; ++s) {
-      if (s > 1 && (units < 2 * s || tiles * s > gs_tc_room(s))) continue;
-      if (forced > 0 && s != forced && s != 1) continue;
-      const int blocks = s > 1 ? (units + s - 1) / s * a.group_blocks : (tiles + sms - 1) / sms * a.k_blocks;
-      const double us = blocks * block_us[i][cls];
-      if (bm == 0 || us < best || (forced > 1 && s == forced)) { best = us; bm = rows; a.splits = s; }
-    }
-  }
-  B2_CHECK(bm != 0 && a.splits >= 1, B200DNN_FAILURE, "bad tile rows %d", forced_bm);      // (B200DNN_GS_TC_BM names no tile)
+  const GsTcPlan p = gs_tc_plan(g.gs, g.M, g.N, g.K);
+  B2_CHECK(p.bm != 0 && p.splits >= 1, B200DNN_FAILURE, "bad tile rows %d", env_int("B200DNN_GS_TC_BM", 0));
+  a.splits = p.splits;
 #define B2_GS_TC(BM) \
   return g.gs == 32 ? launch_gs_tc_t<BM, 4>(g, a, map_w, epi, st) : g.gs == 64 ? launch_gs_tc_t<BM, 2>(g, a, map_w, epi, st) : launch_gs_tc_t<BM, 1>(g, a, map_w, epi, st)
-  if (bm == 16) B2_GS_TC(16);
-  if (bm == 32) B2_GS_TC(32);
-  if (bm == 64) B2_GS_TC(64);
+  if (p.bm == 16) B2_GS_TC(16);
+  if (p.bm == 32) B2_GS_TC(32);
+  if (p.bm == 64) B2_GS_TC(64);
   B2_GS_TC(128);
 #undef B2_GS_TC
 }
@@ -363,15 +393,15 @@ int32_t matmul_group_scaled(const b200dnn_matmul_t *d, cudaStream_t st) {
   };
 
   const bool early = p.dyn && p.src_cols == 1 && !p.src_per_tensor;      // (directly behind the per-token quantisation, which waited for everything in front of it)
-  if (gs_tc_pays(p, d->wei_scale.dt, M, K)) {
+  // (the decode form addresses the weight and the scales with 32-bit offsets)
+  const bool decode_fits = M <= 16 && p.G >= kGsWarps && p.gs % 32 == 0 && d->wei_scale.dt == B200DNN_F32 && N % 2 == 0 &&
+                           (int64_t)(N + 8) * Kp < (int64_t)1 << 32 && (int64_t)p.G * N < (int64_t)1 << 30 && (reinterpret_cast<uintptr_t>(ws_dev) & 7) == 0;
+  if (gs_tc_pays(p, d->wei_scale.dt, M, N, K, decode_fits)) {
     B2_TRY(prepare_source());
     B2_TRY(launch_gs_tc(a, epi, early, st));
     return finish_out({&o_dst, &o_scale}, st);
   }
-  // (the decode form addresses the weight and the scales with 32-bit offsets)
-  if (M <= 16 && p.G >= kGsWarps && p.gs % 32 == 0 && d->wei_scale.dt == B200DNN_F32 && N % 2 == 0 &&
-      (int64_t)(N + 8) * Kp < (int64_t)1 << 32 && (int64_t)p.G * N < (int64_t)1 << 30 &&
-      (reinterpret_cast<uintptr_t>(ws_dev) & 7) == 0 && env_int("B200DNN_GS_DECODE", 1) != 0) {
+  if (decode_fits && env_int("B200DNN_GS_DECODE", 1) != 0) {
     B2_TRY(prepare_source());
     bool done = false;
     int32_t rcd;
