@@ -35,6 +35,8 @@ def test_int8(capi, oracle, monkeypatch, pair, bn, splits, M, K, N):
     dA, dW, dsa, dsw, db = (torch.from_numpy(x).cuda() for x in (A, W, sa, sw, bias))
     s32, out = torch.zeros(M, N, dtype=torch.int32, device="cuda"), torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")
     d32 = capi.make_matmul(M, N, K, dA, dW, s32, src_dt=capi.DT["s8"], dst_dt=capi.DT["s32"], force_kernel=2)
+    f32 = torch.zeros(M, N, device="cuda")
+    df = capi.make_matmul(M, N, K, dA, dW, f32, src_dt=capi.DT["s8"], dst_dt=capi.DT["f32"], src_scale=dsa, wei_scale=dsw, bias=db, postops=["relu"], force_kernel=2)
     d16 = capi.make_matmul(M, N, K, dA, dW, out, src_dt=capi.DT["s8"], dst_dt=capi.DT["bf16"], src_scale=dsa, wei_scale=dsw, bias=db, postops=["gelu_tanh"], force_kernel=2)
     st = torch.cuda.current_stream().cuda_stream
     capi.check(capi.matmul(d16, st))
@@ -45,8 +47,12 @@ def test_int8(capi, oracle, monkeypatch, pair, bn, splits, M, K, N):
     out.zero_()
     capi.check(capi.matmul(d32, st))
     capi.check(capi.matmul(d16, st))
-    assert (s32.cpu().numpy() == oracle.gemm_s32(A, W)).all()
+    capi.check(capi.matmul(df, st))
+    acc = oracle.gemm_s32(A, W)
+    assert (s32.cpu().numpy() == acc).all()
     assert torch.equal(out, default)
+    # one rounding per operation, none of them contracted
+    assert (f32.cpu().numpy() == np.maximum(acc.astype(np.float32) * sa[:, None] * sw[None, :] + bias[None, :], np.float32(0))).all()
     capi.lib.b200dnn_clear_caches()
 
 
@@ -67,3 +73,26 @@ def test_bf16(capi, monkeypatch, pair, bn, splits, M, K, N):
     # f32 sums of K exact products, see test_skinny_gpu.py
     assert ((out - (a @ w + bias)).abs() <= K * 2.0 ** -23 * (a.abs() @ w.abs() + bias.abs())).all()
     capi.lib.b200dnn_clear_caches()
+
+
+@pytest.mark.parametrize("M", [20, 400])
+def test_gelu_tanh_rounds_where_it_did(capi, M):
+    """x / (1 + 2^(-2 u log2 e)) with u = (c x) (1 + (f x) x), the last sum in one rounding (few rows and tiles).  From the argument on, what is left
+    are 2^x (2^-22), the reciprocal (2^-23) and three roundings (2^-24); a rounding more in u moves the result by 14 to 25 times 2^-24 or 2^-23."""
+    import torch
+    rng = np.random.default_rng(M)
+    K, N, f4 = 16, 256, np.float32
+    A, W = np.zeros((M, K), dtype=np.int8), np.zeros((K, N), dtype=np.int8)
+    A[:, 0], W[0] = 1, -(np.arange(N) % 16 + 112).astype(np.int8)
+    s = rng.uniform(4.6 / 112, 5.7 / 127, M).astype(f4)
+    out = torch.zeros(M, N, device="cuda")
+    dA, dW, ds, dw = torch.from_numpy(A).cuda(), torch.from_numpy(W).cuda(), torch.from_numpy(s).cuda(), torch.ones(N, device="cuda")
+    d = capi.make_matmul(M, N, K, dA, dW, out, src_dt=capi.DT["s8"], dst_dt=capi.DT["f32"], src_scale=ds, wei_scale=dw, weights_const=False, postops=["gelu_tanh"])
+    capi.check(capi.matmul(d, torch.cuda.current_stream().cuda_stream))
+    x = W[0].astype(f4)[None, :] * s[:, None]
+    c, f = f4(0.79788458347320556640625), f4(0.044715)
+    t = ((f * x).astype(np.float64) * x + 1).astype(f4)                         # (the product is exact in double)
+    arg = ((c * x) * t) * f4(-2.0 * 1.44269504088896340736)
+    ref = x / (1 + np.exp2(arg.astype(np.float64)))
+    err = np.abs(out.cpu().numpy() - ref) / np.abs(ref)
+    assert err.max() <= 2.0 ** -22 + 2.0 ** -23 + 3 * 2.0 ** -24, err.max()

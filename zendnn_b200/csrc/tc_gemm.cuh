@@ -277,7 +277,7 @@ __device__ __forceinline__ float tc_act(const EpiParams &epi, float x, int m, in
   if (ACT == FA_RELU) return fmaxf(x, 0.0f);
   if (ACT == FA_GELU_TANH) {
     const float c = 0.79788458347320556640625f, f = 0.044715f;
-    const float inner = __fmul_rn(__fmul_rn(c, x), __fadd_rn(1.0f, __fmul_rn(__fmul_rn(f, x), x)));
+    const float inner = __fmul_rn(__fmul_rn(c, x), __fmaf_rn(__fmul_rn(f, x), x, 1.0f));
     return fast_sigmoid_mul(x, 2.0f * inner);
   }
   if (ACT == FA_GELU_ERF) return po_gelu_erf(x);
@@ -299,6 +299,7 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 __device__ __forceinline__ uint64_t tc_pack2(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
 __device__ __forceinline__ void tc_unpack2(uint64_t r, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(r)); }
 __device__ __forceinline__ uint64_t tc_mul2(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ uint64_t tc_fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
 __device__ __forceinline__ uint64_t tc_add2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 
 // x / (1 + exp(-arg)) of two elements, arg2 already times -log2(e): the operations of fast_sigmoid_mul
@@ -308,10 +309,11 @@ __device__ __forceinline__ uint64_t tc_sigmoid_mul2(uint64_t x2, uint64_t arg2) 
   tc_unpack2(tc_add2(tc_pack2(1.0f, 1.0f), tc_pack2(tc_ex2(a0), tc_ex2(a1))), b0, b1);
   return tc_mul2(x2, tc_pack2(tc_rcp(b0), tc_rcp(b1)));
 }
-// gelu_tanh as in tc_act: the factor 2 of its argument is in the constant (exact)
+// gelu_tanh as in tc_act, 1 + (f x) x in one rounding: the factor 2 of its argument is in the constant (exact).  Largest error against double for x from -6
+// to 6: 3.6e-6 of the result (20 rows; 4.4e-6 with a rounding between the product and the sum).
 __device__ __forceinline__ uint64_t tc_gelu_tanh2(uint64_t x2) {
   const uint64_t c2 = tc_pack2(0.79788458347320556640625f, 0.79788458347320556640625f), f2 = tc_pack2(0.044715f, 0.044715f);
-  const uint64_t inner = tc_mul2(tc_mul2(c2, x2), tc_add2(tc_pack2(1.0f, 1.0f), tc_mul2(tc_mul2(f2, x2), x2)));
+  const uint64_t inner = tc_mul2(tc_mul2(c2, x2), tc_fma2(tc_mul2(f2, x2), x2, tc_pack2(1.0f, 1.0f)));
   return tc_sigmoid_mul2(x2, tc_mul2(inner, tc_pack2(2.0f * kTcNegLog2e, 2.0f * kTcNegLog2e)));
 }
 __device__ __forceinline__ uint64_t tc_swish2(uint64_t x2) { return tc_sigmoid_mul2(x2, tc_mul2(x2, tc_pack2(kTcNegLog2e, kTcNegLog2e))); }
