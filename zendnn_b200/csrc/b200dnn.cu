@@ -429,12 +429,14 @@ TcChoice tc_choose(long long M, int N, int k_blocks, bool f16) {
     if (forced < 2) consider(0, bn, 1);
     if (forced == 1 || (forced_bn <= 0 && bn != 64 && bn != 128 && bn != 256)) continue;
     // clusters of 2 to 4 CTAs share a tile, each with K blocks of its own and at least one 32-column chunk to finish; the int32 partial sums are added
-    // through distributed shared memory, so the result is the same bit for bit.  All clusters are resident at once.
+    // through distributed shared memory, so the result is the same bit for bit.  All clusters are resident at once, with room for two more where they
+    // are of three: those do not tile the GPCs, and behind another kernel the last ones wait (M = 100, K = 7168 behind the quantisation, in two and three
+    // shares, us: 45 tiles 15.3 and 20.8, 44 tiles 15.3 and 18.0, 43 tiles 15.2 and 15.4, 42 tiles 15.1 and 14.3).
     const long long tiles = ((M + 127) / 128) * ((N + bn - 1) / bn);
     for (int s = 2; s <= 4; ++s) {
       const int per = (k_blocks + s - 1) / s;
       if ((forced >= 2 && s != forced) || per * (s - 1) >= k_blocks || per < 2 || bn / 32 < s) continue;
-      if (forced < 2 && (split_room(s) <= 0 || tiles * s > split_room(s))) continue;
+      if (forced < 2 && (split_room(s) <= 0 || tiles * s + (s == 3 ? 6 : 0) > split_room(s))) continue;
       consider(0, bn, s);
     }
   }
