@@ -390,21 +390,31 @@ int split_room(int s) { return cluster_room(tc_gemm_kernel<true>, kTcThreads, kT
 // bf16: wide pair tiles keep the tensor pipe so busy that the clock gives way.  Choosing by it is 0.8 % off the best form and width on average;
 // the rules before (waves times width + 16; pairs from two tiles per pair of SMs; a split model of its own) 9.5 %.  Largest differences, us: M = 3615,
 // K = 5824, N = 576 in bf16 43.0 -> 28.4; M = 825, K = 1280, N = 10752 in INT8 22.9 -> 14.6; M = 4096, K = 14336, N = 4096 201 -> 161.
-double tc_cost_us(bool pair, int bn, int splits, long long tiles, int k_blocks, double dram_bytes, bool f16) {
-  static const double floor1[8] = {0.195, 0.20, 0.20, 0.20, 0.225, 0.24, 0.295, 0.315};      // widths 32, 64 ... 256: one CTA a tile
-  static const double floor2[8] = {0.205, 0.205, 0.206, 0.208, 0.217, 0.222, 0.26, 0.29};      // a pair
-  const int i = bn / 32 - 1, kb = (k_blocks + splits - 1) / splits;
-  const long long conc = pair ? rt().sm_count / 2 : rt().sm_count, ctas = tiles * splits, full = ctas / conc, last = ctas % conc;
-  double per_kb = (pair ? floor2 : floor1)[i];
-  if (pair && f16 && bn >= 224 && tiles > conc) per_kb *= 1.08;
-  const double bytes = (double)((pair ? 256 : 128) + bn) * 128.0 / (pair ? 17.5e6 : 20.4e6);       // us per block and tile in flight
-  const double wave = (pair ? 0.63 + 1.9 * bn / 256.0 : 0.32 + 1.7 * bn / 256.0);
+// Every plain call asks for it about forty times: terms of a form and width are in a table, divisions of 32 bits (the choice 0.19 -> 0.10 us of host time).
+struct TcForm { double wave, per_kb, bytes; };      // us of a wave beside its blocks; of a block at least; of a block and tile in flight
+struct TcForms {
+  TcForm f[2][8];                                   // [one CTA a tile, a pair][width / 32 - 1]
+  constexpr TcForms() : f{} {
+    const double floor[2][8] = {{0.195, 0.20, 0.20, 0.20, 0.225, 0.24, 0.295, 0.315}, {0.205, 0.205, 0.206, 0.208, 0.217, 0.222, 0.26, 0.29}};
+    for (int p = 0; p < 2; ++p)
+      for (int i = 0; i < 8; ++i) {
+        const int bn = 32 * (i + 1);
+        f[p][i] = {p ? 0.63 + 1.9 * bn / 256.0 : 0.32 + 1.7 * bn / 256.0, floor[p][i], ((p ? 256 : 128) + bn) * 128.0 / (p ? 17.5e6 : 20.4e6)};
+      }
+  }
+};
+constexpr TcForms kTcForms;
+inline double tc_dram_us(double bytes) { return 4.0 + bytes / 4.15e6; }
+inline double tc_cost_us(bool pair, int bn, int splits, unsigned tiles, int k_blocks, double dram_us, bool f16, unsigned sms) {
+  const TcForm &w = kTcForms.f[pair][bn / 32 - 1];
+  const int kb = splits == 1 ? k_blocks : (k_blocks + splits - 1) / splits;
+  const unsigned conc = pair ? sms / 2 : sms, ctas = tiles * (unsigned)splits, full = ctas / conc, last = ctas - full * conc;
+  const double per_kb = pair && f16 && bn >= 224 && tiles > conc ? 1.08 * w.per_kb : w.per_kb;
   double t = pair ? 5.3 : 4.55;
-  if (splits > 1) t += 1.6 + 0.77 * (splits - 1) * bn / 128.0;
-  t += (double)full * (wave + kb * std::max(per_kb, bytes * (double)conc));
-  if (last) t += wave + kb * std::max(per_kb, bytes * (double)last);
-  const double d = 4.0 + dram_bytes / 4.15e6;
-  return std::max(t, d) + 0.15 * std::min(t, d);
+  if (splits > 1) t += 1.6 + 0.77 / 128.0 * ((splits - 1) * bn);
+  if (full) t += (double)full * (w.wave + kb * std::max(per_kb, w.bytes * (double)conc));
+  if (last) t += w.wave + kb * std::max(per_kb, w.bytes * (double)last);
+  return std::max(t, dram_us) + 0.15 * std::min(t, dram_us);
 }
 
 struct TcChoice { int pair, bn, splits; };
@@ -412,35 +422,36 @@ struct TcChoice { int pair, bn, splits; };
 // Knobs: B200DNN_TC_PAIR -1 (default) by cost, 0 never, 1 whenever the shape allows; B200DNN_TC_BN, B200DNN_TC_KSPLIT (1 never, 2 to 4 that many).
 TcChoice tc_choose(long long M, int N, int k_blocks, bool f16) {
   const int mode = env_int("B200DNN_TC_PAIR", -1), forced_bn = env_int("B200DNN_TC_BN", 0), forced = env_int("B200DNN_TC_KSPLIT", 0);
-  const double bytes = (double)k_blocks * 128.0 * (double)(M + N) + 2.0 * (double)M * N;
+  const double dram_us = tc_dram_us((double)k_blocks * 128.0 * (double)(M + N) + 2.0 * (double)M * N);
+  const unsigned sms = (unsigned)rt().sm_count, m128 = (unsigned)((M + 127) / 128), m256 = (m128 + 1) / 2;
   TcChoice best{0, forced_bn > 0 ? forced_bn : 128, 1};
   double best_us = 1e30;
-  auto consider = [&](int pair, int bn, int s) {
-    const long long tiles = ((M + (pair ? 255 : 127)) / (pair ? 256 : 128)) * ((N + bn - 1) / bn);
-    const double us = tc_cost_us(pair != 0, bn, s, tiles, k_blocks, bytes, f16);
+  auto consider = [&](int pair, int bn, int s, unsigned tiles) {
+    const double us = tc_cost_us(pair != 0, bn, s, tiles, k_blocks, dram_us, f16, sms);
     if (us < best_us) { best_us = us; best = {pair, bn, s}; }
   };
   const bool pair_ok = N >= 128 && mode != 0 && forced < 2, single_ok = !(mode == 1 && N >= 128) || forced >= 2;
   for (int bn = 256; bn >= 32; bn -= 32) {
     const bool width = forced_bn > 0 ? bn == forced_bn : true;
     if (!width) continue;
-    if (pair_ok && bn >= 64) consider(1, bn, 1);
+    const unsigned n_tiles = (unsigned)(N + bn - 1) / (unsigned)bn, tiles = m128 * n_tiles;
+    if (pair_ok && bn >= 64) consider(1, bn, 1, m256 * n_tiles);
     if (!single_ok) continue;
-    if (forced < 2) consider(0, bn, 1);
+    if (forced < 2) consider(0, bn, 1, tiles);
     if (forced == 1 || (forced_bn <= 0 && bn != 64 && bn != 128 && bn != 256)) continue;
     // clusters of 2 to 4 CTAs share a tile, each with K blocks of its own and at least one 32-column chunk to finish; the int32 partial sums are added
     // through distributed shared memory, so the result is the same bit for bit.  All clusters are resident at once, with room for two more where they
     // are of three: those do not tile the GPCs, and behind another kernel the last ones wait (M = 100, K = 7168 behind the quantisation, in two and three
     // shares, us: 45 tiles 15.3 and 20.8, 44 tiles 15.3 and 18.0, 43 tiles 15.2 and 15.4, 42 tiles 15.1 and 14.3).
-    const long long tiles = ((M + 127) / 128) * ((N + bn - 1) / bn);
     for (int s = 2; s <= 4; ++s) {
+      if (bn / 32 < s || (forced >= 2 && s != forced) || (forced < 2 && tiles * s > sms)) continue;
       const int per = (k_blocks + s - 1) / s;
-      if ((forced >= 2 && s != forced) || per * (s - 1) >= k_blocks || per < 2 || bn / 32 < s) continue;
-      if (forced < 2 && (split_room(s) <= 0 || tiles * s + (s == 3 ? 6 : 0) > split_room(s))) continue;
-      consider(0, bn, s);
+      if (per * (s - 1) >= k_blocks || per < 2) continue;
+      if (forced < 2 && (int)(tiles * s) + (s == 3 ? 6 : 0) > split_room(s)) continue;
+      consider(0, bn, s, tiles);
     }
   }
-  if (best_us > 1e29 && forced_bn <= 0) consider(0, 128, 1);        // (a knob that fits no form)
+  if (best_us > 1e29 && forced_bn <= 0) consider(0, 128, 1, m128 * ((unsigned)(N + 127) / 128u));        // (a knob that fits no form)
   return best;
 }
 
@@ -453,7 +464,7 @@ int pick_bn(int m_tiles, int N, int k_blocks, int gated, int pair, bool f16) {
   int best = 0;
   double best_us = 0.0;
   for (int bn = 256; bn >= (gated ? step : 64); bn -= step) {
-    const double us = tc_cost_us(pair != 0, bn, 1, (long long)m_tiles * ((N + bn - 1) / bn), k_blocks, 0.0, f16);
+    const double us = tc_cost_us(pair != 0, bn, 1, (unsigned)m_tiles * ((unsigned)(N + bn - 1) / (unsigned)bn), k_blocks, tc_dram_us(0.0), f16, (unsigned)rt().sm_count);
     if (best == 0 || us < best_us) { best = bn; best_us = us; }
   }
   return best;

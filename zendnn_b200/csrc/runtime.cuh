@@ -49,13 +49,17 @@ inline int env_int(const char *name, int dflt) {
   if (dynamic) { const char *e = getenv(name); return e ? atoi(e) : dflt; }
   struct Slot { const char *name; bool set; int value; };
   static Slot slots[64];
-  static int n_slots = 0;
+  static std::atomic<int> n_slots{0};      // slots below it are written and stay as they are: read without the lock
+  int n = n_slots.load(std::memory_order_acquire), i = 0;
+  for (; i < n; ++i)
+    if (slots[i].name == name) return slots[i].set ? slots[i].value : dflt;
   static std::mutex mu;
   std::lock_guard<std::mutex> lk(mu);
-  for (int i = 0; i < n_slots; ++i)
+  n = n_slots.load(std::memory_order_relaxed);
+  for (; i < n; ++i)
     if (slots[i].name == name) return slots[i].set ? slots[i].value : dflt;
   const char *e = getenv(name);
-  if (n_slots < 64) { slots[n_slots].name = name; slots[n_slots].set = e != nullptr; slots[n_slots].value = e ? atoi(e) : 0; ++n_slots; }
+  if (n < 64) { slots[n] = Slot{name, e != nullptr, e ? atoi(e) : 0}; n_slots.store(n + 1, std::memory_order_release); }
   return e ? atoi(e) : dflt;
 }
 
