@@ -264,6 +264,7 @@ inline bool gs_tc_pays(const GsPlan &p, int32_t ws_dt, int M, int N, int K, bool
   return us + tc[c][1] * gs_tc_plan(p.gs, M, N, K).blocks < 0.92 * other;
 }
 int32_t launch_gs_tc(const GsGemmArgs &g, const EpiParams &epi, bool early, cudaStream_t st) {
+  B2_CHECK(epi.dst_dt == B200DNN_BF16, B200DNN_UNIMPLEMENTED, "the tensor-core form of W4A8 writes bf16");
   GsTcArgs a{};
   a.M = g.M; a.N = g.N; a.k_blocks = (g.K + 127) / 128; a.group_blocks = g.gs > 128 ? g.gs / 128 : 1; a.G = g.G;
   a.n_tiles = (g.N + 127) / 128;

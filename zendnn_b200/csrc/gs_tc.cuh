@@ -1,4 +1,4 @@
-// W4A8 on the 5th-generation tensor cores: bf16 rows quantised per token to s8 x packed s4 weights with {G,N} scales, the contract of gs_gemm.cuh.  Exact
+// W4A8 on the 5th-generation tensor cores: bf16 rows quantised per token to s8 x packed s4 weights with {G,N} scales, bf16 out, the contract of gs_gemm.cuh.  Exact
 // integer sum per group, x weight scale and added in group order in f32 with one rounding (fused), x source scale once at the end: two
 // roundings fewer per group than the scalar definition's product by product.
 //
@@ -354,8 +354,7 @@ gs_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
             const int m = m0 + c * 8 + i;
             if (m >= a.M || n >= a.N) continue;
             const float x = epi_finish(epi, cx, __fmul_rn(__uint_as_float(lds4(outb + (uint32_t)i * kSlot)), a.sa[m] * 0.0625f), m, n);
-            if (epi.dst_dt == DT_BF16) reinterpret_cast<uint16_t *>(epi.dst)[(int64_t)m * epi.ldc + n] = f32_to_bf16_bits(x);
-            else reinterpret_cast<float *>(epi.dst)[(int64_t)m * epi.ldc + n] = x;
+            reinterpret_cast<uint16_t *>(epi.dst)[(int64_t)m * epi.ldc + n] = f32_to_bf16_bits(x);
           }
         }
       }
@@ -372,8 +371,7 @@ gs_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
       const int nt = tile0 / a.m_tiles, m_first = (tile0 - nt * a.m_tiles) * BM, n4 = nt * 128 + lane * 4;
       const int rows = min(BM, a.M - m_first);
       const EpiCtx cx = epi_ctx(epi, 0);
-      const int esz = epi.dst_dt == DT_BF16 ? 2 : 4;
-      const bool whole = n4 + 4 <= a.N && ((reinterpret_cast<uintptr_t>(epi.dst) | (uintptr_t)(epi.ldc * esz)) & (4 * esz - 1)) == 0;
+      const bool whole = n4 + 4 <= a.N && ((reinterpret_cast<uintptr_t>(epi.dst) | (uintptr_t)(epi.ldc * 2)) & 7) == 0;
       for (int r = crank + a.splits * (warp - 10); r < rows && n4 < a.N; r += SW * a.splits) {
         const uint32_t own = smem0 + (uint32_t)(r * 512 + lane * 16);
         float x[4] = {0.f, 0.f, 0.f, 0.f};
@@ -393,19 +391,13 @@ gs_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float z = n4 + i < a.N ? epi_finish(epi, cx, __fmul_rn(x[i], s_row), m, n4 + i) : 0.f;
-          y[i] = esz == 2 ? (uint32_t)f32_to_bf16_bits(z) : __float_as_uint(z);
+          y[i] = f32_to_bf16_bits(z);
         }
-        uint8_t *o = reinterpret_cast<uint8_t *>(epi.dst) + ((int64_t)m * epi.ldc + n4) * esz;
-        if (esz == 2) {
-          if (whole) *reinterpret_cast<uint2 *>(o) = make_uint2(y[0] | (y[1] << 16), y[2] | (y[3] << 16));
-          else {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) if (n4 + i < a.N) reinterpret_cast<uint16_t *>(o)[i] = (uint16_t)y[i];
-          }
-        } else if (whole) *reinterpret_cast<uint4 *>(o) = make_uint4(y[0], y[1], y[2], y[3]);
+        uint16_t *o = reinterpret_cast<uint16_t *>(epi.dst) + (int64_t)m * epi.ldc + n4;
+        if (whole) *reinterpret_cast<uint2 *>(o) = make_uint2(y[0] | (y[1] << 16), y[2] | (y[3] << 16));
         else {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) if (n4 + i < a.N) reinterpret_cast<uint32_t *>(o)[i] = y[i];
+          for (int i = 0; i < 4; ++i) if (n4 + i < a.N) o[i] = (uint16_t)y[i];
         }
       }
     }
