@@ -79,7 +79,9 @@ def test_other_kernel_numbers_stay_with_the_tile_kernel(capi, oracle, kernel):
 # both sides of the lines that the choice of kernel draws: rows against bytes of a column, one wave of column tiles (148 x 128 columns) and
 # how full the last one is, rows of 16 x K that the decode kernel has no room for
 @pytest.mark.parametrize("M,K,N", [(24, 512, 300), (25, 1008, 300), (25, 1024, 300), (33, 1536, 300), (33, 1520, 300), (48, 1024, 18944), (9, 2048, 18945),
-                                   (17, 3072, 18945), (24, 3072, 37889), (25, 512, 25600), (24, 512, 18945), (16, 14336, 18960), (9, 8192, 18944)])
+                                   (17, 3072, 18945), (24, 3072, 37889), (25, 512, 25600), (24, 512, 18945), (16, 14336, 18960), (9, 8192, 18944),
+                                   (49, 2048, 300), (64, 2048, 5120), (64, 2048, 5121), (49, 4096, 5121), (64, 4080, 9472), (33, 3056, 9473), (48, 3072, 9473),
+                                   (48, 8192, 9473), (64, 8192, 9473), (65, 8192, 9473)])
 def test_lines_of_the_choice_int8(capi, M, K, N):
     import torch
     g = torch.Generator(device="cuda").manual_seed(M + K + N)
@@ -91,7 +93,8 @@ def test_lines_of_the_choice_int8(capi, M, K, N):
 
 
 @pytest.mark.parametrize("M,K,N", [(64, 1024, 300), (64, 1016, 300), (48, 768, 300), (48, 760, 300), (8, 512, 18944), (8, 512, 18945), (8, 512, 25300),
-                                   (9, 1536, 25300), (24, 1536, 25300), (24, 1528, 25300), (25, 1536, 25300)])
+                                   (9, 1536, 25300), (24, 1536, 25300), (24, 1528, 25300), (25, 1536, 25300), (64, 1024, 5121), (64, 2048, 5121), (48, 1528, 9473),
+                                   (48, 1536, 9473), (64, 4088, 9473), (64, 4096, 9473)])
 def test_lines_of_the_choice_bf16(capi, M, K, N):
     import torch
     g = torch.Generator(device="cuda").manual_seed(M + K + N)

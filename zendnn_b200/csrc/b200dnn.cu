@@ -690,17 +690,27 @@ int32_t launch_skinny(const uint8_t *A, int64_t lda, bool a_unsigned, bool f16, 
   return B200DNN_SUCCESS;
 }
 
-// Does the few-row kernel beat the tile kernel?  col_bytes: bytes of a weight column.  Over 1400 shapes (M 1 to 64, K 512 to 14336, N 512 to
-// 50176, bf16 and INT8) the choice is 0.7 % off the better of the two on average.
+// Does the few-row kernel beat the tile kernel?  col_bytes: bytes of a weight column.  Up to 24 rows over 1400 shapes (M 1 to 64, K 512 to 14336, N 512
+// to 50176, bf16 and INT8) the choice was 0.7 % off the better of the two on average; above 24 rows, over 840 shapes (M 17 to 64, K 512 to 14336, N 512 to
+// 28672, device time), it is 0.3 % off in INT8 and 0.2 % in bf16, 12 % at worst.  (With the lines fitted to an earlier tile kernel, and none of more than 48
+// INT8 rows: 3.0 and 1.1 %, 75 % at worst: K = 14336, N = 512, M = 56 12.8 us in tiles, 7.3 here; bf16, K = 1024, N = 11008, M = 64 7.4 and 10.9.)
 //   - Column tiles for at most one wave of CTAs: always up to 24 rows (bf16, K = 4096, N = 1024, M = 16: 6.6 us against 12.5); with more rows the
 //     fixed cost of handling them (about 0.04 us a row) must be less than what the tile kernel loses by not sharing K (about 0.9 us a KiB
-//     of column): bf16, M = 64, N = 4096: K = 512 7.5 against 6.2, K = 2048 9.6 against 10.2.
+//     of column).  Above 48 rows and 40 tiles that takes 4096 bytes (K = 2048, N = 9472, M = 64 in INT8: 7.5 in tiles, 9.2 here).  With tiles for more than half the
+//     SMs no CTA shares K and the rows are paid in full: columns of 3072 to 8191 bytes (4096 x 11008, M = 48: 11.2 and 13.3), and above 48 rows shorter ones
+//     too, go to the tile kernel.
 //   - More column tiles than SMs: the kernel is not persistent, so its last wave must be well filled (K = 8192, N = 20480 is 160 tiles: 71
 //     against 60 us for 8 rows; N = 50176 is 392 and K = 4096: 69 against 107), and every tile pays for its rows again (K = 4096, N = 28672:
 //     8 rows 44 against 56, 32 rows 48 against 45).  Columns of at most 512 bytes are one short burst each: 12.9 against 17.1 (N = 50176).
 bool few_rows_pay(int M, int N, int64_t col_bytes) {
   const long long tiles = (N + 127) / 128, sms = rt().sm_count, waves = (tiles + sms - 1) / sms;
-  if (waves == 1) return M <= 24 || col_bytes >= 32ll * ((M + 15) & ~15);
+  if (waves == 1) {
+    if (M <= 24) return true;
+    if (col_bytes < 32ll * ((M + 15) & ~15)) return false;
+    if (M <= 32) return true;
+    if (2 * tiles <= sms) return M <= 48 || tiles <= 40 || col_bytes >= 4096;
+    return col_bytes >= 8192 || (M <= 48 && col_bytes < 3072);
+  }
   if (M <= 24 && col_bytes <= 512) return true;
   return 3 * tiles >= 2 * waves * sms && (M <= 8 || (M <= 24 && col_bytes >= 3072));
 }
@@ -1216,9 +1226,9 @@ int32_t b200dnn_matmul(const b200dnn_matmul_t *d, void *stream) {
   const bool early = !pw.fresh && (dyn || (d->flags & B200DNN_FLAG_STABLE_WEIGHTS) != 0);
   // Few rows on the tensor cores (skinny_gemm.cuh).  Up to 16 rows against the decode kernel, us: K = 4096, N = 11008 12.7 -> 12.2, K = 14336,
   // N = 4096 31.0 -> 16.0, but K = N = 4096 7.2 -> 7.6 (its fixed cost is higher), and with more column tiles than SMs K = 4096, N = 50176
-  // 37.3 -> 41.0: there only rows that the decode kernel has no room for.  Above 48 rows the tile kernel (M = 64, K = N = 4096: 10.4 -> 10.9).
+  // 37.3 -> 41.0: there only rows that the decode kernel has no room for.  From 17 to 64 rows against the tile kernel: few_rows_pay.
   const bool skinny = M <= 16 ? M > 8 && (long long)K * N >= (24ll << 20) && ((N + 127) / 128 <= rt().sm_count || decode_smem(M, N, pw.Kp) > 220 * 1024)
-                              : M <= 48 && few_rows_pay(M, N, K);
+                              : M <= kSkinnyMaxM && few_rows_pay(M, N, K);
   const bool few_rows = d->force_kernel == 0 && tc_ok && skinny;
   B2_CHECK(few_rows || which == 1 || which == 3 || tc_ok, B200DNN_FAILURE, "tcgen05 kernel needs a 16-byte aligned source with lda %% 16 == 0");
   if (few_rows) {

@@ -113,8 +113,8 @@ int32_t matmul_bf16_packed(const b200dnn_matmul_t *d, const PackedWeight &pw, cu
     B2_TRY(repitch_rows(A, lda * 2, M, 2 * K, st, &A, &lda));
     lda /= 2;
   }
-  // few rows (skinny_gemm.cuh); M = 96, K = 4096, N = 11008: 24.7 us in the tile kernel, 27.3 there
-  if (d->force_kernel == 0 && M <= 64 && few_rows_pay(M, N, 2ll * K)) {
+  // few rows (skinny_gemm.cuh)
+  if (d->force_kernel == 0 && M <= kSkinnyMaxM && few_rows_pay(M, N, 2ll * K)) {
     const bool early = (d->flags & B200DNN_FLAG_STABLE_WEIGHTS) != 0 && !pw.fresh;
     B2_TRY(launch_skinny(A, lda * 2, false, true, M, N, 2 * K, pw, epi, fast_act_code(epi), early, st));
     return finish_out({&o_dst}, st);
