@@ -47,6 +47,13 @@ def test_f32_beside_the_middle_of_two_codes(oracle, K, rows):
     _check(oracle, x, "f32", K)
 
 
+@pytest.mark.parametrize("warp", ["0", "1"])
+@pytest.mark.parametrize("dt,K,rows", [("bf16", 2560, 128), ("bf16", 4096, 128), ("f32", 1024, 64), ("f32", 2048, 64)])
+def test_middle_of_two_codes_in_either_kernel(oracle, monkeypatch, warp, dt, K, rows):
+    monkeypatch.setenv("B200DNN_QUANT_WARP", warp)
+    (test_bf16_every_pair_of_significands if dt == "bf16" else test_f32_beside_the_middle_of_two_codes)(oracle, K, rows)
+
+
 # a warp and a CTA per row, one and two vectors past a multiple, the longest rows of a warp, rows beyond a CTA's registers
 @pytest.mark.parametrize("dt", ["bf16", "f32"])
 @pytest.mark.parametrize("rows,K", [(70, 1), (70, 17), (64, 1999), (64, 2047), (5, 1001), (5, 4097), (64, 16385 + 8)])
