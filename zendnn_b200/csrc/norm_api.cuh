@@ -140,32 +140,91 @@ __device__ __forceinline__ void norm_load4(const void *p, int32_t dt, int i4, fl
   }
 }
 
-// One row of the full-width form, held by the CTA as the bf16 pairs it came in: v = input, r = residual (fused add).  red: a buffer per
-// reduction, used by one row in two (so one barrier each).  Same arithmetic as the generic kernel.
-template <int NV>
-__device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, uint32_t (&v)[NV][4], const uint32_t (&r)[NV][4], float (*red)[kNormThreads / 32]) {
-  const int nvec = (int)(a.n >> 3);
+// Parameters of the four columns c0 .. c0 + 3.  ANY: the columns start anywhere (c0 & 3 is the same for all vectors of a row) and may lie partly
+// outside [0, n); f32 parameters come as two aligned float4, of which the wanted four are picked.
+template <bool ANY>
+__device__ __forceinline__ void norm_params4(const void *p, int32_t dt, int c0, int n, float (&g)[4]) {
+  if constexpr (!ANY) norm_load4(p, dt, c0 >> 2, g);
+  else {
+    const int r = c0 & 3;
+    if (dt == B200DNN_F32 && c0 >= 0 && c0 - r + 8 <= n) {
+      const float4 *v = reinterpret_cast<const float4 *>(p) + (c0 >> 2);
+      const float4 x = v[0], y = v[1];
+      const float w[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+      float u[5];
+#pragma unroll
+      for (int e = 0; e < 5; ++e) u[e] = (r & 2) ? w[e + 2] : w[e];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) g[e] = (r & 1) ? u[e + 1] : u[e];
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) g[e] = (unsigned)(c0 + e) < (unsigned)n ? load_as_f32(p, dt, c0 + e) : 0.f;
+    }
+  }
+}
+
+// a sum (or a largest value) over the CTA (sh: one word per warp, not used again before the next barrier)
+template <bool MAX>
+__device__ __forceinline__ float norm_row_reduce(float x, float *sh) {
+  auto op = [](float p, float q) { return MAX ? fmaxf(p, q) : p + q; };
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x = op(x, __shfl_xor_sync(0xffffffffu, x, o));
+  const int warps = (int)(blockDim.x >> 5);
+  if (warps == 1) return x;
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
+  __syncthreads();
+  float t = 0.f;
+  if (warps <= 8) {
+    for (int i = 0; i < warps; ++i) t = op(t, sh[i]);
+  } else {
+    t = (int)(threadIdx.x & 31) < warps ? sh[threadIdx.x & 31] : 0.f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t = op(t, __shfl_xor_sync(0xffffffffu, t, o));
+  }
+  return t;
+}
+
+// eight bf16 of a tensor of `total` elements as a 16-byte vector; at the tensor's end (ANY) element by element
+template <bool ANY>
+__device__ __forceinline__ void norm_load_vec(const uint16_t *base, int64_t at, int64_t total, uint32_t (&w)[4]) {
+  if (!ANY || at + 8 <= total) {
+    const uint4 q = *reinterpret_cast<const uint4 *>(base + at);
+    w[0] = q.x; w[1] = q.y; w[2] = q.z; w[3] = q.w;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const uint32_t l = at + 2 * e < total ? base[at + 2 * e] : 0u, h = at + 2 * e + 1 < total ? base[at + 2 * e + 1] : 0u;
+      w[e] = l | (h << 16);
+    }
+  }
+}
+// the elements of a vector that belong to the row: columns c0 .. c0 + 7 within [0, n)
+template <bool ANY>
+__device__ __forceinline__ void norm_store_vec(uint16_t *base, int64_t at, int c0, int n, const uint32_t (&w)[4]) {
+  if (!ANY || (c0 >= 0 && c0 + 8 <= n)) *reinterpret_cast<uint4 *>(base + at) = make_uint4(w[0], w[1], w[2], w[3]);
+  else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) if ((unsigned)(c0 + e) < (unsigned)n) base[at + e] = (uint16_t)(w[e >> 1] >> ((e & 1) * 16));
+  }
+}
+
+// clears the elements of a vector outside the row (its first column is c0)
+__device__ __forceinline__ void norm_clear_outside(uint32_t (&w)[4], int c0, int n) {
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    if ((unsigned)(c0 + e) >= (unsigned)n) w[e >> 1] &= (e & 1) ? 0x0000FFFFu : 0xFFFF0000u;
+}
+
+// One row of the full-width form, held by the CTA as the bf16 pairs it came in: v = input, r = residual (fused add); vector i holds the columns
+// 8 i - shift .. 8 i - shift + 7 (shift = 0 unless ANY), and elements outside the row are zeros.  red: a buffer per reduction, used by one row in two
+// (so one barrier each).  Same arithmetic as the generic kernel.
+template <int NV, bool ANY>
+__device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, int shift, uint32_t (&v)[NV][4], const uint32_t (&r)[NV][4], float (*red)[32]) {
+  const int n = (int)a.n, nvec = (shift + n + 7) >> 3;
   auto lo = norm_lo; auto hi = norm_hi;
-  const int64_t off = b * a.n;
-  uint4 *rv = a.residual ? reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(a.residual) + off) : nullptr;
-  auto sum = [](float x, float *sh) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
-    __syncthreads();
-    float t = 0.f;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += sh[i];
-    return t;
-  };
-  auto largest = [](float x, float *sh) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
-    __syncthreads();
-    float t = 0.f;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t = fmaxf(t, sh[i]);
-    return t;
-  };
+  const int64_t off = b * a.n - shift;          // element of vector 0
+  auto inside = [&](int c) { return (unsigned)c < (unsigned)n; };
+  auto whole = [&](int c0) { return !ANY || (c0 >= 0 && c0 + 8 <= n); };
   float s1 = 0.f;
   if (a.type == NORM_FUSED_ADD_RMS) {
 #pragma unroll
@@ -179,7 +238,7 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, uint3
           s1 = __fmaf_rn(s_lo, s_lo, s1); s1 = __fmaf_rn(s_hi, s_hi, s1);
           v[j][e] = pack_bf16x2(s_lo, s_hi);
         }
-        rv[i] = make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]);
+        norm_store_vec<ANY>(reinterpret_cast<uint16_t *>(a.residual), off + (int64_t)i * 8, i * 8 - shift, n, v[j]);
       }
     }
   } else if (a.type == NORM_RMS) {
@@ -193,35 +252,42 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, uint3
 #pragma unroll
       for (int e = 0; e < 4; ++e) { s1 = __fadd_rn(s1, lo(v[j][e])); s1 = __fadd_rn(s1, hi(v[j][e])); }
   }
-  s1 = sum(s1, red[0]);
+  s1 = norm_row_reduce<false>(s1, red[0]);
   float mean = 0.f, inv;
   if (a.type == NORM_LAYER) {
     mean = __fdiv_rn(s1, (float)a.n);
     float s2 = 0.f;
 #pragma unroll
-    for (int j = 0; j < NV; ++j)
-      if (threadIdx.x + j * blockDim.x < nvec) {
+    for (int j = 0; j < NV; ++j) {
+      const int i = threadIdx.x + j * blockDim.x, c0 = i * 8 - shift;
+      if (i < nvec && whole(c0)) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float d0 = __fadd_rn(lo(v[j][e]), -mean), d1 = __fadd_rn(hi(v[j][e]), -mean);
           s2 = __fmaf_rn(d0, d0, s2); s2 = __fmaf_rn(d1, d1, s2);
         }
+      } else if (ANY && i < nvec) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float d0 = inside(c0 + 2 * e) ? __fadd_rn(lo(v[j][e]), -mean) : 0.f, d1 = inside(c0 + 2 * e + 1) ? __fadd_rn(hi(v[j][e]), -mean) : 0.f;
+          s2 = __fmaf_rn(d0, d0, s2); s2 = __fmaf_rn(d1, d1, s2);
+        }
       }
-    s2 = sum(s2, red[1]);
+    }
+    s2 = norm_row_reduce<false>(s2, red[1]);
     inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(s2, (float)a.n), a.eps)));
   } else inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(s1, (float)a.n), a.eps)));
-  float amax = 0.f;
-  const bool layer = a.type == NORM_LAYER, shift = a.use_shift && layer;
+  AbsMax<uint16_t> am;
+  const bool layer = a.type == NORM_LAYER, shifted = a.use_shift && layer;
 #pragma unroll
   for (int j = 0; j < NV; ++j) {
-    const int i = threadIdx.x + j * blockDim.x;
+    const int i = threadIdx.x + j * blockDim.x, c0 = i * 8 - shift;
     if (i < nvec) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {          // two halves of four elements
-        float g[4] = {1.f, 1.f, 1.f, 1.f};
-        if (a.use_scale) norm_load4(a.gamma, a.gamma_dt, 2 * i + h, g);
-        float bt[4] = {0.f, 0.f, 0.f, 0.f};
-        if (shift) norm_load4(a.beta, a.beta_dt, 2 * i + h, bt);
+        float g[4] = {1.f, 1.f, 1.f, 1.f}, bt[4] = {0.f, 0.f, 0.f, 0.f};
+        if (a.use_scale) norm_params4<ANY>(a.gamma, a.gamma_dt, c0 + 4 * h, n, g);
+        if (shifted) norm_params4<ANY>(a.beta, a.beta_dt, c0 + 4 * h, n, bt);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const uint32_t w = v[j][2 * h + e];
@@ -229,73 +295,77 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, uint3
           if (layer) { y0 = __fadd_rn(y0, -mean); y1 = __fadd_rn(y1, -mean); }
           y0 = __fmul_rn(y0, inv); y1 = __fmul_rn(y1, inv);
           if (a.use_scale) { y0 = __fmul_rn(y0, g[2 * e]); y1 = __fmul_rn(y1, g[2 * e + 1]); }
-          if (shift) { y0 = __fadd_rn(y0, bt[2 * e]); y1 = __fadd_rn(y1, bt[2 * e + 1]); }
-          const uint32_t o = pack_bf16x2(y0, y1);
-          v[j][2 * h + e] = o;
-          // rounding to bf16 is monotonic: the largest rounded magnitude is the rounded largest magnitude (a NaN does not
-          // enter fmaxf; an infinity does and is dealt with after the loop)
-          if (a.q) amax = fmaxf(amax, fmaxf(fabsf(y0), fabsf(y1)));
+          if (shifted) { y0 = __fadd_rn(y0, bt[2 * e]); y1 = __fadd_rn(y1, bt[2 * e + 1]); }
+          v[j][2 * h + e] = pack_bf16x2(y0, y1);
         }
       }
-      if (a.y) reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(a.y) + off)[i] = make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]);
+      if (!whole(c0)) norm_clear_outside(v[j], c0, n);
+      if (a.q) am.add(make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]));
+      if (a.y) norm_store_vec<ANY>(reinterpret_cast<uint16_t *>(a.y), off + (int64_t)i * 8, c0, n, v[j]);
     }
   }
   if (a.q) {
-    amax = largest(amax, red[2]);
-    amax = __uint_as_float(pack_bf16x2(amax, 0.0f) << 16);
+    float amax = norm_row_reduce<true>(am.finite() ? __uint_as_float(am.bits()) : __int_as_float(0x7F800000), red[2]);
     if (!finite_f32(amax)) {
-      // an infinite element (it quantises to 0): take the maximum over the finite rounded values instead
-      uint32_t mb = 0u;
+      // an infinite or NaN element (it quantises to 0): the maximum over the finite values instead
+      AbsMax<uint16_t> fin;
 #pragma unroll
-      for (int j = 0; j < NV; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint32_t m0 = (v[j][e] << 16) & 0x7FFFFFFFu, m1 = v[j][e] & 0x7FFF0000u;
-          mb = max(mb, m0 < 0x7F800000u ? m0 : 0u);
-          mb = max(mb, m1 < 0x7F800000u ? m1 : 0u);
-        }
-      amax = largest(__uint_as_float(mb), red[3]);
+      for (int j = 0; j < NV; ++j) fin.add_finite(make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]));
+      amax = norm_row_reduce<true>(__uint_as_float(fin.bits()), red[3]);
     }
     const float scale = scale_from_absmax(amax);
     const float rinv = __frcp_rn(scale);
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
-      const int i = threadIdx.x + j * blockDim.x;
-      if (i < nvec)
-        *reinterpret_cast<uint2 *>(a.q + b * a.q_ld + (int64_t)i * 8) =
-            quant_vec<uint16_t>(make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]), scale, rinv);
+      const int i = threadIdx.x + j * blockDim.x, c0 = i * 8 - shift;
+      if (i < nvec) {
+        const uint2 codes = quant_vec<uint16_t>(make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]), scale, rinv);
+        int8_t *o = a.q + b * a.q_ld + c0;
+        if (whole(c0)) *reinterpret_cast<uint2 *>(o) = codes;
+        else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) if (inside(c0 + e)) o[e] = (int8_t)((e < 4 ? codes.x : codes.y) >> ((e & 3) * 8));
+        }
+      }
     }
     if (threadIdx.x == 0) a.q_scale[b] = scale;
   }
 }
 
-// The decoder-layer case at full width: bf16 rows of at most NV * 8 * blockDim elements, 16-byte aligned, bf16 out.  One
+// The decoder-layer case at full width: bf16 rows of at most NV * 8 * blockDim elements in 16-byte aligned tensors, bf16 out.  One
 // CTA per row; a thread keeps its NV vectors of eight elements in registers (as the bf16 pairs they are at every stage that
 // is kept) between the passes, so the row is read once and every access is a 16-byte vector (8 bytes for the s8 codes).
 // Bound by HBM without the quantised output and by instruction issue with it (3.15 of 4 instructions a cycle): all loads of a row (input and
 // residual) are in flight before the first store, each reduction costs one barrier, and the launch overlaps the kernel in front.  4096 rows of 4096 with residual add and s8 codes
 // (151 MB): 36.9 -> 30.5 us (4.9 TB/s); a ring of rows filled by bulk copies ahead of persistent CTAs took 35.7 us (four CTAs per SM where
 // there are six here).
-template <int NV>
-__global__ void __launch_bounds__(kNormThreads, NV <= 2 ? 6 : (NV <= 4 ? 4 : 2)) norm_rows_vec_kernel(const NormArgs a) {
-  __shared__ float red[2][4][kNormThreads / 32];
+// ANY: rows of any length, one behind the other.  A row is covered by the aligned vectors of the tensor that it touches (the first and the last shared with
+// its neighbours, of which it writes its own elements only); input, residual, result and codes then need no shifting, the parameters are picked out of two
+// aligned loads.  Instruction issue again: 8903 x 844 LayerNorm with codes 59 (element by element) -> 30 us, 3000 x 7001 with residual add and codes 197 -> 57,
+// 2000 x 12287 220 -> 55; the sets of registers per thread leave two CTAs an SM or more (one: 85 us for the last).
+template <int NV, int THREADS, int CTAS, bool ANY>
+__global__ void __launch_bounds__(THREADS, CTAS) norm_rows_vec_kernel(const NormArgs a) {
+  __shared__ float red[2][4][32];
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int nvec = (int)(a.n >> 3);
+  const int64_t total = a.batch * a.n;
   int parity = 0;
   for (int64_t b = blockIdx.x; b < a.batch; b += gridDim.x, parity ^= 1) {
-    const uint4 *xv = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(a.x) + b * a.n);
-    const uint4 *rv = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(a.residual) + b * a.n);
+    const int shift = ANY ? (int)((b * a.n) & 7) : 0, n = (int)a.n, nvec = (shift + n + 7) >> 3;
+    const int64_t off = b * a.n - shift;
     uint32_t v[NV][4], r[NV][4];
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
       const int i = threadIdx.x + j * blockDim.x;
-      const uint4 q = i < nvec ? xv[i] : make_uint4(0u, 0u, 0u, 0u);
-      v[j][0] = q.x; v[j][1] = q.y; v[j][2] = q.z; v[j][3] = q.w;
-      const uint4 s = (a.type == NORM_FUSED_ADD_RMS && i < nvec) ? rv[i] : make_uint4(0u, 0u, 0u, 0u);
-      r[j][0] = s.x; r[j][1] = s.y; r[j][2] = s.z; r[j][3] = s.w;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[j][e] = r[j][e] = 0u;
+      if (i < nvec) {
+        norm_load_vec<ANY>(reinterpret_cast<const uint16_t *>(a.x), off + (int64_t)i * 8, total, v[j]);
+        if (a.type == NORM_FUSED_ADD_RMS) norm_load_vec<ANY>(reinterpret_cast<const uint16_t *>(a.residual), off + (int64_t)i * 8, total, r[j]);
+        if (ANY && (i == 0 || i == nvec - 1)) { norm_clear_outside(v[j], i * 8 - shift, n); norm_clear_outside(r[j], i * 8 - shift, n); }
+      }
     }
-    norm_row_vec<NV>(a, b, v, r, red[parity]);
+    norm_row_vec<NV, ANY>(a, b, shift, v, r, red[parity]);
   }
 }
 
@@ -388,26 +458,32 @@ extern "C" int32_t b200dnn_normalization(const b200dnn_norm_t *d, void *stream) 
     B2_TRY(stage_in(d->running_var, (size_t)d->num_channels * 4, st, &v));
     norm_batch_kernel<<<(unsigned)((elems + 255) / 256), 256, 0, st>>>(a, (const float *)m, (const float *)v, d->num_channels, n);
   } else {
-    // full-width form: bf16 in and out, whole 16-byte vectors everywhere, at most 8 vectors per thread
+    // full-width form: bf16 in and out in 16-byte aligned tensors, at most 16384 columns; rows that are no whole vectors (ANY) need codes laid out as the rows are
     auto al16 = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-    const bool vec = d->src_dt == B200DNN_BF16 && d->dst_dt == B200DNN_BF16 && n % 8 == 0 && n <= (int64_t)kNormThreads * 64 &&
+    const bool any = n % 8 != 0;
+    const bool vec = d->src_dt == B200DNN_BF16 && d->dst_dt == B200DNN_BF16 && n <= 16384 - (any ? 14 : 0) &&
                      al16(a.x) && al16(a.y) && al16(a.residual) && (!a.use_scale || al16(a.gamma)) && (!(a.use_shift && !rms) || al16(a.beta)) &&
-                     (!a.q || (a.q_ld % 8 == 0 && (reinterpret_cast<uintptr_t>(a.q) & 7) == 0)) && env_int("B200DNN_NORM_VEC", 1) != 0;
+                     (!a.q || ((any ? a.q_ld == n : a.q_ld % 8 == 0) && (reinterpret_cast<uintptr_t>(a.q) & 7) == 0)) && env_int("B200DNN_NORM_VEC", 1) != 0;
     if (vec) {
-      const int nvec = (int)(n / 8);
-      // two vectors per thread before the CTA grows (measured: 58 us for 16384 rows of 4096 against 122 us with four and
-      // 195 us with eight: registers, and so resident CTAs, matter more than bytes in flight per thread)
-      const int per = env_int("B200DNN_NORM_NV", 2);
-      int threads = 32;
-      while (threads < kNormThreads && threads * per < nvec) threads <<= 1;
+      const int nvec = (int)((n + (any ? 14 : 0)) / 8);          // vectors that a row touches at most
+      // Two vectors per thread while the CTA grows with the row; four for many rows of 2048 columns or more, which pay less for what every thread does once
+      // per row (16384 columns need four).  us with two and four: 4700 x 3328 with codes 24.7, 22.4; 12000 x 2048 LayerNorm 30.6, 28.1; 8830 x 11136 with
+      // codes 143, 138; but 16000 x 1024 26.9, 28.3; 300 x 1001 4.2, 6.6; 92 x 9472 5.1, 5.7.
+      const int per = nvec > 1536 || (batch >= 2048 && nvec >= 256) ? 4 : 2;
+      const int threads = (int)round_up((nvec + per - 1) / per, 32);
       const int nv = (nvec + threads - 1) / threads;
       const long long cap = (long long)R.sm_count * 64;
       const unsigned grid = (unsigned)(batch < cap ? batch : cap);
-      const int nvt = nv <= 1 ? 1 : (nv <= 2 ? 2 : (nv <= 4 ? 4 : 8));
-      if (nvt == 1) B2_TRY(launch_pdl(norm_rows_vec_kernel<1>, grid, (unsigned)threads, 0, st, true, a));
-      else if (nvt == 2) B2_TRY(launch_pdl(norm_rows_vec_kernel<2>, grid, (unsigned)threads, 0, st, true, a));
-      else if (nvt == 4) B2_TRY(launch_pdl(norm_rows_vec_kernel<4>, grid, (unsigned)threads, 0, st, true, a));
-      else B2_TRY(launch_pdl(norm_rows_vec_kernel<8>, grid, (unsigned)threads, 0, st, true, a));
+      auto go = [&](auto kern) { return launch_pdl(kern, grid, (unsigned)threads, 0, st, true, a); };
+      auto pick = [&](auto one, auto two, auto two_512, auto two_768, auto four_128, auto four_256, auto four_512) {
+        if (nv <= 1) return go(one);
+        if (nv <= 2) return threads <= 256 ? go(two) : threads <= 512 ? go(two_512) : go(two_768);
+        return threads <= 128 ? go(four_128) : threads <= 256 ? go(four_256) : go(four_512);
+      };
+      B2_TRY(any ? pick(norm_rows_vec_kernel<1, 256, 4, true>, norm_rows_vec_kernel<2, 256, 5, true>, norm_rows_vec_kernel<2, 512, 2, true>, norm_rows_vec_kernel<2, 768, 2, true>,
+                        norm_rows_vec_kernel<4, 128, 8, true>, norm_rows_vec_kernel<4, 256, 4, true>, norm_rows_vec_kernel<4, 512, 2, true>)
+                 : pick(norm_rows_vec_kernel<1, 256, 6, false>, norm_rows_vec_kernel<2, 256, 6, false>, norm_rows_vec_kernel<2, 512, 3, false>, norm_rows_vec_kernel<2, 768, 2, false>,
+                        norm_rows_vec_kernel<4, 128, 8, false>, norm_rows_vec_kernel<4, 256, 4, false>, norm_rows_vec_kernel<4, 512, 2, false>));
       B2_LAUNCHED();
       B2_CUDA(cudaGetLastError());
       return finish_out({&o_y, &o_res, &o_q, &o_s}, st);
