@@ -56,8 +56,8 @@ template <int BM, int GPB> struct GsTcShape {
 };
 
 __device__ __forceinline__ void tc_mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-               "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n}"
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nelect.sync _|q, 0xffffffff;\n"
+               "@q tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n}"
                ::"r"(d_tmem), "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -147,7 +147,7 @@ gs_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
       const int nt = tile / a.m_tiles, y = nt * 16, m0 = (tile - nt * a.m_tiles) * BM;
       for (int kb = kb0; kb < kb1; ++kb) {
         const uint32_t dst = smem0 + (uint32_t)s * Sh::kStage;
-        if (pre == 0 && ok) ok = mbar_wait(done(s), ph ^ 1u);
+        if (pre == 0 && !mbar_wait_warp(done(s), ph ^ 1u)) { ok = false; break; }
         if (elect_one()) {
           if (acts) {
             mbar_expect_tx(ready(s), (uint32_t)(BM * 128));
@@ -161,7 +161,6 @@ gs_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
         if (pre > 0) --pre;
         if (++s == S) { s = 0; ph ^= 1u; }
       }
-      ok = __all_sync(0xffffffffu, ok) != 0;
       if (!ok) break;
     }
     if (!ok && lane == 0) { s_err = 1; report_status(a.status, 51); }
@@ -170,10 +169,10 @@ gs_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
     const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BM >> 3) << 17) | (8u << 24);      // s32 += s8 x s8, M = 128, N = BM
     int s = 0, b = 0, acc = 0; uint32_t ph = 0, aph = 0;
     bool ok = true;
-    // (the lanes compare notes once per tile: after an expired wait the remaining blocks are issued on what the stages hold; the call has failed)
     auto wait2 = [&](uint32_t bar, uint32_t parity, uint32_t bar2, uint32_t parity2) {        // both first tries in flight
       const uint32_t t1 = mbar_try_wait(bar, parity), t2 = mbar_try_wait(bar2, parity2);
-      return (t1 || mbar_wait(bar, parity)) && (t2 || mbar_wait(bar2, parity2));
+      if (__all_sync(0xffffffffu, t1 & t2)) return true;
+      return mbar_wait_warp(bar, parity) && mbar_wait_warp(bar2, parity2);
     };
     auto next_acc = [&]() { if (++acc == NA) { acc = 0; aph ^= 1u; } };
     for (int tile = tile0; tile < tiles; tile += tile_step) {
@@ -182,44 +181,40 @@ gs_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
         const uint64_t da = make_smem_desc(smem0 + (uint32_t)s * Sh::kStage + 8192u);
         const uint32_t wa = tmem_w + (uint32_t)(b * 32);
         if constexpr (GPB == 1) {
-          if (ok) ok = in_group ? mbar_wait(ready(s), ph) : wait2(ready(s), ph, acc_free(acc), aph ^ 1u);
+          ok = in_group ? mbar_wait_warp(ready(s), ph) : wait2(ready(s), ph, acc_free(acc), aph ^ 1u);
+          if (!ok) break;
           tc_fence_after();
           const uint32_t d = tmem + (uint32_t)(acc * BM);
           const bool last = in_group == gb - 1;
-          if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) tc_mma_i8_ts(d, wa + (uint32_t)(k * 8), da + (uint64_t)(k * 2), idesc, (in_group | k) ? 1u : 0u);
-            tc_commit(done(s));
-            if (last) tc_commit(acc_full(acc));
-          }
-          __syncwarp();
+          for (int k = 0; k < 4; ++k) tc_mma_i8_ts(d, wa + (uint32_t)(k * 8), da + (uint64_t)(k * 2), idesc, (in_group | k) ? 1u : 0u);
+          tc_commit(done(s));
+          if (last) tc_commit(acc_full(acc));
           if (last) { in_group = 0; next_acc(); } else ++in_group;
         } else {
           constexpr int KS = 4 / GPB;
 #pragma unroll
           for (int h = 0; h < GPB / PG; ++h) {
-            if (h > 0 && kb * GPB + h * PG >= a.G) continue;
-            if (ok) ok = h ? mbar_wait(acc_free(acc), aph ^ 1u) : wait2(ready(s), ph, acc_free(acc), aph ^ 1u);
+            if (!ok || (h > 0 && kb * GPB + h * PG >= a.G)) continue;
+            ok = h ? mbar_wait_warp(acc_free(acc), aph ^ 1u) : wait2(ready(s), ph, acc_free(acc), aph ^ 1u);
+            if (!ok) continue;
             tc_fence_after();
             const bool last = h == GPB / PG - 1 || kb * GPB + (h + 1) * PG >= a.G;
-            if (elect_one()) {
-              // (past the last group the stage holds zeros, and nobody reads the sums)
+            // (past the last group the stage holds zeros, and nobody reads the sums)
 #pragma unroll
-              for (int k = 0; k < PG * KS; ++k) {
-                const int kk = h * PG * KS + k;
-                tc_mma_i8_ts(tmem + (uint32_t)((acc * PG + k / KS) * BM), wa + (uint32_t)(kk * 8), da + (uint64_t)(kk * 2), idesc, k % KS ? 1u : 0u);
-              }
-              tc_commit(acc_full(acc));
-              if (last) tc_commit(done(s));
+            for (int k = 0; k < PG * KS; ++k) {
+              const int kk = h * PG * KS + k;
+              tc_mma_i8_ts(tmem + (uint32_t)((acc * PG + k / KS) * BM), wa + (uint32_t)(kk * 8), da + (uint64_t)(kk * 2), idesc, k % KS ? 1u : 0u);
             }
-            __syncwarp();
+            tc_commit(acc_full(acc));
+            if (last) tc_commit(done(s));
             next_acc();
           }
+          if (!ok) break;
         }
         if (++s == S) { s = 0; ph ^= 1u; }
         if (++b == NW) b = 0;
       }
-      ok = __all_sync(0xffffffffu, ok) != 0;
       if (!ok) break;
     }
     if (!ok && lane == 0) { s_err = 1; report_status(a.status, 52); }
@@ -233,7 +228,7 @@ gs_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
     bool ok = true;
     const int mine = tile0 < tiles ? ((tiles - 1 - tile0) / tile_step + 1) * (kb1 - kb0) : 0;       // blocks of this CTA
     for (int n = set; n < mine; n += 2) {
-      if (ok) ok = mbar_wait(codes(s), ph);
+      if (!mbar_wait_warp(codes(s), ph)) { ok = false; break; }
       const uint32_t p = smem0 + (uint32_t)s * Sh::kStage + src;
       const uint4 v0 = ld_shared_v4(p + flip), v1 = ld_shared_v4(p + (flip ^ 16u)), v2 = ld_shared_v4(p + 256u + flip), v3 = ld_shared_v4(p + 256u + (flip ^ 16u));
       const uint4 w0 = flip ? v1 : v0, w1 = flip ? v0 : v1, w2 = flip ? v3 : v2, w3 = flip ? v2 : v3;
@@ -242,7 +237,7 @@ gs_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
 #pragma unroll
       for (int i = 0; i < 16; ++i) { r[2 * i] = (w[i] << 4) & 0xF0F0F0F0u; r[2 * i + 1] = w[i] & 0xF0F0F0F0u; }
       if (n >= NW) {
-        if (ok) ok = mbar_wait(done(sf), phf);
+        if (!mbar_wait_warp(done(sf), phf)) { ok = false; break; }
         if ((sf += 2) >= S) { sf -= S; phf ^= 1u; }
         tc_fence_after();
       }
@@ -254,7 +249,6 @@ gs_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
       if (lane == 0) mbar_arrive(ready(s));
       if ((s += 2) >= S) { s -= S; ph ^= 1u; }
       if ((b += 2) >= NW) b -= NW;
-      if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
     }
     if (!ok && lane == 0) { s_err = 1; report_status(a.status, 53); }
   } else {
@@ -302,7 +296,7 @@ gs_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
           w2[j] = f32x2_pack(w, w);
         }
         c_slot = c_slot + PG == kGsTcScaleSlots ? 0 : c_slot + PG;
-        if (ok) ok = mbar_wait(acc_full(acc), aph);
+        if (!mbar_wait_warp(acc_full(acc), aph)) { ok = false; break; }
         tc_fence_after();
         __syncwarp();
         const uint32_t ta = tq + (uint32_t)(acc * PG * BM);

@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(128, 1) int8_peak_kernel(int iters, int32_t *s
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
   bool ok = true;
-  if (threadIdx.x == 0) {
+  if (warp == 0) {      // (the MMAs elect the lane that issues)
     const uint32_t idesc = make_idesc_i8(0, kPeakBN);
     const uint64_t da = make_smem_desc(smem0), db = make_smem_desc(smem0 + kTcBM * kTcBK);
     for (int it = 0; it < iters; ++it) {
@@ -54,8 +54,8 @@ __global__ void __launch_bounds__(128, 1) int8_peak_kernel(int iters, int32_t *s
       for (int k = 0; k < kTcBK / 32; ++k) tc_mma_i8(d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (it > 1 || k) ? 1u : 0u);
     }
     tc_commit(smem_u32(&bar));
-    ok = mbar_wait(smem_u32(&bar), 0);
-    if (!ok) report_status(status, 31);
+    ok = mbar_wait_warp(smem_u32(&bar), 0);
+    if (!ok && threadIdx.x == 0) report_status(status, 31);
   }
   __syncthreads();
   tc_fence_after();

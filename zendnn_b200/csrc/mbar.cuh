@@ -42,6 +42,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     if (clock64() - t0 > kWaitCycles) return false;
   }
 }
+// The same for a converged warp, one answer for all its lanes.  A lane that waits inside a branch of its own takes 200 clocks when the phase is already complete,
+// a whole warp 80 (the loop behind the first try is out of line: inlined, it costs 20 to 70 in every role that issues copies or products).
+static __device__ __noinline__ bool mbar_wait_warp_more(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0; }
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return mbar_wait_warp_more(bar, parity);
+}
 // one lane of a converged warp
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;

@@ -76,6 +76,15 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map
   asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
                ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar) : "memory");
 }
+// Issued by one lane (the elected one of a converged warp).  (With the election inside the asm statement, as the tile kernels have it, this kernel was 2 to 10 % slower.)
+__device__ __forceinline__ void tc_mma_bf16_lane(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
+               ::"r"(d_tmem), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tc_commit_lane(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
 // A from tensor memory (bf16 pairs, one row per lane), B from shared memory
 __device__ __forceinline__ void tc_mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
@@ -207,8 +216,8 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < 4 * DB; ++k)
-          if (k < ksteps) tc_mma_bf16(d_tmem, qa + (k >> 2) * kBoxD + (k & 3) * 2, ka + (k >> 2) * kBoxD + (k & 3) * 2, idesc_s, k ? 1u : 0u);
-        tc_commit(bar);
+          if (k < ksteps) tc_mma_bf16_lane(d_tmem, qa + (k >> 2) * kBoxD + (k & 3) * 2, ka + (k >> 2) * kBoxD + (k & 3) * 2, idesc_s, k ? 1u : 0u);
+        tc_commit_lane(bar);
       }
       __syncwarp();
     };
@@ -221,7 +230,7 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       }
       __syncwarp();
     };
-    auto commit = [&](uint32_t bar) { if (elect_one()) tc_commit(bar); __syncwarp(); };
+    auto commit = [&](uint32_t bar) { if (elect_one()) tc_commit_lane(bar); __syncwarp(); };
     auto wait = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0; };
     bool ok = wait(q_full, 0);
     int u = 0;

@@ -13,7 +13,7 @@
 //   - Programmatic dependent launch: where the weight does not depend on the kernel before (see SkinnyArgs::early) its ring is
 //     requested before griddepcontrol.wait and streams while, for instance, the activations are still being quantised.
 // Bound by HBM behind a fixed cost of about 5 us (launch, the first copies' latency, the addition).  bf16, M = 8, K = 4096, N = 11008 (90 MB): 31.0 us
-// in the 128-row tile kernel -> 19.8 us (4.6 TB/s).  INT8, M = 32, same sizes: 17.7 -> 13.5 us.
+// in the 128-row tile kernel -> 19.2 us (4.7 TB/s).  INT8, M = 32, same sizes: 17.7 -> 13.5 us.
 // Every wait is bounded, as in tc_gemm.cuh.
 #pragma once
 #include "common.cuh"
@@ -85,48 +85,47 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   const int q = warp & 3, part = (warp - 2) >> 2, col = q * 32 + lane, n4 = tile * 128 + lane * 4;
   float ws[4], bias[4]; int32_t comp[4];
   if (warp == 0) {
-    if (lane == 0) {
-      const int n_it = kb1 - kb0, pre = min(n_it, S);
-      auto load_w = [&](int i, int slot) {
-        mbar_expect_tx(full_bar(slot), stage_bytes);
-        tma_load_wt(smem0 + (uint32_t)slot * stage_bytes, &map_w, kb0 + i, tile * 16, full_bar(slot));
-      };
-      auto load_a = [&](int i, int slot) { tma_load_2d(smem0 + (uint32_t)slot * stage_bytes + w_bytes, &map_a, (kb0 + i) * 128, 0, full_bar(slot)); };
-      if (a.early && !a.test_no_loads) for (int i = 0; i < pre; ++i) load_w(i, i);
-      asm volatile("griddepcontrol.wait;" ::: "memory");
-      if (!a.test_no_loads) {
-        for (int i = 0; i < pre; ++i) { if (!a.early) load_w(i, i); load_a(i, i); }
-        int slot = 0; uint32_t phase = 0;
-        for (int i = pre; i < n_it; ++i) {
-          if (!mbar_wait(empty_bar(slot), phase)) { s_err = 1; report_status(a.status, 31); break; }
-          load_w(i, slot); load_a(i, slot);
-          if (++slot == S) { slot = 0; phase ^= 1u; }
-        }
+    // (the whole warp walks the blocks and waits, one elected lane issues)
+    const int n_it = kb1 - kb0, pre = min(n_it, S);
+    auto load_w = [&](int i, int slot) {
+      mbar_expect_tx(full_bar(slot), stage_bytes);
+      tma_load_wt(smem0 + (uint32_t)slot * stage_bytes, &map_w, kb0 + i, tile * 16, full_bar(slot));
+    };
+    auto load_a = [&](int i, int slot) { tma_load_2d(smem0 + (uint32_t)slot * stage_bytes + w_bytes, &map_a, (kb0 + i) * 128, 0, full_bar(slot)); };
+    if (a.early && !a.test_no_loads && elect_one()) for (int i = 0; i < pre; ++i) load_w(i, i);
+    __syncwarp();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!a.test_no_loads) {
+      if (elect_one()) for (int i = 0; i < pre; ++i) { if (!a.early) load_w(i, i); load_a(i, i); }
+      __syncwarp();
+      int slot = 0; uint32_t phase = 0;
+      for (int i = pre; i < n_it; ++i) {
+        if (!mbar_wait_warp(empty_bar(slot), phase)) { if (lane == 0) { s_err = 1; report_status(a.status, 31); } break; }
+        if (elect_one()) { load_w(i, slot); load_a(i, slot); }
+        __syncwarp();
+        if (++slot == S) { slot = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    // the whole warp walks the blocks and one elected lane issues (operands stay in uniform registers)
+    // the whole warp walks the blocks (operands stay in uniform registers)
     // A = weight (s8, or bf16), B = activations (u8 | s8, or bf16), both K-major; M = 128, N = MP
     const uint32_t idesc = F16 ? make_idesc_bf16(a.MP) : ((2u << 4) | (1u << 7) | ((a.a_unsigned ? 0u : 1u) << 10) | ((uint32_t)(a.MP >> 3) << 17) | (8u << 24));
     int slot = 0; uint32_t phase = 0;
     bool ok = true;
     for (int kb = kb0; kb < kb1; ++kb) {
-      if (ok) ok = mbar_wait(full_bar(slot), phase);
+      if (!mbar_wait_warp(full_bar(slot), phase)) { ok = false; break; }
       tc_fence_after();
       const uint32_t sw = smem0 + (uint32_t)slot * stage_bytes;
       const uint64_t dw = make_smem_desc(sw), da = make_smem_desc(sw + w_bytes);
-      if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if constexpr (F16) tc_mma_bf16(tmem, dw + (uint64_t)(k * 2), da + (uint64_t)(k * 2), idesc, ((kb - kb0) | k) ? 1u : 0u);
-          else tc_mma_i8(tmem, dw + (uint64_t)(k * 2), da + (uint64_t)(k * 2), idesc, ((kb - kb0) | k) ? 1u : 0u);
-        }
-        tc_commit(empty_bar(slot));
+      for (int k = 0; k < 4; ++k) {
+        if constexpr (F16) tc_mma_bf16(tmem, dw + (uint64_t)(k * 2), da + (uint64_t)(k * 2), idesc, ((kb - kb0) | k) ? 1u : 0u);
+        else tc_mma_i8(tmem, dw + (uint64_t)(k * 2), da + (uint64_t)(k * 2), idesc, ((kb - kb0) | k) ? 1u : 0u);
       }
-      __syncwarp();
+      tc_commit(empty_bar(slot));
       if (++slot == S) { slot = 0; phase ^= 1u; }
     }
-    if (__all_sync(0xffffffffu, ok)) { if (elect_one()) tc_commit(tfull_bar); }
+    if (ok) tc_commit(tfull_bar);
     else if (lane == 0) { s_err = 1; report_status(a.status, 32); }
     __syncwarp();
   } else {
@@ -142,7 +141,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       comp[i] = (!F16 && in && epi.has_zp) ? load_zp(epi) * epi.colsum[n] : 0;
     }
     // the partial sums go to shared memory as [row][128 columns], over the ring (every product that read it has completed)
-    const bool ok = __all_sync(0xffffffffu, mbar_wait(tfull_bar, 0));
+    const bool ok = mbar_wait_warp(tfull_bar, 0);
     if (ok) {
       tc_fence_after();
       for (int c = part; c * 16 < a.M; c += 2) {

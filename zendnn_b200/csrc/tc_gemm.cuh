@@ -117,14 +117,17 @@ __device__ __forceinline__ void tma_load_wt_pair(uint32_t dst, const CUtensorMap
   asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
                ::"r"(dst), "l"(map), "r"(0), "r"(0), "r"(kblock), "r"(group), "r"(bar) : "memory");
 }
+// MMAs and commits below are issued by a converged warp: the instruction is predicated on the elected lane (always the same one) inside its asm statement.  With a
+// branch around them the operands no longer count as the same in every lane, and each MMA first moves them: a 128-byte block of K (a wait, four MMAs, a commit) took 370
+// clocks whatever the tile, in a loop of its own; as it is, 227 with N = 16 and the tensor pipe's own 257 with N = 128.
 // completion of the pair's MMAs, signalled on the barrier at the same offset in both CTAs
 __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+  asm volatile("{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}"
                ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
 __device__ __forceinline__ void tc_mma_i8_pair(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-               "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n}"
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nelect.sync _|q, 0xffffffff;\n"
+               "@q tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n}"
                ::"r"(d_tmem), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
 }
 // arrive on a barrier of another CTA of the cluster (shared::cluster address from cluster_map)
@@ -134,11 +137,11 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+  asm volatile("{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-               "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}"
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nelect.sync _|q, 0xffffffff;\n"
+               "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}"
                ::"r"(d_tmem), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
@@ -198,13 +201,13 @@ __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sy
 
 // bf16 x bf16 -> f32, M x N x 16 (32 bytes of K per instruction, as kind::i8)
 __device__ __forceinline__ void tc_mma_bf16_pair(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-               "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n}"
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nelect.sync _|q, 0xffffffff;\n"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n}"
                ::"r"(d_tmem), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
 }
 __device__ __forceinline__ void tc_mma_bf16(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nelect.sync _|q, 0xffffffff;\n"
+               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
                ::"r"(d_tmem), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
 }
 
@@ -677,18 +680,18 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    // (the whole warp walks the tiles so that the group lookup is a warp operation; lane 0 issues the copies)
+    // (the whole warp walks the tiles and waits, one elected lane issues the copies)
     int stage = 0; uint32_t phase = 0;
     bool ok = true;
     for (int tile = tile0; tile < total_tiles && !a.test_no_loads; tile += tile_step) {
       // one decision for the whole warp (the lookup below uses warp-wide operations)
       if (!__shfl_sync(0xffffffffu, (ok && !s_err) ? 1 : 0, 0)) break;
       const TileCoord t = tc_tile_warp(a, tile, m_tiles, lane, tile_m, sub);
-      if (lane == 0) {
-        const CUtensorMap *mb = a.maps_b ? a.maps_b + t.g : &map_b0;
-        for (int kb = kb_begin; kb < kb_end; ++kb) {
-          if (!mbar_wait(empty_bar(stage), phase ^ 1u)) { s_err = 1; report_status(a.status, 1); ok = false; break; }
-          const uint32_t sa = smem0 + (uint32_t)stage * stage_bytes;
+      const CUtensorMap *mb = a.maps_b ? a.maps_b + t.g : &map_b0;
+      for (int kb = kb_begin; kb < kb_end; ++kb) {
+        if (!mbar_wait_warp(empty_bar(stage), phase ^ 1u)) { if (lane == 0) { s_err = 1; report_status(a.status, 1); } ok = false; break; }
+        const uint32_t sa = smem0 + (uint32_t)stage * stage_bytes;
+        if (elect_one()) {
           if constexpr (PAIR) {
             // both CTAs' copies are counted on the leader's barrier; the leader expects the bytes of both
             const uint32_t lead_bar = cluster_map(full_bar(stage), 0);
@@ -700,48 +703,42 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             tma_load_2d(sa, &map_a, kb * kTcBK, t.row0, full_bar(stage));
             tma_load_wt(sa + a_bytes, mb, kb, (t.nt * a.BN) >> 3, full_bar(stage));
           }
-          if (++stage == S) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == S) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    // The whole warp walks the tiles and one elected lane issues, so that operands and control flow are warp-uniform: inside a
-    // single-lane branch every MMA first moves its descriptors to uniform registers (about 100 clocks an MMA, longer than the MMA itself
-    // for tiles up to 128 columns; the pair form gained too: 127 -> 113 us at M = 2048, K = 4096, N = 14336 with the epilogue below).
+    // (the whole warp walks the tiles: operands and control flow are the same in every lane, see the MMAs above)
     if (!PAIR || crank == 0) {      // pair form: the leader issues for both CTAs
       const uint32_t idesc = F16 ? make_idesc_bf16(a.BN, tile_m) : make_idesc_i8(a.a_unsigned, a.BN, tile_m);
       int stage = 0; uint32_t phase = 0; int acc = 0; uint32_t acc_phase = 0;
-      auto wait = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0; };
       auto commit = [&](uint32_t bar) { if constexpr (PAIR) tc_commit_pair(bar); else tc_commit(bar); };
       for (int tile = tile0; tile < total_tiles && __shfl_sync(0xffffffffu, s_err ? 0 : 1, 0); tile += tile_step) {
-        if (!wait(tempty_bar(acc), acc_phase ^ 1u)) { if (lane == 0) { s_err = 2; report_status(a.status, 2); } break; }
+        if (!mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u)) { if (lane == 0) { s_err = 2; report_status(a.status, 2); } break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * a.BN);
-        // (the lanes compare notes once per tile, not per K block: after an expired wait the remaining blocks are issued on what the
-        // stages hold, and the tile is not published)
         bool ok = true;
         for (int kb = kb_begin; kb < kb_end; ++kb) {
-          if (ok) ok = mbar_wait(full_bar(stage), phase);
+          if (!mbar_wait_warp(full_bar(stage), phase)) { ok = false; break; }
           if (lane == 0 && kb == kb_begin && tile == tile0) TC_STAMP(2);
           tc_fence_after();
           const uint32_t sa = smem0 + (uint32_t)stage * stage_bytes;
           const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + a_bytes);
-          if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < kTcBK / 32; ++k) {
-              const uint32_t accum = ((kb - kb_begin) | k) ? 1u : 0u;
-              if constexpr (PAIR && F16) tc_mma_bf16_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
-              else if constexpr (PAIR) tc_mma_i8_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
-              else if constexpr (F16) tc_mma_bf16(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
-              else tc_mma_i8(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
-            }
-            commit(empty_bar(stage));
+          for (int k = 0; k < kTcBK / 32; ++k) {
+            const uint32_t accum = ((kb - kb_begin) | k) ? 1u : 0u;
+            if constexpr (PAIR && F16) tc_mma_bf16_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
+            else if constexpr (PAIR) tc_mma_i8_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
+            else if constexpr (F16) tc_mma_bf16(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
+            else tc_mma_i8(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, accum);
           }
+          commit(empty_bar(stage));
           if (++stage == S) { stage = 0; phase ^= 1u; }
         }
-        if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) { s_err = 3; report_status(a.status, 3); } break; }
-        if (elect_one()) commit(tfull_bar(acc));
+        if (!ok) { if (lane == 0) { s_err = 3; report_status(a.status, 3); } break; }
+        commit(tfull_bar(acc));
         if (lane == 0 && tile == tile0) TC_STAMP(3);
         if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
@@ -802,7 +799,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
       }
       // the buffer is free when the epilogue warps have left the tile that used it two tiles ago
-      if (!__all_sync(0xffffffffu, mbar_wait(cempty_bar(cb), cphase ^ 1u))) { if (lane == 0) { s_err = 6; report_status(a.status, 6); } break; }
+      if (!mbar_wait_warp(cempty_bar(cb), cphase ^ 1u)) { if (lane == 0) { s_err = 6; report_status(a.status, 6); } break; }
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         if (lane + 32 * j < a.BN) { cols[cb].ws[lane + 32 * j] = cw[j]; cols[cb].bias[lane + 32 * j] = cbv[j]; cols[cb].comp[lane + 32 * j] = ck[j]; }
@@ -826,7 +823,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     int ob = 0; uint32_t ophase = 0;            // operand buffer of the current tile
     for (int tile = tile0; tile < total_tiles; tile += tile_step) {
       // everything from global memory was put into shared memory by the operand warp
-      if (!mbar_wait(cfull_bar(ob), ophase)) { if (lane == 0) { s_err = 5; report_status(a.status, 5); } break; }
+      if (!mbar_wait_warp(cfull_bar(ob), ophase)) { if (lane == 0) { s_err = 5; report_status(a.status, 5); } break; }
       const TileMeta tm = meta[ob];
       const TileCols &tcols = cols[ob];
       const bool row_ok = row_in_tile < tm.rows;
@@ -836,7 +833,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       cx.wei_scale = nullptr; cx.colsum = nullptr; cx.bias = nullptr; cx.dst = tm.dst; cx.ldc = tm.ldc;
       cx.s_src = row_scale[ob][row_in_tile];
       const int pc_tile = tm.nt * a.BN;
-      if (!mbar_wait(tfull_bar(acc), acc_phase)) { if (lane == 0) { s_err = 4; report_status(a.status, 4); } break; }
+      if (!mbar_wait_warp(tfull_bar(acc), acc_phase)) { if (lane == 0) { s_err = 4; report_status(a.status, 4); } break; }
       if (warp == 2 && lane == 0 && tile == tile0) TC_STAMP(4);
       tc_fence_after();
       const bool has_bias = tm.has_bias != 0;
