@@ -1,4 +1,6 @@
 // Launchers of the fused attention kernels (sdpa_flash.cuh): which form takes a call, tensor maps, grids.
+#include <algorithm>
+#include <cmath>
 #include <cudaTypedefs.h>
 #include "runtime.cuh"
 #include "sdpa_flash.cuh"
@@ -106,6 +108,9 @@ int32_t launch_sdpa_flash(const SdpaCall &c, cudaStream_t st) {
   // and V stay in the L2 together; head after head otherwise.
   a.bh_major = !c.causal || 4 * heads * c.KV * c.D > (64ll << 20);
   a.scale = c.scale; a.causal = c.causal;
+  const double c_exact = (double)c.scale * 1.44269504088896340736;
+  a.c = (float)c_exact;
+  a.kappa = std::isnormal(a.c) ? (float)((c_exact / (double)a.c - 1.0) * 0.693147180559945309417) : 0.f;
   a.mask = SdpaMask{c.mask, c.mask_dt, c.mb, c.mh, c.mi};
   const int64_t mstep = c.mask_dt == B200DNN_F32 ? 4 : 8;
   a.mask_vec = (reinterpret_cast<uintptr_t>(c.mask) & 15) == 0 && c.mb % mstep == 0 && c.mh % mstep == 0 && c.mi % mstep == 0;
@@ -119,14 +124,19 @@ int32_t launch_sdpa_flash(const SdpaCall &c, cudaStream_t st) {
   B2_TRY(make_map_heads(&mk, c.k, c.D, c.KV, a.kh ? c.H : 1, a.kb ? c.B : 1, c.ks[2], c.ks[1], c.ks[0]));
   B2_TRY(make_map_heads(&mv, c.v, c.D, c.KV, a.vh ? c.H : 1, a.vb ? c.B : 1, c.vs[2], c.vs[1], c.vs[0]));
   const int db = c.D <= 64 ? 1 : 2;
-  const size_t smem = (size_t)(a.tiles + kFlashSlots) * db * 16384 + 1024;
-  const unsigned grid = (unsigned)(heads * a.n_qt);
-  if (db == 1) {
-    if (c.mask) return launch(sdpa_flash_kernel<1, true>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
-    return launch(sdpa_flash_kernel<1, false>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
-  }
-  if (c.mask) return launch(sdpa_flash_kernel<2, true>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
-  return launch(sdpa_flash_kernel<2, false>, grid, kFlashThreads, smem, 1, st, mq, mk, mv, a);
+  // A CTA of one row tile has half the warps and half the tensor memory, so that two fit an SM where shared memory allows it: with one block of keys (two slots of
+  // the ring are used) or a head dimension up to 64.  us before and after: 192 heads of 100 keys, head_dim 128, causal 13.8 -> 10.0; 160 of 90, 64, causal 11.3 -> 8.4;
+  // 320 of 128, 128, causal 23.3 -> 18.2.  But one CTA per SM while there are SMs for all of them (two of one launch on an SM: 24 heads of 310 keys,
+  // 64, with a mask 14.3 -> 18.5).
+  const bool one_block = a.tiles == 1 && (c.KV <= 128 || (c.causal && c.S <= 128));
+  size_t smem = (size_t)(a.tiles + (one_block ? 2 : kFlashSlots)) * db * 16384 + 1024;
+  if (heads * a.n_qt <= sms) smem = std::max(smem, (size_t)120 * 1024);
+  const unsigned grid = (unsigned)(heads * a.n_qt), threads = 32u * (8 * a.tiles + 2);
+  auto go = [&](auto plain, auto masked) { return launch(c.mask ? masked : plain, grid, threads, smem, 1, st, mq, mk, mv, a); };
+  if (c.D <= 64) return go(sdpa_flash_kernel<4, false>, sdpa_flash_kernel<4, true>);
+  if (c.D <= 80) return go(sdpa_flash_kernel<5, false>, sdpa_flash_kernel<5, true>);
+  if (c.D <= 96) return go(sdpa_flash_kernel<6, false>, sdpa_flash_kernel<6, true>);
+  return go(sdpa_flash_kernel<8, false>, sdpa_flash_kernel<8, true>);
 }
 
 }  // namespace

@@ -7,13 +7,13 @@
 // round unnormalised probabilities instead and give other results; so the prompt kernel sweeps the keys twice: the first
 // sweep takes row maximum and row sum, the second recomputes the scores and multiplies the normalised probabilities with V.
 // The extra Q K^T costs half as much again on the tensor pipe and saves every rescale of the accumulator.
-// Score, mask, distance from the row maximum and quotient by the row sum are formed in natural units with the operations of the
-// three-step form (the distance with one rounding less).  Error of the f32 probabilities against double, mean / mean weighted by the
+// Every exponent is formed with one rounding (see flash_frame).  Error of the f32 probabilities against double, mean / mean weighted by the
 // probability / largest, for 2048 keys with scores of spread 1, 4 and 10 at scale 2^-3.5 (head_dim 128), in units of 1e-7:
-//   three-step form   0.94 / 0.79 / 5.3    3.5 / 1.9 / 24    9.4 / 2.4 / 62
-//   here              0.92 / 0.76 / 4.8    3.1 / 0.81 / 17    7.5 / 0.65 / 40
-// and 1.2 / 1.0 / 9 on both sides with a mask of spread 1, 150 / 150 / 330 with one of -1000; head_dim 64 without a mask 0.92 / 0.74 / 5.1 and
-// 0.93 / 0.75 / 4.9.
+//   three-step form                                                    0.94 / 0.79 / 5.3    3.5 / 1.9 / 24     9.4 / 2.4 / 62
+//   distance from the maximum, exponential corrected for its argument   1.03 / 0.89 / 6.1    3.1 / 0.95 / 17    7.5 / 0.95 / 40      (before)
+//   here                                                               1.02 / 0.92 / 6.1    3.0 / 1.05 / 17    7.4 / 1.01 / 30
+// (the last two from one run); with a mask of spread 1, before 1.3 / 1.1 / 10, 3.9 / 2.8 / 34 and 12 / 4.3 / 90, here 1.3 / 1.1 / 9, 3.4 / 2.2 / 25 and 10 / 3.2 / 57;
+// with one of -1000 150 / 150 / 330 on both sides at spread 1.
 #pragma once
 #include "common.cuh"
 #include "mbar.cuh"
@@ -30,6 +30,7 @@ struct SdpaFlashArgs {
   int tiles;                // 128-row tiles per CTA: 1 or 2
   int bh_major;             // work order: all query tiles of a head first, else all heads of the longest query tile first
   float scale;              // > 0
+  float c, kappa;           // scale log2 e in f32; (its relative error) ln 2
   int causal;
   SdpaMask mask; int mask_vec;   // mask_vec: every mask row starts on a 16-byte boundary
   int kb, kh, vb, vh;       // 0 where K / V are broadcast over the batch / the heads (stride 0), else 1
@@ -39,8 +40,7 @@ struct SdpaFlashArgs {
   int test_no_loads;        // test hook, as in SdpaDecodeArgs
 };
 
-constexpr int kFlashSoftmaxWarps = 16;  // two 128-row tiles x two halves of a key block x four lane quadrants
-constexpr int kFlashThreads = 32 * (kFlashSoftmaxWarps + 2);
+constexpr int kFlashThreads = 32 * (16 + 2);      // softmax: two 128-row tiles x two halves of a key block x four lane quadrants; producer, MMAs
 constexpr int kFlashSlots = 4;          // K / V ring
 
 __device__ __forceinline__ float ex2f(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
@@ -50,45 +50,45 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { u
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 
-// exp(-u) of two arguments u >= 0 (infinities included), as 2^(u * -log2 e) with log2 e in two parts.  The plain form rounds the product; it serves
-// the row sum, where the roundings of hundreds of terms average out.  The corrected form multiplies by 1 + (exact product - rounded
-// product) * ln 2, so that what remains is the error of ex2.approx (and of u), of which the part that has one sign is in the sum as well.
+// Exponentials of a row.  z: score (natural units with the mask added; without a mask the raw product, the scale is in c).  With M = fl(zmax c) the exponent
+// x = z c - M is one fused operation and so one rounding, also where all scores share a large part.  M's own rounding moves every x of the row by the same amount and
+// leaves with the row sum, as long as both sweeps use the same M; c = fl(scale log2 e) is off by a factor 1 + kappa, which a factor 1 + kappa ln2 x
+// of the result makes good (for the row sum: the sum of 2^x x beside that of 2^x).  Rows whose M is so large that its rounding would leave the
+// range of an exponential are shifted by r = zmax first (such scores are multiples of 16 or more, their distance is exact); r = 0 otherwise.
+// Exponents stop at -127 (zero), so that an infinite one does not meet a zero in a product; a NaN passes.
 constexpr float kLog2e = 1.44269504088896340736f, kLog2eLo = (float)(1.44269504088896340736 - (double)kLog2e), kLn2 = 0.693147180559945309417f;
+constexpr float kFlashReach = 1.0f;         // the first sweep's frame follows the row maximum once a score's exponent passes this
+struct FlashFrame { float r, M; };
+__device__ __forceinline__ FlashFrame flash_frame(float m, float c) {
+  const float p = __fmul_rn(m, c);
+  const bool large = !(fabsf(p) <= 268435456.0f);
+  return FlashFrame{large ? m : 0.f, large ? 0.f : p};
+}
+// what moving from one frame to another adds to every exponent
+__device__ __forceinline__ float flash_shift(const FlashFrame &from, const FlashFrame &to, float c) {
+  return fmaxf(__fmaf_rn(from.r - to.r, c, from.M - to.M), -1000.f);
+}
+__device__ __forceinline__ uint64_t flash_exponent2(uint64_t z2, uint64_t c2, uint64_t nM2) {
+  float x0, x1;
+  upk2(fma2(z2, c2, nM2), x0, x1);
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x0) : "f"(-127.f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x1) : "f"(-127.f));
+  return pk2(x0, x1);
+}
 __device__ __forceinline__ uint64_t ex2_pair(uint64_t x2) {
   float x0, x1;
   upk2(x2, x0, x1);
   return pk2(ex2f(x0), ex2f(x1));
-}
-__device__ __forceinline__ uint64_t exp_neg2_plain(uint64_t u2) {
-  return ex2_pair(fma2(u2, pk2(-kLog2e, -kLog2e), mul2(u2, pk2(-kLog2eLo, -kLog2eLo))));
-}
-__device__ __forceinline__ uint64_t exp_neg2(uint64_t u2) {
-  float u0, u1;
-  upk2(u2, u0, u1);
-  u2 = pk2(fminf(u0, 1e4f), fminf(u1, 1e4f));      // (already 0; an infinity would meet itself below)
-  const uint64_t x2 = mul2(u2, pk2(-kLog2e, -kLog2e));
-  const uint64_t r2 = fma2(u2, pk2(kLog2eLo, kLog2eLo), fma2(u2, pk2(kLog2e, kLog2e), x2));      // what rounding the product dropped
-  const uint64_t e2 = ex2_pair(x2);
-  return fma2(mul2(e2, pk2(-kLn2, -kLn2)), r2, e2);
 }
 
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, int w, uint32_t bar) {
   asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
                ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar) : "memory");
 }
-// Issued by one lane (the elected one of a converged warp).  (With the election inside the asm statement, as the tile kernels have it, this kernel was 2 to 10 % slower.)
-__device__ __forceinline__ void tc_mma_bf16_lane(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-               ::"r"(d_tmem), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tc_commit_lane(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
 // A from tensor memory (bf16 pairs, one row per lane), B from shared memory
 __device__ __forceinline__ void tc_mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nelect.sync _|q, 0xffffffff;\n"
+               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
                ::"r"(d_tmem), "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -103,20 +103,24 @@ __device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t saddr, uint32_t l
   return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lead >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 
-// Prompt form: one CTA per (batch, head, 256 query rows), 576 threads.
+// Prompt form: one CTA per (batch, head, 256 query rows), 576 threads (128 rows: 320).
 //   warps 0-15      softmax: eight per 128-row tile, of which four take keys 0-63 of a block and four keys 64-127 (two threads per row), scores
-//                   read from tensor memory
-//   warp 16         TMA producer: Q once; K blocks of 128 keys (sweep 1); K and V blocks in turn (sweep 2)
-//   warp 17         MMA issuer
-// Tensor memory (512 columns): S0 S1 O0 O1.  In sweep 1 the O columns are the second score buffer of their tile, so the
+//                   read from tensor memory 32 at a time (64 at once left no registers: 200 bytes spilled, 174 against 134 us with a padding mask)
+//   next            TMA producer: Q once; K blocks of 128 keys (sweep 1); K and V blocks in turn (sweep 2)
+//   last            MMA issuer
+// Tensor memory: S0 S1 O0 O1, 128 columns each.  In sweep 1 the O columns are the second score buffer of their tile, so the
 // tensor pipe runs a block ahead; in sweep 2 the normalised probabilities replace the scores in place as bf16 pairs and are the
-// A operand of the product with V straight from tensor memory, and the two row tiles alternate: while one is in its
-// exponentials the other's products run.
-// Bounds, per pair of 128 x 128 blocks (both row tiles, both sweeps): 4096 clocks of exponentials (two per score, 16 a clock) and 3072 of
-// the tensor pipe (three products a block); it takes about 6900 (32 heads x 2048 without a mask, head_dim 128: 116 us in two waves of CTAs).
-// 256 query rows per CTA, because K and V then pass the L2 half as often as with 128
-// (64 KB per two blocks: 6 TB/s over the device at that rate, against 12 TB/s).
-template <int DB, bool MASK>
+// A operand of the product with V straight from tensor memory.  Sweep 2 goes in four streams, a tile's half of the keys each: as soon as its 64 probabilities a row
+// are there, P V of these keys and the scores of the next block's 64 keys are issued, while the other streams are in their
+// exponentials.  (Whole tiles of 128 keys waited for both halves and for the whole product: 3480 clocks a pair of blocks.)  One block of keys needs no second product: its
+// scores stay in tensor memory.
+// Bounds, per pair of 128 x 128 blocks (both row tiles): the exponentials, one per score and sweep at 16 a clock, 2048 clocks each, and the tensor pipe, 1024 in sweep 1 and
+// 2560 in sweep 2 (64 columns at a time run at two thirds of the rate; head_dim 64: half of each); measured inside a CTA 2500 to 2700 and 3300 (head_dim 64: 2470).
+// A share of the exponentials on the FMA pipe (a polynomial of degree six) was slower, 203 against 196 us: the pipes wait for one another, not for one of them.
+// 32 heads x 2048, us before the streams and the one-rounding exponents and now: causal 64.0 -> 62.9, none 123 -> 118.5, padding mask 160 -> 134; head_dim 64, 240 heads x
+// 1447 with padding 635 -> 538.  256 query rows per CTA, because K and V then pass the L2 half as often as with 128.
+// KS: 16-element steps of the head dimension
+template <int KS, bool MASK>
 __global__ void __launch_bounds__(kFlashThreads, 1)
 sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                   const __grid_constant__ CUtensorMap map_v, const SdpaFlashArgs a) {
@@ -125,9 +129,12 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   __shared__ float2 stats[2][2][128];                  // row maximum and row sum of each half
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile int s_err;
+  constexpr int DB = (KS + 3) / 4;                     // 64-element blocks of the head dimension
   constexpr uint32_t kBox = 128 * 128;                 // [128 rows][64 elements]
   constexpr uint32_t kTile = DB * kBox;                // 128 rows of Q, K or V
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (the same in every lane, and known to be)
+  const int sw = 8 * a.tiles;                          // softmax warps; then the producer's and the MMAs'
+  const uint32_t o_off = 128u * (uint32_t)a.tiles;     // tensor memory: scores of the tiles, then their outputs
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t ring0 = smem0 + (uint32_t)a.tiles * kTile;
   const uint32_t bar0 = smem_u32(bars);
@@ -138,6 +145,8 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   auto s_free = [&](int t, int b) { return bar0 + 8u * (5 + 2 * kFlashSlots + 2 * t + b); };
   auto p_ready = [&](int t, int half) { return bar0 + 8u * (9 + 2 * kFlashSlots + 2 * t + half); };
   auto o_done = [&](int t) { return bar0 + 8u * (13 + 2 * kFlashSlots + t); };
+  // (sweep 2 has barriers of its own: a phase of s_full may pass only when all warps of the tile have met the one before)
+  auto s2_full = [&](int t, int half) { return bar0 + 8u * (15 + 2 * kFlashSlots + 2 * t + half); };
 
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
@@ -146,15 +155,15 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     mbar_init(q_full, 1);
     for (int s = 0; s < kFlashSlots; ++s) { mbar_init(kv_full(s), 1); mbar_init(kv_empty(s), 1); }
     for (int t = 0; t < 2; ++t) {
-      for (int b = 0; b < 2; ++b) { mbar_init(s_full(t, b), 1); mbar_init(s_free(t, b), 8); mbar_init(p_ready(t, b), 4); }
+      for (int b = 0; b < 2; ++b) { mbar_init(s_full(t, b), 1); mbar_init(s2_full(t, b), 1); mbar_init(s_free(t, b), 8); mbar_init(p_ready(t, b), 4); }
       mbar_init(o_done(t), 1);
     }
     s_err = 0;
     mbar_fence_init();
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (warp == kFlashSoftmaxWarps + 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(512u) : "memory");
+  if (warp == sw + 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(2u * o_off) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
@@ -178,8 +187,9 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     return (min(a.KV, a.causal ? r0 + 128 : a.KV) + 127) >> 7;
   };
   const int nb0 = n_blocks(0), nb1 = n_blocks(1), nmax = max(nb0, nb1);
+  const bool keep = nmax == 1;        // one block of keys: its scores stay in tensor memory between the sweeps
 
-  if (warp == kFlashSoftmaxWarps) {
+  if (warp == sw) {
     // ------------------------------------------------------------------ producer
     if (lane == 0 && !a.test_no_loads) {
       const int active = nb1 > 0 ? 2 : 1;
@@ -187,12 +197,12 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       for (int t = 0; t < active; ++t)
         for (int d = 0; d < DB; ++d)
           tma_load_4d(smem0 + (uint32_t)t * kTile + (uint32_t)d * kBox, &map_q, d * 64, q0 + t * 128, h, b, q_full);
-      const int total = 3 * nmax;
+      const int total = keep ? 2 : 3 * nmax;
       for (int u = 0; u < total; ++u) {
         const int slot = u % kFlashSlots;
         if (!mbar_wait(kv_empty(slot), ((uint32_t)(u / kFlashSlots) & 1u) ^ 1u)) { s_err = 1; report_status(a.status, 21); break; }
-        const int w = u - nmax;
-        const bool is_v = w >= 0 && (w & 1);
+        const int w = u - nmax + (keep ? 1 : 0);           // (with one block: K, V)
+        const bool is_v = w > 0 && (w & 1);
         const int blk = w < 0 ? u : (w >> 1);
         mbar_expect_tx(kv_full(slot), kTile);
         const CUtensorMap *m = is_v ? &map_v : &map_k;
@@ -201,40 +211,35 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           tma_load_4d(ring0 + (uint32_t)slot * kTile + (uint32_t)d * kBox, m, d * 64, blk * 128, hh, bb, kv_full(slot));
       }
     }
-  } else if (warp == kFlashSoftmaxWarps + 1) {
+  } else if (warp == sw + 1) {
     // ------------------------------------------------------------------ MMA issuer
-    // The whole warp walks the schedule and one elected lane issues: control flow and operands stay warp-uniform, so the
-    // descriptors live in uniform registers.  (Inside a lane == 0 branch every MMA first moved its operands there, about 100
-    // clocks each: the issue, not the tensor pipe, was the bound -- 1.2 us for two 128 x 128 x 128 products instead of 0.6.)
-    const uint32_t idesc_s = make_idesc_bf16(128);
-    const uint32_t idesc_o = make_idesc_bf16((a.D + 15) & ~15) | (1u << 16);           // B (V) is N-major
-    const int ksteps = (a.D + 15) >> 4;
+    // (the whole warp walks the schedule: control flow and operands are the same in every lane)
+    const uint32_t idesc_s = make_idesc_bf16(128), idesc_h = make_idesc_bf16(64);
+    const uint32_t idesc_o = make_idesc_bf16(KS * 16) | (1u << 16);           // B (V) is N-major
     const uint64_t q_desc = make_smem_desc(smem0), k_desc = make_smem_desc(ring0), v_desc = make_smem_desc_mn(ring0, kBox);
     constexpr uint64_t kTileD = kTile >> 4, kBoxD = kBox >> 4;
     auto qk = [&](int t, uint32_t d_tmem, int slot, uint32_t bar) {
       const uint64_t qa = q_desc + (uint64_t)t * kTileD, ka = k_desc + (uint64_t)slot * kTileD;
-      if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 4 * DB; ++k)
-          if (k < ksteps) tc_mma_bf16_lane(d_tmem, qa + (k >> 2) * kBoxD + (k & 3) * 2, ka + (k >> 2) * kBoxD + (k & 3) * 2, idesc_s, k ? 1u : 0u);
-        tc_commit_lane(bar);
-      }
-      __syncwarp();
+      for (int k = 0; k < KS; ++k) tc_mma_bf16(d_tmem, qa + (k >> 2) * kBoxD + (k & 3) * 2, ka + (k >> 2) * kBoxD + (k & 3) * 2, idesc_s, k ? 1u : 0u);
+      tc_commit(bar);
+    };
+    auto qk_half = [&](int t, int h2, int slot) {              // scores of 64 keys of a block, where that half of the tile's warps expects them
+      const uint64_t qa = q_desc + (uint64_t)t * kTileD, ka = k_desc + (uint64_t)slot * kTileD + (uint64_t)h2 * (64 * 128 >> 4);
+#pragma unroll
+      for (int k = 0; k < KS; ++k)
+        tc_mma_bf16(tmem + (uint32_t)t * 128u + (uint32_t)h2 * 64u, qa + (k >> 2) * kBoxD + (k & 3) * 2, ka + (k >> 2) * kBoxD + (k & 3) * 2, idesc_h, k ? 1u : 0u);
+      tc_commit(s2_full(t, h2));
     };
     auto pv = [&](int t, int slot, bool first, int k0) {       // 64 keys: k0 = 0 or 4
       const uint64_t va = v_desc + (uint64_t)slot * kTileD + (uint64_t)(k0 * 128);
-      const uint32_t pa = tmem + (uint32_t)t * 128u + (k0 ? 64u : 0u), od = tmem + 256u + (uint32_t)t * 128u;
-      if (elect_one()) {
+      const uint32_t pa = tmem + (uint32_t)t * 128u + (k0 ? 64u : 0u), od = tmem + o_off + (uint32_t)t * 128u;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) tc_mma_bf16_ts(od, pa + (uint32_t)k * 8u, va + k * 128, idesc_o, (first && k0 + k == 0) ? 0u : 1u);
-      }
-      __syncwarp();
+      for (int k = 0; k < 4; ++k) tc_mma_bf16_ts(od, pa + (uint32_t)k * 8u, va + k * 128, idesc_o, (first && k0 + k == 0) ? 0u : 1u);
     };
-    auto commit = [&](uint32_t bar) { if (elect_one()) tc_commit_lane(bar); __syncwarp(); };
-    auto wait = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0; };
-    bool ok = wait(q_full, 0);
+    bool ok = mbar_wait_warp(q_full, 0);
     int u = 0;
-    auto full = [&](int uu) { return wait(kv_full(uu % kFlashSlots), (uint32_t)(uu / kFlashSlots) & 1u); };
+    auto full = [&](int uu) { return mbar_wait_warp(kv_full(uu % kFlashSlots), (uint32_t)(uu / kFlashSlots) & 1u); };
     // sweep 1: scores only, two buffers per tile
     for (int j = 0; ok && j < nmax; ++j, ++u) {
       ok = full(u);
@@ -242,46 +247,42 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         if (!ok || j >= (t ? nb1 : nb0)) continue;
-        ok = wait(s_free(t, j & 1), ((uint32_t)(j >> 1) & 1u) ^ 1u);
+        ok = mbar_wait_warp(s_free(t, j & 1), ((uint32_t)(j >> 1) & 1u) ^ 1u);
         if (!ok) break;
         tc_fence_after();
-        qk(t, tmem + (uint32_t)t * 128u + ((j & 1) ? 256u : 0u), u % kFlashSlots, s_full(t, j & 1));
+        qk(t, tmem + (uint32_t)t * 128u + ((j & 1) ? o_off : 0u), u % kFlashSlots, s_full(t, j & 1));
       }
-      commit(kv_empty(u % kFlashSlots));
+      tc_commit(kv_empty(u % kFlashSlots));
     }
-    // sweep 2: first scores
-    if (ok) ok = full(u);
+    // sweep 2: first scores, published to the two halves of a tile's warps
+    if (ok && !keep) ok = full(u);
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
       const int nb = t ? nb1 : nb0;
-      if (!ok || nb == 0) continue;
-      ok = wait(s_free(t, 0), ((uint32_t)((nb + 1) >> 1) & 1u) ^ 1u);
+      if (!ok || keep || nb == 0) continue;
+      ok = mbar_wait_warp(s_free(t, 0), ((uint32_t)((nb + 1) >> 1) & 1u) ^ 1u);
       if (!ok) break;
       tc_fence_after();
-      qk(t, tmem + (uint32_t)t * 128u, u % kFlashSlots, s_full(t, 0));
+      qk_half(t, 0, u % kFlashSlots);
+      qk_half(t, 1, u % kFlashSlots);
     }
-    if (ok) { commit(kv_empty(u % kFlashSlots)); ++u; }
+    if (ok && !keep) { tc_commit(kv_empty(u % kFlashSlots)); ++u; }
+    // then in turn for each tile and half: P V of its 64 keys, and the scores of the next block in place of P
     for (int j = 0; ok && j < nmax; ++j, u += 2) {
+      ok = full(u) && (j + 1 >= nmax || full(u + 1));
 #pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const int nb = t ? nb1 : nb0;
+      for (int i = 0; i < 4; ++i) {
+        const int t = i & 1, h2 = i >> 1, nb = t ? nb1 : nb0;
         if (!ok || j >= nb) continue;
-        ok = wait(p_ready(t, 0), (uint32_t)j & 1u) && full(u);
+        ok = mbar_wait_warp(p_ready(t, h2), (uint32_t)j & 1u);
         if (!ok) break;
         tc_fence_after();
-        pv(t, u % kFlashSlots, j == 0, 0);
-        ok = wait(p_ready(t, 1), (uint32_t)j & 1u);
-        if (!ok) break;
-        tc_fence_after();
-        pv(t, u % kFlashSlots, j == 0, 4);
-        if (j + 1 < nb) {
-          ok = full(u + 1);
-          if (!ok) break;
-          qk(t, tmem + (uint32_t)t * 128u, (u + 1) % kFlashSlots, s_full(t, 0));
-        } else commit(o_done(t));
+        pv(t, u % kFlashSlots, j == 0, 4 * h2);
+        if (j + 1 < nb) qk_half(t, h2, (u + 1) % kFlashSlots);
+        else if (h2) tc_commit(o_done(t));
       }
-      commit(kv_empty(u % kFlashSlots));
-      if (j + 1 < nmax) commit(kv_empty((u + 1) % kFlashSlots));
+      tc_commit(kv_empty(u % kFlashSlots));
+      if (j + 1 < nmax) tc_commit(kv_empty((u + 1) % kFlashSlots));
     }
     if (!ok && lane == 0) { s_err = 1; report_status(a.status, 22); }
   } else {
@@ -290,49 +291,50 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const int t = warp >> 3, half = (warp >> 2) & 1, nb = t ? nb1 : nb0;
     const int row_in_tile = (warp & 3) * 32 + lane, row = q0 + t * 128 + row_in_tile;
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t ts0 = tmem + lane_off + (uint32_t)t * 128u + (uint32_t)half * 64u, to0 = ts0 + 256u;
+    const uint32_t ts0 = tmem + lane_off + (uint32_t)t * 128u + (uint32_t)half * 64u, to0 = ts0 + o_off;
     const float ninf = __int_as_float(0xff800000);
     const int n_keys = min(a.KV, a.causal ? row + 1 : a.KV);         // keys this row sees
     const int64_t moff = MASK ? (int64_t)b * a.mask.mb + (int64_t)h * a.mask.mh + (int64_t)min(row, a.S - 1) * a.mask.mi : 0;
     // a chunk of 32 scores; with a mask, scale and mask are applied here (vector loads where the mask's rows allow it: all lanes read the
     // same bytes when the mask does not depend on the query).  The mask is added as it is: the type's lowest finite value times log2(e)
     // would be an infinity, and a row that carries it throughout is a softmax over equal scores, not a row without keys
-    auto mask32 = [&](uint32_t (&s)[32], int j0) {
-      if constexpr (MASK) {
-        const uint64_t sc2 = pk2(a.scale, a.scale);
-        auto put = [&](int i, float m0, float m1) {
-          float y0, y1;
-          upk2(add2(mul2(pk2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), sc2), pk2(m0, m1)), y0, y1);
-          s[i] = __float_as_uint(y0); s[i + 1] = __float_as_uint(y1);
-        };
-        const bool whole = j0 + 32 <= a.KV;
-        if (a.mask.dt == DT_F32) {
-          const float *mp = reinterpret_cast<const float *>(a.mask.p) + moff + j0;
-          if (a.mask_vec && whole) {
+    auto mask_load = [&](float (&mk)[32], int j0) {
+      const bool whole = a.mask_vec && j0 + 32 <= a.KV;
+      if (a.mask.dt == DT_F32) {
+        const float *mp = reinterpret_cast<const float *>(a.mask.p) + moff + j0;
+        if (whole) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              const float4 v = __ldg(reinterpret_cast<const float4 *>(mp + i));
-              put(i, v.x, v.y); put(i + 2, v.z, v.w);
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) put(i, j0 + i < a.KV ? __ldg(mp + i) : 0.f, j0 + i + 1 < a.KV ? __ldg(mp + i + 1) : 0.f);
+          for (int i = 0; i < 32; i += 4) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(mp + i));
+            mk[i] = v.x; mk[i + 1] = v.y; mk[i + 2] = v.z; mk[i + 3] = v.w;
           }
         } else {
-          const uint16_t *mp = reinterpret_cast<const uint16_t *>(a.mask.p) + moff + j0;
-          if (a.mask_vec && whole) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-              const uint4 v = __ldg(reinterpret_cast<const uint4 *>(mp + i));
-              const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) put(i + 2 * e, __uint_as_float(w[e] << 16), __uint_as_float(w[e] & 0xffff0000u));
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) put(i, j0 + i < a.KV ? bf16_bits_to_f32(__ldg(mp + i)) : 0.f, j0 + i + 1 < a.KV ? bf16_bits_to_f32(__ldg(mp + i + 1)) : 0.f);
-          }
+          for (int i = 0; i < 32; ++i) mk[i] = j0 + i < a.KV ? __ldg(mp + i) : 0.f;
         }
+      } else {
+        const uint16_t *mp = reinterpret_cast<const uint16_t *>(a.mask.p) + moff + j0;
+        if (whole) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 8) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(mp + i));
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { mk[i + 2 * e] = __uint_as_float(w[e] << 16); mk[i + 2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u); }
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) mk[i] = j0 + i < a.KV ? bf16_bits_to_f32(__ldg(mp + i)) : 0.f;
+        }
+      }
+    };
+    auto mask_add = [&](uint32_t (&s)[32], const float (&mk)[32]) {
+      const uint64_t sc2 = pk2(a.scale, a.scale);
+#pragma unroll
+      for (int i = 0; i < 32; i += 2) {
+        float y0, y1;
+        upk2(fma2(pk2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), sc2, pk2(mk[i], mk[i + 1])), y0, y1);
+        s[i] = __float_as_uint(y0); s[i + 1] = __float_as_uint(y1);
       }
     };
     int n_vis = n_keys;
@@ -340,38 +342,64 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
       for (int i = 0; i < 32; ++i) if (j0 + i >= n_vis) s[i] = __float_as_uint(ninf);
     };
-    float m = ninf, l = 0.f;
+    float m = ninf, l = 0.f, lx = 0.f;            // the score whose frame it is (the row's largest, or one just below it), sums of 2^x and of 2^x x
+    FlashFrame fr{0.f, 0.f};
+    bool shifted = false;                       // some lane's frame has an r
     bool ok = true;
     uint32_t ph0 = 0, ph1 = 0;
-    // u = m - s * scale, the distance of two scores from the row maximum m (natural units; with a mask the scale is in s already)
-    const float sc = MASK ? 1.0f : a.scale;
-    auto below = [&](const uint32_t (&s)[32], int i, float m_ref) {
-      return fma2(pk2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), pk2(-sc, -sc), pk2(m_ref, m_ref));
+    const float c = MASK ? kLog2e : a.c, kap = MASK ? kLog2eLo / kLog2e * kLn2 : a.kappa;
+    const uint64_t c2 = pk2(c, c);
+    auto shift32 = [&](uint32_t (&s)[32]) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) s[i] = __float_as_uint(__uint_as_float(s[i]) - fr.r);
     };
-    // ---- sweep 1: row maximum and row sum of this half, 32 scores at a time; the sum is kept relative to the largest score so far,
-    // so a single score far above all others is met wherever it lies.  (fmaxf passes over a NaN; the sum does not)
+    // ---- sweep 1: row maximum and row sum of this half, 32 scores at a time.  The frame is that of the first scores until one lies far above it, so a
+    // single score far above all others is met wherever it lies.  (fmaxf passes over a NaN; the sum does not)
     auto sum_half = [&](uint32_t ta, int k0, bool last) {
-      uint32_t s[2][32];
-      tc_ld32(ta, s[0]);
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
+        uint32_t s[32];
+        tc_ld32(ta + (uint32_t)q * 32u, s);
+        float mk[MASK ? 32 : 1];
+        if constexpr (MASK) mask_load(mk, k0 + q * 32);           // (in flight beside the scores)
         tc_wait_ld();
-        if (q < 1) tc_ld32(ta + 32u, s[1]);
-        mask32(s[q], k0 + q * 32);
-        if (last) limit32(s[q], k0 + q * 32);
-        float mx = ninf;
+        if constexpr (MASK) mask_add(s, mk);
+        if (last) limit32(s, k0 + q * 32);
+        float mx = ninf, my = ninf;
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(s[q][i]), __uint_as_float(s[q][i + 1])));
-        mx = fmaxf(m, __fmul_rn(mx, sc));
-        const float ref = mx == ninf ? 0.f : mx;            // (no key so far: every term is exp(-inf))
-        uint64_t acc[2] = {0ull, 0ull};
+        for (int i = 0; i < 32; i += 4) {
+          mx = fmaxf(mx, fmaxf(__uint_as_float(s[i]), __uint_as_float(s[i + 1])));
+          my = fmaxf(my, fmaxf(__uint_as_float(s[i + 2]), __uint_as_float(s[i + 3])));
+        }
+        mx = fmaxf(mx, my);
+        const bool move = mx > ninf && (m == ninf || !(__fmaf_rn(mx - fr.r, c, -fr.M) <= kFlashReach));
+        if (__any_sync(0xffffffffu, move)) {
+          if (move) {
+            m = mx;
+            const FlashFrame to = flash_frame(m, c);
+            if (l != 0.f) {
+              const float sh = flash_shift(fr, to, c), f = ex2f(sh);
+              lx = f * __fmaf_rn(sh, l, lx);
+              l *= f;
+            }
+            fr = to;
+          }
+          shifted = __any_sync(0xffffffffu, fr.r != 0.f);
+        }
+        if (shifted) shift32(s);
+        const uint64_t nM2 = pk2(-fr.M, -fr.M);
+        uint64_t acc[2] = {0ull, 0ull}, accx[2] = {0ull, 0ull};
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          acc[i & 1] = add2(acc[i & 1], exp_neg2_plain(below(s[q], i, ref)));
+        for (int i = 0; i < 16; ++i) {
+          const uint64_t x2 = flash_exponent2(pk2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), c2, nM2), e2 = ex2_pair(x2);
+          acc[i & 1] = add2(acc[i & 1], e2);
+          accx[i & 1] = fma2(e2, x2, accx[i & 1]);
+        }
         float e0, e1;
         upk2(add2(acc[0], acc[1]), e0, e1);
-        l = __fmaf_rn(l, expf(m - ref), e0 + e1);
-        m = mx;
+        l += e0 + e1;
+        upk2(add2(accx[0], accx[1]), e0, e1);
+        lx += e0 + e1;
       }
     };
     for (int j = 0; ok && j < nb; ++j) {
@@ -386,35 +414,43 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       __syncwarp();
       if (lane == 0) mbar_arrive(s_free(t, bf));
     }
-    // ---- the two halves of a row together
+    // ---- the two halves of a row together, each with its corrected sum, in the higher of the two frames
+    l = __fmaf_rn(kap, lx, l);
     stats[t][half][row_in_tile] = make_float2(m, l);
     asm volatile("bar.sync %0, 256;" ::"r"(1 + t) : "memory");
     {
       const float2 o = stats[t][half ^ 1][row_in_tile];
-      const float mn = fmaxf(m, o.x), ref = mn == ninf ? 0.f : mn;
-      l = l * expf(m - ref) + o.y * expf(o.x - ref);
+      const float mn = fmaxf(m, o.x);
+      fr = flash_frame(mn, c);
+      const float sa = flash_shift(flash_frame(m, c), fr, c), sb = flash_shift(flash_frame(o.x, c), fr, c);
+      l = ex2f(sa) * __fmaf_rn(kap * sa, l, l) + ex2f(sb) * __fmaf_rn(kap * sb, o.y, o.y);
       m = mn;
     }
-    // ---- sweep 2: p = exp(s - m) / l.  A row without a score above -inf gives zeros (all its scores count as masked); a NaN
+    // ---- sweep 2: p = 2^x (1 + kappa ln2 x) / l.  A row without a score above -inf gives zeros (all its scores count as masked); a NaN
     // in the sum makes the whole row NaN
     const bool dead = m == ninf;
-    if (dead) n_vis = 0;
+    if (dead) { n_vis = 0; fr = FlashFrame{0.f, 0.f}; }
     const bool any_dead = __any_sync(0xffffffffu, dead) != 0;
-    const float inv = dead ? 0.f : __fdiv_rn(1.0f, l), ref = dead ? 0.f : m;
+    shifted = __any_sync(0xffffffffu, fr.r != 0.f);
+    const float inv = dead ? 0.f : __fdiv_rn(1.0f, l), kinv = kap * inv;
+    const uint64_t nM2 = pk2(-fr.M, -fr.M), inv2 = pk2(inv, inv), kinv2 = pk2(kinv, kinv);
     auto p_half = [&](int k0, bool last) {
-      uint32_t s[2][32];
-      tc_ld32(ts0, s[0]);
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
+        uint32_t s[32];
+        tc_ld32(ts0 + (uint32_t)q * 32u, s);
+        float mk[MASK ? 32 : 1];
+        if constexpr (MASK) mask_load(mk, k0 + q * 32);           // (in flight beside the scores)
         tc_wait_ld();
-        if (q < 1) tc_ld32(ts0 + 32u, s[1]);
-        mask32(s[q], k0 + q * 32);
-        if (last) limit32(s[q], k0 + q * 32);
+        if constexpr (MASK) mask_add(s, mk);
+        if (last) limit32(s, k0 + q * 32);
+        if (shifted) shift32(s);
         uint32_t p[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
+          const uint64_t x2 = flash_exponent2(pk2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), c2, nM2);
           float x0, x1;
-          upk2(mul2(exp_neg2(below(s[q], i, ref)), pk2(inv, inv)), x0, x1);
+          upk2(mul2(ex2_pair(x2), fma2(x2, kinv2, inv2)), x0, x1);
           p[i] = pack_bf16x2(x0, x1);
         }
         tc_st16(ts0 + (uint32_t)q * 16u, p);      // (over scores of this half that have been read)
@@ -425,9 +461,8 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       if (lane == 0) mbar_arrive(p_ready(t, half));
     };
     for (int j = 0; ok && j < nb; ++j) {
-      ok = __all_sync(0xffffffffu, mbar_wait(s_full(t, 0), ph0));
+      if (!keep) ok = __all_sync(0xffffffffu, mbar_wait(s2_full(t, half), (uint32_t)j & 1u));
       if (!ok) break;
-      ph0 ^= 1u;
       tc_fence_after();
       if (j == nb - 1 || any_dead) p_half(j * 128 + half * 64, true); else p_half(j * 128 + half * 64, false);
     }
@@ -436,7 +471,7 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       tc_fence_after();
       uint16_t *o = a.out + (int64_t)b * a.ob + (int64_t)h * a.oh + (int64_t)row * a.os;
       const int units = (a.D + 15) >> 4, u0 = half ? (units + 1) >> 1 : 0, u1 = half ? units : (units + 1) >> 1;     // the halves share the columns
-      const uint32_t od = tmem + lane_off + 256u + (uint32_t)t * 128u;
+      const uint32_t od = tmem + lane_off + o_off + (uint32_t)t * 128u;
       for (int d0 = u0 * 16; d0 < u1 * 16; d0 += 16) {
         uint32_t r[16], pk[8];
         tc_ld16(od + (uint32_t)d0, r);
@@ -465,9 +500,9 @@ sdpa_flash_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     for (int i = 0; i < 64; ++i) __nanosleep(20000);     // copies still in flight land before shared memory is released
     __syncthreads();
   }
-  if (warp == kFlashSoftmaxWarps + 1) {
+  if (warp == sw + 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * o_off) : "memory");
   }
 }
 
