@@ -279,7 +279,7 @@ size_t decode_smem(int M, int N, int64_t Kp) {
 // Decode-shape kernel (M <= 16): persistent, evenly split over all warps of the device.
 // Returns unimplemented when the shape does not fit it (the caller then uses the tiled streaming kernel).
 int32_t launch_decode(const uint8_t *A, int64_t lda, bool a_unsigned, int M, int N, int K, const PackedWeight &pw,
-                      const EpiParams &epi, bool early_weights, cudaStream_t st) {
+                      const EpiParams &epi, bool early_weights, cudaStream_t st, const DecodeQuant &dq = DecodeQuant{}) {
   Runtime &R = rt();
   DecodeGemmArgs g{};
   g.A = A; g.lda = lda; g.M = M; g.N = N; g.K = K; g.Wt = pw.wt; g.Kp = (int)pw.Kp;
@@ -291,7 +291,7 @@ int32_t launch_decode(const uint8_t *A, int64_t lda, bool a_unsigned, int M, int
   g.tune = env_int("B200DNN_DECODE_TUNE", 0);
   const size_t smem = decode_smem(M, N, pw.Kp);
   if (M > 16 || smem > 220 * 1024) return B200DNN_UNIMPLEMENTED;
-  void (*kern)(DecodeGemmArgs, EpiParams) = a_unsigned ? decode_gemm_kernel<true> : decode_gemm_kernel<false>;
+  void (*kern)(DecodeGemmArgs, EpiParams, DecodeQuant) = dq.src ? decode_gemm_kernel<false, true> : a_unsigned ? decode_gemm_kernel<true> : decode_gemm_kernel<false>;
   B2_TRY(ensure_max_smem((const void *)kern));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid); cfg.blockDim = dim3(kDecodeWarps * 32); cfg.dynamicSmemBytes = smem; cfg.stream = st;
@@ -299,7 +299,7 @@ int32_t launch_decode(const uint8_t *A, int64_t lda, bool a_unsigned, int M, int
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = early_weights ? 1 : 0;
-  B2_CUDA(cudaLaunchKernelEx(&cfg, kern, g, epi));
+  B2_CUDA(cudaLaunchKernelEx(&cfg, kern, g, epi, dq));
   B2_LAUNCHED();
   return B200DNN_SUCCESS;
 }
@@ -307,7 +307,7 @@ int32_t launch_decode(const uint8_t *A, int64_t lda, bool a_unsigned, int M, int
 // Ring form of the decode GEMM (decode_ring.cuh).  unimplemented when the ring would be too shallow.
 template <int R>
 int32_t launch_decode_ring(const uint8_t *A, int64_t lda, bool a_unsigned, int M, int N, int K, const PackedWeight &pw,
-                           const EpiParams &epi, bool early_weights, cudaStream_t st) {
+                           const EpiParams &epi, bool early_weights, cudaStream_t st, const DecodeQuant &dq) {
   Runtime &R_ = rt();
   DecodeRingArgs g{};
   g.A = A; g.lda = lda; g.M = M; g.N = N; g.K = K; g.Wt = pw.wt; g.Kp = (int)pw.Kp;
@@ -331,7 +331,7 @@ int32_t launch_decode_ring(const uint8_t *A, int64_t lda, bool a_unsigned, int M
   if (cap > 1 && stages > cap) stages = cap;
   g.stages = stages;
   const size_t smem = fixed + (size_t)stages * stage_bytes;
-  void (*kern)(DecodeRingArgs, EpiParams) = a_unsigned ? decode_ring_kernel<true, R> : decode_ring_kernel<false, R>;
+  void (*kern)(DecodeRingArgs, EpiParams, DecodeQuant) = dq.src ? decode_ring_kernel<false, R, true> : a_unsigned ? decode_ring_kernel<true, R> : decode_ring_kernel<false, R>;
   B2_TRY(ensure_max_smem((const void *)kern));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid); cfg.blockDim = dim3((kRingWarps + 1) * 32); cfg.dynamicSmemBytes = smem; cfg.stream = st;
@@ -339,7 +339,7 @@ int32_t launch_decode_ring(const uint8_t *A, int64_t lda, bool a_unsigned, int M
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = early_weights ? 1 : 0;
-  B2_CUDA(cudaLaunchKernelEx(&cfg, kern, g, epi));
+  B2_CUDA(cudaLaunchKernelEx(&cfg, kern, g, epi, dq));
   B2_LAUNCHED();
   return B200DNN_SUCCESS;
 }
@@ -1089,6 +1089,32 @@ int32_t launch_expert_rank(const int32_t *ids, int nslots, int nkeys, int32_t *r
   return B200DNN_SUCCESS;
 }
 
+// Few rows on the tensor cores (skinny_gemm.cuh).  Up to 16 rows against the decode kernel, us: K = 4096, N = 11008 12.7 -> 12.2, K = 14336,
+// N = 4096 31.0 -> 16.0, but K = N = 4096 7.2 -> 7.6 (its fixed cost is higher), and with more column tiles than SMs K = 4096, N = 50176
+// 37.3 -> 41.0: there only rows that the decode kernel has no room for.  From 17 to 64 rows against the tile kernel: few_rows_pay.
+bool skinny_decode(int M, int N, int K, int64_t Kp) {
+  return M > 8 && (long long)K * N >= (24ll << 20) && ((N + 127) / 128 <= rt().sm_count || decode_smem(M, N, Kp) > 220 * 1024);
+}
+
+// Dynamic quantisation inside the decode kernel (decode_quant.cuh): aligned bf16 rows that the decode kernels take, few enough elements, and no
+// overlap of the results with the source (every CTA reads all of it, while others may already write).  The line: a kernel of its own costs 0.5 to 4 us, all SMs
+// quantising every row about 0.06 us per 1000 elements, part of it behind a weight that is long in coming.  us, kernel of its own and fused: M = 1,
+// K = 11008, N = 4096 16.5, 12.5; K = 6272, N = 8640 19.3, 14.9; M = 4, K = 4096, N = 11008 14.9, 12.6; K = N = 4096 7.6, 7.4 (M = 8: 8.1, 8.9);
+// M = 8, K = N = 2048 6.1, 5.8 (M = 12: 6.6, 7.1); M = 8, K = 11008, N = 4096 16.1, 17.5.  B200DNN_FUSED_QUANT: 0 never, 1 whenever the rows allow it, -1 by the line.
+bool fused_quant_pays(const b200dnn_matmul_t *d, const void *src, const PackedWeight &pw) {
+  const int M = d->M, N = d->N, K = d->K;
+  if (M > 16 || d->force_kernel != 0 || d->src_dt != B200DNN_BF16 || K % 8 != 0 || d->lda % 8 != 0 || (reinterpret_cast<uintptr_t>(src) & 15) != 0) return false;
+  if (skinny_decode(M, N, K, pw.Kp) || decode_smem(M, N, pw.Kp) > 220 * 1024 || env_int("B200DNN_DECODE_KERNEL", 1) == 0) return false;
+  const int mode = env_int("B200DNN_FUSED_QUANT", -1);
+  if (mode == 0 || (mode < 0 && (long long)M * K > 20000 + (((long long)K * N) >> 20) * 500)) return false;
+  auto apart = [](const void *p, size_t n, const void *q, size_t m) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(q);
+    return !p || !q || a + n <= b || b + m <= a;
+  };
+  const size_t in = span_bytes(M, K, d->lda, d->src_dt);
+  return apart(d->src, in, d->dst, span_bytes(M, N, d->ldc, d->dst_dt)) && apart(d->src, in, d->src_scale.buff, (size_t)M * 4);
+}
+
 extern "C" {
 
 int32_t b200dnn_moe_route(const float *logits, int32_t T, int32_t E, int32_t topk, int32_t renorm, int32_t *ids,
@@ -1151,7 +1177,14 @@ int32_t b200dnn_matmul(const b200dnn_matmul_t *d, void *stream) {
   B2_TRY(stage_in(d->src, span_bytes(M, K, d->lda, d->src_dt), st, &src_dev, &R.small));
   const uint8_t *A = (const uint8_t *)src_dev; int64_t lda = d->lda; bool a_unsigned = d->src_dt == B200DNN_U8;
   Staged o_scale;
-  if (dyn) {
+  DecodeQuant dq{};
+  if (dyn && fused_quant_pays(d, src_dev, pw)) {
+    const int32_t sdt = d->src_scale.buff ? d->src_scale.dt : B200DNN_F32;
+    B2_TRY(stage_out(const_cast<void *>(d->src_scale.buff), (size_t)M * dt_size(sdt), st, &o_scale));
+    dq = DecodeQuant{(const uint16_t *)src_dev, d->lda, o_scale.dev, sdt};
+    A = nullptr; a_unsigned = false;
+    epi.src_scale_dt = B200DNN_F32; epi.src_scale_n = M;      // (the kernel has them in shared memory)
+  } else if (dyn) {
     const int64_t Kq = round_up(K, 16);
     int8_t *q = (int8_t *)R.ws.alloc((size_t)M * Kq);
     B2_CHECK(q, B200DNN_FAILURE, "workspace allocation failed");
@@ -1223,13 +1256,9 @@ int32_t b200dnn_matmul(const b200dnn_matmul_t *d, void *stream) {
   if (which == 0) which = (M <= 16 || !tc_ok) ? 1 : 2;
   // the weight may be read before the kernel in front has finished: that kernel is this call's quantisation, which itself waited for
   // everything before it, or the caller says that its weights are in place (and the library's own copy of them is: see take_cached)
-  const bool early = !pw.fresh && (dyn || (d->flags & B200DNN_FLAG_STABLE_WEIGHTS) != 0);
-  // Few rows on the tensor cores (skinny_gemm.cuh).  Up to 16 rows against the decode kernel, us: K = 4096, N = 11008 12.7 -> 12.2, K = 14336,
-  // N = 4096 31.0 -> 16.0, but K = N = 4096 7.2 -> 7.6 (its fixed cost is higher), and with more column tiles than SMs K = 4096, N = 50176
-  // 37.3 -> 41.0: there only rows that the decode kernel has no room for.  From 17 to 64 rows against the tile kernel: few_rows_pay.
-  const bool skinny = M <= 16 ? M > 8 && (long long)K * N >= (24ll << 20) && ((N + 127) / 128 <= rt().sm_count || decode_smem(M, N, pw.Kp) > 220 * 1024)
-                              : M <= kSkinnyMaxM && few_rows_pay(M, N, K);
-  const bool few_rows = d->force_kernel == 0 && tc_ok && skinny;
+  const bool early = !pw.fresh && ((dyn && !dq.src) || (d->flags & B200DNN_FLAG_STABLE_WEIGHTS) != 0);
+  const bool skinny = M <= 16 ? skinny_decode(M, N, K, pw.Kp) : M <= kSkinnyMaxM && few_rows_pay(M, N, K);
+  const bool few_rows = d->force_kernel == 0 && !dq.src && tc_ok && skinny;
   B2_CHECK(few_rows || which == 1 || which == 3 || tc_ok, B200DNN_FAILURE, "tcgen05 kernel needs a 16-byte aligned source with lda %% 16 == 0");
   if (few_rows) {
     B2_TRY(launch_skinny(A, lda, a_unsigned, false, M, N, K, pw, epi, M <= 16 && epi.n_po > 0 ? FA_GENERIC : fast_act_code(epi), early, st));
@@ -1239,18 +1268,19 @@ int32_t b200dnn_matmul(const b200dnn_matmul_t *d, void *stream) {
     // default: ring for M <= 2 and weights of 24 MB or more (measured faster there: 10.9 against 11.5 us at 45 MB, but
     // 5.9 against 5.7 us at 16.8 MB), register-batch form otherwise
     const int dk = env_int("B200DNN_DECODE_KERNEL", (M <= 2 && (long long)K * N >= (24ll << 20)) ? 2 : 1);
-    const bool pdl = early && env_int("B200DNN_PDL", 1) != 0;
+    dq.late = early ? 0 : 1;
+    const bool pdl = (early || dq.src) && env_int("B200DNN_PDL", 1) != 0;
     if (which == 1 && M <= 16 && dk >= 2) {
       // groups per stage: split the CTA's groups into equal sets of at most five
       const int groups = (N + 7) / 8, grid = groups < rt().sm_count ? groups : rt().sm_count;
       const int local = (groups + grid - 1) / grid, sets = (local + 4) / 5;
       int r = dk > 2 ? dk : (local + sets - 1) / sets;
-      if (r <= 2) rc = launch_decode_ring<2>(A, lda, a_unsigned, M, N, K, pw, epi, pdl, st);
-      else if (r == 3) rc = launch_decode_ring<3>(A, lda, a_unsigned, M, N, K, pw, epi, pdl, st);
-      else if (r == 4) rc = launch_decode_ring<4>(A, lda, a_unsigned, M, N, K, pw, epi, pdl, st);
-      else rc = launch_decode_ring<5>(A, lda, a_unsigned, M, N, K, pw, epi, pdl, st);
+      if (r <= 2) rc = launch_decode_ring<2>(A, lda, a_unsigned, M, N, K, pw, epi, pdl, st, dq);
+      else if (r == 3) rc = launch_decode_ring<3>(A, lda, a_unsigned, M, N, K, pw, epi, pdl, st, dq);
+      else if (r == 4) rc = launch_decode_ring<4>(A, lda, a_unsigned, M, N, K, pw, epi, pdl, st, dq);
+      else rc = launch_decode_ring<5>(A, lda, a_unsigned, M, N, K, pw, epi, pdl, st, dq);
     }
-    if (which == 1 && M <= 16 && dk != 0 && rc == B200DNN_UNIMPLEMENTED) rc = launch_decode(A, lda, a_unsigned, M, N, K, pw, epi, pdl, st);
+    if (which == 1 && M <= 16 && dk != 0 && rc == B200DNN_UNIMPLEMENTED) rc = launch_decode(A, lda, a_unsigned, M, N, K, pw, epi, pdl, st, dq);
     if (rc == B200DNN_UNIMPLEMENTED) rc = launch_stream(A, lda, a_unsigned, M, N, K, pw, epi, st);
     B2_TRY(rc);
   } else {

@@ -12,8 +12,9 @@ struct DecodeEpiSmem {
   float *bias;      // [cols] bias as f32 (0 when absent)
   int32_t *cs;      // [cols] column sums (0 when no zero point)
   float *ss;        // [16] source scale per row (1 when absent)
+  uint32_t *top;    // [16] largest magnitudes of the rows, while the kernel quantises them itself
 };
-__host__ __device__ inline size_t decode_epi_bytes(int max_local_groups) { return (size_t)max_local_groups * 8 * 12 + 64; }
+__host__ __device__ inline size_t decode_epi_bytes(int max_local_groups) { return (size_t)max_local_groups * 8 * 12 + 128; }
 __device__ __forceinline__ DecodeEpiSmem decode_epi_carve(uint8_t *base, int max_local_groups) {
   DecodeEpiSmem s;
   const int cols = max_local_groups * 8;
@@ -21,13 +22,14 @@ __device__ __forceinline__ DecodeEpiSmem decode_epi_carve(uint8_t *base, int max
   s.bias = s.ws + cols;
   s.cs = reinterpret_cast<int32_t *>(s.bias + cols);
   s.ss = reinterpret_cast<float *>(s.cs + cols);
+  s.top = reinterpret_cast<uint32_t *>(s.ss + 16);
   return s;
 }
 
 // Called by `nthreads` threads (tid 0..nthreads-1) after griddepcontrol.wait; a barrier must follow before
 // decode_epilogue.  Columns [n0, n0 + cols) of the GEMM, rows [0, M).
 __device__ __forceinline__ void decode_epi_stage(const EpiParams &epi, const DecodeEpiSmem &s, int n0, int cols, int N, int M,
-                                                 int tid, int nthreads) {
+                                                 int tid, int nthreads, bool rows_scaled = false /* s.ss is filled by the caller */) {
   if (epi.dst_dt == DT_S32) {
     if (epi.has_zp) for (int j = tid; j < cols; j += nthreads) s.cs[j] = (n0 + j < N) ? epi.colsum[n0 + j] : 0;
     return;
@@ -39,7 +41,7 @@ __device__ __forceinline__ void decode_epi_stage(const EpiParams &epi, const Dec
     s.bias[j] = (in && epi.bias) ? load_as_f32(epi.bias, epi.bias_dt, n) : 0.0f;
     s.cs[j] = (in && epi.has_zp) ? epi.colsum[n] : 0;
   }
-  for (int m = tid; m < 16; m += nthreads)
+  if (!rows_scaled) for (int m = tid; m < 16; m += nthreads)
     s.ss[m] = (m < M && epi.src_scale_n) ? load_as_f32(epi.src_scale, epi.src_scale_dt, epi.src_scale_n > 1 ? m : 0) : 1.0f;
 }
 

@@ -23,6 +23,7 @@
 #pragma once
 #include "common.cuh"
 #include "decode_epi.cuh"
+#include "decode_quant.cuh"
 #include "mbar.cuh"
 #include "stream_gemm.cuh"
 
@@ -56,8 +57,9 @@ __device__ __forceinline__ W32 ldg_stream32(const void *p) {
 }
 __device__ __forceinline__ W32 w32_zero() { W32 v; v.a = make_uint4(0, 0, 0, 0); v.b = v.a; return v; }
 
-template <bool A_UNSIGNED>
-__global__ void __launch_bounds__(kDecodeWarps * 32, 1) decode_gemm_kernel(DecodeGemmArgs g, EpiParams epi) {
+// DYN: the activations are bf16 rows that the CTA quantises itself (dq; see decode_quant.cuh)
+template <bool A_UNSIGNED, bool DYN = false>
+__global__ void __launch_bounds__(kDecodeWarps * 32, 1) decode_gemm_kernel(DecodeGemmArgs g, EpiParams epi, DecodeQuant dq) {
   extern __shared__ __align__(16) uint8_t smem[];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -72,6 +74,7 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, 1) decode_gemm_kernel(Decod
 
   // ---- weights first: the first register batch is in flight while the activations are staged
   const int8_t *wlane = g.Wt + (size_t)g0 * g.Kp * 8 + lg * 128 + lt * 32;   // CTA's span is contiguous: item i at i*1024
+  if constexpr (DYN) { if (dq.late) asm volatile("griddepcontrol.wait;" ::: "memory"); }
   W32 w[kDecodeBatch];
 #pragma unroll
   for (int u = 0; u < kDecodeBatch; ++u) w[u] = (item + u < item_end) ? ldg_stream32(wlane + (size_t)(item + u) * 1024) : w32_zero();
@@ -80,10 +83,17 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, 1) decode_gemm_kernel(Decod
     if (lt == 0 && (g.tune & 1)) prefetch_l2(wlane + (size_t)i * 1024);
   }
   for (int i = tid; i < (g1 - g0) * 128; i += kDecodeWarps * 32) red[i] = 0;
+  if constexpr (DYN) {
+    if (tid < 16) es.top[tid] = 0u;
+    __syncthreads();
+  }
 
   // ---- everything below may depend on the previous kernel of the stream
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  {
+  if constexpr (DYN) {
+    decode_quant_rows<kDecodeWarps * 32, 2>(dq, smem, g.a_stride, g.M, g.K, es.top, es.ss, tid, blockIdx.x == 0, [] { __syncthreads(); });
+    decode_epi_stage(epi, es, g0 * 8, (g1 - g0) * 8, g.N, g.M, tid, kDecodeWarps * 32, true);
+  } else {
     const bool vec = ((reinterpret_cast<uintptr_t>(g.A) | (uintptr_t)g.lda) & 15) == 0;
     const int segs = g.Kp >> 4;
     for (int i = tid; i < g.rows_staged * segs; i += kDecodeWarps * 32) {

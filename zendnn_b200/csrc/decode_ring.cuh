@@ -27,6 +27,7 @@
 #pragma once
 #include "common.cuh"
 #include "decode_epi.cuh"
+#include "decode_quant.cuh"
 #include "mbar.cuh"
 #include "stream_gemm.cuh"
 
@@ -58,8 +59,9 @@ __host__ __device__ inline size_t ring_off_ring(int rows_staged, int a_stride, i
   return (ring_off_bars(rows_staged, a_stride, max_local_groups) + (2 * kRingMaxStages + 2) * 8 + 127) & ~(size_t)127;
 }
 
-template <bool A_UNSIGNED, int R>
-__global__ void __launch_bounds__((kRingWarps + 1) * 32, 1) decode_ring_kernel(DecodeRingArgs g, EpiParams epi) {
+// DYN: the activations are bf16 rows that the CTA's consumers quantise themselves (dq; see decode_quant.cuh)
+template <bool A_UNSIGNED, int R, bool DYN = false>
+__global__ void __launch_bounds__((kRingWarps + 1) * 32, 1) decode_ring_kernel(DecodeRingArgs g, EpiParams epi, DecodeQuant dq) {
   extern __shared__ __align__(128) uint8_t ring_smem[];
   uint8_t *const smem = ring_smem;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -83,6 +85,7 @@ __global__ void __launch_bounds__((kRingWarps + 1) * 32, 1) decode_ring_kernel(D
   auto empty_bar = [&](int s) { return bars + 8u * (uint32_t)(kRingMaxStages + s); };
   volatile int &s_err = *reinterpret_cast<volatile int *>(smem + bars_off + 8 * (2 * kRingMaxStages + 1));
 
+  if (DYN && tid < 16) es.top[tid] = 0u;
   if (tid == 0) {
     s_err = 0;
     for (int s = 0; s < S; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), NCW); }
@@ -105,6 +108,7 @@ __global__ void __launch_bounds__((kRingWarps + 1) * 32, 1) decode_ring_kernel(D
         bulk_load(ring_s + (uint32_t)slot * kStageBytes + (uint32_t)lane * kCopyBytes,
                   span + ((size_t)(set * R + lane) * g.blocks + c0) * 1024, (uint32_t)nblk * 1024u, full_bar(slot));
     };
+    if constexpr (DYN) { if (dq.late) asm volatile("griddepcontrol.wait;" ::: "memory"); }
     int st = 0;
     bool ok = true;
     const int pre = g.test_no_loads ? 0 : (n_stages < S ? n_stages : S);
@@ -124,7 +128,11 @@ __global__ void __launch_bounds__((kRingWarps + 1) * 32, 1) decode_ring_kernel(D
     asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int kConsumers = NCW * 32;
     for (int i = tid; i < n_local * 128; i += kConsumers) red[i] = 0;
-    {
+    if constexpr (DYN) {
+      decode_quant_rows<kConsumers, 8>(dq, smem, g.a_stride, g.M, g.K, es.top, es.ss, tid, blockIdx.x == 0,
+                                       [] { asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory"); });
+      decode_epi_stage(epi, es, g0 * 8, n_local * 8, g.N, g.M, tid, kConsumers, true);
+    } else {
       // activations: 16-byte asynchronous copies (cp.async), all in flight at once.  Not bulk copies: those
       // complete in issue order per SM and would queue behind the ring.
       const bool vec = ((reinterpret_cast<uintptr_t>(g.A) | (uintptr_t)g.lda) & 15) == 0;
