@@ -16,6 +16,7 @@
 #include "decode_ring.cuh"
 #include "tc_gemm.cuh"
 #include "skinny_gemm.cuh"
+#include "moe_few.cuh"
 #include "moe_kernels.cuh"
 #include "sdpa_flash_api.cuh"
 
