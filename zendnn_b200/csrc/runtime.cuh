@@ -183,11 +183,11 @@ struct DeviceShared {
 // Descriptor tables that depend only on the caller's weight pointers (per-expert epilogue pointers, tensor maps) are
 // kept on the device and found again by their bytes, so that a steady-state MoE call uploads nothing.
 struct BlobCache {
-  struct Entry { std::vector<uint8_t> bytes; void *dev; };
+  struct Entry { std::vector<uint8_t> bytes; void *dev; bool made; };      // made: the bytes are what the table was made from, not the table
   std::vector<Entry> entries;
-  void *find(const void *host, size_t n) const {
+  void *find(const void *host, size_t n, bool made = false) const {
     for (const Entry &e : entries)
-      if (e.bytes.size() == n && memcmp(e.bytes.data(), host, n) == 0) return e.dev;
+      if (e.made == made && e.bytes.size() == n && memcmp(e.bytes.data(), host, n) == 0) return e.dev;
     return nullptr;
   }
   void release() { for (Entry &e : entries) cudaFree(e.dev); entries.clear(); }
@@ -397,9 +397,11 @@ inline int32_t upload_blob(const void *host, size_t bytes, cudaStream_t st, void
 }
 // The same for tables that depend only on the caller's weight pointers: kept on the device and found again by their
 // bytes, so a repeated call uploads nothing.
-inline int32_t cached_blob(const void *host, size_t bytes, cudaStream_t st, void **dev) {
+inline int32_t cached_blob(const void *host, size_t bytes, cudaStream_t st, void **dev, const void *key = nullptr, size_t key_bytes = 0) {
   Runtime &R = rt();
-  if (void *d = R.blobs.find(host, bytes)) { *dev = d; return B200DNN_SUCCESS; }
+  if (!key) {
+    if (void *d = R.blobs.find(host, bytes)) { *dev = d; return B200DNN_SUCCESS; }
+  }
   if (R.blobs.entries.size() >= 256) {      // bounded: start again (nothing in flight may still read the old tables)
     B2_CUDA(cudaStreamSynchronize(st));
     R.blobs.release();
@@ -411,10 +413,21 @@ inline int32_t cached_blob(const void *host, size_t bytes, cudaStream_t st, void
   }
   B2_CUDA(cudaMemcpyAsync(d, host, bytes, cudaMemcpyHostToDevice, st));
   B2_CUDA(cudaStreamSynchronize(st));
-  BlobCache::Entry e; e.bytes.assign((const uint8_t *)host, (const uint8_t *)host + bytes); e.dev = d;
+  BlobCache::Entry e;
+  if (key) e.bytes.assign((const uint8_t *)key, (const uint8_t *)key + key_bytes); else e.bytes.assign((const uint8_t *)host, (const uint8_t *)host + bytes);
+  e.dev = d; e.made = key != nullptr;
   R.blobs.entries.push_back(std::move(e));
   *dev = d;
   return B200DNN_SUCCESS;
+}
+
+// A table of n elements that follows from `key` (its bytes): make() fills the host copy only when the device has none yet.
+template <typename T, typename Make>
+int32_t cached_table(const void *key, size_t key_bytes, size_t n, Make make, cudaStream_t st, void **dev) {
+  if (void *d = rt().blobs.find(key, key_bytes, true)) { *dev = d; return B200DNN_SUCCESS; }
+  std::vector<T> host(n);
+  B2_TRY(make(host.data()));
+  return cached_blob(host.data(), sizeof(T) * n, st, dev, key, key_bytes);
 }
 
 // 2-D uint8 tensor map [rows][row_bytes used of pitch] with a [box_rows x 128 B] box, SWIZZLE_128B.
