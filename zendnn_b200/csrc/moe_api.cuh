@@ -459,6 +459,19 @@ extern "C" int32_t b200dnn_moe_layer(const void *x, int64_t ldx, const float *lo
     B2_TRY(E <= 32 ? B2_RS(1) : E <= 64 ? B2_RS(2) : E <= 128 ? B2_RS(4) : B2_RS(8));
 #undef B2_RS
     B2_LAUNCHED();
+  } else if (E <= 256 && G <= kRouteSmallGroups && env_int("B200DNN_ROUTE_CHUNKS", 1) != 0) {
+    const int chunk = route_chunk_tokens(T);
+    const unsigned chunks = (unsigned)((T + chunk - 1) / chunk);
+    zmax = (uint32_t *)Rt.ws.alloc((size_t)R * 4);
+    int32_t *counts = (int32_t *)Rt.ws.alloc((size_t)chunks * E * 4);
+    B2_CHECK(zmax && counts, B200DNN_FAILURE, "workspace allocation failed");
+#define B2_RC(PER) launch_pdl(route_count_kernel<PER>, chunks, (unsigned)kRouteChunkThreads, 0, st, true, (const float *)l_dev, T, E, topk, S, chunk, ids, w, counts, zmax)
+    B2_TRY(E <= 32 ? B2_RC(1) : E <= 64 ? B2_RC(2) : E <= 128 ? B2_RC(4) : B2_RC(8));
+#undef B2_RC
+    B2_LAUNCHED();
+    B2_TRY(launch_pdl(route_assign_kernel, chunks, (unsigned)kRouteChunkThreads, 0, st, true, ids, w, counts, T, E, topk, S, chunk, tile_rows, row_off, tile_prefix, slot_rows, slot_w,
+                      row_token));
+    B2_LAUNCHED();
   } else {
     B2_TRY(launch_route_topk((const float *)l_dev, T, E, topk, 1, ids, w, st));
     B2_TRY(launch_expert_rank(ids, T * topk, E, rank, cnt, st));

@@ -288,6 +288,105 @@ __global__ void __launch_bounds__(1024) route_small_kernel(const float *logits, 
   }
 }
 
+// The routing of a larger batch in two launches over chunks of tokens: top-k of the chunk's tokens with the number of slots per expert; then every chunk adds up the
+// counts of all chunks (its own offsets and those in front of it), ranks its slots inside their experts and writes the slot and row maps.  The results are those of the
+// launches it stands for (route, rank in one or three, offsets, maps, memset), which were not overlapped: layers of
+// 173 tokens 58.4 -> 46.5 us, 575 106.6 -> 96.0, 1185 68.9 -> 59.7, 8782 191 -> 174, 16384 1272 -> 1271.  The fewer the chunks, the fewer counts each adds up: 32 tokens,
+// more where there would be more than 256 chunks.
+constexpr int kRouteChunkThreads = 1024, kRouteMaxChunks = 256;
+inline int route_chunk_tokens(int T) { return 32 * (int)((T + 32LL * kRouteMaxChunks - 1) / (32LL * kRouteMaxChunks)); }
+template <int PER>
+__global__ void __launch_bounds__(kRouteChunkThreads) route_count_kernel(const float *logits, int T, int E, int k, int S, int chunk, int32_t *ids, float *w, int32_t *counts,
+                                                                         uint32_t *row_max) {
+  __shared__ int hist[PER * 32];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t0 = blockIdx.x * chunk, t1 = min(T, t0 + chunk), ns = k + S;
+  for (int i = tid; i < E; i += kRouteChunkThreads) hist[i] = 0;
+  for (int i = t0 * ns + tid; i < t1 * ns; i += kRouteChunkThreads) row_max[i] = 0u;
+  __syncthreads();
+  for (int t = t0 + warp; t < t1; t += kRouteChunkThreads / 32) {
+    int32_t id; float weight;
+    route_topk_warp<PER>(logits + (int64_t)t * E, E, k, 1, lane, &id, &weight);
+    // (logits that are all NaN leave no choice: the last expert, so that every index below stays inside its array)
+    id = min(id, E - 1);
+    if (lane < k) { ids[t * k + lane] = id; w[t * k + lane] = weight; atomicAdd(&hist[id], 1); }
+  }
+  __syncthreads();
+  for (int i = tid; i < E; i += kRouteChunkThreads) counts[blockIdx.x * E + i] = hist[i];
+}
+__global__ void __launch_bounds__(kRouteChunkThreads) route_assign_kernel(const int32_t *ids, const float *w, const int32_t *counts, int T, int E, int k, int S, int chunk,
+                                                                          int tile_rows, int32_t *row_off, int32_t *tile_prefix, int32_t *slot_rows, float *slot_w,
+                                                                          int32_t *row_token) {
+  __shared__ int32_t s_cnt[32][kRouteSmallGroups];      // per warp of 32 slots and expert: how many
+  __shared__ int32_t s_off[kRouteSmallGroups + 1];      // first row of a group; the experts' entries then move on to this chunk's next row
+  __shared__ int32_t s_total[kRouteSmallGroups], s_before[kRouteSmallGroups];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, G = E + S, ns = k + S, nchunks = gridDim.x, me = blockIdx.x;
+  const int t0 = me * chunk, t1 = min(T, t0 + chunk);
+  for (int i = tid; i < E; i += kRouteChunkThreads) { s_total[i] = 0; s_before[i] = 0; }
+  __syncthreads();
+  {
+    const int parts = kRouteChunkThreads / E, e = tid % E, part = tid / E;      // (E <= 256)
+    if (part < parts) {
+      int total = 0, before = 0;
+      for (int c = part; c < nchunks; c += parts) {
+        const int n = counts[c * E + e];
+        total += n;
+        if (c < me) before += n;
+      }
+      atomicAdd(&s_total[e], total);
+      atomicAdd(&s_before[e], before);
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+    // offsets: a scan over the groups (shared experts have T rows each)
+    int row_carry = 0, tile_carry = 0;
+    for (int base = 0; base < G; base += 32) {
+      const int g = base + lane, rows = g < E ? s_total[g] : g < G ? T : 0, tiles = (rows + tile_rows - 1) / tile_rows;
+      int rsum = rows, tsum = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int r = __shfl_up_sync(0xffffffffu, rsum, o), t = __shfl_up_sync(0xffffffffu, tsum, o);
+        if (lane >= o) { rsum += r; tsum += t; }
+      }
+      if (g < G) {
+        const int off = row_carry + rsum - rows;
+        s_off[g] = off + (g < E ? s_before[g] : 0);
+        if (me == 0) { row_off[g] = off; tile_prefix[g] = tile_carry + tsum - tiles; }
+      }
+      row_carry += __shfl_sync(0xffffffffu, rsum, 31);
+      tile_carry += __shfl_sync(0xffffffffu, tsum, 31);
+    }
+    if (lane == 0 && me == 0) { row_off[G] = row_carry; tile_prefix[G] = tile_carry; }
+  }
+  for (int s0 = t0 * k; s0 < t1 * k; s0 += kRouteChunkThreads) {
+    for (int i = lane; i < E; i += 32) s_cnt[warp][i] = 0;
+    const int s = s0 + tid;
+    const int key = s < t1 * k ? ids[s] : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, key);
+    const int in_warp = __popc(same & ((1u << lane) - 1u));
+    __syncwarp();
+    if (key >= 0 && in_warp == 0) s_cnt[warp][key] = __popc(same);
+    __syncthreads();
+    if (key >= 0) {
+      int row = s_off[key] + in_warp;
+      for (int i = 0; i < warp; ++i) row += s_cnt[i][key];
+      const int t = s / k, j = s - t * k;
+      slot_rows[t * ns + j] = row; slot_w[t * ns + j] = w[s]; row_token[row] = t;
+    }
+    __syncthreads();
+    for (int i = tid; i < E; i += kRouteChunkThreads) { int n = 0; for (int v = 0; v < 32; ++v) n += s_cnt[v][i]; s_off[i] += n; }
+    __syncthreads();
+  }
+  for (int i = t0 * S + tid; i < t1 * S; i += kRouteChunkThreads) {
+    const int t = i / S, j = i - t * S, row = s_off[E + j] + t;
+    slot_rows[t * ns + k + j] = row; slot_w[t * ns + k + j] = 1.0f; row_token[row] = t;
+  }
+}
+
 // Stable rank of every slot inside its key, in three passes over chunks of 1024 slots (keys <= kRankMaxKeys):
 // per-chunk histograms, a scan over chunks per key, and the in-chunk stable rank.  Same output as expert_rank_kernel.
 constexpr int kRankChunk = 1024;
