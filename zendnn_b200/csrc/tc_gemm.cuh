@@ -359,57 +359,129 @@ __device__ __forceinline__ void warp_store_rows64(uint8_t *sbuf, const uint4 (&v
   warp_store_rows32(sbuf, v[2], v[3], g_row0 + 32, pitch_bytes, rows_valid, lane);
 }
 
-// The same block for a destination without 16-byte alignment (an odd N or ldc): the rows pass through the staging block and leave
-// element by element, but along the rows -- an instruction writes 32 bytes of each of four (4-byte elements) or four (bf16, as
-// aligned words) rows instead of one element in each of 32.  M = 5000, N = 4097, K = 4096, bf16 out: 259 -> 111 us.
-// cols: how many of the block's columns exist.
-__device__ __forceinline__ void warp_stage_rows32(uint8_t *sbuf, const uint4 &v0, const uint4 &v1, int lane) {
-  tc_staging_free(lane);
-  const int sw = (lane >> 2) & 1;
-  *reinterpret_cast<uint4 *>(sbuf + lane * 32 + ((0 ^ sw) << 4)) = v0;
-  *reinterpret_cast<uint4 *>(sbuf + lane * 32 + ((1 ^ sw) << 4)) = v1;
-  __syncwarp();
-}
-__device__ __forceinline__ const uint8_t *warp_staged_byte(const uint8_t *sbuf, int row, int byte) {
-  return sbuf + row * 32 + ((((byte >> 4) ^ (row >> 2)) & 1) << 4) + (byte & 15);
-}
-// [32 rows x 8 four-byte elements]
-__device__ __forceinline__ void warp_store_any32(uint8_t *sbuf, const uint4 &v0, const uint4 &v1, uint8_t *g_row0, int64_t pitch_bytes, int rows_valid,
-                                                 int cols, int lane) {
-  warp_stage_rows32(sbuf, v0, v1, lane);
-  const int c = lane & 7;
+// A destination without 16-byte alignment (an odd N or ldc): every lane writes its own row as aligned 32-byte pieces, put together in registers from sixteen columns and
+// the last words of the sixteen before them.  Three (bf16: four) steps of selects shift the words by the row's distance from a 32-byte boundary; where a run
+// of columns begins or ends inside a piece, its elements are stored one by one.  (Through a staging block, four rows of eight words an instruction, as before: 32 instructions
+// and twice as many partial sectors.)  M = 3027, K = 1280, N = 7295: f32 75.1 -> 46.3 us, bf16
+// 50.4 -> 39.3; whole sectors at N = 7296 take 40.4 and 28.7.
+struct RowCarry { uint32_t w[8]; bool have; };      // the eight words in front of the next ones; have: they are this run's, and not all of them are stored
+template <int STEP, int N>
+__device__ __forceinline__ void shift_words(const uint32_t (&x)[N], bool on, uint32_t (&y)[N - STEP]) {      // y[i] = on ? x[i] : x[i + STEP]
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int R = 4 * j + (lane >> 3);
-    const uint32_t val = *reinterpret_cast<const uint32_t *>(warp_staged_byte(sbuf, R, c * 4));
-    if (R < rows_valid && c < cols) *reinterpret_cast<uint32_t *>(g_row0 + (int64_t)R * pitch_bytes + c * 4) = val;
-  }
-  __syncwarp();
+  for (int i = 0; i < N - STEP; ++i) y[i] = on ? x[i] : x[i + STEP];
 }
-// [32 rows x 16 bf16]
-__device__ __forceinline__ void warp_store_any16(uint8_t *sbuf, const uint4 &v0, const uint4 &v1, uint8_t *g_row0, int64_t pitch_bytes, int rows_valid,
-                                                 int cols, int lane) {
-  warp_stage_rows32(sbuf, v0, v1, lane);
-  const int w = lane & 7;
+// words from s on, or the first n words, of an aligned piece: at most one store of each size
+__device__ __forceinline__ void put_words_from(uint8_t *base, const uint32_t (&o)[8], int s) {
+  if (s & 1) *reinterpret_cast<uint32_t *>(base + 4 * s) = s < 4 ? (s < 2 ? o[1] : o[3]) : (s < 6 ? o[5] : o[7]);
+  const int s2 = (s + 1) & ~1;
+  if (s2 & 2) *reinterpret_cast<uint2 *>(base + 4 * s2) = s2 < 4 ? make_uint2(o[2], o[3]) : make_uint2(o[6], o[7]);
+  const int s4 = (s2 + 2) & ~3;
+  if (s4 <= 4) *reinterpret_cast<uint4 *>(base + 16) = make_uint4(o[4], o[5], o[6], o[7]);
+  if (s4 == 0) *reinterpret_cast<uint4 *>(base) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+__device__ __forceinline__ void put_words_to(uint8_t *base, const uint32_t (&o)[8], int n) {
+  const int h = n & 4, k = n & 6;
+  if (h) *reinterpret_cast<uint4 *>(base) = make_uint4(o[0], o[1], o[2], o[3]);
+  if (n & 2) *reinterpret_cast<uint2 *>(base + 4 * h) = h ? make_uint2(o[4], o[5]) : make_uint2(o[0], o[1]);
+  if (n & 1) *reinterpret_cast<uint32_t *>(base + 4 * k) = k < 4 ? (k < 2 ? o[0] : o[2]) : (k < 6 ? o[4] : o[6]);
+}
+// NV pieces of eight words from x (seven words in front, then 8 * NV words of which the first belongs at p).  Elements, PER to a word and the first of them `off` in front of p, from
+// lo to hi - 1 are written; edge: the element that shares its word with one outside, where off is 1.
+template <int NV, int PER>
+__device__ __forceinline__ void put_pieces(uint8_t *p, const uint32_t (&x)[8 * NV + 7], int off, int lo, int hi, uint16_t edge) {
+  const int r = (int)((reinterpret_cast<uintptr_t>(p) >> 2) & 7);
+  uint32_t t[8 * NV + 6], u[8 * NV + 4], o[8 * NV];
+  shift_words<1>(x, (r & 1) != 0, t);
+  shift_words<2>(t, (r & 2) != 0, u);
+  shift_words<4>(u, (r & 4) != 0, o);
+  uint8_t *base = p - 4 * r;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int R = 4 * j + (lane >> 3);
-    uint8_t *g = g_row0 + (int64_t)R * pitch_bytes;
-    // the row's elements as words of the destination: elements (2w, 2w + 1), or, where the row starts in the middle of a word,
-    // (2w + 1, 2w + 2); the last lane of such a row takes elements 0 and 15
-    const bool odd = (reinterpret_cast<uintptr_t>(g) & 2) != 0;
-    const int e0 = odd ? 2 * w + 1 : 2 * w, e1 = (odd && w == 7) ? 0 : e0 + 1;
-    const uint32_t lo = *reinterpret_cast<const uint16_t *>(warp_staged_byte(sbuf, R, e0 * 2));
-    const uint32_t hi = *reinterpret_cast<const uint16_t *>(warp_staged_byte(sbuf, R, e1 * 2));
-    if (R < rows_valid) {
-      if (e1 == e0 + 1 && e1 < cols) *reinterpret_cast<uint32_t *>(g + e0 * 2) = lo | (hi << 16);
-      else {
-        if (e0 < cols) *reinterpret_cast<uint16_t *>(g + e0 * 2) = (uint16_t)lo;
-        if (e1 < cols) *reinterpret_cast<uint16_t *>(g + e1 * 2) = (uint16_t)hi;
+  for (int v = 0; v < NV; ++v) {
+    const int e0 = (8 * v - r) * PER - off;                  // first element of the piece
+    const uint32_t q[8] = {o[8 * v], o[8 * v + 1], o[8 * v + 2], o[8 * v + 3], o[8 * v + 4], o[8 * v + 5], o[8 * v + 6], o[8 * v + 7]};
+    if (e0 >= lo && e0 + 8 * PER <= hi) st_global_v8(base + 32 * v, q);
+    else if (v == 0 && lo == 0 && e0 + 8 * PER <= hi) {      // the run begins in this piece
+      if (PER == 2 && off) *reinterpret_cast<uint16_t *>(p + 2) = edge;
+      put_words_from(base, q, r + off);
+    } else if (v == 0 && lo < 0 && hi == 0) {                // and here it ends
+      put_words_to(base, q, r);
+      if (PER == 2 && off) *reinterpret_cast<uint16_t *>(p) = edge;
+    } else if (e0 >= lo && e0 < hi) {                        // the last columns of the matrix
+      const int n = hi - e0, k = n / PER;
+      put_words_to(base + 32 * v, q, k);
+      if (PER == 2 && (n & 1)) {
+        const uint32_t w = k < 4 ? (k < 2 ? (k < 1 ? q[0] : q[1]) : (k < 3 ? q[2] : q[3])) : (k < 6 ? (k < 5 ? q[4] : q[5]) : (k < 7 ? q[6] : q[7]));
+        *reinterpret_cast<uint16_t *>(base + 32 * v + 4 * k) = (uint16_t)w;
+      }
+    } else if (e0 < hi) {
+#pragma unroll 1
+      for (int i = 0; i < 8; ++i) {
+        const int e = e0 + i * PER;
+        const uint32_t lo4 = i < 4 ? (i < 2 ? (i < 1 ? q[0] : q[1]) : (i < 3 ? q[2] : q[3])) : (i < 6 ? (i < 5 ? q[4] : q[5]) : (i < 7 ? q[6] : q[7]));
+        uint8_t *at = base + 32 * v + 4 * i;
+        if constexpr (PER == 1) { if (e >= lo && e < hi) *reinterpret_cast<uint32_t *>(at) = lo4; }
+        else {
+          if (e >= lo && e < hi) *reinterpret_cast<uint16_t *>(at) = (uint16_t)lo4;
+          if (e + 1 >= lo && e + 1 < hi) *reinterpret_cast<uint16_t *>(at + 2) = (uint16_t)(lo4 >> 16);
+        }
       }
     }
   }
-  __syncwarp();
+}
+// sixteen 4-byte columns at p, of which the first n exist; last: the run ends here
+__device__ __forceinline__ void row_put32(uint8_t *p, const uint32_t (&w)[16], int n, bool last, bool row_ok, RowCarry &c) {
+  uint32_t x[23];
+#pragma unroll
+  for (int i = 0; i < 7; ++i) x[i] = c.w[i + 1];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) x[7 + i] = w[i];
+  if (row_ok) put_pieces<2, 1>(p, x, 0, c.have ? -7 : 0, n, 0);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) c.w[i] = w[8 + i];
+  c.have = true;
+  if (last || n < 16) {
+    uint32_t y[15];
+#pragma unroll
+    for (int i = 0; i < 15; ++i) y[i] = i < 7 ? c.w[i + 1] : 0u;
+    if (row_ok) put_pieces<1, 1>(p + 64, y, 0, -7, n - 16, 0);
+    c.have = false;
+  }
+}
+// the same for sixteen bf16 columns (eight words)
+__device__ __forceinline__ void row_put16(uint8_t *p, const uint32_t (&w)[8], int n, bool last, bool row_ok, RowCarry &c) {
+  const int odd = (int)((reinterpret_cast<uintptr_t>(p) >> 1) & 1);
+  auto put = [&](uint8_t *at, const uint32_t (&v)[8], int lo, int hi, uint32_t edge) {
+    uint32_t x[15];          // words of the destination: an odd element in front moves all of them by half a word
+#pragma unroll
+    for (int i = 0; i < 15; ++i) {
+      const uint32_t cur = i < 7 ? c.w[i + 1] : v[i - 7], prev = i < 8 ? c.w[i] : v[i - 8];
+      x[i] = odd ? __funnelshift_l(prev, cur, 16) : cur;
+    }
+    if (row_ok) put_pieces<1, 2>(at - 2 * odd, x, odd, lo, hi, (uint16_t)edge);
+  };
+  put(p, w, c.have ? -16 : 0, n, w[0]);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) c.w[i] = w[i];
+  c.have = true;
+  if (last || n < 16) {
+    const uint32_t none[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+    put(p + 32, none, -16, n - 16, c.w[7] >> 16);
+    c.have = false;
+  }
+}
+
+// the last columns of a row that starts on 16 bytes, n of eight (sixteen) words: nothing to shift.  (M = 3000, K = 1024, N = 1000, bf16: 9.1 us, through the
+// shifts above 9.5, through a staging block 9.3.)
+template <int W>
+__device__ __forceinline__ void put_tail_words(uint8_t *p, const uint32_t (&w)[W], int n) {
+#pragma unroll
+  for (int v = 0; v < W / 4; ++v) {
+    if (n >= 4 * v + 4) *reinterpret_cast<uint4 *>(p + 16 * v) = make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
+    else {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) if (4 * v + i < n) *reinterpret_cast<uint32_t *>(p + 16 * v + 4 * i) = w[4 * v + i];
+    }
+  }
 }
 
 // The same [32 rows x 32 bytes] block as one TMA store: the lanes write their rows to the staging block (plain row-major) and one lane hands it
@@ -466,7 +538,7 @@ __device__ __forceinline__ void tc_act16(const EpiParams &epi, float (&x)[16], i
 // instantiated per activation the split form spilled hundreds of registers.)
 template <bool F16>
 __device__ __forceinline__ void tc_epi_half(int fast_act, const EpiParams &epi, const EpiCtx &cx, const uint32_t (&r)[16], const TileCols &tc,
-                                            int c0, int pc, int N, int m_dst, bool has_bias, const EpiStore &es, int lane) {
+                                            int c0, int pc, int N, int m_dst, bool has_bias, const EpiStore &es, int lane, RowCarry &carry, bool last) {
   const bool has_zp = !F16 && epi.has_zp != 0;
   const bool full = pc + 16 <= N;
   if (!F16 && epi.dst_dt == DT_S32) {
@@ -490,11 +562,11 @@ __device__ __forceinline__ void tc_epi_half(int fast_act, const EpiParams &epi, 
       for (int p = 0; p < 4; ++p) v[p] = make_uint4(y[4 * p], y[4 * p + 1], y[4 * p + 2], y[4 * p + 3]);
       warp_store_rows64(es.sbuf, v, es.g_row0 + (size_t)pc * 4, es.pitch_bytes, es.rows_valid, lane);
     } else {
+      uint32_t w[16];
 #pragma unroll
-      for (int p = 0; p < 2; ++p)
-        if (pc + 8 * p < N)
-          warp_store_any32(es.sbuf, make_uint4(y[8 * p], y[8 * p + 1], y[8 * p + 2], y[8 * p + 3]), make_uint4(y[8 * p + 4], y[8 * p + 5], y[8 * p + 6], y[8 * p + 7]),
-                           es.g_row0 + (size_t)(pc + 8 * p) * 4, es.pitch_bytes, es.rows_valid, N - (pc + 8 * p), lane);
+      for (int i = 0; i < 16; ++i) w[i] = (uint32_t)y[i];
+      if (es.coalesce) { if (es.row_ok) put_tail_words(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, N - pc); }
+      else row_put32(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, max(0, min(16, N - pc)), last, es.row_ok, carry);
     }
     return;
   }
@@ -560,9 +632,18 @@ __device__ __forceinline__ void tc_epi_half(int fast_act, const EpiParams &epi, 
       } else if (es.coalesce && full) {
         warp_store_rows32(es.sbuf, make_uint4(pk[0], pk[1], pk[2], pk[3]), make_uint4(pk[4], pk[5], pk[6], pk[7]),
                           es.g_row0 + (size_t)pc * 2, es.pitch_bytes, es.rows_valid, lane);
-      } else if (pc < N) {
-        warp_store_any16(es.sbuf, make_uint4(pk[0], pk[1], pk[2], pk[3]), make_uint4(pk[4], pk[5], pk[6], pk[7]), es.g_row0 + (size_t)pc * 2, es.pitch_bytes,
-                         es.rows_valid, N - pc, lane);
+      } else if (es.coalesce) {
+        if (es.row_ok) {
+          uint8_t *o = reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 2;
+          const int n = N - pc;
+          put_tail_words(o, pk, n >> 1);
+          if (n & 1) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) if (i == n >> 1 && n > 0) *reinterpret_cast<uint16_t *>(o + 4 * i) = (uint16_t)pk[i];
+          }
+        }
+      } else {
+        row_put16(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 2, pk, max(0, min(16, N - pc)), last, es.row_ok, carry);
       }
     } else {
       if (es.v8 && full) {
@@ -583,12 +664,11 @@ __device__ __forceinline__ void tc_epi_half(int fast_act, const EpiParams &epi, 
           v[p] = make_uint4(__float_as_uint(x[4 * p]), __float_as_uint(x[4 * p + 1]), __float_as_uint(x[4 * p + 2]), __float_as_uint(x[4 * p + 3]));
         warp_store_rows64(es.sbuf, v, es.g_row0 + (size_t)pc * 4, es.pitch_bytes, es.rows_valid, lane);
       } else {
+        uint32_t w[16];
 #pragma unroll
-        for (int p = 0; p < 2; ++p)
-          if (pc + 8 * p < N)
-            warp_store_any32(es.sbuf, make_uint4(__float_as_uint(x[8 * p]), __float_as_uint(x[8 * p + 1]), __float_as_uint(x[8 * p + 2]), __float_as_uint(x[8 * p + 3])),
-                             make_uint4(__float_as_uint(x[8 * p + 4]), __float_as_uint(x[8 * p + 5]), __float_as_uint(x[8 * p + 6]), __float_as_uint(x[8 * p + 7])),
-                             es.g_row0 + (size_t)(pc + 8 * p) * 4, es.pitch_bytes, es.rows_valid, N - (pc + 8 * p), lane);
+        for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(x[i]);
+        if (es.coalesce) { if (es.row_ok) put_tail_words(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, N - pc); }
+        else row_put32(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, max(0, min(16, N - pc)), last, es.row_ok, carry);
       }
     }
   }
@@ -881,6 +961,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int nc = min(a.BN / 32, (a.N - pc_tile + 31) / 32);
         const int per = (a.BN / 32 + kTcEpiParts - 1) / kTcEpiParts;
         const int c_begin = part * per, c_end = min(nc, c_begin + per);
+        RowCarry carry;
+        carry.have = false;
         for (int c = c_begin; c < c_end; ++c) {
 #pragma unroll 1
           for (int h = 0; h < 2; ++h) {             // sixteen columns at a time: fewer values live at once
@@ -893,7 +975,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               for (int i = 0; i < 16; ++i) x ^= r[i];
               if (x == 0x12345678u) report_status(a.status, 99); continue; }
 #endif
-            tc_epi_half<F16>(a.fast_act, epi, cx, r, tcols, c * 32 + 16 * h, pc_tile + c * 32 + 16 * h, a.N, m_dst, has_bias, es, lane);
+            tc_epi_half<F16>(a.fast_act, epi, cx, r, tcols, c * 32 + 16 * h, pc_tile + c * 32 + 16 * h, a.N, m_dst, has_bias, es, lane, carry, c == c_end - 1 && h == 1);
           }
         }
       } else {
@@ -1048,6 +1130,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
       cluster_arrive_all();   // this warp reads no neighbour any more
       arrived = true;
+      RowCarry carry;
+      carry.have = false;
       for (int c = (int)crank + a.k_splits * part; c < nc; c += a.k_splits * kTcEpiParts) {
         const uint32_t base = smem0 + (uint32_t)((c * kTcBM + row_in_tile) * 128);
 #pragma unroll 1
@@ -1058,7 +1142,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const uint4 v = ld_shared_v4(base + (uint32_t)(((u + 4 * h) ^ (row_in_tile & 7)) << 4));
             r[4 * u] = v.x; r[4 * u + 1] = v.y; r[4 * u + 2] = v.z; r[4 * u + 3] = v.w;
           }
-          tc_epi_half<F16>(a.fast_act, epi, cx, r, tcols, c * 32 + 16 * h, pc_tile + c * 32 + 16 * h, a.N, m_dst, has_bias, es, lane);
+          tc_epi_half<F16>(a.fast_act, epi, cx, r, tcols, c * 32 + 16 * h, pc_tile + c * 32 + 16 * h, a.N, m_dst, has_bias, es, lane, carry, h == 1);
         }
       }
     }
