@@ -50,3 +50,27 @@ def test_infinities_and_nan_stay_in_their_row(capi, oracle, n):
         for row in (0, 1, 3, 5, 7, 8):
             for i in (1, 3, 4):
                 assert (got[i][row] == want[i][row]).all(), (kind, row, i)
+
+
+@pytest.mark.parametrize("rows", [506, 1100, 2101])
+@pytest.mark.parametrize("n", [505, 844, 1024, 2056, 2999, 4104, 6152, 8192, 8200])
+@pytest.mark.parametrize("kind", ["fused_add_rms_norm", "layer_norm"])
+def test_many_rows(capi, oracle, kind, n, rows):
+    """As many rows as make a thread hold two or four vectors: the same eleven rows again and again."""
+    rng = np.random.default_rng(n)
+    x = oracle.f32_to_bf16(rng.normal(size=(11, n)).astype(np.float32) * 2 + 0.3)
+    res = oracle.f32_to_bf16(rng.normal(size=(11, n)).astype(np.float32)) if kind == "fused_add_rms_norm" else None
+    gamma, beta = (rng.normal(size=n).astype(np.float32) for _ in range(2))
+    if kind != "layer_norm":
+        beta = None
+    times = (rows // 11, 1)
+    st, out, res_out, q, s = run(capi, kind, np.tile(x, times), gamma, beta, residual=None if res is None else np.tile(res, times), quant=True)
+    assert st == capi.SUCCESS, capi.last_error()
+    ref = oracle.normalization(kind, x, gamma, beta, **({} if res is None else dict(residual=res)))
+    if res is not None:
+        ref, ref_res = ref
+        assert (res_out == np.tile(ref_res, times)).all()
+    close(oracle, out, np.tile(ref, times), (kind, n, rows))
+    for part in (slice(0, 11), slice(rows - 11, rows)):
+        qr, sr = oracle.quant_per_token(np.ascontiguousarray(out[part]))
+        assert (q[part] == qr).all() and (s[part] == sr).all(), (kind, n, rows)

@@ -164,17 +164,16 @@ __device__ __forceinline__ void norm_params4(const void *p, int32_t dt, int c0, 
 }
 
 // a sum (or a largest value) over the CTA (sh: one word per warp, not used again before the next barrier)
-template <bool MAX>
+template <bool MAX, int THREADS>
 __device__ __forceinline__ float norm_row_reduce(float x, float *sh) {
   auto op = [](float p, float q) { return MAX ? fmaxf(p, q) : p + q; };
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x = op(x, __shfl_xor_sync(0xffffffffu, x, o));
   const int warps = (int)(blockDim.x >> 5);
-  if (warps == 1) return x;
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
   __syncthreads();
   float t = 0.f;
-  if (warps <= 8) {
+  if (THREADS <= 256) {
     for (int i = 0; i < warps; ++i) t = op(t, sh[i]);
   } else {
     t = (int)(threadIdx.x & 31) < warps ? sh[threadIdx.x & 31] : 0.f;
@@ -218,7 +217,7 @@ __device__ __forceinline__ void norm_clear_outside(uint32_t (&w)[4], int c0, int
 // One row of the full-width form, held by the CTA as the bf16 pairs it came in: v = input, r = residual (fused add); vector i holds the columns
 // 8 i - shift .. 8 i - shift + 7 (shift = 0 unless ANY), and elements outside the row are zeros.  red: a buffer per reduction, used by one row in two
 // (so one barrier each).  Same arithmetic as the generic kernel.
-template <int NV, bool ANY>
+template <int NV, int THREADS, bool ANY>
 __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, int shift, uint32_t (&v)[NV][4], const uint32_t (&r)[NV][4], float (*red)[32]) {
   const int n = (int)a.n, nvec = (shift + n + 7) >> 3;
   auto lo = norm_lo; auto hi = norm_hi;
@@ -252,7 +251,7 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, int s
 #pragma unroll
       for (int e = 0; e < 4; ++e) { s1 = __fadd_rn(s1, lo(v[j][e])); s1 = __fadd_rn(s1, hi(v[j][e])); }
   }
-  s1 = norm_row_reduce<false>(s1, red[0]);
+  s1 = norm_row_reduce<false, THREADS>(s1, red[0]);
   float mean = 0.f, inv;
   if (a.type == NORM_LAYER) {
     mean = __fdiv_rn(s1, (float)a.n);
@@ -274,7 +273,7 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, int s
         }
       }
     }
-    s2 = norm_row_reduce<false>(s2, red[1]);
+    s2 = norm_row_reduce<false, THREADS>(s2, red[1]);
     inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(s2, (float)a.n), a.eps)));
   } else inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(s1, (float)a.n), a.eps)));
   AbsMax<uint16_t> am;
@@ -305,13 +304,13 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, int s
     }
   }
   if (a.q) {
-    float amax = norm_row_reduce<true>(am.finite() ? __uint_as_float(am.bits()) : __int_as_float(0x7F800000), red[2]);
+    float amax = norm_row_reduce<true, THREADS>(am.finite() ? __uint_as_float(am.bits()) : __int_as_float(0x7F800000), red[2]);
     if (!finite_f32(amax)) {
       // an infinite or NaN element (it quantises to 0): the maximum over the finite values instead
       AbsMax<uint16_t> fin;
 #pragma unroll
       for (int j = 0; j < NV; ++j) fin.add_finite(make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]));
-      amax = norm_row_reduce<true>(__uint_as_float(fin.bits()), red[3]);
+      amax = norm_row_reduce<true, THREADS>(__uint_as_float(fin.bits()), red[3]);
     }
     const float scale = scale_from_absmax(amax);
     const float rinv = __frcp_rn(scale);
@@ -337,7 +336,7 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, int s
 // is kept) between the passes, so the row is read once and every access is a 16-byte vector (8 bytes for the s8 codes).
 // Bound by HBM without the quantised output and by instruction issue with it (3.15 of 4 instructions a cycle): all loads of a row (input and
 // residual) are in flight before the first store, each reduction costs one barrier, and the launch overlaps the kernel in front.  4096 rows of 4096 with residual add and s8 codes
-// (151 MB): 36.9 -> 30.5 us (4.9 TB/s); a ring of rows filled by bulk copies ahead of persistent CTAs took 35.7 us (four CTAs per SM where
+// (151 MB): 36.9 -> 28.3 us (5.3 TB/s); a ring of rows filled by bulk copies ahead of persistent CTAs took 35.7 us (four CTAs per SM where
 // there are six here).
 // ANY: rows of any length, one behind the other.  A row is covered by the aligned vectors of the tensor that it touches (the first and the last shared with
 // its neighbours, of which it writes its own elements only); input, residual, result and codes then need no shifting, the parameters are picked out of two
@@ -357,6 +356,14 @@ __global__ void __launch_bounds__(THREADS, CTAS) norm_rows_vec_kernel(const Norm
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
       const int i = threadIdx.x + j * blockDim.x;
+      if constexpr (!ANY) {
+        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+        const uint4 x = i < nvec ? reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(a.x) + off)[i] : zero;
+        const uint4 y = a.type == NORM_FUSED_ADD_RMS && i < nvec ? reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(a.residual) + off)[i] : zero;
+        v[j][0] = x.x; v[j][1] = x.y; v[j][2] = x.z; v[j][3] = x.w;
+        r[j][0] = y.x; r[j][1] = y.y; r[j][2] = y.z; r[j][3] = y.w;
+        continue;
+      }
 #pragma unroll
       for (int e = 0; e < 4; ++e) v[j][e] = r[j][e] = 0u;
       if (i < nvec) {
@@ -365,7 +372,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) norm_rows_vec_kernel(const Norm
         if (ANY && (i == 0 || i == nvec - 1)) { norm_clear_outside(v[j], i * 8 - shift, n); norm_clear_outside(r[j], i * 8 - shift, n); }
       }
     }
-    norm_row_vec<NV, ANY>(a, b, shift, v, r, red[parity]);
+    norm_row_vec<NV, THREADS, ANY>(a, b, shift, v, r, red[parity]);
   }
 }
 
@@ -466,23 +473,30 @@ extern "C" int32_t b200dnn_normalization(const b200dnn_norm_t *d, void *stream) 
                      (!a.q || ((any ? a.q_ld == n : a.q_ld % 8 == 0) && (reinterpret_cast<uintptr_t>(a.q) & 7) == 0)) && env_int("B200DNN_NORM_VEC", 1) != 0;
     if (vec) {
       const int nvec = (int)((n + (any ? 14 : 0)) / 8);          // vectors that a row touches at most
-      // Two vectors per thread while the CTA grows with the row; four for many rows of 2048 columns or more, which pay less for what every thread does once
-      // per row (16384 columns need four).  us with two and four: 4700 x 3328 with codes 24.7, 22.4; 12000 x 2048 LayerNorm 30.6, 28.1; 8830 x 11136 with
-      // codes 143, 138; but 16000 x 1024 26.9, 28.3; 300 x 1001 4.2, 6.6; 92 x 9472 5.1, 5.7.
-      const int per = nvec > 1536 || (batch >= 2048 && nvec >= 256) ? 4 : 2;
-      const int threads = (int)round_up((nvec + per - 1) / per, 32);
+      // One vector per thread where all rows are in flight at once (a row's latency counts): up to three rows an SM of 2048 columns, one of 8192.  us with two and one, residual add
+      // and codes: 130 x 512 3.1, 2.5; 400 x 2048 3.5, 3.2; 130 x 4096 3.5, 2.9; 130 x 2999 5.3, 4.5; but 400 x 4096 4.4, 5.9; 900 x 1024 3.8, 4.5.
+      // Else two while the CTA grows with the row (more CTAs in flight), and four for many long rows, which then pay less for what every thread does once per
+      // row -- from where on depends on the registers a vector takes: two inputs with a residual, and an unaligned row's (any) instructions weigh more.  us with two
+      // and four at 4096 rows: residual add and codes 4096 columns 28.5, 29.2; 6144 41.0, 41.3; 8192 53.8, 51.6, without codes 43.8, 44.5; LayerNorm and codes 2048
+      // 15.8, 16.7; 4096 28.3, 27.2; 8192 55.6, 49.3; unaligned 2999 residual add 34.3, 33.7.  (More than 12288 columns need four.)
+      const int from = any ? 256 : a.type != NORM_FUSED_ADD_RMS ? (batch < 2048 ? 769 : 512) : a.q ? 769 : 1537;
+      const bool one_wave = nvec <= 1024 && batch <= (int64_t)R.sm_count * (nvec <= 256 ? 3 : 1);
+      const int per = one_wave ? 1 : nvec > 1536 || (batch >= (any ? 2048 : 768) && nvec >= from) ? 4 : 2;
+      // up to 1024 rows whole warps for each of an SM's four schedulers (700 x 2560: 160 threads 6.3 us, 256 5.4); beyond, idle warps cost more (4096 x 2560: 22.4, 19.9)
+      int threads = (int)round_up((nvec + per - 1) / per, 32);
+      if (batch < 1024 && threads > 128) threads = (int)round_up(threads, 128);
       const int nv = (nvec + threads - 1) / threads;
       const long long cap = (long long)R.sm_count * 64;
       const unsigned grid = (unsigned)(batch < cap ? batch : cap);
       auto go = [&](auto kern) { return launch_pdl(kern, grid, (unsigned)threads, 0, st, true, a); };
-      auto pick = [&](auto one, auto two, auto two_512, auto two_768, auto four_128, auto four_256, auto four_512) {
-        if (nv <= 1) return go(one);
+      auto pick = [&](auto one, auto one_1024, auto two, auto two_512, auto two_768, auto four_128, auto four_256, auto four_512) {
+        if (nv <= 1) return threads <= 256 ? go(one) : go(one_1024);
         if (nv <= 2) return threads <= 256 ? go(two) : threads <= 512 ? go(two_512) : go(two_768);
         return threads <= 128 ? go(four_128) : threads <= 256 ? go(four_256) : go(four_512);
       };
-      B2_TRY(any ? pick(norm_rows_vec_kernel<1, 256, 4, true>, norm_rows_vec_kernel<2, 256, 5, true>, norm_rows_vec_kernel<2, 512, 2, true>, norm_rows_vec_kernel<2, 768, 2, true>,
+      B2_TRY(any ? pick(norm_rows_vec_kernel<1, 256, 4, true>, norm_rows_vec_kernel<1, 1024, 1, true>, norm_rows_vec_kernel<2, 256, 5, true>, norm_rows_vec_kernel<2, 512, 2, true>, norm_rows_vec_kernel<2, 768, 2, true>,
                         norm_rows_vec_kernel<4, 128, 8, true>, norm_rows_vec_kernel<4, 256, 4, true>, norm_rows_vec_kernel<4, 512, 2, true>)
-                 : pick(norm_rows_vec_kernel<1, 256, 6, false>, norm_rows_vec_kernel<2, 256, 6, false>, norm_rows_vec_kernel<2, 512, 3, false>, norm_rows_vec_kernel<2, 768, 2, false>,
+                 : pick(norm_rows_vec_kernel<1, 256, 6, false>, norm_rows_vec_kernel<1, 1024, 1, false>, norm_rows_vec_kernel<2, 256, 6, false>, norm_rows_vec_kernel<2, 512, 3, false>, norm_rows_vec_kernel<2, 768, 2, false>,
                         norm_rows_vec_kernel<4, 128, 8, false>, norm_rows_vec_kernel<4, 256, 4, false>, norm_rows_vec_kernel<4, 512, 2, false>));
       B2_LAUNCHED();
       B2_CUDA(cudaGetLastError());
