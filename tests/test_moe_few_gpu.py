@@ -1,5 +1,6 @@
 """The grouped GEMM for a few rows per expert (MoE layers of up to 64 tokens) against the tile kernel: the same layer, bit for bit (INT8 sums are exact and the epilogue's
-operations the same; bf16 within the order of the f32 sums), at the edges of its row counts, of its 128-column tiles and of the routing, and its bounded waits."""
+operations the same; bf16 within the order of the f32 sums), at the edges of its row counts, of its 128-column tiles and of the routing, with tokens that name no expert, and its
+bounded waits."""
 import numpy as np
 import pytest
 
@@ -58,6 +59,42 @@ def test_against_the_tile_kernel(capi, monkeypatch, T, H, I, E, S, topk, skew, k
     else:                                                # two products of f32 sums with a rounding to bf16 between and behind them
         d = (out.float() - want.float()).abs()
         assert (d <= 2.0 ** -7 * want.float().abs() + 2.0 ** -7 * want.float().abs().max()).all()
+    capi.lib.b200dnn_clear_caches()
+
+
+@pytest.mark.parametrize("T", [9, 16, 64])
+@pytest.mark.parametrize("topk,E,S", [(2, 4, 0), (8, 11, 1), (2, 300, 0)])
+@pytest.mark.parametrize("wdt", ["s8", "bf16"])
+def test_tokens_without_a_choice(capi, monkeypatch, T, topk, E, S, wdt):
+    """Logits that are NaN or minus infinity throughout, or infinite once, name no expert, and all choices of such tokens may fall on one expert: more rows than there are
+    tokens.  The other tokens keep their results, and (s8) all of them are those of the tile kernel; a few such tokens, and all of them."""
+    import torch
+    call, out, keep = layer(capi, torch, T, 136, 96, E, S, topk, wdt=wdt, skew=True, seed=T + topk)
+    logits = keep[-2]
+    st = torch.cuda.current_stream().cuda_stream
+
+    def run(few):
+        monkeypatch.setenv("B200DNN_MOE_FEW", few)
+        out.zero_()
+        capi.check(call())
+        assert capi.lib.b200dnn_stream_status(st) == capi.SUCCESS, capi.last_error()
+        return out.clone()
+
+    want = run("64")
+    assert want.abs().max() > 0
+    inf = float("inf")
+    for rows in (slice(1, None, 3), slice(None)):
+        bad = torch.zeros(T, dtype=torch.bool, device="cuda")
+        bad[rows] = True
+        logits[rows] = -inf
+        logits[rows][::3, E // 2] = float("nan")
+        logits[rows][1::3] = float("nan")
+        logits[rows][2::3, 0] = inf
+        torch.cuda.synchronize()
+        got, tile = run("64"), run("0")
+        assert torch.equal(got[~bad], want[~bad])
+        if wdt == "s8":
+            assert torch.equal(got.view(torch.int16), tile.view(torch.int16))
     capi.lib.b200dnn_clear_caches()
 
 

@@ -17,13 +17,10 @@ namespace {
 int32_t grouped_gemm(const uint8_t *A, int64_t lda, int R, int N, int K, const std::vector<PackedWeight> &pws,
                      const int32_t *row_off_dev, const int32_t *tile_prefix_dev, const TcGroupDesc *groups_dev,
                      int m_tiles_bound, EpiParams epi, bool shared_dst, cudaStream_t st, int tile_rows = kTcBM, bool f16 = false,
-                     int max_rows = 0 /* no expert has more rows; 0: not known */) {
+                     int few_rows = 0 /* tile_prefix_dev counts tiles of so many rows for moe_few_kernel (bf16 results back to back) */) {
   Runtime &Rt = rt();
   const int G = (int)pws.size();
-  // Few rows per expert: the weight as the 128-row operand (moe_few.cuh).  72 layers of 1 to 64 tokens, one call after the other in either form: 1.1 to 1.7 times as fast
-  // up to 16 tokens, 1.0 to 1.4 up to 40, 0.98 to 1.11 (1.04 on average) up to 64, as far as its rows go.  B200DNN_MOE_FEW: the largest number of rows it takes.
-  const bool few = max_rows > 0 && max_rows <= env_int("B200DNN_MOE_FEW", kMoeFewMaxRows) && max_rows <= kMoeFewMaxRows && tile_rows == kTcBM && shared_dst && groups_dev &&
-                   epi.dst_dt == B200DNN_BF16;
+  const bool few = few_rows > 0;
   TcGemmArgs ta{};
   ta.pair = tile_rows > kTcBM ? 1 : 0;  // tile_prefix_dev and m_tiles_bound count tiles of tile_rows rows
   ta.f16 = f16 ? 1 : 0;                 // bf16 form: lda and K count bytes, pws hold bf16 packs
@@ -48,7 +45,7 @@ int32_t grouped_gemm(const uint8_t *A, int64_t lda, int R, int N, int K, const s
   }, st, &maps_dev));
   if (few) {
     MoeFewArgs fa{};
-    fa.n_groups = G; fa.n_tiles = (N + 127) / 128; fa.N = N; fa.k_blocks = (int)(p0.Kp / 128); fa.MP = (max_rows + 15) & ~15;
+    fa.n_groups = G; fa.n_tiles = (N + 127) / 128; fa.N = N; fa.k_blocks = (int)(p0.Kp / 128); fa.MP = few_rows;
     fa.gated = p0.gated; fa.row_off = row_off_dev; fa.tile_prefix = tile_prefix_dev; fa.maps_w = (const CUtensorMap *)maps_dev; fa.groups = groups_dev;
     fa.status = Rt.status; fa.test_no_loads = env_int("B200DNN_TEST_NO_LOADS", 0);
     const int stage_bytes = (128 + fa.MP) * 128, parts = 2 * fa.MP * 512;
@@ -121,7 +118,7 @@ __global__ void __launch_bounds__(256) moe_place_rows_bf16_kernel(const uint16_t
 int32_t moe_core_bf16(int G, const std::vector<ExpertWeightsIn> &ew, int K, int I, int H, int transB, int act, int weights_const,
                       RowQuantArgs qa, int32_t src_dt, int R, const int32_t *row_off_dev, const int32_t *tile_prefix_dev,
                       int m_tiles_bound, const std::vector<void *> *dst_down_dev, const std::vector<int64_t> *ldc_down,
-                      void **O_out, int64_t *ldO_out, cudaStream_t st, void *O_given, int tile_rows, const uint16_t **Z_out, int max_rows) {
+                      void **O_out, int64_t *ldO_out, cudaStream_t st, void *O_given, int tile_rows, const uint16_t **Z_out, int few_rows) {
   Runtime &Rt = rt();
   B2_CHECK(src_dt == B200DNN_BF16, B200DNN_UNIMPLEMENTED, "bf16 experts take bf16 rows");
   B2_CHECK(!qa.scatter_peer && !qa.n_rows_dev, B200DNN_UNIMPLEMENTED, "the expert-parallel exchange is built for s8 experts");
@@ -177,7 +174,7 @@ int32_t moe_core_bf16(int G, const std::vector<ExpertWeightsIn> &ew, int K, int 
   EpiParams e1{};
   e1.dst = Z; e1.ldc = I; e1.dst_dt = B200DNN_BF16; e1.gated_act = act; e1.gated_I = I; e1.bias_dt = b13_dt;
   B2_TRY(grouped_gemm((const uint8_t *)X, ldx * 2, R, 2 * I, 2 * K, p13, row_off_dev, tile_prefix_dev, (const TcGroupDesc *)g13_dev,
-                      m_tiles_bound, e1, true, st, tile_rows, true, max_rows));
+                      m_tiles_bound, e1, true, st, tile_rows, true, few_rows));
   rt().mark(4);
 
   // 3. second GEMM reads Z as it is -> O
@@ -186,7 +183,7 @@ int32_t moe_core_bf16(int G, const std::vector<ExpertWeightsIn> &ew, int K, int 
   EpiParams e2{};
   e2.dst = O; e2.ldc = H; e2.dst_dt = B200DNN_BF16; e2.bias_dt = b2_dt;
   B2_TRY(grouped_gemm((const uint8_t *)Z, (int64_t)I * 2, R, H, 2 * I, p2, row_off_dev, tile_prefix_dev, (const TcGroupDesc *)g2_dev,
-                      m_tiles_bound, e2, dst_down_dev == nullptr, st, tile_rows, true, max_rows));
+                      m_tiles_bound, e2, dst_down_dev == nullptr, st, tile_rows, true, few_rows));
   rt().mark(6);
   if (Z_out) *Z_out = Z;
   if (O_out) { *O_out = O; *ldO_out = H; }
@@ -199,7 +196,7 @@ int32_t moe_core(int G, const std::vector<ExpertWeightsIn> &ew, int K, int I, in
                  int m_tiles_bound, const std::vector<void *> *dst_down_dev, const std::vector<int64_t> *ldc_down,
                  void **O_out, int64_t *ldO_out, cudaStream_t st, void *O_given = nullptr, int tile_rows = kTcBM,
                  const uint16_t **Z_out = nullptr, uint32_t *zmax = nullptr /* row maxima already set to zero, or null */,
-                 int max_rows = 0 /* see grouped_gemm */) {
+                 int few_rows = 0 /* see grouped_gemm */) {
   Runtime &Rt = rt();
   B2_CHECK(act >= 1 && act <= 3, B200DNN_UNIMPLEMENTED, "fused MoE needs a gated activation (got %d)", act);
   B2_CHECK(I % kGateGranule == 0, B200DNN_UNIMPLEMENTED, "expert FFN width must be a multiple of %d", kGateGranule);
@@ -209,7 +206,7 @@ int32_t moe_core(int G, const std::vector<ExpertWeightsIn> &ew, int K, int I, in
     B2_CHECK((ew[g].wei_dt == B200DNN_BF16) == wbf16 && (wbf16 || ew[g].wei_dt == 0 || ew[g].wei_dt == B200DNN_S8), B200DNN_UNIMPLEMENTED,
              "expert %d: weight dtype %d (all experts s8, or all bf16)", g, ew[g].wei_dt);
   if (wbf16) return moe_core_bf16(G, ew, K, I, H, transB, act, weights_const, qa, src_dt, R, row_off_dev, tile_prefix_dev, m_tiles_bound,
-                                  dst_down_dev, ldc_down, O_out, ldO_out, st, O_given, tile_rows, Z_out, max_rows);
+                                  dst_down_dev, ldc_down, O_out, ldO_out, st, O_given, tile_rows, Z_out, few_rows);
   std::vector<PackedWeight> p13(G), p2(G);
   std::vector<TcGroupDesc> g13(G), g2(G);
   int32_t b13_dt = 0, b2_dt = 0;
@@ -272,7 +269,7 @@ int32_t moe_core(int G, const std::vector<ExpertWeightsIn> &ew, int K, int I, in
   e1.dst = Z; e1.ldc = I; e1.dst_dt = B200DNN_BF16; e1.gated_act = act; e1.gated_I = I; e1.row_absmax = zmax;
   e1.bias_dt = b13_dt;
   B2_TRY(grouped_gemm(A1_in, lda1, R, 2 * I, K, p13, row_off_dev, tile_prefix_dev, (const TcGroupDesc *)g13_dev,
-                      m_tiles_bound, e1, true, st, tile_rows, false, max_rows));
+                      m_tiles_bound, e1, true, st, tile_rows, false, few_rows));
   rt().mark(4);
 
   // 3. re-quantise the activated rows (from their bf16 values, as the reference does)
@@ -290,7 +287,7 @@ int32_t moe_core(int G, const std::vector<ExpertWeightsIn> &ew, int K, int I, in
   e2.wei_scale_dt = B200DNN_F32; e2.wei_scale_n = H;
   e2.dst = O; e2.ldc = H; e2.dst_dt = B200DNN_BF16; e2.bias_dt = b2_dt;
   B2_TRY(grouped_gemm((const uint8_t *)A2, Iq, R, H, I, p2, row_off_dev, tile_prefix_dev, (const TcGroupDesc *)g2_dev,
-                      m_tiles_bound, e2, dst_down_dev == nullptr, st, tile_rows, false, max_rows));
+                      m_tiles_bound, e2, dst_down_dev == nullptr, st, tile_rows, false, few_rows));
   rt().mark(6);
   if (Z_out) *Z_out = Z;
   if (O_out) { *O_out = O; *ldO_out = H; }
@@ -451,11 +448,15 @@ extern "C" int32_t b200dnn_moe_layer(const void *x, int64_t ldx, const float *lo
   B2_CHECK(ids && w && rank && cnt && row_off && tile_prefix && slot_rows && slot_w && row_token, B200DNN_FAILURE, "workspace allocation failed");
   rt().mark(-1);
   const int tile_rows = tc_tile_rows(R, H < 2 * I ? H : 2 * I);
+  // Few rows per expert: the weight as the 128-row operand (moe_few.cuh).  72 layers of 1 to 64 tokens, one call after the other in either form: 1.1 to 1.7 times as fast
+  // up to 16 tokens, 1.0 to 1.4 up to 40, 0.98 to 1.11 (1.04 on average) up to 64, as far as its rows go.  B200DNN_MOE_FEW: the largest number of tokens that it takes.
+  const int few_rows = tile_rows == kTcBM && T <= std::min(env_int("B200DNN_MOE_FEW", kMoeFewMaxRows), kMoeFewMaxRows) ? (T + 15) & ~15 : 0;
+  const int route_rows = few_rows ? few_rows : tile_rows;      // what the tile counts count
   uint32_t *zmax = nullptr;
   if (T <= kRouteSmallT && T * topk <= kRouteSmallSlots && G <= kRouteSmallGroups) {
     zmax = (uint32_t *)Rt.ws.alloc((size_t)R * 4);
     B2_CHECK(zmax, B200DNN_FAILURE, "workspace allocation failed");
-#define B2_RS(PER) launch_pdl(route_small_kernel<PER>, 1u, 1024u, 0, st, true, (const float *)l_dev, T, E, topk, S, tile_rows, row_off, tile_prefix, slot_rows, slot_w, row_token, zmax)
+#define B2_RS(PER) launch_pdl(route_small_kernel<PER>, 1u, 1024u, 0, st, true, (const float *)l_dev, T, E, topk, S, route_rows, row_off, tile_prefix, slot_rows, slot_w, row_token, zmax)
     B2_TRY(E <= 32 ? B2_RS(1) : E <= 64 ? B2_RS(2) : E <= 128 ? B2_RS(4) : B2_RS(8));
 #undef B2_RS
     B2_LAUNCHED();
@@ -469,13 +470,13 @@ extern "C" int32_t b200dnn_moe_layer(const void *x, int64_t ldx, const float *lo
     B2_TRY(E <= 32 ? B2_RC(1) : E <= 64 ? B2_RC(2) : E <= 128 ? B2_RC(4) : B2_RC(8));
 #undef B2_RC
     B2_LAUNCHED();
-    B2_TRY(launch_pdl(route_assign_kernel, chunks, (unsigned)kRouteChunkThreads, 0, st, true, ids, w, counts, T, E, topk, S, chunk, tile_rows, row_off, tile_prefix, slot_rows, slot_w,
+    B2_TRY(launch_pdl(route_assign_kernel, chunks, (unsigned)kRouteChunkThreads, 0, st, true, ids, w, counts, T, E, topk, S, chunk, route_rows, row_off, tile_prefix, slot_rows, slot_w,
                       row_token));
     B2_LAUNCHED();
   } else {
     B2_TRY(launch_route_topk((const float *)l_dev, T, E, topk, 1, ids, w, st));
     B2_TRY(launch_expert_rank(ids, T * topk, E, rank, cnt, st));
-    expert_offsets_kernel<<<1, 32, 0, st>>>(cnt, E, S, T, row_off, tile_prefix, tile_rows);
+    expert_offsets_kernel<<<1, 32, 0, st>>>(cnt, E, S, T, row_off, tile_prefix, route_rows);
     B2_LAUNCHED();
     build_maps_kernel<<<(unsigned)((R + 255) / 256), 256, 0, st>>>(ids, rank, w, row_off, T, topk, E, S, slot_rows, slot_w, row_token);
     B2_LAUNCHED();
@@ -491,10 +492,10 @@ extern "C" int32_t b200dnn_moe_layer(const void *x, int64_t ldx, const float *lo
   if (ns <= 32) { qa.scatter = slot_rows; qa.scatter_n = ns; qa.scatter_rows = T; }
   else qa.gather = row_token;
   void *O = nullptr; int64_t ldO = 0;
-  // row tiles: whole ones, and one that is not for every expert that can have rows (a few tokens meet a few experts)
+  // row tiles of tile_rows: whole ones, and one that is not for every expert that can have rows (a few tokens meet a few experts)
   const int m_tiles_bound = R / tile_rows + (int)std::min<long long>(E, (long long)T * topk) + S;
   B2_TRY(moe_core(G, ew, K, I, H, transB, act, 1, qa, B200DNN_BF16, R, row_off, tile_prefix, m_tiles_bound, nullptr, nullptr, &O, &ldO, st,
-                  nullptr, tile_rows, nullptr, zmax, T));
+                  nullptr, tile_rows, nullptr, zmax, few_rows));
 
   Staged o_out;
   B2_TRY(stage_out(out, span_bytes(T, H, ld_out, B200DNN_BF16), st, &o_out, ld_out != H));

@@ -4,7 +4,8 @@
 // As in skinny_gemm.cuh the operands change places: the MMA's M = 128 rows are 128 packed output columns of one expert, its N is the rows rounded up to 16.  The
 // tile kernel's 128-row box of activations per 128 bytes of K, nearly all of it other experts' rows or padding, costs as many bytes from L2 to shared memory as
 // the weight itself; here it is MP x 128 bytes beside 16 KiB of weight, and an accumulator holds no padding.
-//   - One persistent CTA per SM over the tiles (expert with rows, 128 packed columns); the experts that have rows are found on the device (tile_prefix).
+//   - One persistent CTA per SM over the tiles (MP rows of an expert, 128 packed columns); an expert's tiles are found on the device (tile_prefix).  MP holds all rows of an
+//     expert that every token asks for once; a token whose logits name no expert (NaN) has the same one k times, and its expert more tiles.
 //   - warp 0 copies, warp 1 issues MMAs, warps 2-9 finish; two accumulators and a ring that runs across tiles keep the weight stream going behind the epilogue.
 //   - The accumulators pass through shared memory as [row][128 columns]; then a warp takes whole rows, four columns a lane, or (gated) two outputs, with the
 //     arithmetic of the tile kernel's epilogue.
@@ -25,9 +26,9 @@ constexpr int kMoeFewSmem = 216 * 1024;
 struct MoeFewArgs {
   int n_groups, n_tiles;          // experts; column tiles of 128 per expert
   int N, k_blocks;                // packed columns; 128-byte blocks of K
-  int MP, stages;                 // rows rounded up to 16 (no expert has more); ring depth
+  int MP, stages;                 // rows of a tile, a multiple of 16; ring depth
   int gated;                      // packed gate/up interleave, see pack_kernels.cuh
-  const int32_t *row_off, *tile_prefix;      // [n_groups + 1] first row of each expert; how many experts in front have rows
+  const int32_t *row_off, *tile_prefix;      // [n_groups + 1] first row of each expert; how many tiles of MP rows the experts in front have
   const CUtensorMap *maps_w;      // [n_groups], boxes of 128 packed rows
   const TcGroupDesc *groups;      // [n_groups] scales and biases
   int32_t *status;
@@ -75,23 +76,26 @@ moe_few_kernel(const __grid_constant__ CUtensorMap map_a, const MoeFewArgs a, co
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   const int total = a.tile_prefix[a.n_groups] * a.n_tiles;
-  // a tile's expert (by a whole warp): the number of prefix entries up to its place among the experts that have rows
-  auto group_of = [&](int tile) {
+  // a tile's expert (by a whole warp): the number of prefix entries up to its place among the row tiles; its first row and its rows, MP at most
+  struct Rows { int g, row0, rows; };
+  auto rows_of = [&](int tile) {
     const int mt = tile / a.n_tiles;
     int g = 0;
     for (int base = 1; base < a.n_groups; base += 32) {
       const int i = base + lane;
       g += __popc(__ballot_sync(0xffffffffu, i < a.n_groups && a.tile_prefix[i] <= mt));
     }
-    return g;
+    const int row0 = a.row_off[g] + (mt - a.tile_prefix[g]) * a.MP;
+    return Rows{g, row0, min(a.MP, a.row_off[g + 1] - row0)};
   };
 
   if (warp == 0) {
     int slot = 0; uint32_t phase = 0;
     bool ok = true;
     for (int tile = blockIdx.x; ok && tile < total && !a.test_no_loads; tile += gridDim.x) {
-      const int g = group_of(tile), nt = tile % a.n_tiles, row0 = a.row_off[g];
-      const CUtensorMap *mw = a.maps_w + g;
+      const Rows t = rows_of(tile);
+      const int nt = tile % a.n_tiles, row0 = t.row0;
+      const CUtensorMap *mw = a.maps_w + t.g;
       for (int kb = 0; kb < a.k_blocks; ++kb) {
         if (!mbar_wait_warp(empty_bar(slot), phase ^ 1u)) { if (lane == 0) { s_err = 1; report_status(a.status, 61); } ok = false; break; }
         const uint32_t sw = smem0 + (uint32_t)slot * stage_bytes;
@@ -135,8 +139,9 @@ moe_few_kernel(const __grid_constant__ CUtensorMap map_a, const MoeFewArgs a, co
     const int gc = (lane >> 4) * 64 + ((2 * lane) & 31);              // gated: this lane's first gate column of the tile (its up columns are 32 further)
     int acc = 0; uint32_t acc_phase = 0;
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
-      const int g = group_of(tile), nt = tile % a.n_tiles, row0 = a.row_off[g], rows = a.row_off[g + 1] - row0;
-      const TcGroupDesc gd = a.groups[g];
+      const Rows t = rows_of(tile);
+      const int nt = tile % a.n_tiles, row0 = t.row0, rows = t.rows;
+      const TcGroupDesc gd = a.groups[t.g];
       // this lane's columns: four in a row, or two gate and two up columns
       float ws[4] = {1.f, 1.f, 1.f, 1.f}, bias[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
