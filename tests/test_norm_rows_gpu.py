@@ -52,8 +52,8 @@ def test_infinities_and_nan_stay_in_their_row(capi, oracle, n):
                 assert (got[i][row] == want[i][row]).all(), (kind, row, i)
 
 
-@pytest.mark.parametrize("rows", [506, 1100, 2101])
-@pytest.mark.parametrize("n", [505, 844, 1024, 2056, 2999, 4104, 6152, 8192, 8200])
+@pytest.mark.parametrize("rows", [253, 506, 1100, 1265, 2101])
+@pytest.mark.parametrize("n", [505, 844, 1024, 1536, 2056, 2999, 4104, 6152, 6400, 8192, 8200])
 @pytest.mark.parametrize("kind", ["fused_add_rms_norm", "layer_norm"])
 def test_many_rows(capi, oracle, kind, n, rows):
     """As many rows as make a thread hold two or four vectors: the same eleven rows again and again."""

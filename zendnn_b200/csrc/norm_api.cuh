@@ -496,10 +496,21 @@ extern "C" int32_t b200dnn_normalization(const b200dnn_norm_t *d, void *stream) 
       // 15.8, 16.7; 4096 28.3, 27.2; 8192 55.6, 49.3; unaligned 2999 residual add 34.3, 33.7.  (More than 12288 columns need four.)
       const int from = any ? 256 : a.type != NORM_FUSED_ADD_RMS ? (batch < 2048 ? 769 : 512) : a.q ? 769 : 1537;
       const bool one_wave = nvec <= 1024 && batch <= (int64_t)R.sm_count * (nvec <= 256 ? 3 : 1);
-      const int per = one_wave ? 1 : nvec > 1536 || (batch >= (any ? 2048 : 768) && nvec >= from) ? 4 : 2;
-      // up to 1024 rows whole warps for each of an SM's four schedulers (700 x 2560: 160 threads 6.3 us, 256 5.4); beyond, idle warps cost more (4096 x 2560: 22.4, 19.9)
+      // Aligned rows of more than 512 vectors in fewer than 768 rows: an SM holds three CTAs of 512 threads with two vectors, four of 384, and four of 256 with four.  Launches overlap, so
+      // that up to half of what the device holds runs as in an idle one, and more as if it were full.  us with two and four, residual add and codes: 230 x 6400 5.7, 5.1;
+      // 360 x 6656 5.9, 6.6; 520 x 6400 8.6, 6.7; 520 x 8192 9.8, 8.5; 360 x 5120 5.9, 5.7; 640 x 5120 8.2, 8.8; 160 x 5120 4.0, 4.3.
+      const int64_t sm = R.sm_count;
+      const bool four = !any && nvec > 512 && nvec <= 1024 && batch <= 4 * sm && (nvec <= 768 ? batch > 2 * sm : batch > 3 * sm || (2 * batch > 3 * sm && batch <= 2 * sm));
+      // (many rows with residual add and no codes: 8000 x 6400 68.7, 65.2; 2100 x 7168 23.0, 23.3; 8192 columns see above)
+      const bool four_plain = !any && nvec > 768 && nvec <= 960 && batch >= 2560;
+      const int per = one_wave ? 1 : nvec > 1536 || four || four_plain || (batch >= (any ? 2048 : 768) && nvec >= from) ? 4 : 2;
+      // up to 1024 rows whole warps for each of an SM's four schedulers (700 x 2560: 160 threads 6.3 us, 256 5.4); beyond, idle warps cost more (4096 x 2560: 22.4, 19.9),
+      // but one in eight does not (4100 x 6400 with residual add and codes: 224 threads 45.1, 256 44.3)
       int threads = (int)round_up((nvec + per - 1) / per, 32);
       if (batch < 1024 && threads > 128) threads = (int)round_up(threads, 128);
+      if (!any && per == 4 && threads == 224) threads = 256;
+      // 96 threads (16 CTAs an SM) or 128 (12), as above: 760 x 1536 3.9, 3.8; 1024 4.2, 5.6; 1300 6.4, 5.6; 2100 6.5, 7.4
+      if (!any && per == 2 && threads == 96 && (batch <= 6 * sm || (batch > 8 * sm && batch <= 12 * sm))) threads = 128;
       const int nv = (nvec + threads - 1) / threads;
       const long long cap = (long long)R.sm_count * 64;
       const unsigned grid = (unsigned)(batch < cap ? batch : cap);
