@@ -32,8 +32,6 @@ def weights(torch, K, N):
 @pytest.mark.parametrize("K", [8, 264, 2048, 6152])
 def test_bits_of_the_separate_kernel(capi, monkeypatch, M, K, ring):
     import torch
-    if ring and M > 2:
-        pytest.skip("the ring form takes one or two rows here")
     torch.manual_seed(M + K)
     w, ws = weights(torch, K, 136)
     x = (torch.randn(M, K, device="cuda") * torch.logspace(-3, 3, M, device="cuda")[:, None]).bfloat16()
@@ -42,7 +40,8 @@ def test_bits_of_the_separate_kernel(capi, monkeypatch, M, K, ring):
     for sdt in ("f32", "bf16"):
         want, want_s, n0 = call(capi, monkeypatch, "0", x, w, ws, sdt, ring=ring)
         got, got_s, n1 = call(capi, monkeypatch, "1", x, w, ws, sdt, ring=ring)
-        assert n1 == n0 - 1 and torch.equal(got, want) and torch.equal(got_s, want_s), (M, K, sdt)
+        # (the ring form has eight warps, and a row needs one at least)
+        assert n1 == (n0 if ring and M > 8 else n0 - 1) and torch.equal(got, want) and torch.equal(got_s, want_s), (M, K, sdt)
     capi.lib.b200dnn_clear_caches()
 
 

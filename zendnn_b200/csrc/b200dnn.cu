@@ -305,7 +305,7 @@ int32_t launch_decode(const uint8_t *A, int64_t lda, bool a_unsigned, int M, int
   return B200DNN_SUCCESS;
 }
 
-// Ring form of the decode GEMM (decode_ring.cuh).  unimplemented when the ring would be too shallow.
+// Ring form of the decode GEMM (decode_ring.cuh).  unimplemented when the ring would be too shallow, or has fewer warps than rows to quantise.
 template <int R>
 int32_t launch_decode_ring(const uint8_t *A, int64_t lda, bool a_unsigned, int M, int N, int K, const PackedWeight &pw,
                            const EpiParams &epi, bool early_weights, cudaStream_t st, const DecodeQuant &dq) {
@@ -322,7 +322,7 @@ int32_t launch_decode_ring(const uint8_t *A, int64_t lda, bool a_unsigned, int M
   const size_t stage_bytes = (size_t)R * kRingWarps * 1024;
   const size_t fixed = ring_off_ring(g.rows_staged, g.a_stride, g.max_local_groups);
   const size_t budget = 227 * 1024;
-  if (M > 16 || fixed + 3 * stage_bytes > budget) return B200DNN_UNIMPLEMENTED;
+  if (M > 16 || fixed + 3 * stage_bytes > budget || (dq.src && M > kRingWarps)) return B200DNN_UNIMPLEMENTED;
   int stages = (int)((budget - fixed) / stage_bytes);
   const int need = ((g.max_local_groups + R - 1) / R) * ((g.blocks + kRingWarps - 1) / kRingWarps);
   if (stages > kRingMaxStages) stages = kRingMaxStages;
@@ -1097,6 +1097,11 @@ bool skinny_decode(int M, int N, int K, int64_t Kp) {
   return M > 8 && (long long)K * N >= (24ll << 20) && ((N + 127) / 128 <= rt().sm_count || decode_smem(M, N, Kp) > 220 * 1024);
 }
 
+// decode kernel: 0 tiled only, 1 register-batch form, 2 ring form, 3..5 ring with that many groups per stage;
+// default: ring for M <= 2 and weights of 24 MB or more (measured faster there: 10.9 against 11.5 us at 45 MB, but
+// 5.9 against 5.7 us at 16.8 MB), register-batch form otherwise
+int decode_form(int M, int N, int K) { return env_int("B200DNN_DECODE_KERNEL", (M <= 2 && (long long)K * N >= (24ll << 20)) ? 2 : 1); }
+
 // Dynamic quantisation inside the decode kernel (decode_quant.cuh): aligned bf16 rows that the decode kernels take, few enough elements, and no
 // overlap of the results with the source (every CTA reads all of it, while others may already write).  The line: a kernel of its own costs 0.5 to 4 us, all SMs
 // quantising every row about 0.06 us per 1000 elements, part of it behind a weight that is long in coming.  us, kernel of its own and fused: M = 1,
@@ -1105,7 +1110,8 @@ bool skinny_decode(int M, int N, int K, int64_t Kp) {
 bool fused_quant_pays(const b200dnn_matmul_t *d, const void *src, const PackedWeight &pw) {
   const int M = d->M, N = d->N, K = d->K;
   if (M > 16 || d->force_kernel != 0 || d->src_dt != B200DNN_BF16 || K % 8 != 0 || d->lda % 8 != 0 || (reinterpret_cast<uintptr_t>(src) & 15) != 0) return false;
-  if (skinny_decode(M, N, K, pw.Kp) || decode_smem(M, N, pw.Kp) > 220 * 1024 || env_int("B200DNN_DECODE_KERNEL", 1) == 0) return false;
+  const int form = decode_form(M, N, K);
+  if (skinny_decode(M, N, K, pw.Kp) || decode_smem(M, N, pw.Kp) > 220 * 1024 || form == 0 || (form >= 2 && M > kRingWarps)) return false;      // (a warp per row at least)
   const int mode = env_int("B200DNN_FUSED_QUANT", -1);
   if (mode == 0 || (mode < 0 && (long long)M * K > 20000 + (((long long)K * N) >> 20) * 500)) return false;
   auto apart = [](const void *p, size_t n, const void *q, size_t m) {
@@ -1265,10 +1271,7 @@ int32_t b200dnn_matmul(const b200dnn_matmul_t *d, void *stream) {
     B2_TRY(launch_skinny(A, lda, a_unsigned, false, M, N, K, pw, epi, M <= 16 && epi.n_po > 0 ? FA_GENERIC : fast_act_code(epi), early, st));
   } else if (which == 1 || which == 3) {
     int32_t rc = B200DNN_UNIMPLEMENTED;
-    // decode kernel: 0 tiled only, 1 register-batch form, 2 ring form, 3..5 ring with that many groups per stage;
-    // default: ring for M <= 2 and weights of 24 MB or more (measured faster there: 10.9 against 11.5 us at 45 MB, but
-    // 5.9 against 5.7 us at 16.8 MB), register-batch form otherwise
-    const int dk = env_int("B200DNN_DECODE_KERNEL", (M <= 2 && (long long)K * N >= (24ll << 20)) ? 2 : 1);
+    const int dk = decode_form(M, N, K);
     dq.late = early ? 0 : 1;
     const bool pdl = (early || dq.src) && env_int("B200DNN_PDL", 1) != 0;
     if (which == 1 && M <= 16 && dk >= 2) {

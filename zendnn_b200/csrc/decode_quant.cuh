@@ -21,7 +21,7 @@ struct DecodeQuant {
 // ss gets the row scales; codes and scales may be read behind a barrier of the caller's.
 template <int THREADS, int NJ, typename Sync>
 __device__ __forceinline__ void decode_quant_rows(const DecodeQuant &q, uint8_t *rows, int stride, int M, int K, uint32_t *top, float *ss, int tid, bool publish, Sync sync) {
-  const int lane = tid & 31, warp = tid >> 5, per_row = (THREADS / 32) / M;          // M <= 16 (8 warps: M <= 8)
+  const int lane = tid & 31, warp = tid >> 5, per_row = (THREADS / 32) / M;          // M <= 16 and no more rows than warps: see fused_quant_pays
   const int r = warp / per_row, step = per_row * 32, i0 = (warp - r * per_row) * 32 + lane, nv = r < M ? K >> 3 : 0;
   const uint4 *src = reinterpret_cast<const uint4 *>(q.src + (int64_t)min(r, M - 1) * q.ld);
   uint4 v[NJ];
