@@ -183,12 +183,20 @@ struct DeviceShared {
 // Descriptor tables that depend only on the caller's weight pointers (per-expert epilogue pointers, tensor maps) are
 // kept on the device and found again by their bytes, so that a steady-state MoE call uploads nothing.
 struct BlobCache {
-  struct Entry { std::vector<uint8_t> bytes; void *dev; bool made; };      // made: the bytes are what the table was made from, not the table
+  // made: the bytes are what the table was made from, not the table; call: the last one that asked for it
+  struct Entry { std::vector<uint8_t> bytes; void *dev; bool made; uint64_t call; };
   std::vector<Entry> entries;
-  void *find(const void *host, size_t n, bool made = false) const {
-    for (const Entry &e : entries)
-      if (e.made == made && e.bytes.size() == n && memcmp(e.bytes.data(), host, n) == 0) return e.dev;
+  uint64_t call = 0;      // counted by CallGuard::enter
+  void *find(const void *host, size_t n, bool made = false) {
+    for (Entry &e : entries)
+      if (e.made == made && e.bytes.size() == n && memcmp(e.bytes.data(), host, n) == 0) { e.call = call; return e.dev; }
     return nullptr;
+  }
+  // frees all but what the current call holds pointers to
+  void release_others() {
+    std::vector<Entry> kept;
+    for (Entry &e : entries) if (e.call == call) kept.push_back(std::move(e)); else cudaFree(e.dev);
+    entries.swap(kept);
   }
   void release() { for (Entry &e : entries) cudaFree(e.dev); entries.clear(); }
 };
@@ -358,6 +366,7 @@ struct CallGuard {
     prev = current_rt(); current_rt() = r;
     r->ws.rewind();
     r->small.begin();
+    ++r->blobs.call;
     return B200DNN_SUCCESS;
   }
   ~CallGuard() { if (r) { current_rt() = prev; r->mu.unlock(); } }
@@ -402,9 +411,9 @@ inline int32_t cached_blob(const void *host, size_t bytes, cudaStream_t st, void
   if (!key) {
     if (void *d = R.blobs.find(host, bytes)) { *dev = d; return B200DNN_SUCCESS; }
   }
-  if (R.blobs.entries.size() >= 256) {      // bounded: start again (nothing in flight may still read the old tables)
+  if (R.blobs.entries.size() >= 256) {      // bounded: start again (nothing in flight may still read the old tables; this call's own stay)
     B2_CUDA(cudaStreamSynchronize(st));
-    R.blobs.release();
+    R.blobs.release_others();
   }
   void *d = nullptr;
   {
@@ -415,7 +424,7 @@ inline int32_t cached_blob(const void *host, size_t bytes, cudaStream_t st, void
   B2_CUDA(cudaStreamSynchronize(st));
   BlobCache::Entry e;
   if (key) e.bytes.assign((const uint8_t *)key, (const uint8_t *)key + key_bytes); else e.bytes.assign((const uint8_t *)host, (const uint8_t *)host + bytes);
-  e.dev = d; e.made = key != nullptr;
+  e.dev = d; e.made = key != nullptr; e.call = R.blobs.call;
   R.blobs.entries.push_back(std::move(e));
   *dev = d;
   return B200DNN_SUCCESS;
