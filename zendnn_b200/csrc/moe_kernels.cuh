@@ -174,6 +174,7 @@ __global__ void __launch_bounds__(1024) expert_rank_kernel(const int32_t *ids, i
 // Warp-per-token form of route_topk_kernel for E <= 32*PER: every probability is computed once, the sum runs
 // in expert order (lane e%32 holds expert e), the k selections are warp arg-max reductions with ties to the
 // lower expert id.  Same results as route_topk_kernel bit for bit.  Lane j < k returns the token's j-th expert and its weight.
+// Logits without a softmax (a NaN, an infinity, or minus infinity throughout) leave nothing to choose: the last expert, so that every index made from it stays inside its array.
 template <int PER>
 __device__ __forceinline__ void route_topk_warp(const float *l, int E, int k, int renorm, int lane, int32_t *id, float *weight) {
   const float ninf = __int_as_float(0xff800000);
@@ -210,7 +211,7 @@ __device__ __forceinline__ void route_topk_warp(const float *l, int E, int k, in
     if (lane == jj) { my_p = bp; my_id = be; }
     tot = __fadd_rn(tot, bp);
   }
-  *id = my_id;
+  *id = min(my_id, E - 1);
   *weight = renorm ? __fdiv_rn(my_p, tot) : my_p;
 }
 template <int PER>
@@ -245,8 +246,7 @@ __global__ void __launch_bounds__(1024) route_small_kernel(const float *logits, 
   for (int t = warp; t < T; t += 32) {
     int32_t id; float weight;
     route_topk_warp<PER>(logits + (int64_t)t * E, E, k, 1, lane, &id, &weight);
-    // (logits that are all NaN leave no choice: the last expert, so that every index below stays inside its array)
-    if (lane < k) { s_id[t * k + lane] = min(id, E - 1); s_w[t * k + lane] = weight; }
+    if (lane < k) { s_id[t * k + lane] = id; s_w[t * k + lane] = weight; }
   }
   __syncthreads();
   const int key = tid < T * k ? s_id[tid] : -1;
@@ -308,8 +308,6 @@ __global__ void __launch_bounds__(kRouteChunkThreads) route_count_kernel(const f
   for (int t = t0 + warp; t < t1; t += kRouteChunkThreads / 32) {
     int32_t id; float weight;
     route_topk_warp<PER>(logits + (int64_t)t * E, E, k, 1, lane, &id, &weight);
-    // (logits that are all NaN leave no choice: the last expert, so that every index below stays inside its array)
-    id = min(id, E - 1);
     if (lane < k) { ids[t * k + lane] = id; w[t * k + lane] = weight; atomicAdd(&hist[id], 1); }
   }
   __syncthreads();
