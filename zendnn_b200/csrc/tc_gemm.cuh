@@ -428,7 +428,7 @@ __device__ __forceinline__ void put_pieces(uint8_t *p, const uint32_t (&x)[8 * N
     }
   }
 }
-// sixteen 4-byte columns at p, of which the first n exist (n > 0); last: the run ends here (there are no columns behind it, or they are another's)
+// sixteen 4-byte columns at p, of which the first n exist; last: the run ends here
 __device__ __forceinline__ void row_put32(uint8_t *p, const uint32_t (&w)[16], int n, bool last, bool row_ok, RowCarry &c) {
   uint32_t x[23];
 #pragma unroll
@@ -439,7 +439,7 @@ __device__ __forceinline__ void row_put32(uint8_t *p, const uint32_t (&w)[16], i
 #pragma unroll
   for (int i = 0; i < 8; ++i) c.w[i] = w[8 + i];
   c.have = true;
-  if (last) {
+  if (last || n < 16) {
     uint32_t y[15];
 #pragma unroll
     for (int i = 0; i < 15; ++i) y[i] = i < 7 ? c.w[i + 1] : 0u;
@@ -459,11 +459,12 @@ __device__ __forceinline__ void row_put16(uint8_t *p, const uint32_t (&w)[8], in
     }
     if (row_ok) put_pieces<1, 2>(at - 2 * odd, x, odd, lo, hi, (uint16_t)edge);
   };
-  put(p, w, c.have ? -16 : 0, n, w[0]);
+  // (no columns left: this ends the run, and the word that its last element shares with one outside is the last of those before)
+  put(p, w, c.have ? -16 : 0, n, n > 0 ? w[0] : c.w[7] >> 16);
 #pragma unroll
   for (int i = 0; i < 8; ++i) c.w[i] = w[i];
   c.have = true;
-  if (last) {
+  if (last || n < 16) {
     const uint32_t none[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
     put(p + 32, none, -16, n - 16, c.w[7] >> 16);
     c.have = false;
@@ -566,7 +567,7 @@ __device__ __forceinline__ void tc_epi_half(int fast_act, const EpiParams &epi, 
 #pragma unroll
       for (int i = 0; i < 16; ++i) w[i] = (uint32_t)y[i];
       if (es.coalesce) { if (es.row_ok) put_tail_words(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, N - pc); }
-      else if (pc < N) row_put32(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, min(16, N - pc), last || pc + 16 >= N, es.row_ok, carry);
+      else row_put32(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, max(0, min(16, N - pc)), last, es.row_ok, carry);
     }
     return;
   }
@@ -642,8 +643,8 @@ __device__ __forceinline__ void tc_epi_half(int fast_act, const EpiParams &epi, 
             for (int i = 0; i < 8; ++i) if (i == n >> 1 && n > 0) *reinterpret_cast<uint16_t *>(o + 4 * i) = (uint16_t)pk[i];
           }
         }
-      } else if (pc < N) {
-        row_put16(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 2, pk, min(16, N - pc), last || pc + 16 >= N, es.row_ok, carry);
+      } else {
+        row_put16(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 2, pk, max(0, min(16, N - pc)), last, es.row_ok, carry);
       }
     } else {
       if (es.v8 && full) {
@@ -668,7 +669,7 @@ __device__ __forceinline__ void tc_epi_half(int fast_act, const EpiParams &epi, 
 #pragma unroll
         for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(x[i]);
         if (es.coalesce) { if (es.row_ok) put_tail_words(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, N - pc); }
-        else if (pc < N) row_put32(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, min(16, N - pc), last || pc + 16 >= N, es.row_ok, carry);
+        else row_put32(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, max(0, min(16, N - pc)), last, es.row_ok, carry);
       }
     }
   }
