@@ -385,65 +385,62 @@ __device__ __forceinline__ void put_words_to(uint8_t *base, const uint32_t (&o)[
   if (n & 2) *reinterpret_cast<uint2 *>(base + 4 * h) = h ? make_uint2(o[4], o[5]) : make_uint2(o[0], o[1]);
   if (n & 1) *reinterpret_cast<uint32_t *>(base + 4 * k) = k < 4 ? (k < 2 ? o[0] : o[2]) : (k < 6 ? o[4] : o[6]);
 }
-// NV pieces of eight words from x (seven words in front, then 8 * NV words of which the first belongs at p).  Elements, PER to a word and the first of them `off` in front of p, from
+// A piece of eight words from x (seven words in front, then eight of which the first belongs at p).  Elements, PER to a word and the first of them `off` in front of p, from
 // lo to hi - 1 are written; edge: the element that shares its word with one outside, where off is 1.
-template <int NV, int PER>
-__device__ __forceinline__ void put_pieces(uint8_t *p, const uint32_t (&x)[8 * NV + 7], int off, int lo, int hi, uint16_t edge) {
+template <int PER>
+__device__ __forceinline__ void put_piece(uint8_t *p, const uint32_t (&x)[15], int off, int lo, int hi, uint16_t edge) {
   const int r = (int)((reinterpret_cast<uintptr_t>(p) >> 2) & 7);
-  uint32_t t[8 * NV + 6], u[8 * NV + 4], o[8 * NV];
+  uint32_t t[14], u[12], q[8];
   shift_words<1>(x, (r & 1) != 0, t);
   shift_words<2>(t, (r & 2) != 0, u);
-  shift_words<4>(u, (r & 4) != 0, o);
+  shift_words<4>(u, (r & 4) != 0, q);
   uint8_t *base = p - 4 * r;
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    const int e0 = (8 * v - r) * PER - off;                  // first element of the piece
-    const uint32_t q[8] = {o[8 * v], o[8 * v + 1], o[8 * v + 2], o[8 * v + 3], o[8 * v + 4], o[8 * v + 5], o[8 * v + 6], o[8 * v + 7]};
-    if (e0 >= lo && e0 + 8 * PER <= hi) st_global_v8(base + 32 * v, q);
-    else if (v == 0 && lo == 0 && e0 + 8 * PER <= hi) {      // the run begins in this piece
-      if (PER == 2 && off) *reinterpret_cast<uint16_t *>(p + 2) = edge;
-      put_words_from(base, q, r + off);
-    } else if (v == 0 && lo < 0 && hi == 0) {                // and here it ends
-      put_words_to(base, q, r);
-      if (PER == 2 && off) *reinterpret_cast<uint16_t *>(p) = edge;
-    } else if (e0 >= lo && e0 < hi) {                        // the last columns of the matrix
-      const int n = hi - e0, k = n / PER;
-      put_words_to(base + 32 * v, q, k);
-      if (PER == 2 && (n & 1)) {
-        const uint32_t w = k < 4 ? (k < 2 ? (k < 1 ? q[0] : q[1]) : (k < 3 ? q[2] : q[3])) : (k < 6 ? (k < 5 ? q[4] : q[5]) : (k < 7 ? q[6] : q[7]));
-        *reinterpret_cast<uint16_t *>(base + 32 * v + 4 * k) = (uint16_t)w;
-      }
-    } else if (e0 < hi) {
+  const int e0 = -r * PER - off;                           // first element of the piece
+  if (e0 >= lo && e0 + 8 * PER <= hi) st_global_v8(base, q);
+  else if (lo == 0 && e0 + 8 * PER <= hi) {                // the run begins in this piece
+    if (PER == 2 && off) *reinterpret_cast<uint16_t *>(p + 2) = edge;
+    put_words_from(base, q, r + off);
+  } else if (lo < 0 && hi == 0) {                          // and here it ends
+    put_words_to(base, q, r);
+    if (PER == 2 && off) *reinterpret_cast<uint16_t *>(p) = edge;
+  } else if (e0 >= lo && e0 < hi) {                        // the last columns of the matrix
+    const int n = hi - e0, k = n / PER;
+    put_words_to(base, q, k);
+    if (PER == 2 && (n & 1)) {
+      const uint32_t w = k < 4 ? (k < 2 ? (k < 1 ? q[0] : q[1]) : (k < 3 ? q[2] : q[3])) : (k < 6 ? (k < 5 ? q[4] : q[5]) : (k < 7 ? q[6] : q[7]));
+      *reinterpret_cast<uint16_t *>(base + 4 * k) = (uint16_t)w;
+    }
+  } else if (e0 < hi) {
 #pragma unroll 1
-      for (int i = 0; i < 8; ++i) {
-        const int e = e0 + i * PER;
-        const uint32_t lo4 = i < 4 ? (i < 2 ? (i < 1 ? q[0] : q[1]) : (i < 3 ? q[2] : q[3])) : (i < 6 ? (i < 5 ? q[4] : q[5]) : (i < 7 ? q[6] : q[7]));
-        uint8_t *at = base + 32 * v + 4 * i;
-        if constexpr (PER == 1) { if (e >= lo && e < hi) *reinterpret_cast<uint32_t *>(at) = lo4; }
-        else {
-          if (e >= lo && e < hi) *reinterpret_cast<uint16_t *>(at) = (uint16_t)lo4;
-          if (e + 1 >= lo && e + 1 < hi) *reinterpret_cast<uint16_t *>(at + 2) = (uint16_t)(lo4 >> 16);
-        }
+    for (int i = 0; i < 8; ++i) {
+      const int e = e0 + i * PER;
+      const uint32_t lo4 = i < 4 ? (i < 2 ? (i < 1 ? q[0] : q[1]) : (i < 3 ? q[2] : q[3])) : (i < 6 ? (i < 5 ? q[4] : q[5]) : (i < 7 ? q[6] : q[7]));
+      uint8_t *at = base + 4 * i;
+      if constexpr (PER == 1) { if (e >= lo && e < hi) *reinterpret_cast<uint32_t *>(at) = lo4; }
+      else {
+        if (e >= lo && e < hi) *reinterpret_cast<uint16_t *>(at) = (uint16_t)lo4;
+        if (e + 1 >= lo && e + 1 < hi) *reinterpret_cast<uint16_t *>(at + 2) = (uint16_t)(lo4 >> 16);
       }
     }
   }
 }
-// sixteen 4-byte columns at p, of which the first n exist; last: the run ends here
+// sixteen 4-byte columns at p, of which the first n exist (n > 0); last: the run ends here.  (Eight columns a piece: sixteen at once held 23 words, and small results paid for
+// it, INT8, f32 out, 371 x 419, K = 768 5.8 us before rows left as pieces, 6.5 with, 5.7 now; 313 x 518, K = 896 8.2, 8.65, 8.2.)
 __device__ __forceinline__ void row_put32(uint8_t *p, const uint32_t (&w)[16], int n, bool last, bool row_ok, RowCarry &c) {
-  uint32_t x[23];
+  auto put = [&](uint8_t *at, const uint32_t *u, const uint32_t *v, int lo, int hi) {
+    uint32_t x[15];
 #pragma unroll
-  for (int i = 0; i < 7; ++i) x[i] = c.w[i + 1];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) x[7 + i] = w[i];
-  if (row_ok) put_pieces<2, 1>(p, x, 0, c.have ? -7 : 0, n, 0);
+    for (int i = 0; i < 15; ++i) x[i] = i < 7 ? u[i + 1] : v[i - 7];
+    if (row_ok) put_piece<1>(at, x, 0, lo, hi, 0);
+  };
+  const uint32_t none[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+  put(p, c.w, w, c.have ? -7 : 0, n);
+  put(p + 32, w, w + 8, -7, n - 8);
 #pragma unroll
   for (int i = 0; i < 8; ++i) c.w[i] = w[8 + i];
   c.have = true;
-  if (last || n < 16) {
-    uint32_t y[15];
-#pragma unroll
-    for (int i = 0; i < 15; ++i) y[i] = i < 7 ? c.w[i + 1] : 0u;
-    if (row_ok) put_pieces<1, 1>(p + 64, y, 0, -7, n - 16, 0);
+  if (last) {
+    put(p + 64, w + 8, none, -7, n - 16);
     c.have = false;
   }
 }
@@ -457,7 +454,7 @@ __device__ __forceinline__ void row_put16(uint8_t *p, const uint32_t (&w)[8], in
       const uint32_t cur = i < 7 ? c.w[i + 1] : v[i - 7], prev = i < 8 ? c.w[i] : v[i - 8];
       x[i] = odd ? __funnelshift_l(prev, cur, 16) : cur;
     }
-    if (row_ok) put_pieces<1, 2>(at - 2 * odd, x, odd, lo, hi, (uint16_t)edge);
+    if (row_ok) put_piece<2>(at - 2 * odd, x, odd, lo, hi, (uint16_t)edge);
   };
   // (no columns left: this ends the run, and the word that its last element shares with one outside is the last of those before)
   put(p, w, c.have ? -16 : 0, n, n > 0 ? w[0] : c.w[7] >> 16);
@@ -567,7 +564,7 @@ __device__ __forceinline__ void tc_epi_half(int fast_act, const EpiParams &epi, 
 #pragma unroll
       for (int i = 0; i < 16; ++i) w[i] = (uint32_t)y[i];
       if (es.coalesce) { if (es.row_ok) put_tail_words(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, N - pc); }
-      else row_put32(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, max(0, min(16, N - pc)), last, es.row_ok, carry);
+      else if (pc < N) row_put32(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, min(16, N - pc), last || pc + 16 >= N, es.row_ok, carry);
     }
     return;
   }
@@ -669,7 +666,7 @@ __device__ __forceinline__ void tc_epi_half(int fast_act, const EpiParams &epi, 
 #pragma unroll
         for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(x[i]);
         if (es.coalesce) { if (es.row_ok) put_tail_words(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, N - pc); }
-        else row_put32(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, max(0, min(16, N - pc)), last, es.row_ok, carry);
+        else if (pc < N) row_put32(reinterpret_cast<uint8_t *>(cx.dst) + ((int64_t)m_dst * cx.ldc + pc) * 4, w, min(16, N - pc), last || pc + 16 >= N, es.row_ok, carry);
       }
     }
   }
