@@ -217,15 +217,11 @@ __device__ __forceinline__ void norm_clear_outside(uint32_t (&w)[4], int c0, int
 // One row of the full-width form, held by the CTA as the bf16 pairs it came in: v = input, r = residual (fused add); vector i holds the columns
 // 8 i - shift .. 8 i - shift + 7 (shift = 0 unless ANY), and elements outside the row are zeros.  red: a buffer per reduction, used by one row in two
 // (so one barrier each).  Same arithmetic as the generic kernel.
-// kNormByFloats: two aligned vectors a thread in up to 256 threads take the abs-max on the values before they are rounded (rounding to bf16 is monotonic: the largest rounded
-// magnitude is the rounded largest one) and store from row pointers; the other forms take it on the rounded words.  The results are the same; it is what nvcc makes of either, us
-// words and floats: 160 x 4096 residual add and codes 3.75, 3.61, RMSNorm 2.82, 2.74; 900 x 1024 3.86, 3.74; 8000 x 1024 LayerNorm and codes 15.3, 15.0; but one
-// vector a thread 1 x 4096 2.62, 2.81, and two in more threads 420 x 4800 6.5, 7.2.
-template <int NV, int THREADS, bool ANY> constexpr bool kNormByFloats = !ANY && NV == 2 && THREADS <= 256;
-template <int NV, int THREADS, bool ANY>
+// FLOATS (aligned rows): the abs-max is taken on the values before they are rounded (rounding to bf16 is monotonic: the largest rounded magnitude is the rounded largest one)
+// and rows are stored from row pointers; without, on the rounded words and through norm_store_vec.  The results are the same, what nvcc makes of either is not: see the rule.
+template <int NV, int THREADS, bool ANY, bool FLOATS>
 __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, int shift, uint32_t (&v)[NV][4], const uint32_t (&r)[NV][4], float (*red)[32]) {
-  constexpr bool kFloats = kNormByFloats<NV, THREADS, ANY>;
-  const int n = (int)a.n, nvec = kFloats ? (int)(a.n >> 3) : (shift + n + 7) >> 3;
+  const int n = (int)a.n, nvec = FLOATS ? (int)(a.n >> 3) : (shift + n + 7) >> 3;
   auto lo = norm_lo; auto hi = norm_hi;
   const int64_t off = b * a.n - shift;          // element of vector 0
   uint4 *rv = a.residual ? reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(a.residual) + off) : nullptr;
@@ -244,7 +240,7 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, int s
           s1 = __fmaf_rn(s_lo, s_lo, s1); s1 = __fmaf_rn(s_hi, s_hi, s1);
           v[j][e] = pack_bf16x2(s_lo, s_hi);
         }
-        if constexpr (kFloats) rv[i] = make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]);
+        if constexpr (FLOATS) rv[i] = make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]);
         else norm_store_vec<ANY>(reinterpret_cast<uint16_t *>(a.residual), off + (int64_t)i * 8, i * 8 - shift, n, v[j]);
       }
     }
@@ -305,11 +301,11 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, int s
           if (a.use_scale) { y0 = __fmul_rn(y0, g[2 * e]); y1 = __fmul_rn(y1, g[2 * e + 1]); }
           if (shifted) { y0 = __fadd_rn(y0, bt[2 * e]); y1 = __fadd_rn(y1, bt[2 * e + 1]); }
           v[j][2 * h + e] = pack_bf16x2(y0, y1);
-          if constexpr (kFloats) { if (a.q) top = fmaxf(top, fmaxf(fabsf(y0), fabsf(y1))); }      // (a NaN does not enter fmaxf, an infinity does)
+          if constexpr (FLOATS) { if (a.q) top = fmaxf(top, fmaxf(fabsf(y0), fabsf(y1))); }      // (a NaN does not enter fmaxf, an infinity does)
         }
       }
       if (!whole(c0)) norm_clear_outside(v[j], c0, n);
-      if constexpr (kFloats) {
+      if constexpr (FLOATS) {
         if (a.y) reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(a.y) + off)[i] = make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]);
       } else {
         if (a.q) am.add(make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]));
@@ -318,8 +314,8 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, int s
     }
   }
   if (a.q) {
-    float amax = norm_row_reduce<true, THREADS>(kFloats ? top : am.finite() ? __uint_as_float(am.bits()) : __int_as_float(0x7F800000), red[2]);
-    if constexpr (kFloats) amax = __uint_as_float(pack_bf16x2(amax, 0.0f) << 16);
+    float amax = norm_row_reduce<true, THREADS>(FLOATS ? top : am.finite() ? __uint_as_float(am.bits()) : __int_as_float(0x7F800000), red[2]);
+    if constexpr (FLOATS) amax = __uint_as_float(pack_bf16x2(amax, 0.0f) << 16);
     if (!finite_f32(amax)) {
       // an infinite or NaN element (it quantises to 0): the maximum over the finite values instead
       AbsMax<uint16_t> fin;
@@ -356,8 +352,8 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, int s
 // ANY: rows of any length, one behind the other.  A row is covered by the aligned vectors of the tensor that it touches (the first and the last shared with
 // its neighbours, of which it writes its own elements only); input, residual, result and codes then need no shifting, the parameters are picked out of two
 // aligned loads.  Instruction issue again: 8903 x 844 LayerNorm with codes 59 (element by element) -> 30 us, 3000 x 7001 with residual add and codes 197 -> 57,
-// 2000 x 12287 220 -> 55; the sets of registers per thread leave two CTAs an SM or more (one: 85 us for the last).
-template <int NV, int THREADS, int CTAS, bool ANY>
+// 2000 x 12287 220 -> 55; the registers of two and four vectors a thread leave two CTAs an SM or more (one: 85 us for the last).
+template <int NV, int THREADS, int CTAS, bool ANY, bool FLOATS = false>
 __global__ void __launch_bounds__(THREADS, CTAS) norm_rows_vec_kernel(const NormArgs a) {
   __shared__ float red[2][4][32];
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -365,7 +361,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) norm_rows_vec_kernel(const Norm
   const int64_t total = a.batch * a.n;
   int parity = 0;
   for (int64_t b = blockIdx.x; b < a.batch; b += gridDim.x, parity ^= 1) {
-    const int shift = ANY ? (int)((b * a.n) & 7) : 0, n = (int)a.n, nvec = kNormByFloats<NV, THREADS, ANY> ? (int)(a.n >> 3) : (shift + n + 7) >> 3;
+    const int shift = ANY ? (int)((b * a.n) & 7) : 0, n = (int)a.n, nvec = FLOATS ? (int)(a.n >> 3) : (shift + n + 7) >> 3;
     const int64_t off = b * a.n - shift;
     uint32_t v[NV][4], r[NV][4];
 #pragma unroll
@@ -387,7 +383,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) norm_rows_vec_kernel(const Norm
         if (ANY && (i == 0 || i == nvec - 1)) { norm_clear_outside(v[j], i * 8 - shift, n); norm_clear_outside(r[j], i * 8 - shift, n); }
       }
     }
-    norm_row_vec<NV, THREADS, ANY>(a, b, shift, v, r, red[parity]);
+    norm_row_vec<NV, THREADS, ANY, FLOATS>(a, b, shift, v, r, red[parity]);
   }
 }
 
@@ -512,6 +508,10 @@ extern "C" int32_t b200dnn_normalization(const b200dnn_norm_t *d, void *stream) 
       // 96 threads (16 CTAs an SM) or 128 (12), as above: 760 x 1536 3.9, 3.8; 1024 4.2, 5.6; 1300 6.4, 5.6; 2100 6.5, 7.4
       if (!any && per == 2 && threads == 96 && (batch <= 6 * sm || (batch > 8 * sm && batch <= 12 * sm))) threads = 128;
       const int nv = (nvec + threads - 1) / threads;
+      // FLOATS for two vectors in up to 256 threads, with codes or where at most half of the rows that the device holds (six CTAs of 256 threads an SM) are there, RMSNorm in 256 threads up to seven rows an SM.  us without and with:
+      // 160 x 4096 residual add and codes 3.75, 3.61, RMSNorm 2.82, 2.74; 8000 x 1024 LayerNorm and codes 15.3, 15.0; 900 x 4096 RMSNorm 5.24, 5.09; but 2000 x 768 residual add
+      // 1.055 times as long, 900 x 1920 1.05, 460 x 4096 1.025; one vector a thread 1 x 4096 2.62, 2.81, and two in more threads 420 x 4800 6.5, 7.2.
+      const bool floats = a.q || batch * threads <= sm * 3 * 256 || (a.type == NORM_RMS && threads == 256 && batch <= 7 * sm);
       const long long cap = (long long)R.sm_count * 64;
       const unsigned grid = (unsigned)(batch < cap ? batch : cap);
       auto go = [&](auto kern) { return launch_pdl(kern, grid, (unsigned)threads, 0, st, true, a); };
@@ -522,7 +522,7 @@ extern "C" int32_t b200dnn_normalization(const b200dnn_norm_t *d, void *stream) 
       };
       B2_TRY(any ? pick(norm_rows_vec_kernel<1, 256, 4, true>, norm_rows_vec_kernel<1, 1024, 1, true>, norm_rows_vec_kernel<2, 256, 5, true>, norm_rows_vec_kernel<2, 512, 2, true>, norm_rows_vec_kernel<2, 768, 2, true>,
                         norm_rows_vec_kernel<4, 128, 8, true>, norm_rows_vec_kernel<4, 256, 4, true>, norm_rows_vec_kernel<4, 512, 2, true>)
-                 : pick(norm_rows_vec_kernel<1, 256, 6, false>, norm_rows_vec_kernel<1, 1024, 1, false>, norm_rows_vec_kernel<2, 256, 6, false>, norm_rows_vec_kernel<2, 512, 3, false>, norm_rows_vec_kernel<2, 768, 2, false>,
+                 : pick(norm_rows_vec_kernel<1, 256, 6, false>, norm_rows_vec_kernel<1, 1024, 1, false>, floats ? norm_rows_vec_kernel<2, 256, 6, false, true> : norm_rows_vec_kernel<2, 256, 6, false>, norm_rows_vec_kernel<2, 512, 3, false>, norm_rows_vec_kernel<2, 768, 2, false>,
                         norm_rows_vec_kernel<4, 128, 8, false>, norm_rows_vec_kernel<4, 256, 4, false>, norm_rows_vec_kernel<4, 512, 2, false>));
       B2_LAUNCHED();
       B2_CUDA(cudaGetLastError());
