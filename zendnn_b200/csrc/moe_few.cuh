@@ -1,5 +1,5 @@
 // Grouped tcgen05 GEMM for a few rows per expert (MoE decode batches), INT8 and bf16: stands in for the tile micro-kernel under group_matmul_direct
-// (matmul/group_matmul/custom_kernel/ukernel/int8_microkernel.hpp:39-56) where an expert has at most 64 rows.
+// (matmul/group_matmul/custom_kernel/ukernel/int8_microkernel.hpp:39-56) where a layer has at most 64 tokens.
 //
 // As in skinny_gemm.cuh the operands change places: the MMA's M = 128 rows are 128 packed output columns of one expert, its N is the rows rounded up to 16.  The
 // tile kernel's 128-row box of activations per 128 bytes of K, nearly all of it other experts' rows or padding, costs as many bytes from L2 to shared memory as
@@ -80,12 +80,14 @@ moe_few_kernel(const __grid_constant__ CUtensorMap map_a, const MoeFewArgs a, co
   struct Rows { int g, row0, rows; };
   auto rows_of = [&](int tile) {
     const int mt = tile / a.n_tiles;
-    int g = 0;
+    int g = 0, first = 0;             // (first: the expert's first row tile, the last entry that does not lie beyond mt)
     for (int base = 1; base < a.n_groups; base += 32) {
-      const int i = base + lane;
-      g += __popc(__ballot_sync(0xffffffffu, i < a.n_groups && a.tile_prefix[i] <= mt));
+      const int i = base + lane, p = i < a.n_groups ? a.tile_prefix[i] : 0x7fffffff;
+      const unsigned up = __ballot_sync(0xffffffffu, p <= mt);
+      g += __popc(up);
+      if (up) first = __shfl_sync(0xffffffffu, p, 31 - __clz(up));
     }
-    const int row0 = a.row_off[g] + (mt - a.tile_prefix[g]) * a.MP;
+    const int row0 = a.row_off[g] + (mt - first) * a.MP;
     return Rows{g, row0, min(a.MP, a.row_off[g + 1] - row0)};
   };
 
