@@ -857,7 +857,7 @@ def run_single_gpu_extras(torch, capi, dev, peaks, int8_peak):
     del xs, rs, y, q, sc
     torch.cuda.synchronize()
 
-    # ---- attention beside the block (BMM form on the bf16 kernels: the scores pass through HBM)
+    # ---- attention beside the block (the fused prompt kernel: scores stay in tensor memory)
     Bs, Hs, Ss, Ds = 1, 32, 2048, 128
     qkv = [torch.randn(Bs, Hs, Ss, Ds, generator=gd, device=dev).to(torch.bfloat16) for _ in range(3)]
     oa = torch.empty_like(qkv[0])
@@ -871,7 +871,7 @@ def run_single_gpu_extras(torch, capi, dev, peaks, int8_peak):
     ms = _time_events(torch, lambda: capi.check(capi.lib.b200dnn_sdpa(C.byref(sd), st)), 5)
     tf = 4.0 * Bs * Hs * Ss * Ss * Ds / ms / 1e9
     out["sdpa_bf16_H32_S2048_D128_causal"] = {"us": round(ms * 1e3, 1), "tflops_of_4BHSSD": round(tf, 1), "roofline": bf16_roof(tf),
-                                              "note": "BMM form (scores, softmax, P V as separate steps): bound by the scores' HBM round trip"}
+                                              "note": "fused prompt kernel, two sweeps over the keys (final row maximum and sum before the probabilities): bound by the exponentials and the waits between its pipes"}
     del qkv, oa
     torch.cuda.synchronize()
 

@@ -345,7 +345,7 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, int s
 // The decoder-layer case at full width: bf16 rows of at most NV * 8 * blockDim elements in 16-byte aligned tensors, bf16 out.  One
 // CTA per row; a thread keeps its NV vectors of eight elements in registers (as the bf16 pairs they are at every stage that
 // is kept) between the passes, so the row is read once and every access is a 16-byte vector (8 bytes for the s8 codes).
-// Bound by HBM without the quantised output and by instruction issue with it (3.07 of 4 instructions a cycle): all loads of a row (input and
+// Bound by HBM without the quantised output and by instruction issue with it (3.10 of 4 instructions a cycle): all loads of a row (input and
 // residual) are in flight before the first store, each reduction costs one barrier, and the launch overlaps the kernel in front.  4096 rows of 4096 with residual add and s8 codes
 // (151 MB): 36.9 -> 28.3 us (5.3 TB/s); a ring of rows filled by bulk copies ahead of persistent CTAs took 35.7 us (four CTAs per SM where
 // there are six here).

@@ -125,9 +125,9 @@ int32_t launch_sdpa_flash(const SdpaCall &c, cudaStream_t st) {
   B2_TRY(make_map_heads(&mv, c.v, c.D, c.KV, a.vh ? c.H : 1, a.vb ? c.B : 1, c.vs[2], c.vs[1], c.vs[0]));
   const int db = c.D <= 64 ? 1 : 2;
   // A CTA of one row tile has half the warps and half the tensor memory, so that two fit an SM where shared memory allows it: with one block of keys (two slots of
-  // the ring are used) or a head dimension up to 64.  us before and after: 192 heads of 100 keys, head_dim 128, causal 13.8 -> 10.0; 160 of 90, 64, causal 11.3 -> 8.4;
-  // 320 of 128, 128, causal 23.3 -> 18.2.  But one CTA per SM while there are SMs for all of them (two of one launch on an SM: 24 heads of 310 keys,
-  // 64, with a mask 14.3 -> 18.5).
+  // the ring are used) or a head dimension up to 64.  us before and after: 192 heads of 100 keys, head_dim 128, causal 13.8 -> 9.2; 160 of 90, 64, causal 11.4 -> 7.7;
+  // 320 of 128, 128, causal 23.5 -> 17.6.  But one CTA per SM while there are SMs for all of them (two of one launch on an SM: 24 heads of 310 keys,
+  // 64, with a mask 14.3 -> 18.5, one an SM 13.5).
   const bool one_block = a.tiles == 1 && (c.KV <= 128 || (c.causal && c.S <= 128));
   size_t smem = (size_t)(a.tiles + (one_block ? 2 : kFlashSlots)) * db * 16384 + 1024;
   if (heads * a.n_qt <= sms) smem = std::max(smem, (size_t)120 * 1024);

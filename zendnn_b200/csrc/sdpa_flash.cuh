@@ -10,9 +10,11 @@
 // Every exponent is formed with one rounding (see flash_frame).  Error of the f32 probabilities against double, mean / mean weighted by the
 // probability / largest, for 2048 keys with scores of spread 1, 4 and 10 at scale 2^-3.5 (head_dim 128), in units of 1e-7:
 //   three-step form                                                    0.94 / 0.79 / 5.3    3.5 / 1.9 / 24     9.4 / 2.4 / 62
-//   distance from the maximum, exponential corrected for its argument   1.03 / 0.89 / 6.1    3.1 / 0.95 / 17    7.5 / 0.95 / 40      (before)
+//   distance from the maximum, exponential corrected for its argument   1.03 / 0.89 / 6.1    3.1 / 0.95 / 17    7.5 / 0.95 / 40      (before; first measured as
+//                                                                       0.92 / 0.76 / 4.8    3.1 / 0.81 / 17    7.5 / 0.65 / 40)
 //   here                                                               1.02 / 0.92 / 6.1    3.0 / 1.05 / 17    7.4 / 1.01 / 30
-// (the last two from one run); with a mask of spread 1, before 1.3 / 1.1 / 10, 3.9 / 2.8 / 34 and 12 / 4.3 / 90, here 1.3 / 1.1 / 9, 3.4 / 2.2 / 25 and 10 / 3.2 / 57;
+// (the last two from one run: their weighted means differ by no more than two measurements of one form do, all of it far below the rounding to bf16 behind).
+// Results against double, head_dim 64 and 128, spread 1, 4, 10, with and without masks: 2.07e-3 to 2.36e-3 (bf16) in either form, within 1e-7 of one another.  With a mask of spread 1, before 1.3 / 1.1 / 10, 3.9 / 2.8 / 34 and 12 / 4.3 / 90, here 1.3 / 1.1 / 9, 3.4 / 2.2 / 25 and 10 / 3.2 / 57;
 // with one of -1000 150 / 150 / 330 on both sides at spread 1.
 #pragma once
 #include "common.cuh"
@@ -117,8 +119,8 @@ __device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t saddr, uint32_t l
 // Bounds, per pair of 128 x 128 blocks (both row tiles): the exponentials, one per score and sweep at 16 a clock, 2048 clocks each, and the tensor pipe, 1024 in sweep 1 and
 // 2560 in sweep 2 (64 columns at a time run at two thirds of the rate; head_dim 64: half of each); measured inside a CTA 2500 to 2700 and 3300 (head_dim 64: 2470).
 // A share of the exponentials on the FMA pipe (a polynomial of degree six) was slower, 203 against 196 us: the pipes wait for one another, not for one of them.
-// 32 heads x 2048, us before the streams and the one-rounding exponents and now: causal 64.0 -> 62.9, none 123 -> 118.5, padding mask 160 -> 134; head_dim 64, 240 heads x
-// 1447 with padding 635 -> 538.  256 query rows per CTA, because K and V then pass the L2 half as often as with 128.
+// 32 heads x 2048, us before the streams and the one-rounding exponents and now: causal 63.8 -> 62.2, none 122 -> 117, padding mask 160 -> 130; head_dim 64, 240 heads x
+// 1447 with padding 637 -> 527.  256 query rows per CTA, because K and V then pass the L2 half as often as with 128.
 // KS: 16-element steps of the head dimension
 template <int KS, bool MASK>
 __global__ void __launch_bounds__(kFlashThreads, 1)

@@ -359,11 +359,11 @@ __device__ __forceinline__ void warp_store_rows64(uint8_t *sbuf, const uint4 (&v
   warp_store_rows32(sbuf, v[2], v[3], g_row0 + 32, pitch_bytes, rows_valid, lane);
 }
 
-// A destination without 16-byte alignment (an odd N or ldc): every lane writes its own row as aligned 32-byte pieces, put together in registers from sixteen columns and
-// the last words of the sixteen before them.  Three (bf16: four) steps of selects shift the words by the row's distance from a 32-byte boundary; where a run
+// A destination without 16-byte alignment (an odd N or ldc): every lane writes its own row as aligned 32-byte pieces, put together in registers from eight words and
+// the last of the eight before them.  Three (bf16: four) steps of selects shift the words by the row's distance from a 32-byte boundary; where a run
 // of columns begins or ends inside a piece, its elements are stored one by one.  (Through a staging block, four rows of eight words an instruction, as before: 32 instructions
-// and twice as many partial sectors.)  M = 3027, K = 1280, N = 7295: f32 75.1 -> 46.3 us, bf16
-// 50.4 -> 39.3; whole sectors at N = 7296 take 40.4 and 28.7.
+// and twice as many partial sectors.)  M = 3027, K = 1280, N = 7295, INT8: f32 75.5 -> 45.4 us, bf16
+// 49.9 -> 37.6; whole sectors at N = 7296 take 40.4 and 28.7.
 struct RowCarry { uint32_t w[8]; bool have; };      // the eight words in front of the next ones; have: they are this run's, and not all of them are stored
 template <int STEP, int N>
 __device__ __forceinline__ void shift_words(const uint32_t (&x)[N], bool on, uint32_t (&y)[N - STEP]) {      // y[i] = on ? x[i] : x[i + STEP]
