@@ -1103,17 +1103,23 @@ bool skinny_decode(int M, int N, int K, int64_t Kp) {
 int decode_form(int M, int N, int K) { return env_int("B200DNN_DECODE_KERNEL", (M <= 2 && (long long)K * N >= (24ll << 20)) ? 2 : 1); }
 
 // Dynamic quantisation inside the decode kernel (decode_quant.cuh): aligned bf16 rows that the decode kernels take, few enough elements, and no
-// overlap of the results with the source (every CTA reads all of it, while others may already write).  The line: a kernel of its own costs 0.5 to 4 us, all SMs
-// quantising every row about 0.06 us per 1000 elements, part of it behind a weight that is long in coming.  us, kernel of its own and fused: M = 1,
-// K = 11008, N = 4096 16.5, 12.5; K = 6272, N = 8640 19.3, 14.9; M = 4, K = 4096, N = 11008 14.9, 12.6; K = N = 4096 7.6, 7.4 (M = 8: 8.1, 8.9);
-// M = 8, K = N = 2048 6.1, 5.8 (M = 12: 6.6, 7.1); M = 8, K = 11008, N = 4096 16.1, 17.5.  B200DNN_FUSED_QUANT: 0 never, 1 whenever the rows allow it, -1 by the line.
+// overlap of the results with the source (every CTA reads all of it, while others may already write).  The line, by the elements that every SM quantises: a kernel of its own
+// costs 0.3 to 5 us, all SMs quantising every row about 0.06 us per 1000 elements, part of it behind a weight that is long in coming -- if that may be read before the kernel in front
+// has finished (STABLE_WEIGHTS); where it may not, only the kernel of its own has it read meanwhile.  From 37 MB on a weight came from HBM in these measurements (three in turn pass the L2),
+// and its stream hides more.  us, kernel of its own and fused, weights in place: M = 1, K = 11008, N = 4096 15.8, 11.7; M = 4, K = N = 4096 7.6, 7.3, N = 11008 14.9, 12.7; M = 3, K = 11008,
+// N = 4096 15.5, 14.4; M = 8, K = N = 2048 6.1, 5.8; but M = 8, K = 4096, N = 8192 10.7, 12.1; M = 4, K = 8192, N = 4096 10.8, 11.7; M = 10, K = 2048, N = 1024 5.4, 5.9; weights that wait:
+// M = 4, K = N = 4096 7.6, 7.6; M = 4, K = 8192, N = 4096 10.9, 12.6; M = 4, K = 2048, N = 14336 8.8, 9.3.  Over 874 (549) sizes the slowest call is 2 (3) % behind a kernel of its
+// own, and 6.4 (4.6) % are gained on average.  B200DNN_FUSED_QUANT: 0 never, 1 whenever the rows allow it, -1 by the line.
 bool fused_quant_pays(const b200dnn_matmul_t *d, const void *src, const PackedWeight &pw) {
   const int M = d->M, N = d->N, K = d->K;
   if (M > 16 || d->force_kernel != 0 || d->src_dt != B200DNN_BF16 || K % 8 != 0 || d->lda % 8 != 0 || (reinterpret_cast<uintptr_t>(src) & 15) != 0) return false;
   const int form = decode_form(M, N, K);
   if (skinny_decode(M, N, K, pw.Kp) || decode_smem(M, N, pw.Kp) > 220 * 1024 || form == 0 || (form >= 2 && M > kRingWarps)) return false;      // (a warp per row at least)
   const int mode = env_int("B200DNN_FUSED_QUANT", -1);
-  if (mode == 0 || (mode < 0 && (long long)M * K > 20000 + (((long long)K * N) >> 20) * 500)) return false;
+  const bool hbm = (long long)K * N >= 37000000;
+  const int most = (d->flags & B200DNN_FLAG_STABLE_WEIGHTS) == 0 ? (M <= 2 || K <= 1024 ? 16384 : N < 8192 ? 12288 : 0)
+                   : M <= 2 ? 32768 : hbm ? (N <= 6144 ? 45056 : K <= 4096 ? 32768 : 24576) : N <= 768 ? 24576 : 16384;
+  if (mode == 0 || (mode < 0 && M * K > most)) return false;
   auto apart = [](const void *p, size_t n, const void *q, size_t m) {
     const uintptr_t a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(q);
     return !p || !q || a + n <= b || b + m <= a;
