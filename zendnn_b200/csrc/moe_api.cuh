@@ -449,8 +449,15 @@ extern "C" int32_t b200dnn_moe_layer(const void *x, int64_t ldx, const float *lo
   rt().mark(-1);
   const int tile_rows = tc_tile_rows(R, H < 2 * I ? H : 2 * I);
   // Few rows per expert: the weight as the 128-row operand (moe_few.cuh).  72 layers of 1 to 64 tokens, one call after the other in either form: 1.1 to 1.7 times as fast
-  // up to 16 tokens, 1.0 to 1.4 up to 40, 0.98 to 1.11 (1.04 on average) up to 64, as far as its rows go.  B200DNN_MOE_FEW: the largest number of tokens that it takes.
-  const int few_rows = tile_rows == kTcBM && T <= std::min(env_int("B200DNN_MOE_FEW", kMoeFewMaxRows), kMoeFewMaxRows) ? (T + 15) & ~15 : 0;
+  // up to 16 tokens, 1.0 to 1.4 up to 40, 1.04 on average up to 64, as far as its rows go.  But where a CTA takes tile after tile (more than four), the first GEMM's few blocks of K
+  // have to hide the epilogue of MP rows: 63 tokens, 16 experts of 1024 x 2720, top 5, 63 us in the tile kernel, 71 here; 46 tokens, 16 of 1216 x 4736 87, 95.  The line: more
+  // than four rows a block, and more than six in an expert.  Of 1446 layers 50 are 1.5 % or more slower here than there, 28 with the line (5 % at most, 11 without), and six are by it.
+  // B200DNN_MOE_FEW: the largest number of tokens that it takes, -1 by this line.
+  const int few_most = env_int("B200DNN_MOE_FEW", -1), MP = (T + 15) & ~15, kb1 = (int)(((int64_t)K * (ex[0].wei_dt == B200DNN_BF16 ? 2 : 1) + 127) / 128);
+  const long long groups = std::min<long long>(E, (long long)T * topk) + S;
+  const bool late_epilogue = MP > 4 * kb1 && groups * ((2 * (long long)I + 127) / 128) > 4ll * Rt.sm_count && R > 6 * groups;
+  const bool few = few_most < 0 ? !late_epilogue : T <= few_most;
+  const int few_rows = tile_rows == kTcBM && T <= kMoeFewMaxRows && few ? MP : 0;
   const int route_rows = few_rows ? few_rows : tile_rows;      // what the tile counts count
   uint32_t *zmax = nullptr;
   if (T <= kRouteSmallT && T * topk <= kRouteSmallSlots && G <= kRouteSmallGroups) {
