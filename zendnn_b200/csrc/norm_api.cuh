@@ -345,7 +345,7 @@ __device__ __forceinline__ void norm_row_vec(const NormArgs &a, int64_t b, int s
 // The decoder-layer case at full width: bf16 rows of at most NV * 8 * blockDim elements in 16-byte aligned tensors, bf16 out.  One
 // CTA per row; a thread keeps its NV vectors of eight elements in registers (as the bf16 pairs they are at every stage that
 // is kept) between the passes, so the row is read once and every access is a 16-byte vector (8 bytes for the s8 codes).
-// Bound by HBM without the quantised output and by instruction issue with it (3.10 of 4 instructions a cycle): all loads of a row (input and
+// Bound by HBM without the quantised output and by instruction issue with it (3.05 of 4 instructions a cycle): all loads of a row (input and
 // residual) are in flight before the first store, each reduction costs one barrier, and the launch overlaps the kernel in front.  4096 rows of 4096 with residual add and s8 codes
 // (151 MB): 36.9 -> 28.3 us (5.3 TB/s); a ring of rows filled by bulk copies ahead of persistent CTAs took 35.7 us (four CTAs per SM where
 // there are six here).
@@ -508,10 +508,10 @@ extern "C" int32_t b200dnn_normalization(const b200dnn_norm_t *d, void *stream) 
       // 96 threads (16 CTAs an SM) or 128 (12), as above: 760 x 1536 3.9, 3.8; 1024 4.2, 5.6; 1300 6.4, 5.6; 2100 6.5, 7.4
       if (!any && per == 2 && threads == 96 && (batch <= 6 * sm || (batch > 8 * sm && batch <= 12 * sm))) threads = 128;
       const int nv = (nvec + threads - 1) / threads;
-      // FLOATS for two vectors in up to 256 threads, with codes or where at most half of the rows that the device holds (six CTAs of 256 threads an SM) are there, RMSNorm in 256 threads up to seven rows an SM.  us without and with:
+      // FLOATS for two vectors in up to 256 threads, with codes (but 2048 rows and more with residual add: 3000 x 1024 1.018 times as long, 4096 x 4096 1.005) or where at most half of the rows that the device holds (six CTAs of 256 threads an SM) are there, RMSNorm in 256 threads up to seven rows an SM.  us without and with:
       // 160 x 4096 residual add and codes 3.75, 3.61, RMSNorm 2.82, 2.74; 8000 x 1024 LayerNorm and codes 15.3, 15.0; 900 x 4096 RMSNorm 5.24, 5.09; but 2000 x 768 residual add
       // 1.055 times as long, 900 x 1920 1.05, 460 x 4096 1.025; one vector a thread 1 x 4096 2.62, 2.81, and two in more threads 420 x 4800 6.5, 7.2.
-      const bool floats = a.q || batch * threads <= sm * 3 * 256 || (a.type == NORM_RMS && threads == 256 && batch <= 7 * sm);
+      const bool floats = (a.q && (a.type != NORM_FUSED_ADD_RMS || batch < 2048)) || batch * threads <= sm * 3 * 256 || (a.type == NORM_RMS && threads == 256 && batch <= 7 * sm);
       const long long cap = (long long)R.sm_count * 64;
       const unsigned grid = (unsigned)(batch < cap ? batch : cap);
       auto go = [&](auto kern) { return launch_pdl(kern, grid, (unsigned)threads, 0, st, true, a); };
